@@ -224,6 +224,8 @@ InstDesc make_inst_desc(const aderdg_config* cfg) {
   in.dy = (cfg->xr[1] - cfg->xl[1]) / cfg->jmax;
   in.idxf = (float)(1.0 / in.dx);
   in.idyf = (float)(1.0 / in.dy);
+  in.rdx = 1.0 / in.dx;
+  in.rdy = 1.0 / in.dy;
   in.xl0 = cfg->xl[0];
   in.xl1 = cfg->xl[1];
   for (int s = 0; s < 4; ++s) in.bc[s] = cfg->bc[s];

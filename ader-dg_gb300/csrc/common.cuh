@@ -56,6 +56,7 @@ struct InstDesc {
   // (Advection-Diffusion/calc_time_step.f90:37-50)
   double ad_smax[2];
   double ad_denom;
+  double rdx, rdy;             // 1/dx, 1/dy (the FP64 predictor)
 };
 
 // Mutable per-instance state, device resident.
@@ -92,7 +93,13 @@ struct DevOps {
   R g[P];            // sum_l iK1(l',l)*F0(l)
   R ts[P];           // sum_l T(l',l)
   R tw[P];           // sum_l' w(l') T(l',l)
+  R iw[P];           // 1/w
   R wg;              // sum_l' w(l') g(l')
+  // Kxi, T, the end values FL and FR, and the time weights w and tw in 58-bit
+  // fixed point (predictor_fix.cuh): entry = (h 2^29 + l) 2^-s, h and l signed,
+  // |h| <= 2^28
+  int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];
+  int sK, sT, sE, sW;
   R FL[P], FR[P];
   double wd[P], FLd[P], FRd[P];
   float wf[P], FLf[P], FRf[P];  // FP32-mixed surface integral and update

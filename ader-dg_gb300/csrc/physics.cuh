@@ -253,10 +253,13 @@ struct EulerSys {
     R gm1;
     __device__ explicit PConst(const Phys& ph) : gm1(R(ph.gamma - 1.0)) {}
   };
-  // predictor flux: Fx, Fy of the same state
-  template <class R>
+  // predictor flux: Fx, Fy of the same state; kNewton: the refined reciprocal
+  // (3 FP64 instructions) in place of the division
+  template <class R, bool kNewton = false>
   __device__ __forceinline__ static void pflux(const PConst<R>& pc, const R* Q, R* Fx, R* Fy) {
-    const R ir = R(1) / Q[0];
+    R ir;
+    if constexpr (kNewton) ir = mrcp<R>(Q[0]);
+    else ir = R(1) / Q[0];
     const R u = Q[1] * ir, v = Q[2] * ir;
     const R p = pc.gm1 * (Q[3] - R(0.5) * (Q[1] * u + Q[2] * v));
     const R e = Q[3] + p;
@@ -265,7 +268,8 @@ struct EulerSys {
     Fx[2] = Q[2] * u;
     Fx[3] = e * u;
     Fy[0] = Q[2];
-    Fy[1] = Q[1] * v;
+    if constexpr (kNewton) Fy[1] = Fx[2];  // rho u v, one product for both
+    else Fy[1] = Q[1] * v;
     Fy[2] = Q[2] * v + p;
     Fy[3] = e * v;
   }
@@ -639,17 +643,26 @@ struct BNSys {
     __device__ explicit PConst(const Phys& ph)
         : gs1(R(ph.gs - 1.0)), gg1(R(ph.gg - 1.0)), gsps(R(ph.gs * ph.ps)), ggpg(R(ph.gg * ph.pg)) {}
   };
-  // predictor flux plus the three scalars the NCP needs (p_g, u_s, v_s)
-  template <class R>
+  // predictor flux plus the three scalars the NCP needs (p_g, u_s, v_s);
+  // kNewton: refined reciprocals in place of the divisions
+  template <class R, bool kNewton = false>
   __device__ __forceinline__ static void pflux(const PConst<R>& pc, const R* Q, R* Fx, R* Fy, R& p_g, R& u_s, R& v_s) {
     const R a = Q[8], b = R(1) - Q[8];
-    const R irs = R(1) / Q[0], irg = R(1) / Q[4];
+    R irs, irg;
+    if constexpr (kNewton) {
+      irs = mrcp<R>(Q[0]);
+      irg = mrcp<R>(Q[4]);
+    } else {
+      irs = R(1) / Q[0];
+      irg = R(1) / Q[4];
+    }
     u_s = Q[1] * irs;
     v_s = Q[2] * irs;
     const R u_g = Q[5] * irg, v_g = Q[6] * irg;
     const R Ps = pc.gs1 * (Q[3] - R(0.5) * (Q[1] * u_s + Q[2] * v_s)) - a * pc.gsps;  // phi_s p_s
     const R Pg = pc.gg1 * (Q[7] - R(0.5) * (Q[5] * u_g + Q[6] * v_g)) - b * pc.ggpg;  // phi_g p_g
-    p_g = Pg / b;
+    if constexpr (kNewton) p_g = Pg * mrcp<R>(b);
+    else p_g = Pg / b;
     const R es = Q[3] + Ps, eg = Q[7] + Pg;
     Fx[0] = Q[1];
     Fx[1] = Q[1] * u_s + Ps;
@@ -661,11 +674,13 @@ struct BNSys {
     Fx[7] = eg * u_g;
     Fx[8] = R(0);
     Fy[0] = Q[2];
-    Fy[1] = Q[1] * v_s;
+    if constexpr (kNewton) Fy[1] = Fx[2];
+    else Fy[1] = Q[1] * v_s;
     Fy[2] = Q[2] * v_s + Ps;
     Fy[3] = es * v_s;
     Fy[4] = Q[6];
-    Fy[5] = Q[5] * v_g;
+    if constexpr (kNewton) Fy[5] = Fx[6];
+    else Fy[5] = Q[5] * v_g;
     Fy[6] = Q[6] * v_g + Pg;
     Fy[7] = eg * v_g;
     Fy[8] = R(0);

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "physics.cuh"
+#include "predictor_fix.cuh"
 
 namespace aderdg {
 
@@ -58,13 +59,16 @@ constexpr int kPredVariants = 7;
 template <class Sys, int N, class R, class Tune = PredTune<>>
 struct PredCfg {
   static constexpr int P = N + 1, P2 = P * P, V = Sys::V;
+  // FP64 Euler / Baer-Nunziato with at least two full Picard iterations: their
+  // linear algebra in fixed point on the integer pipe (predictor_fix.cuh)
+  static constexpr bool FIX = sizeof(R) == 8 && Sys::ID != kSysAD && P >= 4;
   // variables of one node padded to whole 16-byte vectors (AD: scalar)
   static constexpr int VEC = 16 / (int)sizeof(R);
   // flux components stored and contracted: Baer-Nunziato's volume fraction
   // has no conservative flux (its ninth component is 0, Baer-Nunziato/pde.f90:74-119),
   // so FP32 stores 8 (two float4) where that is faster (N <= 4; at N = 5
   // the larger cells-per-CTA it allows spill registers); elsewhere all 9 (measured)
-  static constexpr int VF = (Sys::ID == kSysBN && sizeof(R) == 4 && N <= 4) ? 8 : V;
+  static constexpr int VF = (Sys::ID == kSysBN && (FIX || (sizeof(R) == 4 && N <= 4))) ? 8 : V;
   // FP32: pad to whole float4; FP64: double2 when VF is even
   static constexpr int VP = (VF == 1) ? 1 : (sizeof(R) == 4 ? ((VF + VEC - 1) / VEC) * VEC : VF);
   // Flux buffer layout.  FP64 and AD: [P][2][P2][VP], a node's variables
@@ -89,28 +93,35 @@ struct PredCfg {
   // then meet no bank group twice at these paddings).
   static constexpr bool ROWCOL = PLANAR && P >= 4 && !Tune::NO_ROWCOL;
   static constexpr bool MMA = ROWCOL && Tune::MMA;  // the row/column pass on the tensor cores
-  static constexpr int XL = ROWCOL ? P2 + ((P == 5) ? 0 : 1) : 2 * P2;  // nodes from x level to x level
-  static constexpr int YL = ROWCOL ? P2 + ((P == 5) ? 4 : 2) : 2 * P2;
-  static constexpr int Y0 = ROWCOL ? P * XL : P2;  // node offset of the y fluxes of level 0
+  // FIX: planes [variable][P x levels, P y levels] of doubles, levels an odd
+  // number of doubles apart (P = 4, y: 20, where the column pass then meets no bank twice)
+  static constexpr int XL = FIX ? (P2 | 1) : ROWCOL ? P2 + ((P == 5) ? 0 : 1) : 2 * P2;  // nodes from x level to x level
+  static constexpr int YL = FIX ? (P == 4 ? 20 : P2 | 1) : ROWCOL ? P2 + ((P == 5) ? 4 : 2) : 2 * P2;
+  static constexpr int Y0 = FIX || ROWCOL ? P * XL : P2;  // node offset of the y fluxes of level 0
   static constexpr int PC_PAD = (PLANAR && !ROWCOL && Sys::ID == kSysBN) ? (P == 2 ? 1 : 0) : 0;
   static constexpr int CE_PAD =
       !PLANAR   ? 0
       : ROWCOL  ? (P == 5 ? (Sys::ID == kSysBN ? 5 : 3) : (P == 6 && Sys::ID == kSysEuler) ? 2 : 0)
                 : (Sys::ID == kSysBN ? (P == 3 ? 1 : 0) : (P == 2 ? 4 : P == 3 ? 6 : 0));
-  static constexpr int PLANE = (ROWCOL ? Y0 + P * YL : 2 * P * P2) + PC_PAD;  // float4 per chunk plane
+  static constexpr int PLANE = (FIX || ROWCOL ? Y0 + P * YL : 2 * P * P2) + PC_PAD;  // float4 per chunk plane; FIX: doubles
   static constexpr int NS = PLANAR ? 4 : VP;            // elements from node to node
   static constexpr int CS = PLANAR ? 4 * PLANE : VEC;   // elements from chunk to chunk of a node
-  static constexpr int FLUX_ELEMS = PLANAR ? 4 * NCH * PLANE : 2 * VP * P * P2;
+  static constexpr int FLUX_ELEMS = FIX ? VF * PLANE : PLANAR ? 4 * NCH * PLANE : 2 * VP * P * P2;
+  static constexpr int EXP_ELEMS = FIX ? VF * P2 : 0;  // line exponents [VF][2][P][P] (int, in doubles)
+  static constexpr int MAT_ELEMS = FIX && Sys::ID == kSysBN ? P2 : 0;  // dudx, once per CTA
   // shared-memory elements per cell: flux buffer (+ BN volume fraction [P][P2];
   // AD: flux [P][2][P2] + state [P][P2]), rounded to 16 bytes (+ CE_PAD);
   // the epilogue reuses it as [V][P2] x 3 (AD: x 5)
-  static constexpr int RAW = (Sys::ID == kSysAD) ? 3 * P * P2 : FLUX_ELEMS + (Sys::ID == kSysBN ? P * P2 : 0);
+  static constexpr int RAW = (Sys::ID == kSysAD) ? 3 * P * P2 : FLUX_ELEMS + EXP_ELEMS + (Sys::ID == kSysBN ? P * P2 : 0);
   static constexpr int CELL_ELEMS = ((RAW + VEC - 1) / VEC) * VEC + 4 * CE_PAD;
-  static_assert(CELL_ELEMS >= 3 * V * P2 && (Sys::ID != kSysAD || CELL_ELEMS >= 5 * P2), "epilogue layout");
+  static_assert(CELL_ELEMS >= 3 * V * P2 + (FIX ? V * P : 0) && (Sys::ID != kSysAD || CELL_ELEMS >= 5 * P2), "epilogue layout");
   // FP32 up to N = 4: CTAs of at most 128 threads, twice as many per SM (each
   // Picard iteration's barriers then wait on fewer warps); N = 5 keeps 256,
-  // whose 36-thread cells fill 128 badly; FP64 is pipe-bound either way
-  static constexpr int MAX_THREADS0 = (sizeof(R) == 4 && N <= 4) ? 128 : 256;
+  // whose 36-thread cells fill 128 badly; FP64 AD and N <= 2 are pipe-bound
+  // either way.  FIX: shared memory (5 to 32 KB a cell) sets the resident warps;
+  // Baer-Nunziato N = 3 fits five CTAs of 4 cells, but two of 8
+  static constexpr int MAX_THREADS0 =
+      (FIX && Sys::ID == kSysBN && P == 4) ? 64 : (FIX || (sizeof(R) == 4 && N <= 4)) ? 128 : 256;
   static constexpr int MAX_THREADS = Tune::CTA > 0 ? 2 * MAX_THREADS0 : Tune::CTA < 0 ? MAX_THREADS0 / 2 : MAX_THREADS0;
   static constexpr int SMEM_BUDGET = 100 * 1024;
   static constexpr int CPB_T = MAX_THREADS / P2;
@@ -120,18 +131,21 @@ struct PredCfg {
   // FP32: CTAs per SM the register allocation aims at, measured per system
   // and degree (more resident warps hide the shared-memory latency of the
   // contractions; Baer-Nunziato's time column does not fit in fewer
-  // registers without spilling at N >= 3); FP64 is pipe-bound either way
+  // registers without spilling at N >= 3); FP64 AD and N <= 2 are pipe-bound
+  // either way; FIX: as many as shared memory admits
   static constexpr int BLOCK_UNITS =
       (Sys::ID == kSysAD ? 4 : Sys::ID == kSysEuler ? (N <= 3 ? 4 : 3) : (N <= 2 ? 3 : 2)) + Tune::BLOCKS;
   static constexpr int MIN_BLOCKS =
+      FIX ? (Sys::ID == kSysEuler ? (P <= 5 ? 5 : 4) : P == 4 ? 5 : 2) :
       (sizeof(R) == 4 && THREADS > 64) ? (BLOCK_UNITS * 256 / MAX_THREADS < 1 ? 1 : BLOCK_UNITS * 256 / MAX_THREADS)
                                        : 1;
   // the middle Picard iterations: a loop (default) or unrolled
   static constexpr int UNROLL = (Tune::UNROLL && P > 3) ? P - 2 : 1;
   // threads past CPB*P2 (the tail of the last warp) take part in the barriers
   // and get a scratch slot of their own so they never touch a real cell's data
-  static constexpr int SLOTS = CPB + (THREADS > CPB * P2 ? 1 : 0);
-  static constexpr int SMEM_BYTES = SLOTS * CELL_ELEMS * (int)sizeof(R);
+  // (FIX: they store nothing and need none)
+  static constexpr int SLOTS = CPB + (!FIX && THREADS > CPB * P2 ? 1 : 0);
+  static constexpr int SMEM_BYTES = (SLOTS * CELL_ELEMS + MAT_ELEMS) * (int)sizeof(R);
 };
 
 // Loads the VP (padded) variables of one node with 16-byte vector loads;
@@ -415,7 +429,7 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
   const bool in_cta = lc < CPB;
   const int k_found = (in_cta && cell < a.ncells) ? find_inst_cell(a.inst, a.ninst, cell) : -1;
   const bool valid = k_found >= 0;
-  R* cs = sm + (size_t)(lc < CPB ? lc : CPB) * C::CELL_ELEMS;  // lc >= CPB: the scratch slot
+  R* cs = sm + (size_t)(lc < CPB ? lc : C::FIX ? 0 : CPB) * C::CELL_ELEMS;  // lc >= CPB: the scratch slot (FIX: reads only)
 
   const int k_inst = valid ? k_found : 0;
   const InstDesc& in = a.inst[k_inst];
@@ -429,7 +443,13 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
   // per-thread contraction rows: Dx(i,k) = Kxi(k,i) dt/(dx w_i), Dy(j,k) likewise
   R Dx[P], Dy[P], Gx[P], Gy[P];
   R cxw, cyw;  // dt/(dx w_i), dt/(dy w_j)
-  {
+  if constexpr (C::FIX) {
+    // 1 in inactive lanes: their arithmetic stays in the fixed-point range
+    cxw = (act ? dt * in.rdx : 1.0) * op.iw[i];
+    cyw = (act ? dt * in.rdy : 1.0) * op.iw[j];
+    if constexpr (C::MAT_ELEMS > 0)
+      for (int k = t; k < P2; k += C::THREADS) sm[C::SLOTS * C::CELL_ELEMS + k] = op.dudx[k];
+  } else {
     // FP32: the reciprocals 1/dx, 1/dy held in FP32 (no FP64 divisions per thread)
     R idx, idy;
     if constexpr (sizeof(R) == 4) {
@@ -477,7 +497,11 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
     return ((d == 0 ? (size_t)l * C::XL : (size_t)C::Y0 + (size_t)l * C::YL) + node) * C::NS + v;
   };
 
-  if constexpr (Sys::ID == kSysAD) {
+  if constexpr (C::FIX) {
+    picard_fix<Sys, N, C>(cs, sm + C::SLOTS * C::CELL_ELEMS, op, pc,
+                          uh_in + ((size_t)(valid ? cell : 0) * P2 + node) * V, act, i, j, cxw, cyw, in.rdx, in.rdy, dt,
+                          qh, Fh, Sh, in_cta);
+  } else if constexpr (Sys::ID == kSysAD) {
     // -------------------------------------------------------------- AD
     // state buffer [P][P2] after the flux buffer [P][2][P2]
     R* qs = cs + 2 * P * P2;
@@ -747,20 +771,22 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
   R* sQ = cs;
   R* sX = cs + V * P2;
   R* sY = cs + 2 * V * P2;
+  if (!C::FIX || in_cta) {
 #pragma unroll
-  for (int v = 0; v < V; ++v) {
-    sQ[v * P2 + node] = qh[v];
-    sX[v * P2 + node] = Fh[0][v];
-    sY[v * P2 + node] = Fh[1][v];
+    for (int v = 0; v < V; ++v) {
+      sQ[v * P2 + node] = qh[v];
+      sX[v * P2 + node] = Fh[0][v];
+      sY[v * P2 + node] = Fh[1][v];
+    }
   }
   if constexpr (Sys::ID == kSysAD) {
     cs[3 * P2 + node] = Gh[0];
     cs[4 * P2 + node] = Gh[1];
   }
   __syncthreads();
-  if (!act) return;
+  if (!C::FIX && !act) return;
 
-  if constexpr (kPhase) {
+  if constexpr (kPhase) if (act) {
     // qhi(v,i,j), Fhi(v,d,i,j), Shi(v,i,j) in the reference layout
     const size_t base = (size_t)cell * P2 + node;
 #pragma unroll
@@ -770,10 +796,12 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
       a.fhi[(base * 2 + 1) * V + v] = (double)Fh[1][v];
       if constexpr (Sys::ID == kSysBN) a.shi[base * V + v] = (double)Sh[v];
     }
-    predictor_outputs<Sys, N, R, false>(a, op, in, cs, cell, node, i, j, Sh);
-  } else {
-    predictor_outputs<Sys, N, R, true>(a, op, in, cs, cell, node, i, j, Sh);
   }
+  if constexpr (C::FIX)
+    outputs_fix<Sys, N, !kPhase>(a, op, in.rdx, in.rdy, cs, reinterpret_cast<int*>(cs + 3 * V * P2), cell, node, i, j, Sh,
+                                 act);
+  else
+    predictor_outputs<Sys, N, R, !kPhase>(a, op, in, cs, cell, node, i, j, Sh);
 }
 
 }  // namespace aderdg
