@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/aderdg_gpu.h"
+#include "cells.cuh"
 #include "control.cuh"
 #include "tables.h"
 
@@ -40,6 +41,7 @@ struct aderdg_ctx {
   size_t bytes = 0;
   bool uploaded = false;
   bool pending = false;  // between element_update and the limiter commit (phase API)
+  bool lmin_bounds = false;  // lminmax holds a fused step's bounds (FP64: exact values on request)
   cudaGraphExec_t gexec = nullptr;
   void* flush_buf = nullptr;
   size_t flush_bytes = 0;
@@ -129,7 +131,7 @@ int cur_par(aderdg_ctx* c) { return (int)(c->h_st->steps & 1); }
 int cells(aderdg_ctx* c, int mode) {
   c->args.mode = mode;
   CK(c, aderdg::launch_cells(c->kt, c->args, c->ops64.data(), c->prec, c->stream));
-  // FP32-mixed: the DMP decisions the FP32 bounds left open
+  // the DMP decisions the FP32 bounds left open
   if (c->args.settle && (mode == aderdg::kCellFused || mode == aderdg::kCellUpdate || mode == aderdg::kCellInitDmp))
     CK(c, c->kt->settle(c->args, c->ops64.data(), c->num_sms, c->stream));
   return ADERDG_OK;
@@ -152,6 +154,47 @@ int set_clock(aderdg_ctx* c, double time, double tend) {
     c->h_st->nonfinite = 0;
     return push_state(c);
   }
+  return ADERDG_OK;
+}
+
+// neighbourhood min/max (get_min_max step 2, Euler/limiter.f90:147-167) of the
+// per-cell values mm[par ^ 1] of a context's single instance
+__global__ void k_neighbourhood(BatchArgs a, int V) {
+  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= a.ncells * V) return;
+  const long long cell = k / V;
+  const int v = (int)(k - cell * V);
+  const InstDesc& in = a.inst[0];
+  const int ci = (int)(cell % in.imax), cj = (int)(cell / in.imax);
+  const double* mm = a.mm[aderdg::parity(a.st[0])];
+  double lo = mm[cell * 2 * V + v], hi = mm[cell * 2 * V + V + v];
+  for (int jj = -1; jj <= 1; ++jj)
+    for (int ii = -1; ii <= 1; ++ii) {
+      const long long nc = aderdg::nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]) +
+                           (long long)in.imax * aderdg::nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
+      lo = fmin(lo, mm[nc * 2 * V + v]);
+      hi = fmax(hi, mm[nc * 2 * V + V + v]);
+    }
+  a.lminmax[cell * 2 * V + v] = lo;
+  a.lminmax[cell * 2 * V + V + v] = hi;
+}
+
+// FP64: a fused step decides its DMP from bounds on the per-cell min/max; the
+// exact lmin/lmax of that step, from its start-of-step state, which the other
+// parity's buffers still hold
+int exact_lminmax(aderdg_ctx* c) {
+  BatchArgs z = c->args;
+  std::swap(z.uh[0], z.uh[1]);
+  std::swap(z.status[0], z.status[1]);
+  std::swap(z.lh[0], z.lh[1]);
+  std::swap(z.mm[0], z.mm[1]);
+  std::swap(z.mme[0], z.mme[1]);
+  z.mode = aderdg::kCellPrime;
+  CK(c, c->kt->cells(z, c->ops64.data(), 0, c->stream));
+  const long long n = c->ncells * c->V;
+  k_neighbourhood<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(z, c->V);
+  CK(c, cudaGetLastError());
+  c->lmin_bounds = false;
   return ADERDG_OK;
 }
 
@@ -180,6 +223,7 @@ void free_all(aderdg_ctx* c) {
 }
 
 int ensure_graph(aderdg_ctx* c) {
+  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
   if (c->gexec) return ADERDG_OK;
   cudaGraph_t g = nullptr;
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -214,8 +258,9 @@ int ensure_phase_buffers(aderdg_ctx* c) {
 namespace aderdg {
 void set_last_error(const std::string& msg) { g_err = msg; }
 int validate_config(const aderdg_config* c, std::string* why) { return validate(c, why); }
-// Instance description of a configuration (cell and face bases 0).
-InstDesc make_inst_desc(const aderdg_config* cfg) {
+// Instance description of a configuration (cell and face bases 0; without
+// ops, the surface integral's w/dx and w/dy are left 0).
+InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops) {
   InstDesc in{};
   in.imax = cfg->imax;
   in.jmax = cfg->jmax;
@@ -226,6 +271,10 @@ InstDesc make_inst_desc(const aderdg_config* cfg) {
   in.idyf = (float)(1.0 / in.dy);
   in.rdx = 1.0 / in.dx;
   in.rdy = 1.0 / in.dy;
+  for (int k = 0; k < 6; ++k) {
+    in.wdx[k] = ops && k < ops->P ? ops->w[k] / in.dx : 0.0;
+    in.wdy[k] = ops && k < ops->P ? ops->w[k] / in.dy : 0.0;
+  }
   in.xl0 = cfg->xl[0];
   in.xl1 = cfg->xl[1];
   for (int s = 0; s < 4; ++s) in.bc[s] = cfg->bc[s];
@@ -364,9 +413,9 @@ int aderdg_create(const aderdg_config* cfg, aderdg_ctx** out) {
     if (!r) r = dalloc(c, &a.lh[1], nc * S * S * V);
     if (!r) r = dalloc(c, &a.mm[0], nc * 2 * V);
     if (!r) r = dalloc(c, &a.mm[1], nc * 2 * V);
-    if (!r && c->prec == ADERDG_FP32_MIXED) r = dalloc(c, &a.mme[0], nc * V);
-    if (!r && c->prec == ADERDG_FP32_MIXED) r = dalloc(c, &a.mme[1], nc * V);
-    if (!r && c->prec == ADERDG_FP32_MIXED) r = dalloc(c, &a.settle, nc);
+    if (!r && c->prec != ADERDG_FP32_WIDE) r = dalloc(c, &a.mme[0], nc * V);
+    if (!r && c->prec != ADERDG_FP32_WIDE) r = dalloc(c, &a.mme[1], nc * V);
+    if (!r && c->prec != ADERDG_FP32_WIDE) r = dalloc(c, &a.settle, nc);
     if (!r) r = dalloc(c, &a.lminmax, nc * 2 * V);
     if (!r) r = dalloc(c, &a.troubled, nc);
     if (!r) r = dalloc(c, &a.recompute, nc);
@@ -384,7 +433,7 @@ int aderdg_create(const aderdg_config* cfg, aderdg_ctx** out) {
   a.nfy = c->nfy;
 
   InstDesc& in = c->h_inst;
-  in = aderdg::make_inst_desc(cfg);
+  in = aderdg::make_inst_desc(cfg, &c->ops);
   e = cudaMemcpyAsync(c->d_inst, &in, sizeof(InstDesc), cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return bail(fail_cuda(nullptr, "cudaMemcpy inst", e));
@@ -424,6 +473,7 @@ int aderdg_destroy(aderdg_ctx* ctx) {
 
 int aderdg_upload(aderdg_ctx* c, const double* uh) {
   if (!c || !uh) return fail(c, ADERDG_EINVAL, "null argument");
+  c->lmin_bounds = false;
   const int par = cur_par(c);
   const size_t n = (size_t)c->ncells * c->P * c->P * c->V;
   CK(c, cudaMemcpyAsync(c->args.uh[par], uh, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -467,6 +517,7 @@ int aderdg_init_limiter(aderdg_ctx* c, const double* lh_ic, int* n_limited) {
 int aderdg_initial_condition(aderdg_ctx* c, int ic, const double* params, int* n_limited) {
   if (!c) return fail(c, ADERDG_EINVAL, "null context");
   if (n_limited) *n_limited = 0;
+  c->lmin_bounds = false;
   const int par = cur_par(c);
   // the subcell candidates are formed after the initial DMP, for the cells it
   // limits only, in both Lh buffers
@@ -648,6 +699,7 @@ int aderdg_surface_integral(aderdg_ctx* c) {
 int aderdg_element_update(aderdg_ctx* c, int* n_recompute) {
   if (!c) return fail(c, ADERDG_EINVAL, "null context");
   if (c->pending) return fail(c, ADERDG_ESTATE, "element update already applied");
+  c->lmin_bounds = false;
   CK(c, cudaMemsetAsync(&c->d_st->n_recompute, 0, sizeof(int), c->stream));
   CK(c, cudaMemsetAsync(&c->d_st->denom_next, 0, sizeof(unsigned long long), c->stream));
   int r = cells(c, aderdg::kCellUpdate);
@@ -679,6 +731,7 @@ int aderdg_step(aderdg_ctx* c, double* time, double tend, double* dt, int* n_rec
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
+  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
   r = launch_step(c);
   if (r) return r;
   r = pull_state(c);
@@ -785,6 +838,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
+  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
   cudaEvent_t ev[8];
   for (auto& e : ev) CK(c, cudaEventCreate(&e));
   CK(c, cudaEventRecord(ev[0], c->stream));
@@ -894,6 +948,9 @@ int aderdg_get_array(aderdg_ctx* c, int which, void* out) {
     case ADERDG_A_STATUS: src = a.status[par]; esz = sizeof(int); break;
     case ADERDG_A_LMIN:
     case ADERDG_A_LMAX: {
+      if (c->lmin_bounds) {
+        if (int r = exact_lminmax(c)) return r;
+      }
       std::vector<double> mm((size_t)n * 2);
       CK(c, cudaMemcpyAsync(mm.data(), a.lminmax, mm.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
       CK(c, cudaStreamSynchronize(c->stream));

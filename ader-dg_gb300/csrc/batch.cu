@@ -31,7 +31,7 @@ namespace aderdg {
 void set_last_error(const std::string& msg);
 int validate_config(const aderdg_config* c, std::string* why);
 FaceConst make_face_const(const HostOps& ops);
-InstDesc make_inst_desc(const aderdg_config* cfg);
+InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops);
 }  // namespace aderdg
 
 using aderdg::BatchArgs;
@@ -112,7 +112,7 @@ long long unit_bytes(int system, int N, int precision, int limiter) {
   b += rb * P * V * (system == ADERDG_SYS_BN ? 4 : 2);              // face fluxes
   if (limiter && system != ADERDG_SYS_ADVDIFF) {
     b += 8 * V * S * S * 2 + 4 * 2 + 8 * 2 * V * 2 + 1 + 4 + 4 + 8;  // Lh[2], status[2], mm[2], flags, list, denom
-    if (precision == ADERDG_FP32_MIXED) b += 4 * V * 2 + 4;           // mme[2], settle list
+    if (precision != ADERDG_FP32_WIDE) b += 4 * V * 2 + 4;             // mme[2], settle list
   }
   return b;
 }
@@ -358,9 +358,9 @@ int aderdg_batch_create(int system, int N, int precision, int limiter, long capa
     if (!r) r = balloc(b, &a.lh[1], U * S * S * V);
     if (!r) r = balloc(b, &a.mm[0], U * 2 * V);
     if (!r) r = balloc(b, &a.mm[1], U * 2 * V);
-    if (!r && precision == ADERDG_FP32_MIXED) r = balloc(b, &a.mme[0], U * V);
-    if (!r && precision == ADERDG_FP32_MIXED) r = balloc(b, &a.mme[1], U * V);
-    if (!r && precision == ADERDG_FP32_MIXED) r = balloc(b, &a.settle, U);
+    if (!r && precision != ADERDG_FP32_WIDE) r = balloc(b, &a.mme[0], U * V);
+    if (!r && precision != ADERDG_FP32_WIDE) r = balloc(b, &a.mme[1], U * V);
+    if (!r && precision != ADERDG_FP32_WIDE) r = balloc(b, &a.settle, U);
     // no lminmax: the neighbourhood bounds are an introspection output of
     // the single-simulation API only
     if (!r) r = balloc(b, &a.troubled, U);
@@ -464,7 +464,7 @@ int badmit(aderdg_batch* b, const aderdg_config* cfg, const double* uh, const do
   b->cfg_of[s] = *cfg;
   ++b->n_used;
   InstDesc& in = b->h_inst[pos];
-  in = aderdg::make_inst_desc(cfg);
+  in = aderdg::make_inst_desc(cfg, &b->ops);
   in.cell_base = in.fx_base = in.fy_base = base;
   InstState st;
   std::memset(&st, 0, sizeof(st));

@@ -200,6 +200,19 @@ __device__ __forceinline__ int nb_index(int x, int d, int n, int bc_lo, int bc_h
   return y;
 }
 
+// a / b, correctly rounded, for a constant b with y = 1/b correctly rounded
+// (Markstein: a faithful quotient plus one exact-remainder correction is the
+// rounded quotient; the first step makes it faithful): 5 FP64 instructions in
+// place of the division's sequence.  Outside 2^-700 .. 2^700, where the
+// remainders could leave the normal range, the division itself.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+  const unsigned e = ((unsigned)__double2hiint(a) >> 20) & 0x7ff;
+  if (e - 323u >= 1400u && a != 0.0) return a / b;
+  const double q0 = __dmul_rn(a, y);
+  const double q1 = __fma_rn(__fma_rn(-q0, b, a), y, q0);
+  return __fma_rn(__fma_rn(-q1, b, a), y, q1);
+}
+
 // CFL denominator at one node (calc_time_step.f90: Euler/BN :31-45, AD :37-50)
 template <class Sys, int N>
 __device__ __forceinline__ double cfl_denom(const InstDesc& in, const double* Q) {
@@ -286,11 +299,18 @@ struct CellCfg {
   }
 };
 
-template <class Sys, int N, bool kFast, int VAR = 0>
-__global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast))
+// kFast: DMP projections in FP32 with an error bound (settled from FP64 where
+// the bound leaves a decision open) and, without kExact, the FP32 modes'
+// storage and surface integral.  kExact: FP64 storage, surface integral, update
+// and CFL in reference order beside those projections: the FP64 mode's fused
+// step, whose decisions and state are those of the FP64 projections bit for
+// bit.
+template <class Sys, int N, bool kFast, int VAR = 0, bool kExact = false>
+__global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast && !kExact))
     k_cells(BatchArgs a, DevOps<N, double> op) {
   using C = CellCfg<Sys, N, VAR>;
   constexpr int P = N + 1, P2 = P * P, S = 2 * N + 1, V = Sys::V, CPB = C::CPB;
+  constexpr bool kF32 = kFast && !kExact;  // FP32 storage and update
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* sm = reinterpret_cast<double*>(smem_raw);
   double* opsm = sm + CPB * C::CELL_DBL;
@@ -369,6 +389,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const long long nc = in.cell_base + in_ + (long long)in.imax * jn_;
           nlmin = fmin(nlmin, mmi[(size_t)nc * 2 * V + v]);
           nlmax = fmax(nlmax, mmi[(size_t)nc * 2 * V + V + v]);
+          if (a.mme[0]) nen = fmaxf(nen, a.mme[par][(size_t)nc * V + v]);
         }
     }
   }
@@ -397,7 +418,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       const long long fxl = in.fx_base + ci + (long long)(in.imax + 1) * cj;
       const long long fyb = in.fy_base + ci + (long long)in.imax * cj;
       const long long fyt = fyb + in.imax;
-      if constexpr (kFast) {
+      if constexpr (kF32) {
         // FP32-mixed: duh and the face fluxes are stored in FP32; the surface
         // contraction and the scaling by 1/(w_i w_j) in FP32, the update of
         // the FP64 state in FP64
@@ -445,7 +466,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const double* XR = (Sys::ID == kSysBN) ? a.fp : a.fu;
           const double* YB = a.gu;
           const double* YT = (Sys::ID == kSysBN) ? a.gp : a.gu;
-          const double cx = op.wd[j] / in.dx, cy = op.wd[i] / in.dy;
+          const double cx = in.wdx[j], cy = in.wdy[i];  // w_j / dx, w_i / dy
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             const double fl = XL[((size_t)fxl * P + j) * V + v], fr = XR[((size_t)(fxl + 1) * P + j) * V + v];
@@ -467,7 +488,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           double* un = a.uh[par ^ 1] + off;
 #pragma unroll
           for (int v = 0; v < V; ++v) {
-            d[v] = d[v] / (op.wd[i] * op.wd[j]);
+            d[v] = div_by(d[v], op.wd[i] * op.wd[j], op.iwwd[i + P * j]);
             u[v] = uo[v] + dt * d[v];
             un[v] = u[v];
           }
@@ -502,7 +523,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       unsigned long long bits = 0ull;
       if (act) {
         double dn;
-        if constexpr (kFast) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+        if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
         else dn = cfl_denom<Sys, N>(in, u);
         bits = (unsigned long long)__double_as_longlong(dn);
       }
@@ -511,7 +532,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     }
   } else if (act && want_cfl) {
     double dn;
-    if constexpr (kFast) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+    if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
     else dn = cfl_denom<Sys, N>(in, u);
     // advection-diffusion: the denominator is the instance's constant, folded below
     if constexpr (Sys::ID != kSysAD) atomicMax(&cmax[lc], (unsigned long long)__double_as_longlong(dn));
@@ -716,10 +737,10 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       }
     }
     __syncthreads();
-    if constexpr (kFast) {
-      // FP32-mixed: a cell whose DMP the error bounds left open (bit 4) and
-      // that nothing else marked goes on the list k_settle decides from FP64
-      // values; here it counts as not troubled
+    {
+      // a cell whose DMP the error bounds left open (bit 4) and that nothing
+      // else marked goes on the list k_settle decides from FP64 values; here it
+      // counts as not troubled
       if (act && node == 0 && a.settle && (cflag[lc] & 7) == 4 &&
           (mode == kCellFused || mode == kCellUpdate || mode == kCellInitDmp))
         a.settle[atomicAdd(&a.list_count[1], 1)] = (int)cell;

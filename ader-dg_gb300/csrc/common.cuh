@@ -12,7 +12,7 @@
 //           (FP32 in the FP32 modes)
 //   lh      [cell][S*S][V]         subcell state of limited cells
 //   mm      [cell][2][V]           per-cell min/max for the DMP neighbourhood
-//   mme     [cell][V]              FP32-mixed: a bound on the error of mm (0: exact FP64 value)
+//   mme     [cell][V]              FP64, FP32-mixed: a bound on the error of mm (0: exact FP64 value)
 #pragma once
 
 #include <cstdint>
@@ -57,6 +57,7 @@ struct InstDesc {
   double ad_smax[2];
   double ad_denom;
   double rdx, rdy;             // 1/dx, 1/dy (the FP64 predictor)
+  double wdx[6], wdy[6];       // w_k/dx, w_k/dy (the FP64 surface integral)
 };
 
 // Mutable per-instance state, device resident.
@@ -104,6 +105,7 @@ struct DevOps {
   double wd[P], FLd[P], FRd[P];
   float wf[P], FLf[P], FRf[P];  // FP32-mixed surface integral and update
   float iwwf[P * P];            // 1 / (w_i w_j) at [i + P*j]
+  double iwwd[P * P];           // the same in FP64, correctly rounded from the rounded product
   double xid[P];
   double uh2lim[S * P];  // (s,k) at [s + S*k]
   double lim2uh[P * S];  // (k,s) at [k + P*s]
@@ -146,7 +148,7 @@ struct BatchArgs {
   int* status[2];                    // limiter status per cell
   double* lh[2];                     // subcell data [cell][S*S][V]
   double* mm[2];                     // per-cell min/max [cell][2][V] (lmin_old/lmax_old)
-  // FP32-mixed mode only (null otherwise): a bound on |mm - the FP64
+  // FP64 and FP32-mixed modes (null in FP32-wide): a bound on |mm - the FP64
   // reference-order min/max| per cell and variable [cell][V], 0 where mm holds
   // the FP64 value itself; double-buffered like mm.  The DMP decisions use it
   // to settle each comparison exactly (see k_cells / k_subcell).
@@ -156,7 +158,7 @@ struct BatchArgs {
   int* recompute;                    // 0, 1, 2
   int* list;                         // cells with recompute > 0
   int* list_count;                   // [0]: entries of list, [1]: entries of settle
-  int* settle;                       // FP32-mixed only (null otherwise): cells whose DMP
+  int* settle;                       // with mme (null otherwise): cells whose DMP
                                      // decision k_settle takes from FP64 values
   double* denom;                     // per-cell CFL denominator
   const double* lh_ic;               // initial-limiter candidates

@@ -63,25 +63,29 @@ cudaError_t faces(const BatchArgs& a, const FaceConst& fc, int fp32, cudaStream_
   return cudaGetLastError();
 }
 
-template <bool kFast>
+template <bool kFast, bool kExact = false>
 cudaError_t launch_cells(const BatchArgs& a, const void* ops, cudaStream_t s) {
   using C = CellCfg<Sys, N>;
   static bool attr = false;
   if (!attr) {
     cudaError_t e =
-        cudaFuncSetAttribute(k_cells<Sys, N, kFast>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+        cudaFuncSetAttribute(k_cells<Sys, N, kFast, 0, kExact>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     attr = true;
   }
   const long long grid = (a.ncells - a.cell0 + C::CPB - 1) / C::CPB;
   if (grid <= 0) return cudaSuccess;
-  k_cells<Sys, N, kFast><<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, double>*>(ops));
+  k_cells<Sys, N, kFast, 0, kExact><<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, double>*>(ops));
   return cudaGetLastError();
 }
 
 // fast = 1 (the FP32 modes): FP32 surface integral and DMP projections, the
-// FP64 update as one fused multiply-add; fast = 0: FP64 in reference order
+// FP64 update as one fused multiply-add; fast = 0: FP64 in reference order;
+// fast = 2: FP64 in reference order with certified FP32 DMP projections
 cudaError_t cells(const BatchArgs& a, const void* ops, int fast, cudaStream_t s) {
+#if ADERDG_SYS != 0
+  if (fast == 2) return launch_cells<true, true>(a, ops, s);
+#endif
   return fast ? launch_cells<true>(a, ops, s) : launch_cells<false>(a, ops, s);
 }
 

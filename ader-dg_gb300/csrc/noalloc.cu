@@ -39,7 +39,7 @@
 namespace aderdg {
 void set_last_error(const std::string& msg);
 int validate_config(const aderdg_config* c, std::string* why);
-InstDesc make_inst_desc(const aderdg_config* cfg);
+InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops);
 }
 
 namespace {
@@ -201,7 +201,7 @@ extern "C" int aderdg_calc_time_step_noalloc(const aderdg_config* cfg, const dou
   unsigned long long* scratch = nullptr;
   int r = scratch_address(&scratch);
   if (r) return r;
-  const aderdg::InstDesc in = aderdg::make_inst_desc(cfg);
+  const aderdg::InstDesc in = aderdg::make_inst_desc(cfg, nullptr);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   cudaError_t e = cudaMemsetAsync(scratch + kMaxBlocks, 0, sizeof(unsigned long long), s);
   if (e != cudaSuccess) {

@@ -48,7 +48,10 @@ void make_ops(const HostOps& h, void* out) {
     o.FRf[a] = (float)h.FR[a];
   }
   for (int j = 0; j < P; ++j)
-    for (int i = 0; i < P; ++i) o.iwwf[i + P * j] = (float)(1.0 / (h.w[i] * h.w[j]));
+    for (int i = 0; i < P; ++i) {
+      o.iwwd[i + P * j] = 1.0 / (h.w[i] * h.w[j]);
+      o.iwwf[i + P * j] = (float)o.iwwd[i + P * j];
+    }
   for (int k = 0; k < P * P; ++k) {
     o.Kxi[k] = (R)h.Kxi[k];
     o.dudx[k] = (R)h.dudx[k];

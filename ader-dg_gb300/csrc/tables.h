@@ -44,6 +44,7 @@ struct KernelTable {
   int (*subcell_grid_mixed)(int num_sms) = nullptr;
   // exact translation unit
   cudaError_t (*faces)(const BatchArgs&, const FaceConst&, int fp32, cudaStream_t) = nullptr;
+  // fast: 0 FP64 in reference order, 1 the FP32 modes, 2 FP64 with certified FP32 projections
   cudaError_t (*cells)(const BatchArgs&, const void* ops64, int fast, cudaStream_t) = nullptr;
   cudaError_t (*volume)(const BatchArgs&, const void* ops64, cudaStream_t) = nullptr;
   cudaError_t (*mark)(const BatchArgs&, cudaStream_t) = nullptr;
@@ -79,8 +80,9 @@ const KernelTable* kernel_table(int sys, int N);
 // The tuner's choice for (system, N, precision) (registry.cu; zeros: the defaults).
 aderdg_tuning tuning_of(int sys, int N, int precision);
 
-// The FP32 modes' predictor and cell kernel in the tuned variant; FP64 keeps
-// the reference-order kernels of its own.
+// The FP32 modes' predictor and cell kernel in the tuned variant; FP64 has
+// kernels of its own (the cell kernel: reference order throughout in the phase
+// API and the priming passes, whose min/max are introspection outputs).
 inline cudaError_t launch_predictor(const KernelTable* kt, const BatchArgs& a, const void* ops, int precision,
                                     cudaStream_t s) {
   const int fp32 = precision != ADERDG_FP64 ? 1 : 0;
@@ -96,6 +98,8 @@ inline cudaError_t launch_cells(const KernelTable* kt, const BatchArgs& a, const
   if (fast) {
     const int v = tuning_of(kt->sys, kt->N, precision).cells;
     if (v > 0 && v < kCellVariantsMax && kt->cells_var[v]) return kt->cells_var[v](a, ops64, s);
+  } else if (a.mode == kCellFused && a.mme[0]) {
+    return kt->cells(a, ops64, 2, s);  // FP64 update, certified FP32 projections
   }
   return kt->cells(a, ops64, fast, s);
 }
