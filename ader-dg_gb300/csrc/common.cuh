@@ -94,13 +94,7 @@ struct DevOps {
   R g[P];            // sum_l iK1(l',l)*F0(l)
   R ts[P];           // sum_l T(l',l)
   R tw[P];           // sum_l' w(l') T(l',l)
-  R iw[P];           // 1/w
   R wg;              // sum_l' w(l') g(l')
-  // Kxi, T, the end values FL and FR, and the time weights w and tw in 58-bit
-  // fixed point (predictor_fix.cuh): entry = (h 2^29 + l) 2^-s, h and l signed,
-  // |h| <= 2^28
-  int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];
-  int sK, sT, sE, sW;
   R FL[P], FR[P];
   double wd[P], FLd[P], FRd[P];
   float wf[P], FLf[P], FRf[P];  // FP32-mixed surface integral and update
@@ -118,6 +112,23 @@ struct DevOps {
   // deviations d = fl(fl(uh) - ubar) formed in FP32 from the FP32-rounded
   // state: their rounding adds at most pdev * (|ubar| + 2 max|d|) to the projections
   float pdev;
+};
+
+// The FP64 predictor's operators: the above (first, so that the other FP64
+// kernels take them from the same host copy) and its fixed-point tables, kept
+// out of the other kernels' parameters: every launch copies its parameters, and
+// 0.6 KB more of them cost a small step 2%.
+template <int N, class R>
+struct PredOps : DevOps<N, R> {};
+template <int N>
+struct PredOps<N, double> : DevOps<N, double> {
+  static constexpr int P = N + 1;
+  double iw[P];  // 1/w
+  // Kxi, T, the end values FL and FR, and the time weights w and tw in 58-bit
+  // fixed point (predictor_fix.cuh): entry = (h 2^29 + l) 2^-s, h and l signed,
+  // |h| <= 2^28
+  int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];
+  int sK, sT, sE, sW;
 };
 
 // Arguments shared by all kernels of one (system, N) batch.  The state that

@@ -110,8 +110,9 @@ struct SubCfg {
   static constexpr int DMP_DBL = V * P2 + V * S * P + V * P * P + 2 * V * (THREADS / 32);
   static constexpr bool DMP_IN_EF = sizeof(T) == 8 && DMP_DBL <= NEF;
   static constexpr int DEL = (DMP_IN_EF ? 0 : DMP_DBL) + OPS_DBL;
-  // misc: flags, CFL max, neighbour cells and their status
-  static constexpr int MISC = 16 + 9 * 8 + 9 * 4 + 4 * V + 12;
+  // misc: flags, CFL max, neighbour cells and their status, |UN - UN(node 0)|
+  // maxima, FP32 uh2lim and uh2lob (T = double)
+  static constexpr int MISC = 16 + 9 * 8 + 9 * 4 + 4 * V + 12 + (sizeof(T) == 8 ? 4 * OPS_DBL : 0);
   static constexpr int SMEM_BYTES = TBYTES + DEL * 8 + MISC;
 };
 
@@ -134,7 +135,8 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
 }
 
 // Subgrid Rusanov flux (Euler/limiter.f90:361-378; BN :359-383 adds D = B~ dQ);
-// kRcp: the reciprocal-sharing physics forms (FP32-mixed mode)
+// kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
+// flux (the update takes half its factor: one FP64 instruction less a variable)
 template <class Sys, class T, bool kRcp = false>
 __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const T* QR, int d, T* F, T* D) {
   constexpr int V = Sys::V;
@@ -146,7 +148,7 @@ __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const
     Sys::flux_dir_eig_r(pc, QR, d, FRf, eR);
     smax = tmax(eL, eR);
 #pragma unroll
-    for (int v = 0; v < V; ++v) F[v] = T(0.5) * (FLf[v] + FRf[v]) - T(0.5) * smax * (QR[v] - QL[v]);
+    for (int v = 0; v < V; ++v) F[v] = (FLf[v] + FRf[v]) - smax * (QR[v] - QL[v]);
   } else {
     smax = tmax(Sys::max_eig(pc, QL, d), Sys::max_eig(pc, QR, d));
     Sys::flux(pc, QL, FLf);
@@ -222,14 +224,18 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
   unsigned long long* cmaxp = reinterpret_cast<unsigned long long*>(misc + 8);
   long long* nbc = reinterpret_cast<long long*>(misc + 16);  // 3x3 neighbour cells, n = (bi+1) + 3 (bj+1)
   int* nbs = reinterpret_cast<int*>(misc + 16 + 9 * 8);     // their status (0: project olduh)
-  unsigned* amax = reinterpret_cast<unsigned*>(nbs + 9);     // FP32-wide: max |UN - UN(node 0)| per variable
+  unsigned* amax = reinterpret_cast<unsigned*>(nbs + 9);     // max |UN - UN(node 0)| per variable
+  float* limf = reinterpret_cast<float*>(amax + V);          // T = double: uh2lim and uh2lob in FP32
   float* UNf = reinterpret_cast<float*>(wLy);                // FP32 DMP (after the re-solve)
   float* LYf = UNf + V * P2;
   float* LBf = LYf + V * S * P;
   float* redf = reinterpret_cast<float*>(red);              // [2][V][NW]
 
   const int t = threadIdx.x;
-  for (int k = t; k < C::OPS_DBL; k += NT) opsm[k] = k < S * P ? op.uh2lim[k] : op.uh2lob[k - S * P];
+  for (int k = t; k < C::OPS_DBL; k += NT) {
+    opsm[k] = k < S * P ? op.uh2lim[k] : op.uh2lob[k - S * P];
+    if constexpr (sizeof(T) == 8) limf[k] = k < S * P ? op.uh2limf[k] : op.uh2lobf[k - S * P];
+  }
   for (int k = t; k < S * P; k += NT) {
     limT[k] = (T)op.uh2lim[k];
     l2uT[k] = (T)op.lim2uh[k];
@@ -529,7 +535,8 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
         for (int v = 0; v < V; ++v) dst[v * NE + q] = F[v];
         if constexpr (BN) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) dst[(V + v) * NE + q] = Dd[v];
+          for (int v = 0; v < V; ++v)
+            if (!kRcp || (v != 0 && v != 4)) dst[(V + v) * NE + q] = Dd[v];
         }
       }
       __syncthreads();
@@ -537,24 +544,36 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
         const int ii = p % S + 1, jj = p / S + 1;
         const int xp = ii + (S + 1) * (jj - 1), xm = (ii - 1) + (S + 1) * (jj - 1);
         const int yp = (ii - 1) + S * jj, ym = (ii - 1) + S * (jj - 1);
+        // kRcp: EX, EY hold twice the flux
+        const T fX = kRcp ? T(0.5) * divx(dt) : divx(dt), fY = kRcp ? T(0.5) * divy(dt) : divy(dt);
         if constexpr (!BN) {
           // first-order FV update, Euler/limiter.f90:592-597
 #pragma unroll
           for (int v = 0; v < V; ++v)
-            sub1[v * S * S + p] = SU(v, ii, jj) - divx(dt) * (EX[v * NE + xp] - EX[v * NE + xm]) -
-                                  divy(dt) * (EY[v * NE + yp] - EY[v * NE + ym]);
+            sub1[v * S * S + p] = SU(v, ii, jj) - fX * (EX[v * NE + xp] - EX[v * NE + xm]) -
+                                  fY * (EY[v * NE + yp] - EY[v * NE + ym]);
         } else {
           T qh[V], src[V];
 #pragma unroll
           for (int v = 0; v < V; ++v) qh[v] = SU(v, ii, jj) + T(0.5) * dt * slt[hx(v, ii, jj)];
           ncp(qh, divx(sa8[ii + H * jj]), divy(sa8[H * H + ii + H * jj]), src);
 #pragma unroll
-          for (int v = 0; v < V; ++v)
-            sub1[v * S * S + p] = SU(v, ii, jj) - divx(dt) * (EX[v * NE + xp] - EX[v * NE + xm]) -
-                                  divy(dt) * (EY[v * NE + yp] - EY[v * NE + ym]) -
-                                  divx(dt) * T(0.5) * (EX[(V + v) * NE + xp] + EX[(V + v) * NE + xm]) -
-                                  divy(dt) * T(0.5) * (EY[(V + v) * NE + yp] + EY[(V + v) * NE + ym]) +
-                                  dt * src[v];
+          for (int v = 0; v < V; ++v) {
+            if constexpr (kRcp) {
+              // the fluctuation of an x (y) edge has no component along y (x),
+              // nor in the two densities
+              T q = SU(v, ii, jj) - fX * (EX[v * NE + xp] - EX[v * NE + xm]) - fY * (EY[v * NE + yp] - EY[v * NE + ym]);
+              if (v != 0 && v != 2 && v != 4 && v != 6) q = q - fX * (EX[(V + v) * NE + xp] + EX[(V + v) * NE + xm]);
+              if (v != 0 && v != 1 && v != 4 && v != 5) q = q - fY * (EY[(V + v) * NE + yp] + EY[(V + v) * NE + ym]);
+              sub1[v * S * S + p] = v != 0 && v != 4 ? q + dt * src[v] : q;
+            } else {
+              sub1[v * S * S + p] = SU(v, ii, jj) - divx(dt) * (EX[v * NE + xp] - EX[v * NE + xm]) -
+                                    divy(dt) * (EY[v * NE + yp] - EY[v * NE + ym]) -
+                                    divx(dt) * T(0.5) * (EX[(V + v) * NE + xp] + EX[(V + v) * NE + xm]) -
+                                    divy(dt) * T(0.5) * (EY[(V + v) * NE + yp] + EY[(V + v) * NE + ym]) +
+                                    dt * src[v];
+            }
+          }
         }
       }
     }
@@ -585,36 +604,35 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     __syncthreads();
     // ---- DMP of the new polynomial: recompute = 2 cells only (a recompute =
     // 1 cell is limited whatever it gives, and its next min/max come from
-    // its subcell data), uniform per CTA.
-    const bool dmp = rec == 2;
-    if constexpr (sizeof(T) == 4) {
-      // FP32-wide DMP: deviations from the new polynomial's node-0 state
-      if (dmp) {
-        for (int p = t; p < P2; p += NT)
-#pragma unroll
-          for (int v = 0; v < V; ++v) {
-            const float d = (float)(UN[v * P2 + p] - UN[v * P2]);
-            UNf[v * P2 + p] = d;
-            atomicMax(&amax[v], __float_as_uint(fabsf(d)));
-          }
-      }
-      __syncthreads();
-    }
-    // FP32-wide (T = float): FP32 projections when their error bound stays
+    // its subcell data), uniform per CTA.  FP32 projections of the deviations
+    // from the new polynomial's node-0 state when their error bound stays
     // within the DMP's absolute tolerance, else FP64 (as in the cell kernel).
-    float err[V];
-    bool f32 = false;
-    if constexpr (sizeof(T) == 4) {
-      f32 = true;
+    // T = double: a comparison the bounds leave open is decided from FP64 values
+    // below; T = float (FP32-wide): the FP32 values are taken as they are.  (The
+    // FP64 re-solve projected in FP64 throughout before: a fifth of its FP64
+    // instructions on a recompute = 2 cell.)
+    const bool dmp = rec == 2;
+    const bool try32 = sizeof(T) == 4 || a.mme[0] != nullptr;
+    const float* lim32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(limT) : limf;
+    const float* lob32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(lobT) : limf + S * P;
+    if (dmp && try32) {
+      for (int p = t; p < P2; p += NT)
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        err[v] = op.perr * __uint_as_float(amax[v]);
-        f32 = f32 && err[v] <= 1.0e-4f;
-      }
+        for (int v = 0; v < V; ++v) {
+          const float d = (float)(UN[v * P2 + p] - UN[v * P2]);
+          UNf[v * P2 + p] = d;
+          atomicMax(&amax[v], __float_as_uint(fabsf(d)));
+        }
     }
-    if constexpr (sizeof(T) == 4) {
-      if (dmp && f32) Proj<N, V, float>::template ypass<true>(UNf, LYf, LBf, limT, lobT, t, NT);
+    __syncthreads();
+    float err[V];
+    bool f32 = try32;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      err[v] = op.perr * __uint_as_float(amax[v]);
+      f32 = f32 && err[v] <= 1.0e-4f;
     }
+    if (dmp && f32) Proj<N, V, float>::template ypass<true>(UNf, LYf, LBf, lim32, lob32, t, NT);
     if (dmp && !f32) Proj<N, V, double>::ypass(UN, LY, LB, opsm, opsm + S * P, t, NT);
     __syncthreads();
     double mn[V], mx[V];
@@ -622,19 +640,16 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     if (!dmp) {
       // no projections: the CFL part below only
     } else if (f32) {
-      float fmn[V], fmx[V];
+      float fmn[V], fmx[V], ubf[V];
 #pragma unroll
       for (int v = 0; v < V; ++v) { fmn[v] = __int_as_float(0x7f800000); fmx[v] = -__int_as_float(0x7f800000); }
       for (int p = t; p < P2; p += NT)
 #pragma unroll
         for (int v = 0; v < V; ++v) { fmn[v] = fminf(fmn[v], UNf[v * P2 + p]); fmx[v] = fmaxf(fmx[v], UNf[v * P2 + p]); }
-      if constexpr (sizeof(T) == 4) {
-        float ubf[V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) ubf[v] = (float)UN[v * P2];
-        Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, limT, lobT, UN, opsm, typename Sys::FConst(ph), err,
-                                                          ubf, ph, t, NT, fmn, fmx, posfail);
-      }
+      for (int v = 0; v < V; ++v) ubf[v] = (float)UN[v * P2];
+      Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, lim32, lob32, UN, opsm, typename Sys::FConst(ph), err,
+                                                        ubf, ph, t, NT, fmn, fmx, posfail);
       warp_minmax_store<float, V, NW>(fmn, fmx, redf, t);
     } else {
 #pragma unroll
@@ -654,6 +669,10 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
 #pragma unroll
         for (int v = 0; v < V; ++v) q[v] = (float)Q[v];
         dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(ph), q, Q);
+      } else if constexpr (kRcp) {
+        double ex, ey;
+        Sys::max_eig2_r(pc, Q, ex, ey);
+        dn = fma(ex, in.rdx, ey * in.rdy);
       } else {
         dn = cfl_denom<Sys, N>(in, Q);
       }
@@ -663,14 +682,21 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     __syncthreads();
     double* mmo = a.mm[par ^ 1] + (size_t)c * 2 * V;
     double dmn = 0.0, dmx = 0.0;  // thread v < V: min/max of the new polynomial's variable v
+    float dme = 0.0f;             // and the bound on their error (0: FP64 values)
     if (dmp && t < V) {
       const int v = t;
       double cmn, cmx;
+      float fmn = 0.0f, fmx = 0.0f;
       if (f32) {
-        float fmn = redf[v * NW], fmx = redf[(V + v) * NW];
+        fmn = redf[v * NW];
+        fmx = redf[(V + v) * NW];
         for (int q = 1; q < NW; ++q) { fmn = fminf(fmn, redf[v * NW + q]); fmx = fmaxf(fmx, redf[(V + v) * NW + q]); }
         cmn = UN[v * P2] + (double)fmn;
         cmx = UN[v * P2] + (double)fmx;
+        // the projections' bound, and the FP64 roundings of the reference-order
+        // values (generously 1e-12 relative)
+        const float am = __uint_as_float(amax[v]);
+        if (sizeof(T) == 8) dme = op.perr * am * 1.0001f + 1.0e-12f * (fabsf((float)UN[v * P2]) + am);
       } else {
         cmn = red[v * NW];
         cmx = red[(V + v) * NW];
@@ -678,40 +704,68 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       }
       dmn = cmn;
       dmx = cmx;
-      if (rec == 2) {
-        const double* mmi = a.mm[par];
-        double lmin = mmi[(size_t)c * 2 * V + v], lmax = mmi[(size_t)c * 2 * V + V + v];
-        float en = 0.0f;  // FP32-mixed: largest error bound of the folded min/max
-        for (int jj = -1; jj <= 1; ++jj)
-          for (int ii = -1; ii <= 1; ++ii) {
-            const int in_ = nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]);
-            const int jn_ = nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
-            const long long nc = in.cell_base + in_ + (long long)in.imax * jn_;
-            lmin = fmin(lmin, mmi[(size_t)nc * 2 * V + v]);
-            lmax = fmax(lmax, mmi[(size_t)nc * 2 * V + V + v]);
-            if (a.mme[0]) en = fmaxf(en, a.mme[par][(size_t)nc * V + v]);
-          }
-        const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (lmax - lmin)), 0.0);
-        if (en == 0.0f) {
-          if (cmn < lmin - ldiff || cmx > lmax + ldiff) atomicOr(&flag[0], 2);
-        } else {
-          // FP32-mixed: the own values are FP64; the neighbourhood bounds
-          // carry at most en, so the threshold moves by at most en (1 + 2e-3).
-          // Comparisons inside that margin are settled below (bit 4).
-          const double M = 1.002 * (double)en + 1.0e-13 * (fabs(lmin) + fabs(lmax) + fabs(cmn) + fabs(cmx));
-          if (cmn < lmin - ldiff - M || cmx > lmax + ldiff + M) atomicOr(&flag[0], 2);
-          else if (!(cmn >= lmin - ldiff + M) || !(cmx <= lmax + ldiff - M)) atomicOr(&flag[0], 4);
+      const double* mmi = a.mm[par];
+      double lmin = mmi[(size_t)c * 2 * V + v], lmax = mmi[(size_t)c * 2 * V + V + v];
+      float en = 0.0f;  // largest error bound of the folded min/max
+      for (int jj = -1; jj <= 1; ++jj)
+        for (int ii = -1; ii <= 1; ++ii) {
+          const int in_ = nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]);
+          const int jn_ = nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
+          const long long nc = in.cell_base + in_ + (long long)in.imax * jn_;
+          lmin = fmin(lmin, mmi[(size_t)nc * 2 * V + v]);
+          lmax = fmax(lmax, mmi[(size_t)nc * 2 * V + V + v]);
+          if (a.mme[0]) en = fmaxf(en, a.mme[par][(size_t)nc * V + v]);
         }
+      if (en == 0.0f && dme == 0.0f) {
+        const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (lmax - lmin)), 0.0);
+        if (cmn < lmin - ldiff || cmx > lmax + ldiff) atomicOr(&flag[0], 2);
+      } else {
+        // the cell kernel's certified comparison, in the deviation space of
+        // the node-0 state: the own values carry dme, the neighbourhood bounds
+        // at most en (so the thresholds move by at most en (1 + 2e-3)), and the
+        // FP32 forms at most 2.5e-7 of the magnitudes involved; inside that
+        // margin the comparison is settled from FP64 values below (bit 4)
+        const double ub = UN[v * P2];
+        const float Lmin = (float)(lmin - ub), Lmax = (float)(lmax - ub);
+        const float ld = fmaxf(1.0e-4f, 1.0e-3f * (Lmax - Lmin));
+        const float xl = f32 ? fmn : (float)(cmn - ub), xh = f32 ? fmx : (float)(cmx - ub);
+        const float e = dme + 1.002f * en + 2.5e-7f * (fabsf(Lmin) + fabsf(Lmax) + ld) + 1.0e-11f + 1.0e-12f * fabsf((float)ub);
+        const float ml = e + 1.2e-7f * fabsf(xl), mh = e + 1.2e-7f * fabsf(xh);
+        const float gl = xl - (Lmin - ld), gh = (Lmax + ld) - xh;
+        if (gl < -ml || gh < -mh) atomicOr(&flag[0], 2);
+        else if (!(gl >= ml) || !(gh >= mh)) atomicOr(&flag[0], 4);
       }
     }
     __syncthreads();
     if constexpr (sizeof(T) == 8) {
-      if (rec == 2 && a.mme[0] != nullptr && (flag[0] & 7) == 4) {
-        // FP32-mixed, a recompute = 2 DMP the bounds left open: the min/max
-        // of every neighbour whose stored values carry an error bound are
-        // recomputed from its start-of-step state in FP64 reference order,
-        // so that the decision is the FP64 path's on this state
+      if (dmp && a.mme[0] != nullptr && (flag[0] & 7) == 4) {
+        // a DMP the bounds left open: the new polynomial's min/max, and those
+        // of every neighbour whose stored values carry an error bound from its
+        // start-of-step state, in FP64 reference order, so that the decision
+        // is the FP64 path's on this state
         if (t == 0) atomicAdd(&a.st[k].n_settled, 1);
+        // FP64 min/max of the polynomial in UN: thread v < V gets variable v's
+        auto minmax64 = [&](double& lo, double& hi) {
+          Proj<N, V, double>::ypass(UN, LY, LB, opsm, opsm + S * P, t, NT);
+          __syncthreads();
+          double nmn[V], nmx[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) { nmn[v] = kInf; nmx[v] = -kInf; }
+          bool pdummy = false;
+          Proj<N, V, double>::template xpass_minmax<Sys>(UN, LY, LB, opsm, opsm + S * P, ph, t, NT, nmn, nmx, pdummy);
+          warp_minmax_store<double, V, NW>(nmn, nmx, red, t);
+          __syncthreads();
+          if (t < V) {
+            lo = red[t * NW];
+            hi = red[(V + t) * NW];
+            for (int q = 1; q < NW; ++q) { lo = fmin(lo, red[t * NW + q]); hi = fmax(hi, red[(V + t) * NW + q]); }
+          }
+          __syncthreads();
+        };
+        if (f32) {
+          minmax64(dmn, dmx);
+          dme = 0.0f;
+        }
         double elmin = kInf, elmax = -kInf;
         for (int n = 0; n < 9; ++n) {
           const long long nc = nbc[n];
@@ -720,38 +774,21 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
 #pragma unroll
             for (int v = 0; v < V; ++v) comp = comp || a.mme[par][(size_t)nc * V + v] > 0.0f;
           }
-          if (comp) {
+          double lo = 0.0, hi = 0.0;
+          if (comp) {  // uniform over the CTA
             const double* un = a.uh[par] + (size_t)nc * P2 * V;
             for (int p = t; p < P2 * V; p += NT) {
               const int node = p / V, v = p - node * V;
               UN[v * P2 + node] = un[p];
             }
+            __syncthreads();
+            minmax64(lo, hi);
+          } else if (t < V) {
+            lo = a.mm[par][(size_t)nc * 2 * V + t];
+            hi = a.mm[par][(size_t)nc * 2 * V + V + t];
           }
-          __syncthreads();
-          if (comp) Proj<N, V, double>::ypass(UN, LY, LB, opsm, opsm + S * P, t, NT);
-          __syncthreads();
-          double nmn[V], nmx[V];
-#pragma unroll
-          for (int v = 0; v < V; ++v) { nmn[v] = kInf; nmx[v] = -kInf; }
-          bool pdummy = false;
-          if (comp) Proj<N, V, double>::template xpass_minmax<Sys>(UN, LY, LB, opsm, opsm + S * P, ph, t, NT, nmn, nmx, pdummy);
-          warp_minmax_store<double, V, NW>(nmn, nmx, red, t);
-          __syncthreads();
-          if (t < V) {
-            const int v = t;
-            double lo, hi;
-            if (comp) {
-              lo = red[v * NW];
-              hi = red[(V + v) * NW];
-              for (int q = 1; q < NW; ++q) { lo = fmin(lo, red[v * NW + q]); hi = fmax(hi, red[(V + v) * NW + q]); }
-            } else {
-              lo = a.mm[par][(size_t)nc * 2 * V + v];
-              hi = a.mm[par][(size_t)nc * 2 * V + V + v];
-            }
-            elmin = fmin(elmin, lo);
-            elmax = fmax(elmax, hi);
-          }
-          __syncthreads();
+          elmin = fmin(elmin, lo);
+          elmax = fmax(elmax, hi);
         }
         if (t < V) {
           const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (elmax - elmin)), 0.0);
@@ -784,7 +821,9 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     if (t < V) {
       const int v = t;
       double cmn = dmn, cmx = dmx;
+      float cme = dme;
       if (limited) {
+        cme = 0.0f;
         T lo = redt[v * NW], hi = redt[(V + v) * NW];
         for (int q = 1; q < NW; ++q) { lo = tmin(lo, redt[v * NW + q]); hi = tmax(hi, redt[(V + v) * NW + q]); }
         cmn = (double)lo;
@@ -792,7 +831,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       }
       mmo[v] = cmn;
       mmo[V + v] = cmx;
-      if (a.mme[0]) a.mme[par ^ 1][(size_t)c * V + v] = 0.0f;  // FP64 values
+      if (a.mme[0]) a.mme[par ^ 1][(size_t)c * V + v] = cme;
     }
     if (t == 0) {
       a.status[par ^ 1][c] = limited ? 1 : 0;

@@ -170,6 +170,17 @@ struct EulerSys {
     flux_eig_r<T>(pc, Q, d, nullptr, e);
     return e;
   }
+  // maxval(abs(Lambda)) along both axes; a NaN sound speed leaves the velocity,
+  // as the maxima of max_eig2 do
+  template <class T>
+  __device__ static void max_eig2_r(const PhysC<T>& pc, const T* Q, T& ex, T& ey) {
+    const T irho = mrcp<T>(Q[0]);
+    const T u = Q[1] * irho, v = Q[2] * irho;
+    const T p = pc.gm1 * (Q[3] - T(0.5) * (Q[1] * u + Q[2] * v));
+    const T c = msqrt<T>(pc.gamma * p * irho);
+    ex = tmax(tabs(u), tabs(u) + c);
+    ey = tmax(tabs(v), tabs(v) + c);
+  }
   // The flux along axis d only, F[v] (Fx = F[0..3], Fy = F[4..7] of
   // flux_eig_r; Q1 v = Q2 u), and maxval(abs(Lambda)) along d
   template <class T>
@@ -487,6 +498,21 @@ struct BNSys {
     T e;
     flux_eig_r<T>(pc, Q, d, nullptr, e);
     return e;
+  }
+  // maxval(abs(Lambda)) along both axes; a NaN sound speed leaves the velocity,
+  // as the maxima of max_eig2 do
+  template <class T>
+  __device__ static void max_eig2_r(const PhysC<T>& pc, const T* Q, T& ex, T& ey) {
+    const T r = mrcp<T>(Q[0] * Q[4]);
+    const T i0 = Q[4] * r, i4 = Q[0] * r;
+    const T u_s = Q[1] * i0, v_s = Q[2] * i0, u_g = Q[5] * i4, v_g = Q[6] * i4;
+    const T phi_s = Q[8], phi_g = T(1) - Q[8];
+    const T pps = pc.gs1 * (Q[3] - T(0.5) * (Q[1] * u_s + Q[2] * v_s)) - pc.gsps * phi_s;
+    const T ppg = pc.gg1 * (Q[7] - T(0.5) * (Q[5] * u_g + Q[6] * v_g)) - pc.ggpg * phi_g;
+    const T a_s = msqrt<T>(pc.gs * (pps + pc.ps * phi_s) * i0);
+    const T a_g = msqrt<T>(pc.gg * (ppg + pc.pg * phi_g) * i4);
+    ex = tmax(tmax(tabs(u_g), tabs(u_g) + a_g), tmax(tabs(u_s), tabs(u_s) + a_s));
+    ey = tmax(tmax(tabs(v_g), tabs(v_g) + a_g), tmax(tabs(v_s), tabs(v_s) + a_s));
   }
   // The flux along axis d only, F[v] (the d-th half of flux_eig_r's F; Q1 v_s
   // = Q2 u_s), and maxval(abs(Lambda)) along d

@@ -415,7 +415,7 @@ __device__ __forceinline__ void predictor_outputs(const BatchArgs& a, const DevO
 
 template <class Sys, int N, class R, bool kPhase, class Tune = PredTune<>>
 __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys, N, R, Tune>::MIN_BLOCKS)
-    k_predictor(BatchArgs a, DevOps<N, R> op) {
+    k_predictor(BatchArgs a, PredOps<N, R> op) {
   using C = PredCfg<Sys, N, R, Tune>;
   constexpr int P = N + 1, P2 = P * P, V = Sys::V, CPB = C::CPB, VP = C::VP;
   extern __shared__ __align__(16) unsigned char smem_raw[];

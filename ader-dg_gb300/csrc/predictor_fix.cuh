@@ -159,7 +159,7 @@ __device__ __forceinline__ void fix_line(double* __restrict__ p, int stride, int
 // the CTA's last cell, which take part in the barriers only.
 template <class Sys, int N, class C, class PC>
 __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double* __restrict__ sG,
-                                           const DevOps<N, double>& op, const PC& pc, const double* __restrict__ un,
+                                           const PredOps<N, double>& op, const PC& pc, const double* __restrict__ un,
                                            bool act, int i, int j, double cxw, double cyw, double idx, double idy,
                                            double dt, double* qh, double (*Fh)[Sys::V], double* Sh, bool live) {
   constexpr int P = N + 1, P2 = P * P, V = Sys::V, VF = C::VF;
@@ -413,7 +413,7 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
 // over the cell's threads; ex: room for their exponents.  All threads of the
 // CTA call it (one barrier); only those of active cells (act) do work.
 template <class Sys, int N, bool kVolume>
-__device__ __forceinline__ void outputs_fix(const BatchArgs& a, const DevOps<N, double>& op, double rdx, double rdy,
+__device__ __forceinline__ void outputs_fix(const BatchArgs& a, const PredOps<N, double>& op, double rdx, double rdy,
                                             double* __restrict__ cs, int* __restrict__ ex, long long cell, int node,
                                             int i, int j, const double* Sh, bool act) {
   constexpr int P = N + 1, P2 = P * P, V = Sys::V;

@@ -31,10 +31,9 @@ constexpr int N = ADERDG_N;
 template <class R>
 void make_ops(const HostOps& h, void* out) {
   constexpr int P = N + 1, S = 2 * N + 1;
-  DevOps<N, R> o;
+  PredOps<N, R> o;
   for (int a = 0; a < P; ++a) {
     o.w[a] = (R)h.w[a];
-    o.iw[a] = (R)(1.0 / h.w[a]);
     o.FL[a] = (R)h.FL[a];
     o.FR[a] = (R)h.FR[a];
     o.wd[a] = h.w[a];
@@ -79,52 +78,55 @@ void make_ops(const HostOps& h, void* out) {
     tws[l] = tw;
   }
   o.wg = (R)wg;
-  // fixed-point limbs under one scale per operator: every entry below 2^57,
-  // every sum of magnitudes the kernel forms (bounded by `sum`) below 2^59
-  auto limbs = [](const double* M, int n, int sh, int* hi, int* lo) {
-    for (int k = 0; k < n; ++k) {
-      const long long x = std::llrint(std::ldexp(M[k], sh));
-      long long l = x & ((1ll << 29) - 1);
-      if (l >= (1ll << 28)) l -= 1ll << 29;
-      lo[k] = (int)l;
-      hi[k] = (int)((x - l) >> 29);
+  if constexpr (sizeof(R) == 8) {
+    // fixed-point limbs under one scale per operator: every entry below 2^57,
+    // every sum of magnitudes the kernel forms (bounded by `sum`) below 2^59
+    auto limbs = [](const double* M, int n, int sh, int* hi, int* lo) {
+      for (int k = 0; k < n; ++k) {
+        const long long x = std::llrint(std::ldexp(M[k], sh));
+        long long l = x & ((1ll << 29) - 1);
+        if (l >= (1ll << 28)) l -= 1ll << 29;
+        lo[k] = (int)l;
+        hi[k] = (int)((x - l) >> 29);
+      }
+    };
+    auto scale = [](const double* M, int n, double sum) {
+      double big = 0.0;
+      for (int k = 0; k < n; ++k) big = std::fmax(big, std::fabs(M[k]));
+      int sh = 56 - std::ilogb(big);
+      while (std::ldexp(sum, sh) >= std::ldexp(1.0, 59)) --sh;
+      return sh;
+    };
+    double Tm[P * P], ends[2 * P], times[2 * P];
+    double sumK = 0.0, sumT = 0.0, sumE = 0.0, sumW = 0.0;
+    for (int l = 0; l < P; ++l) {
+      double rK = 0.0, cK = 0.0, rT = 0.0;
+      for (int m = 0; m < P; ++m) {
+        Tm[l + P * m] = T[l][m];
+        rK += std::fabs(h.Kxi[l + P * m]);
+        cK += std::fabs(h.Kxi[m + P * l]);
+        rT += std::fabs(T[l][m]);
+      }
+      sumK = std::fmax(sumK, std::fmax(rK, cK));
+      sumT = std::fmax(sumT, rT);
+      ends[l] = h.FL[l];
+      ends[P + l] = h.FR[l];
+      times[l] = h.w[l];
+      times[P + l] = tws[l];
+      sumE += std::fabs(h.FL[l]) + std::fabs(h.FR[l]);
+      sumW += std::fabs(h.w[l]) + std::fabs(tws[l]);
     }
-  };
-  auto scale = [](const double* M, int n, double sum) {
-    double big = 0.0;
-    for (int k = 0; k < n; ++k) big = std::fmax(big, std::fabs(M[k]));
-    int sh = 56 - std::ilogb(big);
-    while (std::ldexp(sum, sh) >= std::ldexp(1.0, 59)) --sh;
-    return sh;
-  };
-  double Tm[P * P], ends[2 * P], times[2 * P];
-  double sumK = 0.0, sumT = 0.0, sumE = 0.0, sumW = 0.0;
-  for (int l = 0; l < P; ++l) {
-    double rK = 0.0, cK = 0.0, rT = 0.0;
-    for (int m = 0; m < P; ++m) {
-      Tm[l + P * m] = T[l][m];
-      rK += std::fabs(h.Kxi[l + P * m]);
-      cK += std::fabs(h.Kxi[m + P * l]);
-      rT += std::fabs(T[l][m]);
-    }
-    sumK = std::fmax(sumK, std::fmax(rK, cK));
-    sumT = std::fmax(sumT, rT);
-    ends[l] = h.FL[l];
-    ends[P + l] = h.FR[l];
-    times[l] = h.w[l];
-    times[P + l] = tws[l];
-    sumE += std::fabs(h.FL[l]) + std::fabs(h.FR[l]);
-    sumW += std::fabs(h.w[l]) + std::fabs(tws[l]);
+    o.sK = scale(h.Kxi.data(), P * P, sumK);
+    o.sT = scale(Tm, P * P, sumT);
+    o.sE = scale(ends, 2 * P, sumE);
+    o.sW = scale(times, 2 * P, sumW);
+    limbs(h.Kxi.data(), P * P, o.sK, o.Kh, o.Kl);
+    limbs(Tm, P * P, o.sT, o.Th, o.Tl);
+    limbs(ends, 2 * P, o.sE, o.Eh, o.El);
+    limbs(times, P, o.sW, o.Wh, o.Wl);
+    limbs(times + P, P, o.sW, o.TWh, o.TWl);
+    for (int k = 0; k < P; ++k) o.iw[k] = 1.0 / h.w[k];
   }
-  o.sK = scale(h.Kxi.data(), P * P, sumK);
-  o.sT = scale(Tm, P * P, sumT);
-  o.sE = scale(ends, 2 * P, sumE);
-  o.sW = scale(times, 2 * P, sumW);
-  limbs(h.Kxi.data(), P * P, o.sK, o.Kh, o.Kl);
-  limbs(Tm, P * P, o.sT, o.Th, o.Tl);
-  limbs(ends, 2 * P, o.sE, o.Eh, o.El);
-  limbs(times, P, o.sW, o.Wh, o.Wl);
-  limbs(times + P, P, o.sW, o.TWh, o.TWl);
   for (int k = 0; k < S * P; ++k) {
     o.uh2lim[k] = h.uh2lim[k];
     o.lim2uh[k] = h.lim2uh[k];
@@ -150,7 +152,7 @@ void make_ops(const HostOps& h, void* out) {
   o.perr = (float)(4.0 * (2 * P + 4) * std::ldexp(1.0, -24) * lam * lam);
   // a rounding of 2^-24 (|uh| + |d|) per node, through the two passes; factor 2 of safety
   o.pdev = (float)(2.0 * std::ldexp(1.0, -24) * lam * lam);
-  *reinterpret_cast<DevOps<N, R>*>(out) = o;
+  *reinterpret_cast<PredOps<N, R>*>(out) = o;
 }
 
 template <class R, bool kPhase>
@@ -165,7 +167,7 @@ cudaError_t launch_pred(const BatchArgs& a, const void* ops, cudaStream_t s) {
   }
   const long long grid = (a.ncells - a.cell0 + C::CPB - 1) / C::CPB;
   if (grid <= 0) return cudaSuccess;
-  kern<<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, R>*>(ops));
+  kern<<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const PredOps<N, R>*>(ops));
   return cudaGetLastError();
 }
 
@@ -221,8 +223,8 @@ cudaError_t faces_mixed(const BatchArgs& a, const FaceConst& fc, cudaStream_t s)
 void ADERDG_CAT(register_predictor_, ADERDG_SYS, ADERDG_N)(KernelTable& t) {
   t.sys = ADERDG_SYS;
   t.N = N;
-  t.ops64_size = sizeof(DevOps<N, double>);
-  t.ops32_size = sizeof(DevOps<N, float>);
+  t.ops64_size = sizeof(PredOps<N, double>);
+  t.ops32_size = sizeof(PredOps<N, float>);
   t.make_ops64 = &make_ops<double>;
   t.make_ops32 = &make_ops<float>;
   t.predictor = &predictor;

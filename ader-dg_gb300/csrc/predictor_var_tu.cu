@@ -39,7 +39,7 @@ cudaError_t predictor_var(const BatchArgs& a, const void* ops, cudaStream_t s) {
   }
   const long long grid = (a.ncells - a.cell0 + C::CPB - 1) / C::CPB;
   if (grid <= 0) return cudaSuccess;
-  kern<<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, float>*>(ops));
+  kern<<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const PredOps<N, float>*>(ops));
   return cudaGetLastError();
 }
 
