@@ -124,9 +124,8 @@ template <int N>
 struct PredOps<N, double> : DevOps<N, double> {
   static constexpr int P = N + 1;
   double iw[P];  // 1/w
-  // Kxi, T, the end values FL and FR, and the time weights w and tw in 58-bit
-  // fixed point (predictor_fix.cuh): entry = (h 2^29 + l) 2^-s, h and l signed,
-  // |h| <= 2^28
+  // Kxi, T, the end values FL and FR, and the time weights w and tw in 60-bit
+  // fixed point (predictor_fix.cuh): entry = (h 2^31 + l) 2^-s, 0 <= l < 2^31
   int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];
   int sK, sT, sE, sW;
 };

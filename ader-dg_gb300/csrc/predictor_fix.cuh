@@ -1,24 +1,26 @@
-// predictor_fix.cuh -- the FP64 predictor with its linear algebra in 58-bit
+// predictor_fix.cuh -- the FP64 predictor with its linear algebra in 60-bit
 // fixed point on the integer multiply-add pipe.
 //
 // Why: the FP64 pipe issues one warp instruction per 20 SM cycles (1.6 lanes
 // per clock, measured), the 32x32+64-bit multiply-add (IMAD.WIDE) one per 1.6.
 // Most of the predictor's FP64 instructions are products with constant
 // matrices: flux derivatives (Kxi), time update (T), time averages, volume
-// integral and face extrapolation.  A product of two 58-bit numbers in 29-bit
-// limbs takes three IMAD.WIDE (the low x low product is below the last bit
-// kept) = 4.9 cycles instead of 20, and the pipes overlap: the FP64 pipe keeps
+// integral and face extrapolation.  A product of two 60-bit numbers in 31-bit
+// limbs takes one IMAD.WIDE and two IMAD.HI (the cross products' upper halves;
+// the low x low product is below the last bit kept) = 3.8 cycles instead of 20,
+// and the pipes overlap: the FP64 pipe keeps
 // the pointwise fluxes and one conversion per result.  Measured (FP64 mode, all
-// in registers and FP64 before): Euler vortex N = 4, 256^2 5.02 -> 2.36 ms,
-// Riemann problem N = 3, 257 x 193 1.32 -> 0.61 ms, Baer-Nunziato cylinder N = 3,
-// 200^2 3.28 -> 1.91 ms.  On the vortex the FP64 pipe is then 53% and the
-// multiply-add pipe 48% busy.  N >= 3: below, the Picard iterations between the
+// in registers and FP64 before): Euler vortex N = 4, 256^2 5.02 -> 1.94 ms,
+// Riemann problem N = 3, 257 x 193 1.32 -> 0.55 ms, Baer-Nunziato cylinder N = 3,
+// 200^2 3.28 -> 1.76 ms (with 29-bit limbs, three IMAD.WIDE a product and the
+// loops less rolled: 2.36, 0.61 and 1.91 ms).  On the vortex the FP64 pipe is
+// then 62% and the multiply-add pipe 45% busy.  N >= 3: below, the Picard iterations between the
 // first and the last, which this is for, are at most one.
 //
 // Accuracy: each operand line takes its own power-of-two scale from its
-// largest magnitude, so a value's error is at most 2^-57 of that magnitude and
-// the constants' 2^-57 of the matrix's largest entry: every sum has an absolute
-// error of a few 2^-56 of its terms' size, where the FP64 chain rounds each
+// largest magnitude, so a value's error is at most 2^-60 of that magnitude and
+// the constants' 2^-60 of the matrix's largest row sum: every sum has an absolute
+// error of a few 2^-57 of its terms' size, where the FP64 chain rounds each
 // partial sum to 2^-53.  Lines holding infinities or NaNs, or whose largest
 // magnitude is beyond 2^900 or below 2^-823, are contracted in FP64 and their
 // nodes take the FP64 time update.
@@ -33,22 +35,24 @@ constexpr int kFixMin = 200;           // lines whose largest biased exponent li
 constexpr int kFixMax = 1023 + 900;    // or from here on take FP64
 constexpr int kFixOut = 1 << 20;       // "exponent" of a line contracted in FP64
 
-// (a * b) with a = (ah, al), b = (bh, bl) in 29-bit limbs, in units of 2^58:
-// ah*bh accumulates in s, ah*bl + al*bh in units of 2^29 in m.
-__device__ __forceinline__ void fix_madd(long long& s, long long& m, int ah, int al, int bh, int bl) {
+// Numbers are (h, l) with value h 2^31 + l, l >= 0 in 31 bits.  A product in
+// units of 2^62: h*h exactly (IMAD.WIDE, into s), and the upper 32 bits of the
+// two cross products (IMAD.HI, 1.1 cycles against IMAD.WIDE's 1.6, into m, in
+// units of two of the sum's; n products start m at n, half the roundings down,
+// unless all are 0: zeros stay exact).
+__device__ __forceinline__ void fix_madd(long long& s, int& m, int ah, int al, int bh, int bl) {
   s += (long long)ah * bh;
-  m += (long long)ah * bl;
-  m += (long long)al * bh;
+  asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(ah), "r"(bl));
+  asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(al), "r"(bh));
 }
-constexpr long long kFixHalf = 1ll << 28;  // start of m: rounds m >> 29 to nearest
-__device__ __forceinline__ long long fix_sum(long long s, long long m) { return s + (m >> 29); }
-__device__ __forceinline__ int fix_hi(long long x) { return (int)(x >> 29); }
-__device__ __forceinline__ int fix_lo(long long x) { return (int)x & ((1 << 29) - 1); }
+__device__ __forceinline__ long long fix_sum(long long s, int m) { return s + 2 * (long long)m; }
+__device__ __forceinline__ int fix_hi(long long x) { return (int)(x >> 31); }
+__device__ __forceinline__ int fix_lo(long long x) { return (int)x & 0x7fffffff; }
 // x >> d, 0 <= d, floor; everything beyond 63 is the sign
 __device__ __forceinline__ long long fix_shift(long long x, int d) { return x >> (d < 63 ? d : 63); }
 // signed integer X, |X| < 2^(53 + kUp), of the finite double (hi, lo) relative
 // to a biased exponent E >= its own: x = X 2^(E - 1023 - 52 - kUp)
-template <int kUp = 4>
+template <int kUp = 7>
 __device__ __forceinline__ long long fix_int(int hi, int lo, int E) {
   const int d = E - ((hi >> 20) & 0x7ff);
   const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
@@ -62,19 +66,20 @@ __device__ __forceinline__ double fix_double(long long x, int e) {
   const double r = (double)x;
   return __hiloint2double(__double2hiint(r) + (x != 0 ? e << 20 : 0), __double2loint(r));
 }
-// a positive factor c = C 2^(e - 1023 - 58), C = (h, l) in [2^58, 2^59)
+// a positive factor c = C 2^(e - 1023 - 61), C = (h, l) in [2^61, 2^62)
 struct FixFactor {
   int h, l, e;
   __device__ explicit FixFactor(double c) {
     const int hi = __double2hiint(c), lo = __double2loint(c);
     e = (hi >> 20) & 0x7ff;
     const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
-    const long long x = (long long)(((unsigned long long)__funnelshift_l((unsigned)lo, mh, 6) << 32) | ((unsigned)lo << 6));
+    const long long x = (long long)(((unsigned long long)__funnelshift_l((unsigned)lo, mh, 9) << 32) | ((unsigned)lo << 9));
     h = fix_hi(x);
     l = fix_lo(x);
   }
-  __device__ __forceinline__ long long times(long long r) const {  // r C / 2^58
-    long long s = 0, m = kFixHalf;
+  __device__ __forceinline__ long long times(long long r) const {  // r C / 2^62
+    long long s = 0;
+    int m = r != 0;
     fix_madd(s, m, fix_hi(r), fix_lo(r), h, l);
     return fix_sum(s, m);
   }
@@ -82,14 +87,14 @@ struct FixFactor {
 // value of a contracted entry with matrix scale 2^sh, out of line (rare): the
 // bits of a double where E says so, else in fixed point
 static __device__ __noinline__ double fix_value(double bits, int E, int sh) {
-  return E == kFixOut ? bits : scalbn((double)__double_as_longlong(bits), E - 1021 - sh);
+  return E == kFixOut ? bits : scalbn((double)__double_as_longlong(bits), E - 1020 - sh);
 }
 
 // P values p[0], p[stride], .. as limbs relative to their largest exponent E.
 // f: the values; false where they need FP64.
 template <int P>
 struct FixLine {
-  int hi[P], lo[P], E;
+  int hi[P], lo[P], E, m0;
   __device__ __forceinline__ bool load(const double* __restrict__ p, int stride) {
     int top = 0;
 #pragma unroll
@@ -102,6 +107,7 @@ struct FixLine {
     }
     E = top >> 20;
     if (top == 0) E = kFixMin;  // all zero
+    m0 = top == 0 ? 0 : P;
     return E >= kFixMin && E < kFixMax;
   }
   __device__ __forceinline__ double value(int k) const { return __hiloint2double(hi[k], lo[k]); }
@@ -113,9 +119,10 @@ struct FixLine {
       lo[k] = fix_lo(x);
     }
   }
-  // sum_k M[k * st] x_k, in units of 2^(E - 1021 - scale of M)
+  // sum_k M[k * st] x_k, in units of 2^(E - 1020 - scale of M)
   __device__ __forceinline__ long long dot(const int* Mh, const int* Ml, int st) const {
-    long long s = 0, m = kFixHalf;
+    long long s = 0;
+    int m = m0;
 #pragma unroll
     for (int k = 0; k < P; ++k) fix_madd(s, m, hi[k], lo[k], Mh[k * st], Ml[k * st]);
     return fix_sum(s, m);
@@ -193,8 +200,9 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
       }
     }
   };
+  constexpr int kLevels = BN ? P : 1;  // unrolled where the NCP's scalars stay in registers
   auto fluxes = [&]() {  // of the column
-#pragma unroll
+#pragma unroll kLevels
     for (int l = 0; l < P; ++l) {
       double Q[V];
 #pragma unroll
@@ -241,19 +249,19 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
       fix_line<P, false>(cs + v * C::PLANE + (d ? C::Y0 + ln : P * ln), d ? P : 1, ex + (2 * v + d) * P2 + ln, op);
     }
   };
-  // dt (dFx/dx + dFy/dy) of variable v at level l: b = value 2^-(A - 2043 - sK) for A at
-  // least the exponents' maximum; |b| < 2^60
+  // dt (dFx/dx + dFy/dy) of variable v at level l: b = value 2^-(A - 2042 - sK) for A at
+  // least the exponents' maximum; |b| < 2^59
   auto divergence = [&](int v, int l, int A) -> long long {
     const long long x = fix_shift(cx.times(__double_as_longlong(fx(v, l))), A - exx(v, l) - cx.e);
     const long long y = fix_shift(cy.times(__double_as_longlong(fy(v, l))), A - exy(v, l) - cy.e);
-    return (x + y) >> 1;
+    return x + y;
   };
   auto divergence64 = [&](int v, int l) -> double {  // the same in FP64 (rare)
     return fma(cxw, fix_value(fx(v, l), exx(v, l), op.sK), cyw * fix_value(fy(v, l), exy(v, l), op.sK));
   };
   // level 0 in FP64
   auto divergence0 = [&](int v) -> double {
-    const int A = max(exx(v, 0) + cx.e, exy(v, 0) + cy.e), e = A - 2043 - op.sK;
+    const int A = max(exx(v, 0) + cx.e, exy(v, 0) + cy.e), e = A - 2042 - op.sK;
     return e > -1000 && e < 900 ? fix_double(divergence(v, 0, A), e) : divergence64(v, 0);
   };
 
@@ -284,10 +292,10 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
     __syncthreads();
     // this thread's lines: x row j and y column j of level i, every variable
 #pragma unroll 1
-    for (int v = 0; v < (live ? VF : 0); ++v) {
-      double* pl = cs + v * C::PLANE;
-      fix_line<P, false>(pl + i * C::XL + P * j, 1, ex + (2 * v * P + i) * P + j, op);
-      fix_line<P, false>(pl + C::Y0 + i * C::YL + j, P, ex + ((2 * v + 1) * P + i) * P + j, op);
+    for (int r = 0; r < (live ? 2 * VF : 0); ++r) {
+      const int v = r >> 1, d = r & 1;
+      fix_line<P, false>(cs + v * C::PLANE + (d ? C::Y0 + i * C::YL + j : i * C::XL + P * j), d ? P : 1,
+                         ex + (r * P + i) * P + j, op);
     }
     if constexpr (BN) {
 #pragma unroll
@@ -309,29 +317,32 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
           nl[l] = __double2loint(n);
           int e = (nh[l] >> 20) & 0x7ff;
           e = e > kFixMin ? e : kFixMin;
-          A = max(A, e >= kFixMax ? kFixOut : e + 964 + op.sK);
+          A = max(A, e >= kFixMax ? kFixOut : e + 962 + op.sK);
         }
       }
-      const int sc = A - 1985 - op.sT - op.sK;  // the update is W 2^sc
+      const int sc = A - 1980 - op.sT - op.sK;  // the update is W 2^sc
       const double u0 = u(v);
       const int uh = __double2hiint(u0), ul = __double2loint(u0);
       const int ue = u0 == 0.0 ? kFixMin : (uh >> 20) & 0x7ff;
       if (sc > -1000 && sc < 900 && ue >= kFixMin && ue < kFixMax) {
-        int bh[P], bl[P];
+        int bh[P], bl[P], m0 = 0;
 #pragma unroll
         for (int l = 0; l < P; ++l) {
           long long b = has_f ? divergence(v, l, A) : 0;
-          if (has_n) b += fix_int(nh[l], nl[l], A - 964 - op.sK);
+          if (has_n) b += fix_int<5>(nh[l], nl[l], A - 962 - op.sK);
           bh[l] = fix_hi(b);
           bl[l] = fix_lo(b);
+          m0 |= bh[l] | bl[l];
         }
+        m0 = m0 ? P : 0;
         // q = u - W 2^sc as one integer in the coarser of the two units, 2^(ue - 1083) and 2^sc
         const int unit = max(ue - 1083, sc);
         const long long U = fix_int<8>(uh, ul, unit + 1083);
         const int dw = unit - sc;
 #pragma unroll
         for (int lp = 0; lp < P; ++lp) {
-          long long s = 0, m = kFixHalf;
+          long long s = 0;
+          int m = m0;
 #pragma unroll
           for (int l = 0; l < P; ++l) fix_madd(s, m, bh[l], bl[l], op.Th[lp + P * l], op.Tl[lp + P * l]);
           col(v, lp) = fix_double(U - fix_shift(fix_sum(s, m), dw), unit);
@@ -369,7 +380,7 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
       if (!live) continue;
       if (x.load(p, d == 0 ? C::XL : C::YL)) {
         x.limbs();
-        const int e = x.E - 1021 - op.sW;
+        const int e = x.E - 1020 - op.sW;
         Fh[d][v] = fix_double(x.dot(op.Wh, op.Wl, 1), e);
         h = fix_double(x.dot(op.TWh, op.TWl, 1), e);
       } else {
@@ -431,7 +442,7 @@ __device__ __forceinline__ void outputs_fix(const BatchArgs& a, const PredOps<N,
     const bool fix = x.load(p, st);
     if (fix) {
       x.limbs();
-      const int e = x.E - 1021 - op.sE;
+      const int e = x.E - 1020 - op.sE;
       lo = fix_double(x.dot(op.Eh, op.El, 1), e);
       hi = fix_double(x.dot(op.Eh + P, op.El + P, 1), e);
     } else {
@@ -471,8 +482,8 @@ __device__ __forceinline__ void outputs_fix(const BatchArgs& a, const PredOps<N,
       for (int v = 0; v < V; ++v) {
         const double bx = cs[(V + v) * P2 + node], by = cs[(2 * V + v) * P2 + node];
         const int ex_ = ex[v * P + j], ey_ = ex[(V + v) * P + i];
-        const double sx = ex_ == kFixOut ? bx : fix_double(__double_as_longlong(bx), ex_ - 1021 - op.sK);
-        const double sy = ey_ == kFixOut ? by : fix_double(__double_as_longlong(by), ey_ - 1021 - op.sK);
+        const double sx = ex_ == kFixOut ? bx : fix_double(__double_as_longlong(bx), ex_ - 1020 - op.sK);
+        const double sy = ey_ == kFixOut ? by : fix_double(__double_as_longlong(by), ey_ - 1020 - op.sK);
         double s = sx * vx + sy * vy;
         if constexpr (Sys::ID == kSysBN) s = fma(op.w[i] * op.w[j], Sh[v], s);
         dst[v] = s;

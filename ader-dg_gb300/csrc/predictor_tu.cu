@@ -79,24 +79,17 @@ void make_ops(const HostOps& h, void* out) {
   }
   o.wg = (R)wg;
   if constexpr (sizeof(R) == 8) {
-    // fixed-point limbs under one scale per operator: every entry below 2^57,
-    // every sum of magnitudes the kernel forms (bounded by `sum`) below 2^59
+    // fixed-point limbs under one scale per operator: every sum of magnitudes
+    // the kernel forms (bounded by `sum`) below 2^60, which keeps its 64-bit sums
+    // and 32-bit cross sums in range (operands below 2^60 and P <= 6 terms)
     auto limbs = [](const double* M, int n, int sh, int* hi, int* lo) {
       for (int k = 0; k < n; ++k) {
         const long long x = std::llrint(std::ldexp(M[k], sh));
-        long long l = x & ((1ll << 29) - 1);
-        if (l >= (1ll << 28)) l -= 1ll << 29;
-        lo[k] = (int)l;
-        hi[k] = (int)((x - l) >> 29);
+        lo[k] = (int)(x & 0x7fffffffll);
+        hi[k] = (int)((x - lo[k]) / (1ll << 31));
       }
     };
-    auto scale = [](const double* M, int n, double sum) {
-      double big = 0.0;
-      for (int k = 0; k < n; ++k) big = std::fmax(big, std::fabs(M[k]));
-      int sh = 56 - std::ilogb(big);
-      while (std::ldexp(sum, sh) >= std::ldexp(1.0, 59)) --sh;
-      return sh;
-    };
+    auto scale = [](double sum) { return 59 - std::ilogb(sum); };
     double Tm[P * P], ends[2 * P], times[2 * P];
     double sumK = 0.0, sumT = 0.0, sumE = 0.0, sumW = 0.0;
     for (int l = 0; l < P; ++l) {
@@ -116,10 +109,10 @@ void make_ops(const HostOps& h, void* out) {
       sumE += std::fabs(h.FL[l]) + std::fabs(h.FR[l]);
       sumW += std::fabs(h.w[l]) + std::fabs(tws[l]);
     }
-    o.sK = scale(h.Kxi.data(), P * P, sumK);
-    o.sT = scale(Tm, P * P, sumT);
-    o.sE = scale(ends, 2 * P, sumE);
-    o.sW = scale(times, 2 * P, sumW);
+    o.sK = scale(sumK);
+    o.sT = scale(sumT);
+    o.sE = scale(sumE);
+    o.sW = scale(sumW);
     limbs(h.Kxi.data(), P * P, o.sK, o.Kh, o.Kl);
     limbs(Tm, P * P, o.sT, o.Th, o.Tl);
     limbs(ends, 2 * P, o.sE, o.Eh, o.El);
