@@ -21,6 +21,8 @@
 //                other cells' min/max and the CFL are those of kCellPrime
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "physics.cuh"
 
@@ -299,6 +301,10 @@ struct CellCfg {
   }
 };
 
+// the operators of a cell-kernel variant: 1/(w_i w_j) in FP64 for the FP64 updates
+template <int N, bool kFast, bool kExact>
+using CellOps = typename std::conditional<kExact || !kFast, ExactOps<N>, DevOps<N, double>>::type;
+
 // kFast: DMP projections in FP32 with an error bound (settled from FP64 where
 // the bound leaves a decision open) and, without kExact, the FP32 modes'
 // storage and surface integral.  kExact: FP64 storage, surface integral, update
@@ -307,7 +313,7 @@ struct CellCfg {
 // bit.
 template <class Sys, int N, bool kFast, int VAR = 0, bool kExact = false>
 __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast && !kExact))
-    k_cells(BatchArgs a, DevOps<N, double> op) {
+    k_cells(BatchArgs a, CellOps<N, kFast, kExact> op) {
   using C = CellCfg<Sys, N, VAR>;
   constexpr int P = N + 1, P2 = P * P, S = 2 * N + 1, V = Sys::V, CPB = C::CPB;
   constexpr bool kF32 = kFast && !kExact;  // FP32 storage and update

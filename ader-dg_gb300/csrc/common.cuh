@@ -99,7 +99,6 @@ struct DevOps {
   double wd[P], FLd[P], FRd[P];
   float wf[P], FLf[P], FRf[P];  // FP32-mixed surface integral and update
   float iwwf[P * P];            // 1 / (w_i w_j) at [i + P*j]
-  double iwwd[P * P];           // the same in FP64, correctly rounded from the rounded product
   double xid[P];
   double uh2lim[S * P];  // (s,k) at [s + S*k]
   double lim2uh[P * S];  // (k,s) at [k + P*s]
@@ -114,16 +113,22 @@ struct DevOps {
   float pdev;
 };
 
-// The FP64 predictor's operators: the above (first, so that the other FP64
-// kernels take them from the same host copy) and its fixed-point tables, kept
-// out of the other kernels' parameters: every launch copies its parameters, and
-// 0.6 KB more of them cost a small step 2%.
+// Operators that only some kernels take, kept out of the other kernels'
+// parameters (every launch copies its parameters: 0.6 KB more of them cost a
+// step of small grids 2%).  One host copy serves all: each struct begins with
+// the previous one.
+template <int N>
+struct ExactOps : DevOps<N, double> {  // the FP64 mode's cell kernel
+  static constexpr int P = N + 1;
+  double iwwd[P * P];  // 1 / (w_i w_j) at [i + P*j], correctly rounded from the rounded product
+};
 template <int N, class R>
 struct PredOps : DevOps<N, R> {};
 template <int N>
-struct PredOps<N, double> : DevOps<N, double> {
+struct PredOps<N, double> : ExactOps<N> {  // the FP64 predictor
   static constexpr int P = N + 1;
-  double iw[P];  // 1/w
+  double iw[P];   // 1/w
+  double tsx[P];  // sum_l T(l',l), rounded once
   // Kxi, T, the end values FL and FR, and the time weights w and tw in 60-bit
   // fixed point (predictor_fix.cuh): entry = (h 2^31 + l) 2^-s, 0 <= l < 2^31
   int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];

@@ -75,7 +75,8 @@ cudaError_t launch_cells(const BatchArgs& a, const void* ops, cudaStream_t s) {
   }
   const long long grid = (a.ncells - a.cell0 + C::CPB - 1) / C::CPB;
   if (grid <= 0) return cudaSuccess;
-  k_cells<Sys, N, kFast, 0, kExact><<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, double>*>(ops));
+  k_cells<Sys, N, kFast, 0, kExact><<<(unsigned)grid, C::THREADS, C::SMEM_BYTES, s>>>(
+      a, *reinterpret_cast<const CellOps<N, kFast, kExact>*>(ops));
   return cudaGetLastError();
 }
 

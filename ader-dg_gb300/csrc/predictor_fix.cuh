@@ -6,25 +6,30 @@
 // Most of the predictor's FP64 instructions are products with constant
 // matrices: flux derivatives (Kxi), time update (T), time averages, volume
 // integral and face extrapolation.  A product of two 60-bit numbers in 31-bit
-// limbs takes one IMAD.WIDE and two IMAD.HI (the cross products' upper halves;
-// the low x low product is below the last bit kept) = 3.8 cycles instead of 20,
-// and the pipes overlap: the FP64 pipe keeps
-// the pointwise fluxes and one conversion per result.  Measured (FP64 mode, all
-// in registers and FP64 before): Euler vortex N = 4, 256^2 5.02 -> 1.94 ms,
-// Riemann problem N = 3, 257 x 193 1.32 -> 0.55 ms, Baer-Nunziato cylinder N = 3,
-// 200^2 3.28 -> 1.76 ms (with 29-bit limbs, three IMAD.WIDE a product and the
-// loops less rolled: 2.36, 0.61 and 1.91 ms).  On the vortex the FP64 pipe is
-// then 62% and the multiply-add pipe 45% busy.  N >= 3: below, the Picard iterations between the
-// first and the last, which this is for, are at most one.
+// limbs takes three IMAD.WIDE (the low x low product is below the last bit
+// kept), or one and two IMAD.HI (the cross products' upper halves) = 4.9 or 3.8
+// cycles instead of 20, and the pipes overlap: the FP64 pipe keeps the
+// pointwise fluxes and one conversion per result.  Measured (FP64 mode, all in
+// registers and FP64 before): Euler vortex N = 4, 256^2 5.02 -> 2.05 ms, Riemann
+// problem N = 3, 257 x 193 1.32 -> 0.56 ms, Baer-Nunziato cylinder N = 3, 200^2
+// 3.28 -> 1.83 ms.  With IMAD.HI throughout the vortex takes 1.91 ms, but the
+// average flux then loses up to a factor 6 of its accuracy; with IMAD.WIDE
+// throughout 2.29 ms.  N >= 3: below, the Picard iterations between the first and
+// the last, which this is for, are at most one.
 //
 // Accuracy: each operand line takes its own power-of-two scale from its
-// largest magnitude, so a value's error is at most 2^-60 of that magnitude and
-// the constants' 2^-60 of the matrix's largest row sum: every sum has an absolute
-// error of a few 2^-57 of its terms' size, where the FP64 chain rounds each
-// partial sum to 2^-53.  Lines holding infinities or NaNs, or whose largest
-// magnitude is beyond 2^900 or below 2^-823, are contracted in FP64 and their
-// nodes take the FP64 time update.
+// largest magnitude, so a value's error is at most 2^-60 of that magnitude, and
+// the constants are formed to twice FP64 and rounded to 2^-60 of the matrix's
+// largest row sum (the FP64 ones miss the exact sums by up to 4e-15).  Against
+// the predictor evaluated in 80-bit arithmetic (Euler and Baer-Nunziato, N = 3..5,
+// smooth and discontinuous states, with and without noise) the error of the
+// averages and face values is 0.25 to 0.39 times that of the FP64 chain.
+// Lines holding infinities or NaNs, or whose largest magnitude is beyond 2^900
+// or below 2^-823, are contracted in FP64 and their nodes take the FP64 time
+// update.
 #pragma once
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "physics.cuh"
@@ -35,17 +40,36 @@ constexpr int kFixMin = 200;           // lines whose largest biased exponent li
 constexpr int kFixMax = 1023 + 900;    // or from here on take FP64
 constexpr int kFixOut = 1 << 20;       // "exponent" of a line contracted in FP64
 
-// Numbers are (h, l) with value h 2^31 + l, l >= 0 in 31 bits.  A product in
-// units of 2^62: h*h exactly (IMAD.WIDE, into s), and the upper 32 bits of the
-// two cross products (IMAD.HI, 1.1 cycles against IMAD.WIDE's 1.6, into m, in
-// units of two of the sum's; n products start m at n, half the roundings down,
-// unless all are 0: zeros stay exact).
-__device__ __forceinline__ void fix_madd(long long& s, int& m, int ah, int al, int bh, int bl) {
-  s += (long long)ah * bh;
-  asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(ah), "r"(bl));
-  asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(al), "r"(bh));
-}
-__device__ __forceinline__ long long fix_sum(long long s, int m) { return s + 2 * (long long)m; }
+// Numbers are (h, l) with value h 2^31 + l, l >= 0 in 31 bits.  A sum of n
+// products in units of 2^62: h*h exactly (IMAD.WIDE, into s); of the two cross
+// products (units of 2^31), with kFine the whole (IMAD.WIDE into 64 bits), else
+// the upper 32 bits (IMAD.HI into 32 bits: two units each, half of them rounded
+// away on average).  The start value holds the mean of what is left out (and,
+// with kFine, the rounding half), unless all operands are 0: zeros stay exact.
+template <bool kFine>
+struct FixSum {
+  using M = typename std::conditional<kFine, long long, int>::type;
+  long long s = 0;
+  M m;
+  __device__ __forceinline__ FixSum(bool any, int n) {
+    if constexpr (kFine) m = any ? ((long long)n << 29) + (1ll << 30) : 0;
+    else m = any ? n : 0;
+  }
+  __device__ __forceinline__ void madd(int ah, int al, int bh, int bl) {
+    s += (long long)ah * bh;
+    if constexpr (kFine) {
+      m += (long long)ah * bl;
+      m += (long long)al * bh;
+    } else {
+      asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(ah), "r"(bl));
+      asm("mad.hi.s32 %0, %1, %2, %0;" : "+r"(m) : "r"(al), "r"(bh));
+    }
+  }
+  __device__ __forceinline__ long long sum() const {
+    if constexpr (kFine) return s + (m >> 31);
+    else return s + 2 * (long long)m;
+  }
+};
 __device__ __forceinline__ int fix_hi(long long x) { return (int)(x >> 31); }
 __device__ __forceinline__ int fix_lo(long long x) { return (int)x & 0x7fffffff; }
 // x >> d, 0 <= d, floor; everything beyond 63 is the sign
@@ -78,10 +102,9 @@ struct FixFactor {
     l = fix_lo(x);
   }
   __device__ __forceinline__ long long times(long long r) const {  // r C / 2^62
-    long long s = 0;
-    int m = r != 0;
-    fix_madd(s, m, fix_hi(r), fix_lo(r), h, l);
-    return fix_sum(s, m);
+    FixSum<true> s(r != 0, 1);
+    s.madd(fix_hi(r), fix_lo(r), h, l);
+    return s.sum();
   }
 };
 // value of a contracted entry with matrix scale 2^sh, out of line (rare): the
@@ -91,10 +114,11 @@ static __device__ __noinline__ double fix_value(double bits, int E, int sh) {
 }
 
 // P values p[0], p[stride], .. as limbs relative to their largest exponent E.
-// f: the values; false where they need FP64.
 template <int P>
 struct FixLine {
-  int hi[P], lo[P], E, m0;
+  int hi[P], lo[P], E;
+  bool any;
+  // false where the values need FP64
   __device__ __forceinline__ bool load(const double* __restrict__ p, int stride) {
     int top = 0;
 #pragma unroll
@@ -105,9 +129,8 @@ struct FixLine {
       const int m = hi[k] & 0x7fffffff;
       top = top > m ? top : m;
     }
-    E = top >> 20;
-    if (top == 0) E = kFixMin;  // all zero
-    m0 = top == 0 ? 0 : P;
+    any = top != 0;
+    E = any ? top >> 20 : kFixMin;
     return E >= kFixMin && E < kFixMax;
   }
   __device__ __forceinline__ double value(int k) const { return __hiloint2double(hi[k], lo[k]); }
@@ -119,37 +142,52 @@ struct FixLine {
       lo[k] = fix_lo(x);
     }
   }
-  // sum_k M[k * st] x_k, in units of 2^(E - 1020 - scale of M)
-  __device__ __forceinline__ long long dot(const int* Mh, const int* Ml, int st) const {
-    long long s = 0;
-    int m = m0;
+  // the values' differences from value 0 (k >= 1), exactly; E as for values
+  // twice as large
+  __device__ __forceinline__ void deviations() {
+    const long long x0 = fix_int<6>(hi[0], lo[0], E);
+    any = false;
 #pragma unroll
-    for (int k = 0; k < P; ++k) fix_madd(s, m, hi[k], lo[k], Mh[k * st], Ml[k * st]);
-    return fix_sum(s, m);
+    for (int k = 1; k < P; ++k) {
+      const long long x = fix_int<6>(hi[k], lo[k], E) - x0;
+      hi[k] = fix_hi(x);
+      lo[k] = fix_lo(x);
+      any = any || x != 0;
+    }
+    ++E;
+  }
+  // sum over k >= kFirst of M[k * st] x_k, in units of 2^(E - 1020 - scale of M)
+  template <bool kFine, int kFirst = 0>
+  __device__ __forceinline__ long long dot(const int* Mh, const int* Ml, int st) const {
+    FixSum<kFine> s(any, P - kFirst);
+#pragma unroll
+    for (int k = kFirst; k < P; ++k) s.madd(hi[k], lo[k], Mh[k * st], Ml[k * st]);
+    return s.sum();
   }
 };
 
-// One line contracted in place, p[o] <- sum_k M(k, o) p[k] as the integer R
-// and the line's exponent; M = Kxi (derivative, kT = false) or its transpose
-// (volume integral, kT = true).
-template <int P, bool kT, class Ops>
+// The derivative of one line in place, p[o] <- sum_k Kxi(k, o) p[k] as the
+// integer R and the line's exponent.  The derivative of a constant is 0 (the
+// 60-bit columns of Kxi sum to 0), so the line's differences from its first value
+// are contracted: one product less an output, and 0 for a constant line.
+template <int P, bool kFine, class Ops>
 __device__ __forceinline__ void fix_line(double* __restrict__ p, int stride, int* __restrict__ ex, const Ops& op) {
-  constexpr int SK = kT ? P : 1, SO = kT ? 1 : P;
   FixLine<P> x;
   if (!x.load(p, stride)) {
 #pragma unroll 1
     for (int o = 0; o < P; ++o) {
       double s = 0.0;
 #pragma unroll
-      for (int k = 0; k < P; ++k) s = fma(op.Kxi[SK * k + SO * o], x.value(k), s);
+      for (int k = 0; k < P; ++k) s = fma(op.Kxi[k + P * o], x.value(k), s);
       p[o * stride] = s;
     }
     *ex = kFixOut;
     return;
   }
-  x.limbs();
+  x.deviations();
 #pragma unroll
-  for (int o = 0; o < P; ++o) p[o * stride] = __longlong_as_double(x.dot(op.Kh + SO * o, op.Kl + SO * o, SK));
+  for (int o = 0; o < P; ++o)
+    p[o * stride] = __longlong_as_double(x.template dot<kFine, 1>(op.Kh + P * o, op.Kl + P * o, 1));
   *ex = x.E;
 }
 
@@ -246,7 +284,7 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
 #pragma unroll 1
     for (int q0 = live ? node : 2 * P * VF; q0 < 2 * P * VF; q0 += P2) {
       const int v = q0 / (2 * P), r = q0 - v * (2 * P), d = r / P, ln = r - d * P;
-      fix_line<P, false>(cs + v * C::PLANE + (d ? C::Y0 + ln : P * ln), d ? P : 1, ex + (2 * v + d) * P2 + ln, op);
+      fix_line<P, true>(cs + v * C::PLANE + (d ? C::Y0 + ln : P * ln), d ? P : 1, ex + (2 * v + d) * P2 + ln, op);
     }
   };
   // dt (dFx/dx + dFy/dy) of variable v at level l: b = value 2^-(A - 2042 - sK) for A at
@@ -282,7 +320,7 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
     if (BN && (v & 3 || v == 8)) b += ncp(0, v);
     const double u0 = u(v);
 #pragma unroll
-    for (int l = 0; l < P; ++l) col(v, l) = fma(-op.ts[l], b, u0);
+    for (int l = 0; l < P; ++l) col(v, l) = fma(-op.tsx[l], b, u0);
   }
 
   // iterations 2 .. P-1
@@ -325,27 +363,26 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
       const int uh = __double2hiint(u0), ul = __double2loint(u0);
       const int ue = u0 == 0.0 ? kFixMin : (uh >> 20) & 0x7ff;
       if (sc > -1000 && sc < 900 && ue >= kFixMin && ue < kFixMax) {
-        int bh[P], bl[P], m0 = 0;
+        int bh[P], bl[P];
+        bool any = false;
 #pragma unroll
         for (int l = 0; l < P; ++l) {
           long long b = has_f ? divergence(v, l, A) : 0;
           if (has_n) b += fix_int<5>(nh[l], nl[l], A - 962 - op.sK);
           bh[l] = fix_hi(b);
           bl[l] = fix_lo(b);
-          m0 |= bh[l] | bl[l];
+          any = any || b != 0;
         }
-        m0 = m0 ? P : 0;
         // q = u - W 2^sc as one integer in the coarser of the two units, 2^(ue - 1083) and 2^sc
         const int unit = max(ue - 1083, sc);
         const long long U = fix_int<8>(uh, ul, unit + 1083);
         const int dw = unit - sc;
 #pragma unroll
         for (int lp = 0; lp < P; ++lp) {
-          long long s = 0;
-          int m = m0;
+          FixSum<true> s(any, P);
 #pragma unroll
-          for (int l = 0; l < P; ++l) fix_madd(s, m, bh[l], bl[l], op.Th[lp + P * l], op.Tl[lp + P * l]);
-          col(v, lp) = fix_double(U - fix_shift(fix_sum(s, m), dw), unit);
+          for (int l = 0; l < P; ++l) s.madd(bh[l], bl[l], op.Th[lp + P * l], op.Tl[lp + P * l]);
+          col(v, lp) = fix_double(U - fix_shift(s.sum(), dw), unit);
         }
       } else {
         double b[P];
@@ -381,8 +418,8 @@ __device__ __forceinline__ void picard_fix(double* __restrict__ cs, const double
       if (x.load(p, d == 0 ? C::XL : C::YL)) {
         x.limbs();
         const int e = x.E - 1020 - op.sW;
-        Fh[d][v] = fix_double(x.dot(op.Wh, op.Wl, 1), e);
-        h = fix_double(x.dot(op.TWh, op.TWl, 1), e);
+        Fh[d][v] = fix_double(x.template dot<true>(op.Wh, op.Wl, 1), e);
+        h = fix_double(x.template dot<true>(op.TWh, op.TWl, 1), e);
       } else {
 #pragma unroll
         for (int l = 0; l < P; ++l) {
@@ -443,8 +480,8 @@ __device__ __forceinline__ void outputs_fix(const BatchArgs& a, const PredOps<N,
     if (fix) {
       x.limbs();
       const int e = x.E - 1020 - op.sE;
-      lo = fix_double(x.dot(op.Eh, op.El, 1), e);
-      hi = fix_double(x.dot(op.Eh + P, op.El + P, 1), e);
+      lo = fix_double(x.template dot<true>(op.Eh, op.El, 1), e);
+      hi = fix_double(x.template dot<true>(op.Eh + P, op.El + P, 1), e);
     } else {
       lo = hi = 0.0;
 #pragma unroll
@@ -459,7 +496,7 @@ __device__ __forceinline__ void outputs_fix(const BatchArgs& a, const PredOps<N,
     if (kVolume && flux) {
       if (fix) {
 #pragma unroll
-        for (int k = 0; k < P; ++k) p[k * st] = __longlong_as_double(x.dot(op.Kh + k, op.Kl + k, P));
+        for (int k = 0; k < P; ++k) p[k * st] = __longlong_as_double(x.template dot<true>(op.Kh + k, op.Kl + k, P));
       } else {
 #pragma unroll 1
         for (int k = 0; k < P; ++k) {

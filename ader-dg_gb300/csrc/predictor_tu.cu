@@ -48,8 +48,9 @@ void make_ops(const HostOps& h, void* out) {
   }
   for (int j = 0; j < P; ++j)
     for (int i = 0; i < P; ++i) {
-      o.iwwd[i + P * j] = 1.0 / (h.w[i] * h.w[j]);
-      o.iwwf[i + P * j] = (float)o.iwwd[i + P * j];
+      const double y = 1.0 / (h.w[i] * h.w[j]);
+      o.iwwf[i + P * j] = (float)y;
+      if constexpr (sizeof(R) == 8) o.iwwd[i + P * j] = y;
     }
   for (int k = 0; k < P * P; ++k) {
     o.Kxi[k] = (R)h.Kxi[k];
@@ -59,7 +60,7 @@ void make_ops(const HostOps& h, void* out) {
   double T[P][P];
   for (int lp = 0; lp < P; ++lp)
     for (int l = 0; l < P; ++l) T[lp][l] = h.iK1[lp + P * l] * h.w[l];
-  double wg = 0.0, tws[P];
+  double wg = 0.0;
   for (int lp = 0; lp < P; ++lp) {
     double g = 0.0, ts = 0.0;
     for (int l = 0; l < P; ++l) {
@@ -75,49 +76,54 @@ void make_ops(const HostOps& h, void* out) {
     double tw = 0.0;
     for (int lp = 0; lp < P; ++lp) tw += h.w[lp] * T[lp][l];
     o.tw[l] = (R)tw;
-    tws[l] = tw;
   }
   o.wg = (R)wg;
   if constexpr (sizeof(R) == 8) {
-    // fixed-point limbs under one scale per operator: every sum of magnitudes
-    // the kernel forms (bounded by `sum`) below 2^60, which keeps its 64-bit sums
-    // and 32-bit cross sums in range (operands below 2^60 and P <= 6 terms)
-    auto limbs = [](const double* M, int n, int sh, int* hi, int* lo) {
+    // fixed-point limbs (h 2^31 + l) 2^-sh under one scale per operator: every
+    // sum of P magnitudes the kernel forms stays below 2^60, which keeps its
+    // 64-bit sums and 32-bit cross sums in range (operands below 2^60, P <= 6).
+    auto limbs = [](const HostOps::Fine& f, int n, double sum, int* hi, int* lo) {
+      const int sh = 59 - std::ilogb(sum);
       for (int k = 0; k < n; ++k) {
-        const long long x = std::llrint(std::ldexp(M[k], sh));
+        const double s = std::ldexp(f.hi[k], sh);
+        const long long a = std::llrint(s);
+        const long long x = a + std::llrint((s - (double)a) + std::ldexp(f.lo[k], sh));
         lo[k] = (int)(x & 0x7fffffffll);
         hi[k] = (int)((x - lo[k]) / (1ll << 31));
       }
+      return sh;
     };
-    auto scale = [](double sum) { return 59 - std::ilogb(sum); };
-    double Tm[P * P], ends[2 * P], times[2 * P];
     double sumK = 0.0, sumT = 0.0, sumE = 0.0, sumW = 0.0;
     for (int l = 0; l < P; ++l) {
       double rK = 0.0, cK = 0.0, rT = 0.0;
       for (int m = 0; m < P; ++m) {
-        Tm[l + P * m] = T[l][m];
         rK += std::fabs(h.Kxi[l + P * m]);
         cK += std::fabs(h.Kxi[m + P * l]);
         rT += std::fabs(T[l][m]);
       }
       sumK = std::fmax(sumK, std::fmax(rK, cK));
       sumT = std::fmax(sumT, rT);
-      ends[l] = h.FL[l];
-      ends[P + l] = h.FR[l];
-      times[l] = h.w[l];
-      times[P + l] = tws[l];
-      sumE += std::fabs(h.FL[l]) + std::fabs(h.FR[l]);
-      sumW += std::fabs(h.w[l]) + std::fabs(tws[l]);
+      sumE += std::fmax(std::fabs(h.FL[l]), std::fabs(h.FR[l]));
+      sumW += std::fabs(h.w[l]);
     }
-    o.sK = scale(sumK);
-    o.sT = scale(sumT);
-    o.sE = scale(sumE);
-    o.sW = scale(sumW);
-    limbs(h.Kxi.data(), P * P, o.sK, o.Kh, o.Kl);
-    limbs(Tm, P * P, o.sT, o.Th, o.Tl);
-    limbs(ends, 2 * P, o.sE, o.Eh, o.El);
-    limbs(times, P, o.sW, o.Wh, o.Wl);
-    limbs(times + P, P, o.sW, o.TWh, o.TWl);
+    // (a margin for the roundings of these FP64 bounds; tw(l) <= w(l))
+    const double up = 1.0 + 1.0e-9;
+    int end_l[2 * P], end_h[2 * P], time_l[2 * P], time_h[2 * P];
+    o.sK = limbs(h.fKxi, P * P, sumK * up, o.Kh, o.Kl);
+    o.sT = limbs(h.fT, P * P, sumT * up, o.Th, o.Tl);
+    o.sE = limbs(h.fEnds, 2 * P, sumE * up, end_h, end_l);
+    o.sW = limbs(h.fTimes, 2 * P, sumW * up, time_h, time_l);
+    for (int k = 0; k < P; ++k) {
+      o.Wh[k] = time_h[k];
+      o.Wl[k] = time_l[k];
+      o.TWh[k] = time_h[P + k];
+      o.TWl[k] = time_l[P + k];
+      o.tsx[k] = h.fTs.hi[k];
+    }
+    for (int k = 0; k < 2 * P; ++k) {
+      o.Eh[k] = end_h[k];
+      o.El[k] = end_l[k];
+    }
     for (int k = 0; k < P; ++k) o.iw[k] = 1.0 / h.w[k];
   }
   for (int k = 0; k < S * P; ++k) {

@@ -139,6 +139,125 @@ bool invert(const Mat& A, Mat& inv) {
   return true;
 }
 
+// Unevaluated sum of two doubles, about 106 bits (two-sum and fma error-free
+// transformations; plain double operations, so every host gives the same bits).
+struct Dd {
+  double h = 0.0, l = 0.0;
+  Dd() = default;
+  Dd(double x) : h(x) {}
+  Dd(double a, double b) : h(a + b), l(0.0) {
+    const double t = h - a;
+    l = (a - (h - t)) + (b - t);
+  }
+};
+Dd operator+(Dd a, Dd b) {
+  const Dd s(a.h, b.h), t(a.l, b.l), u(s.h, s.l + t.h);
+  return Dd(u.h, u.l + t.l);
+}
+Dd operator-(Dd a) {
+  a.h = -a.h;
+  a.l = -a.l;
+  return a;
+}
+Dd operator-(Dd a, Dd b) { return a + (-b); }
+Dd operator*(Dd a, Dd b) {
+  const double p = a.h * b.h;
+  return Dd(p, std::fma(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+Dd operator/(Dd a, Dd b) {
+  const double q0 = a.h / b.h;
+  Dd r = a - b * Dd(q0);
+  const double q1 = r.h / b.h;
+  r = r - b * Dd(q1);
+  return Dd(q0, q1) + Dd(r.h / b.h);
+}
+
+// HostOps::Fine from the FP64 nodes and iK1: Newton steps on the Legendre
+// polynomial and on the inverse.
+void build_fine(HostOps& o) {
+  const int P = o.P;
+  std::vector<Dd> x(P), w(P);
+  for (int i = 0; i < P; ++i) {
+    Dd z = Dd(o.xi[i]) * Dd(2.0) - Dd(1.0), dp;
+    for (int it = 0; it < 3; ++it) {
+      Dd pa(1.0), pb(0.0);
+      for (int k = 1; k <= P; ++k) {
+        const Dd pc = pb;
+        pb = pa;
+        pa = (Dd(2.0 * k - 1.0) * z * pb - Dd(k - 1.0) * pc) / Dd((double)k);
+      }
+      dp = Dd((double)P) * (z * pa - pb) / (z * z - Dd(1.0));
+      if (it < 2) z = z - pa / dp;
+    }
+    x[i] = (z + Dd(1.0)) * Dd(0.5);
+    w[i] = Dd(1.0) / ((Dd(1.0) - z * z) * dp * dp);
+  }
+  auto phi = [&](int k, Dd s) {
+    Dd v(1.0);
+    for (int j = 0; j < P; ++j)
+      if (j != k) v = v * (s - x[j]) / (x[k] - x[j]);
+    return v;
+  };
+  auto dphi = [&](int k, Dd s) {
+    Dd d(0.0);
+    for (int m = 0; m < P; ++m) {
+      if (m == k) continue;
+      Dd t = Dd(1.0) / (x[k] - x[m]);
+      for (int j = 0; j < P; ++j)
+        if (j != k && j != m) t = t * (s - x[j]) / (x[k] - x[j]);
+      d = d + t;
+    }
+    return d;
+  };
+  std::vector<Dd> K(P * P), K1(P * P), X(P * P), T(P * P), ends(2 * P), times(2 * P), ts(P);
+  for (int k = 0; k < P; ++k) {
+    ends[k] = phi(k, Dd(0.0));
+    ends[P + k] = phi(k, Dd(1.0));
+  }
+  for (int k = 0; k < P; ++k)
+    for (int i = 0; i < P; ++i) {
+      K[k + P * i] = w[i] * dphi(k, x[i]);
+      K1[k + P * i] = ends[P + k] * ends[P + i] - K[k + P * i];
+      X[k + P * i] = Dd(o.iK1[k + P * i]);
+    }
+  for (int it = 0; it < 2; ++it) {  // X <- X (2 I - K1 X)
+    std::vector<Dd> R(P * P), Y(P * P);
+    for (int a = 0; a < P; ++a)
+      for (int b = 0; b < P; ++b) {
+        Dd s(a == b ? 2.0 : 0.0);
+        for (int k = 0; k < P; ++k) s = s - K1[a + P * k] * X[k + P * b];
+        R[a + P * b] = s;
+      }
+    for (int a = 0; a < P; ++a)
+      for (int b = 0; b < P; ++b) {
+        Dd s(0.0);
+        for (int k = 0; k < P; ++k) s = s + X[a + P * k] * R[k + P * b];
+        Y[a + P * b] = s;
+      }
+    X = Y;
+  }
+  for (int a = 0; a < P; ++a)
+    for (int l = 0; l < P; ++l) {
+      T[a + P * l] = X[a + P * l] * w[l];
+      ts[a] = ts[a] + T[a + P * l];
+    }
+  for (int l = 0; l < P; ++l) {
+    times[l] = w[l];
+    for (int a = 0; a < P; ++a) times[P + l] = times[P + l] + w[a] * T[a + P * l];
+  }
+  auto split = [](const std::vector<Dd>& v, HostOps::Fine& f) {
+    for (const Dd& d : v) {
+      f.hi.push_back(d.h);
+      f.lo.push_back(d.l);
+    }
+  };
+  split(K, o.fKxi);
+  split(T, o.fT);
+  split(ends, o.fEnds);
+  split(times, o.fTimes);
+  split(ts, o.fTs);
+}
+
 }  // namespace
 
 double pi_value() { return kPi; }
@@ -201,6 +320,8 @@ bool build_ops(int N, HostOps& o, std::string* err) {
   }
   o.K1 = K1.a;
   o.iK1 = iK1.a;
+
+  build_fine(o);
 
   // subcell limiter maps (Euler/initialize.f90:171-213)
   Mat U(S, P);

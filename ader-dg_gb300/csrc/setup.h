@@ -21,6 +21,16 @@ struct HostOps {
   std::vector<double> lim2uh;        // P x S: subcell averages -> DG (constrained LSQ)
   std::vector<double> uh2lob;        // P x P: DG -> Gauss-Lobatto point values
   std::vector<double> xilimbary;     // S subcell barycentres on [0,1]
+  // Operators to twice FP64 (value = hi + lo), for the 60-bit constants of the
+  // FP64 predictor: the FP64 ones above sum to zero (derivative of a constant)
+  // or one (time operator of a constant) only to a few 1e-16.
+  struct Fine {
+    std::vector<double> hi, lo;
+  };
+  Fine fKxi, fT;     // Kxi(k,i) at [k + P*i]; T(l',l) = iK1(l',l) w(l) at [l' + P*l]
+  Fine fEnds;        // FL, FR
+  Fine fTimes;       // w(l), tw(l) = sum_l' w(l') T(l',l)
+  Fine fTs;          // sum_l T(l',l)
 };
 
 bool build_ops(int N, HostOps& ops, std::string* err);
