@@ -290,7 +290,13 @@ struct CellCfg {
   static_assert(8 * V * P2 + 4 * (3 * V * P2 + V * S * P + V * P * P) <= 8 * CELL_DBL, "FP32 cell layout");
   static constexpr int OPS_DBL = S * P + P * P;  // uh2lim, uh2lob (FP64, then FP32 in the FP32 modes)
   static constexpr int SMEM_BYTES = CPB * CELL_DBL * 8 + OPS_DBL * 12 + CPB * 8 /*cell max*/ + CPB * 4 /*flags*/ +
-                                    CPB * V * 4 /*|U| max*/ + CPB * V * 4 /*FP32 reference state*/ + 16;
+                                    CPB * V * 4 /*|U| max*/ + CPB * V * 4 /*FP32 reference state*/ +
+                                    CPB * 4 /*instances*/ + 16;
+  // (cell, variable) pairs of the DMP comparison per thread: consecutive
+  // threads take them, so that they fill whole warps (with the pairs of a cell
+  // on its own first V threads every warp issued the comparison's FP64
+  // instructions for a few lanes: 2.5 of 6.8 FP64 slots per DOF)
+  static constexpr int NPAIR = (CPB * V + THREADS - 1) / THREADS;
   // blocks per SM the register allocation aims at, in 256-thread units:
   // Euler's FP32-mixed cell kernel is latency-bound and gains from a fourth;
   // the other variants keep the allocation they reach unconstrained
@@ -325,6 +331,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   int* cflag = reinterpret_cast<int*>(cmax + CPB);
   unsigned* amax_all = reinterpret_cast<unsigned*>(cflag + CPB);  // [CPB][V]
   float* ubs_all = reinterpret_cast<float*>(amax_all + CPB * V);  // [CPB][V]
+  int* cinst = reinterpret_cast<int*>(ubs_all + CPB * V);  // instance of each active cell, else -1
 
   const int mode = a.mode;
   const int t = threadIdx.x;
@@ -341,6 +348,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   const bool priming = mode == kCellPrime || mode == kCellInitDmp || mode == kCellCfl || mode == kCellPrimeLimited;
   const bool act = valid && (priming ? (a.only_inst < 0 || kc == a.only_inst) : st.active != 0) &&
                    (mode != kCellPrimeLimited || a.status[parity(st)][cell] != 0);
+  if (in_cta && node == 0) cinst[lc] = act ? kc : -1;
   if (!__syncthreads_or(act)) return;  // nothing to do in this CTA
   const int par = parity(st);
   const long long lcell = cell - in.cell_base;
@@ -359,49 +367,54 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   float* ubs = ubs_all + (in_cta ? lc : 0) * V;
 
   // DMP neighbourhood bounds (get_min_max step 2, Euler/limiter.f90:147-167):
-  // thread v < V of a cell folds its 3x3 Voronoi neighbourhood now, so the
-  // global loads overlap the update and the projections
-  double nlmin = 0.0, nlmax = 0.0;
-  float nen = 0.0f;  // FP32-mixed: largest error bound of the folded min/max
-  if (limiter && act && node < V && (mode == kCellFused || mode == kCellUpdate)) {
-    const int v = node;
-    const double* mmi = a.mm[par];
-    nlmin = mmi[(size_t)cell * 2 * V + v];
-    nlmax = mmi[(size_t)cell * 2 * V + V + v];
-    if constexpr (kFast) {
-      // integer-key min/max (the integer pipe, not FP64)
-      long long kmn = okey(nlmin), kmx = okey(nlmax);
-      const float* mei = a.mme[par];
+  // the thread of a (cell, variable) pair folds the cell's 3x3 Voronoi
+  // neighbourhood now, so the global loads overlap the update and the
+  // projections
+  double nlmin[C::NPAIR], nlmax[C::NPAIR];
+  float nen[C::NPAIR];  // largest error bound of the folded min/max
+  if (limiter && (mode == kCellFused || mode == kCellUpdate)) {
+#pragma unroll
+    for (int q = 0; q < C::NPAIR; ++q) {
+      const int pr = t + q * C::THREADS, lc2 = pr / V, v = pr - lc2 * V;
+      nlmin[q] = nlmax[q] = 0.0;
+      nen[q] = 0.0f;
+      const int k2 = pr < CPB * V ? cinst[lc2] : -1;
+      if (k2 < 0) continue;
+      const InstDesc& in2 = a.inst[k2];
+      const int par2 = parity(a.st[k2]);
+      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2, l2 = cell2 - in2.cell_base;
+      const int ci2 = (int)(l2 % in2.imax), cj2 = (int)(l2 / in2.imax);
+      const double* mmi = a.mm[par2];
+      const float* mei = a.mme[par2];
+      // integer-key min/max (the integer pipe, not FP64) in the fast kernels
+      double lo = mmi[(size_t)cell2 * 2 * V + v], hi = mmi[(size_t)cell2 * 2 * V + V + v];
+      long long klo = okey(lo), khi = okey(hi);
+      float en = 0.0f;
 #pragma unroll
       for (int jj = -1; jj <= 1; ++jj)
 #pragma unroll
         for (int ii = -1; ii <= 1; ++ii) {
-          const int in_ = nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]);
-          const int jn_ = nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
-          const long long nc = in.cell_base + in_ + (long long)in.imax * jn_;
-          kmn = min(kmn, okey(mmi[(size_t)nc * 2 * V + v]));
-          kmx = max(kmx, okey(mmi[(size_t)nc * 2 * V + V + v]));
-          if (mei) nen = fmaxf(nen, mei[(size_t)nc * V + v]);
+          const int in_ = nb_index(ci2, ii, in2.imax, in2.bc[0], in2.bc[1]);
+          const int jn_ = nb_index(cj2, jj, in2.jmax, in2.bc[2], in2.bc[3]);
+          const long long nc = in2.cell_base + in_ + (long long)in2.imax * jn_;
+          const double a_lo = mmi[(size_t)nc * 2 * V + v], a_hi = mmi[(size_t)nc * 2 * V + V + v];
+          if constexpr (kFast) {
+            klo = min(klo, okey(a_lo));
+            khi = max(khi, okey(a_hi));
+          } else {
+            lo = fmin(lo, a_lo);
+            hi = fmax(hi, a_hi);
+          }
+          if (mei) en = fmaxf(en, mei[(size_t)nc * V + v]);
         }
-      nlmin = okey_inv(kmn);
-      nlmax = okey_inv(kmx);
-    } else {
-#pragma unroll
-      for (int jj = -1; jj <= 1; ++jj)
-#pragma unroll
-        for (int ii = -1; ii <= 1; ++ii) {
-          const int in_ = nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]);
-          const int jn_ = nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
-          const long long nc = in.cell_base + in_ + (long long)in.imax * jn_;
-          nlmin = fmin(nlmin, mmi[(size_t)nc * 2 * V + v]);
-          nlmax = fmax(nlmax, mmi[(size_t)nc * 2 * V + V + v]);
-          if (a.mme[0]) nen = fmaxf(nen, a.mme[par][(size_t)nc * V + v]);
-        }
+      nlmin[q] = kFast ? okey_inv(klo) : lo;
+      nlmax[q] = kFast ? okey_inv(khi) : hi;
+      nen[q] = en;
     }
   }
 
   // projection operators into shared memory (lanes index them by subcell)
-  for (int k = t; k < C::OPS_DBL; k += blockDim.x) {
+  if constexpr (Sys::ID != kSysAD) for (int k = t; k < C::OPS_DBL; k += C::THREADS) {
     opsm[k] = k < S * P ? op.uh2lim[k] : op.uh2lob[k - S * P];
     if constexpr (kFast) opsf[k] = k < S * P ? op.uh2limf[k] : op.uh2lobf[k - S * P];
   }
@@ -409,10 +422,14 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     cmax[lc] = 0ull;
     cflag[lc] = 0;
   }
-  if (kFast && in_cta && node < V) {
-    // the cell's FP32 reference state ubar: its start-of-step state at node 0, rounded to FP32
-    amax[node] = 0u;
-    ubs[node] = act ? (float)a.uh[par][(size_t)cell * P2 * V + node] : 0.0f;
+  if constexpr (kFast && Sys::ID != kSysAD) {
+    // a cell's FP32 reference state ubar: its start-of-step state at node 0, rounded to FP32
+    for (int pr = t; pr < CPB * V; pr += C::THREADS) {
+      const int lc2 = pr / V, v = pr - lc2 * V, k2 = cinst[lc2];
+      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2;
+      amax_all[pr] = 0u;
+      ubs_all[pr] = k2 >= 0 ? (float)a.uh[parity(a.st[k2])][(size_t)cell2 * P2 * V + v] : 0.0f;
+    }
   }
   __syncthreads();
 
@@ -510,7 +527,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   // FP32-mixed: the node's state in FP32, and its deviation from the cell's
   // FP32 reference state ubar, formed in FP32 (one conversion per value)
   float uf[V], du[V], ubf[V];
-  if constexpr (kFast) {
+  if constexpr (kFast && Sys::ID != kSysAD) {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       ubf[v] = ubs[v];
@@ -550,7 +567,6 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     // Cells whose limiter is active keep their min/max from the subcell data
     // (get_min_max, Euler/limiter.f90:134-139) in the priming pass.
     const bool from_lh = act && (mode == kCellPrime || mode == kCellPrimeLimited) && a.status[par][valid ? cell : 0] != 0;
-    bool f32red = false;  // the cell's partial min/max are in REDf (FP32)
     if constexpr (kFast) {
       if (act) {
 #pragma unroll
@@ -627,7 +643,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         }
         if (posfail) atomicOr(&cflag[lc], 1);
       }
-      f32red = f32ok && !from_lh;
+      if (act && node == 0 && f32ok && !from_lh) atomicOr(&cflag[lc], 8);  // the cell's partial min/max are in REDf (FP32)
     } else {
       if (act) {
 #pragma unroll
@@ -660,63 +676,72 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       }
     }
     __syncthreads();
-    if (act && node < V) {
-      const int v = node;
+#pragma unroll
+    for (int q = 0; q < C::NPAIR; ++q) {
+      const int pr = t + q * C::THREADS, lc2 = pr / V, v = pr - lc2 * V;
+      const int k2 = pr < CPB * V ? cinst[lc2] : -1;
+      if (k2 < 0) continue;
+      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2;
+      const int par2 = parity(a.st[k2]);
+      const double* U2 = sm + (size_t)lc2 * C::CELL_DBL;
+      const double* RED2 = U2 + V * P2 + V * S * P + V * P * P;
+      const float* REDf2 = reinterpret_cast<const float*>(U2 + V * P2) + V * P2 + V * S * P + V * P * P;
+      const bool f32red = (cflag[lc2] & 8) != 0;
+      const float am = kFast ? __uint_as_float(amax_all[pr]) : 0.0f, ub32 = kFast ? ubs_all[pr] : 0.0f;
       double cmn, cmx;
-      const double ubar = kFast ? (double)ubs[v] : 0.0;  // the cell's FP32 reference state (FP32-mixed)
+      const double ubar = kFast ? (double)ub32 : 0.0;  // the cell's FP32 reference state
       // FP32 projections: the cell's deviation min/max from its FP32 reference
       // state ubar, and a bound on |ubar + fmn - FP64 value| (and fmx): the
       // projections' bound as formed above (rounded up), plus the FP64
       // roundings of the reference-order values (generously 1e-12 relative)
       float fmn = 0.0f, fmx = 0.0f, ecell = 0.0f;
       if (f32red) {
-        fmn = REDf[v * P2];
-        fmx = REDf[(V + v) * P2];
+        fmn = REDf2[v * P2];
+        fmx = REDf2[(V + v) * P2];
 #pragma unroll
-        for (int k = 1; k < P2; ++k) { fmn = fminf(fmn, REDf[v * P2 + k]); fmx = fmaxf(fmx, REDf[(V + v) * P2 + k]); }
+        for (int k = 1; k < P2; ++k) { fmn = fminf(fmn, REDf2[v * P2 + k]); fmx = fmaxf(fmx, REDf2[(V + v) * P2 + k]); }
         cmn = ubar + (double)fmn;
         cmx = ubar + (double)fmx;
-        const float am = __uint_as_float(amax[v]);
-        ecell = (op.perr * am + op.pdev * (fabsf(ubs[v]) + 2.0f * am)) * 1.0001f + 1.0e-12f * (fabsf(ubs[v]) + am);
+        ecell = (op.perr * am + op.pdev * (fabsf(ub32) + 2.0f * am)) * 1.0001f + 1.0e-12f * (fabsf(ub32) + am);
       } else {
-        cmn = RED[v * P2];
-        cmx = RED[(V + v) * P2];
+        cmn = RED2[v * P2];
+        cmx = RED2[(V + v) * P2];
 #pragma unroll
-        for (int k = 1; k < P2; ++k) { cmn = fmin(cmn, RED[v * P2 + k]); cmx = fmax(cmx, RED[(V + v) * P2 + k]); }
+        for (int k = 1; k < P2; ++k) { cmn = fmin(cmn, RED2[v * P2 + k]); cmx = fmax(cmx, RED2[(V + v) * P2 + k]); }
       }
       if (mode == kCellPrime || mode == kCellPrimeLimited) {
-        a.mm[par][(size_t)cell * 2 * V + v] = cmn;
-        a.mm[par][(size_t)cell * 2 * V + V + v] = cmx;
-        if (a.mme[0]) a.mme[par][(size_t)cell * V + v] = ecell;
+        a.mm[par2][(size_t)cell2 * 2 * V + v] = cmn;
+        a.mm[par2][(size_t)cell2 * 2 * V + V + v] = cmx;
+        if (a.mme[0]) a.mme[par2][(size_t)cell2 * V + v] = ecell;
       } else {
         double lmin, lmax, argmax;
         float en = 0.0f;
         if (mode == kCellInitDmp) {
           // Euler/initialize.f90:291-294: the cell's own nodal min/max
-          lmin = U[v * P2];
-          lmax = U[v * P2];
-          for (int k = 1; k < P2; ++k) { lmin = fmin(lmin, U[v * P2 + k]); lmax = fmax(lmax, U[v * P2 + k]); }
+          lmin = U2[v * P2];
+          lmax = U2[v * P2];
+          for (int k = 1; k < P2; ++k) { lmin = fmin(lmin, U2[v * P2 + k]); lmax = fmax(lmax, U2[v * P2 + k]); }
           argmax = 1.0e-1;
         } else {
           // get_min_max step 2: the neighbourhood bounds folded at the start
-          lmin = nlmin;
-          lmax = nlmax;
-          en = nen;
+          lmin = nlmin[q];
+          lmax = nlmax[q];
+          en = nen[q];
           argmax = 0.0;
           if (a.lminmax) {
-            a.lminmax[(size_t)cell * 2 * V + v] = lmin;
-            a.lminmax[(size_t)cell * 2 * V + V + v] = lmax;
+            a.lminmax[(size_t)cell2 * 2 * V + v] = lmin;
+            a.lminmax[(size_t)cell2 * 2 * V + V + v] = lmax;
           }
           // candidate min/max for the next step (status 0)
-          a.mm[par ^ 1][(size_t)cell * 2 * V + v] = cmn;
-          a.mm[par ^ 1][(size_t)cell * 2 * V + V + v] = cmx;
-          if (a.mme[0]) a.mme[par ^ 1][(size_t)cell * V + v] = ecell;
+          a.mm[par2 ^ 1][(size_t)cell2 * 2 * V + v] = cmn;
+          a.mm[par2 ^ 1][(size_t)cell2 * 2 * V + V + v] = cmx;
+          if (a.mme[0]) a.mme[par2 ^ 1][(size_t)cell2 * V + v] = ecell;
         }
         if (a.mme[0] == nullptr || (!f32red && en == 0.0f)) {
           // FP64 values (FP32-wide mode: FP32 projections taken as they are);
           // Euler/limiter.f90:210-220
           const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (lmax - lmin)), argmax);
-          if (cmn < lmin - ldiff || cmx > lmax + ldiff) atomicOr(&cflag[lc], 2);
+          if (cmn < lmin - ldiff || cmx > lmax + ldiff) atomicOr(&cflag[lc2], 2);
         } else {
           // FP32-mixed: the same comparisons in FP32, in the deviation space
           // of the cell's FP32 reference state ub (FP64 work is the costly
@@ -734,11 +759,11 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const float dl = Lmin - ld, dh = Lmax + ld;
           const float xl = f32red ? fmn : (float)(cmn - ub), xh = f32red ? fmx : (float)(cmx - ub);
           const float e = ecell + 1.002f * en + 2.5e-7f * (fabsf(Lmin) + fabsf(Lmax) + ld) + 1.0e-11f +
-                          1.0e-12f * fabsf(ubs[v]);
+                          1.0e-12f * fabsf(ub32);
           const float ml = e + 1.2e-7f * fabsf(xl), mh = e + 1.2e-7f * fabsf(xh);
           const float gl = xl - dl, gh = dh - xh;  // >= 0: not below lmin - ldiff / not above lmax + ldiff
-          if (gl < -ml || gh < -mh) atomicOr(&cflag[lc], 2);
-          else if (!(gl >= ml) || !(gh >= mh)) atomicOr(&cflag[lc], 4);
+          if (gl < -ml || gh < -mh) atomicOr(&cflag[lc2], 2);
+          else if (!(gl >= ml) || !(gh >= mh)) atomicOr(&cflag[lc2], 4);
         }
       }
     }
