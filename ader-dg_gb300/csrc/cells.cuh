@@ -169,27 +169,111 @@ struct Proj {
 #pragma unroll
       for (int v = 0; v < V; ++v) { mn[v] = fminf(mn[v], val[v]); mx[v] = fmaxf(mx[v], val[v]); }
     }
-    // the subcells left open, in FP64 in the reference's order (the y pass
-    // of get_subcell_data, then x; lim64 = uh2lim (s,k) at [s + S*k]): the
-    // FP64 path's value and decision bit for bit
-    if constexpr (Sys::ID != kSysAD) while (open) {
-      const int idx = r + (__ffs(open) - 1) * nr;
-      open &= open - 1u;
-      const int s1 = idx % S, s2 = idx / S;
-      double qd[V];
-#pragma unroll 1
-      for (int v = 0; v < V; ++v) {
-        double acc = 0.0;
-#pragma unroll 1
-        for (int k = 0; k < P; ++k) {
-          double ly = 0.0;
-          for (int m = 0; m < P; ++m) ly = ly + U64[v * P2 + k + P * m] * lim64[s2 + S * m];
-          acc = acc + ly * lim64[s1 + S * k];
-        }
-        qd[v] = acc;
+    if constexpr (Sys::ID != kSysAD)
+      while (open) {
+        const int idx = r + (__ffs(open) - 1) * nr;
+        open &= open - 1u;
+        if (!positive64<Sys>(U64, lim64, ph, idx % S, idx / S)) posfail = true;
       }
-      if (!Sys::positive(ph, qd)) posfail = true;
+  }
+  // a subcell left open, in FP64 in the reference's order (the y pass of
+  // get_subcell_data, then x; lim64 = uh2lim (s,k) at [s + S*k]): the FP64 path's
+  // value and decision bit for bit
+  template <class Sys>
+  __device__ static bool positive64(const double* U64, const double* lim64, const Phys& ph, int s1, int s2) {
+    double qd[V];
+#pragma unroll 1
+    for (int v = 0; v < V; ++v) {
+      double acc = 0.0;
+#pragma unroll 1
+      for (int k = 0; k < P; ++k) {
+        double ly = 0.0;
+        for (int m = 0; m < P; ++m) ly = __dadd_rn(ly, __dmul_rn(U64[v * P2 + k + P * m], lim64[s2 + S * m]));
+        acc = __dadd_rn(acc, __dmul_rn(ly, lim64[s1 + S * k]));
+      }
+      qd[v] = acc;
     }
+    return Sys::positive(ph, qd);
+  }
+  // The FP32 passes of a team of P2 threads (the cell kernel), each thread
+  // taking several outputs that share operands: the y pass column ii = r % P
+  // and the outputs r / P, + P, .. of the S subcell and P Lobatto rows; the x
+  // pass row s2 and a chunk of its subcells.  One output at a time read 2P (V +
+  // 1) shared-memory words for every V P products, and the kernel waited on
+  // them.  Same sums in the same order.
+  __device__ static void ypass_team(const float* U, float* LY, float* LB, const float* lim, const float* lob, int r) {
+    constexpr int NO = (S + P + P - 1) / P;  // outputs of a thread
+    const int ii = r % P, o0 = r / P;
+    float c[NO][P];
+#pragma unroll
+    for (int q = 0; q < NO; ++q) {
+      const int o = o0 + q * P;
+#pragma unroll
+      for (int k = 0; k < P; ++k) c[q][k] = o < S ? lim[o + S * k] : o < S + P ? lob[o - S + P * k] : 0.0f;
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      float x[P];
+#pragma unroll
+      for (int k = 0; k < P; ++k) x[k] = U[v * P2 + ii + P * k];
+#pragma unroll
+      for (int q = 0; q < NO; ++q) {
+        const int o = o0 + q * P;
+        float acc = 0.0f;
+#pragma unroll
+        for (int k = 0; k < P; ++k) acc = fmaf(x[k], c[q][k], acc);
+        if (o < S) LY[(v * S + o) * P + ii] = acc;
+        else if (o < S + P) LB[(v * P + o - S) * P + ii] = acc;
+      }
+    }
+  }
+  template <class Sys>
+  __device__ static void xpass_team(const float* LY, const float* LB, const float* lim, const float* lob,
+                                    const double* U64, const double* lim64, const typename Sys::FConst& fc,
+                                    const float* err, const float* ubf, const Phys& ph, int r, float* mn, float* mx,
+                                    bool& posfail) {
+    constexpr int C = P2 / S;             // chunks of a row
+    constexpr int CH = (S + C - 1) / C;   // subcells of a chunk
+    float val[V];
+    if (r < C * S) {
+      const int s2 = r / C, c0 = r - s2 * C;
+      float e[V], ly[V][P];
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        e[v] = err[v] + 2.5e-7f * fabsf(ubf[v]);
+#pragma unroll
+        for (int k = 0; k < P; ++k) ly[v][k] = LY[(v * S + s2) * P + k];
+      }
+      unsigned open = 0u;  // bit q: the chunk's q-th subcell needs the FP64 test
+#pragma unroll 1
+      for (int q = 0; q < CH; ++q) {
+        const int s1 = c0 + q * C;
+        if (s1 >= S) break;
+        float c[P], qv[V];
+#pragma unroll
+        for (int k = 0; k < P; ++k) c[k] = lim[s1 + S * k];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          float acc = 0.0f;
+#pragma unroll
+          for (int k = 0; k < P; ++k) acc = fmaf(ly[v][k], c[k], acc);
+          mn[v] = fminf(mn[v], acc);
+          mx[v] = fmaxf(mx[v], acc);
+          qv[v] = ubf[v] + acc;
+        }
+        if constexpr (Sys::ID != kSysAD)
+          if (!Sys::admissible_box_f32(fc, qv, e)) open |= 1u << q;
+      }
+      if constexpr (Sys::ID != kSysAD)
+        while (open) {
+          const int q = __ffs(open) - 1;
+          open &= open - 1u;
+          if (!positive64<Sys>(U64, lim64, ph, c0 + q * C, s2)) posfail = true;
+        }
+    }
+    lobatto<true>(LB, lob, r % P, r / P, val);
+#pragma unroll
+    for (int v = 0; v < V; ++v) { mn[v] = fminf(mn[v], val[v]); mx[v] = fmaxf(mx[v], val[v]); }
   }
 };
 
@@ -323,6 +407,10 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   using C = CellCfg<Sys, N, VAR>;
   constexpr int P = N + 1, P2 = P * P, S = 2 * N + 1, V = Sys::V, CPB = C::CPB;
   constexpr bool kF32 = kFast && !kExact;  // FP32 storage and update
+  // the team passes where they are faster (measured): N = 3, 344 -> 328 us on the
+  // Riemann problem 512^2; at N = 4 their chunks leave a quarter of the lanes idle
+  // (156 -> 170 us on the vortex), at N = 5 and 2 they cost 7% and 6%
+  constexpr bool kTeam = P == 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* sm = reinterpret_cast<double*>(smem_raw);
   double* opsm = sm + CPB * C::CELL_DBL;
@@ -598,7 +686,10 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         f32ok = f32ok && err[v] <= 1.0e-4f;
       }
       if (act && !from_lh) {
-        if (f32ok) Proj<N, V, float>::template ypass<true>(Uf, LYf, LBf, opsf, opsf + S * P, node, P2);
+        if (f32ok) {
+          if constexpr (kTeam) Proj<N, V, float>::ypass_team(Uf, LYf, LBf, opsf, opsf + S * P, node);
+          else Proj<N, V, float>::template ypass<true>(Uf, LYf, LBf, opsf, opsf + S * P, node, P2);
+        }
         else Proj<N, V, double>::template ypass<false>(U, LY, LB, opsm, opsm + S * P, node, P2);
       }
       __syncthreads();
@@ -621,9 +712,14 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           float mn[V], mx[V];
 #pragma unroll
           for (int v = 0; v < V; ++v) { mn[v] = du[v]; mx[v] = du[v]; }
-          Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, opsf, opsf + S * P, U, opsm,
-                                                            typename Sys::FConst(in.ph), err, ubf, in.ph, node, P2,
-                                                            mn, mx, posfail);
+          if constexpr (kTeam)
+            Proj<N, V, float>::template xpass_team<Sys>(LYf, LBf, opsf, opsf + S * P, U, opsm,
+                                                        typename Sys::FConst(in.ph), err, ubf, in.ph, node, mn, mx,
+                                                        posfail);
+          else
+            Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, opsf, opsf + S * P, U, opsm,
+                                                              typename Sys::FConst(in.ph), err, ubf, in.ph, node, P2,
+                                                              mn, mx, posfail);
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             REDf[v * P2 + node] = mn[v];
