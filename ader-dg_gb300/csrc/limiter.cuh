@@ -134,6 +134,7 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
   return ma < mb ? a : b;
 }
 
+__device__ __forceinline__ double max_nonneg(double a, double b);
 // Subgrid Rusanov flux (Euler/limiter.f90:361-378; BN :359-383 adds D = B~ dQ);
 // kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
 // flux (the update takes half its factor: one FP64 instruction less a variable)
@@ -146,7 +147,8 @@ __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const
     T eL, eR;
     Sys::flux_dir_eig_r(pc, QL, d, FLf, eL);
     Sys::flux_dir_eig_r(pc, QR, d, FRf, eR);
-    smax = tmax(eL, eR);
+    if constexpr (sizeof(T) == 8) smax = max_nonneg(eL, eR);
+    else smax = tmax(eL, eR);
 #pragma unroll
     for (int v = 0; v < V; ++v) F[v] = (FLf[v] + FRf[v]) - smax * (QR[v] - QL[v]);
   } else {
@@ -164,23 +166,55 @@ __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const
   }
 }
 
+// Keys that leave a NaN out of a minimum / maximum, as fmin / fmax do.
+__device__ __forceinline__ bool is_nan_bits(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ long long okey_min(double x) { return is_nan_bits(x) ? 0x7ff0000000000000LL : okey(x); }
+__device__ __forceinline__ long long okey_max(double x) {
+  return is_nan_bits(x) ? okey(__longlong_as_double((long long)0xfff0000000000000ull)) : okey(x);
+}
+// fmax of two values that are >= 0 or NaN, on the integer pipe
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  const long long ka = is_nan_bits(a) ? -1 : __double_as_longlong(a), kb = is_nan_bits(b) ? -1 : __double_as_longlong(b);
+  return ka >= kb ? a : b;
+}
+
 // Warp-wide min/max of V values per lane (butterfly), then lane 0 of warp w
-// stores them at red[v * NW + w] (min) and red[(V + v) * NW + w] (max).
+// stores them at red[v * NW + w] (min) and red[(V + v) * NW + w] (max).  FP64
+// values as integer keys (okey, cells.cuh): the ten FP64 comparisons a value
+// took on the pipe that bounds the re-solve were 13% of its FP64 slots.
 template <class R, int V, int NW>
 __device__ __forceinline__ void warp_minmax_store(R* mn, R* mx, R* red, int t) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      mn[v] = tmin(mn[v], __shfl_xor_sync(0xffffffffu, mn[v], o));
-      mx[v] = tmax(mx[v], __shfl_xor_sync(0xffffffffu, mx[v], o));
-    }
-  if ((t & 31) == 0)
+  if constexpr (sizeof(R) == 8) {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-      red[v * NW + (t >> 5)] = mn[v];
-      red[(V + v) * NW + (t >> 5)] = mx[v];
+      long long lo = okey_min(mn[v]), hi = okey_max(mx[v]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      }
+      if ((t & 31) == 0) {
+        red[v * NW + (t >> 5)] = okey_inv(lo);
+        red[(V + v) * NW + (t >> 5)] = okey_inv(hi);
+      }
     }
+  } else {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        mn[v] = tmin(mn[v], __shfl_xor_sync(0xffffffffu, mn[v], o));
+        mx[v] = tmax(mx[v], __shfl_xor_sync(0xffffffffu, mx[v], o));
+      }
+    if ((t & 31) == 0)
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        red[v * NW + (t >> 5)] = mn[v];
+        red[(V + v) * NW + (t >> 5)] = mx[v];
+      }
+  }
 }
 
 // T = double: the reference's FP64 arithmetic in its order (bit for bit),
@@ -580,26 +614,23 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     __syncthreads();
 
     // ---- put_subcell_data (Euler/limiter.f90:74-98): luhy then luh
-    for (int p = t; p < S * P; p += NT) {
-      const int iii = p % S, s = p / S;
+    // (variable, item) pairs, so that few lanes idle
+    for (int q = t; q < V * S * P; q += NT) {
+      const int v = q / (S * P), p = q - v * (S * P), iii = p % S, s = p / S;
+      T acc = T(0);
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        T acc = T(0);
-        for (int kk = 0; kk < S; ++kk) acc = acc + sub1[v * S * S + iii + S * kk] * l2uT[s + P * kk];
-        LUY[(v * P + s) * S + iii] = acc;
-      }
+      for (int kk = 0; kk < S; ++kk) acc = acc + sub1[v * S * S + iii + S * kk] * l2uT[s + P * kk];
+      LUY[(v * P + s) * S + iii] = acc;
     }
     __syncthreads();
     double* uout = a.uh[par ^ 1] + (size_t)c * P2 * V;
-    for (int p = t; p < P2; p += NT) {
-      const int s1 = p % P, jjj = p / P;
+    for (int q = t; q < V * P2; q += NT) {
+      const int p = q / V, v = q - p * V, s1 = p % P, jjj = p / P;
+      T acc = T(0);
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        T acc = T(0);
-        for (int kk = 0; kk < S; ++kk) acc = acc + LUY[(v * P + jjj) * S + kk] * l2uT[s1 + P * kk];
-        UN[v * P2 + p] = (double)acc;
-        uout[p * V + v] = (double)acc;
-      }
+      for (int kk = 0; kk < S; ++kk) acc = acc + LUY[(v * P + jjj) * S + kk] * l2uT[s1 + P * kk];
+      UN[v * P2 + p] = (double)acc;
+      uout[q] = (double)acc;
     }
     __syncthreads();
     // ---- DMP of the new polynomial: recompute = 2 cells only (a recompute =
@@ -807,14 +838,29 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
 #pragma unroll
         for (int v = 0; v < V; ++v) nl[p * V + v] = (double)sub1[v * S * S + p];
       T tmn[V], tmx[V];
+      if constexpr (sizeof(T) == 8) {
+        long long lo[V], hi[V];
 #pragma unroll
-      for (int v = 0; v < V; ++v) { tmn[v] = T(kInf); tmx[v] = T(-kInf); }
-      for (int p = t; p < S * S; p += NT)
+        for (int v = 0; v < V; ++v) { lo[v] = okey_min(kInf); hi[v] = okey_max(-kInf); }
+        for (int p = t; p < S * S; p += NT)
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          tmn[v] = tmin(tmn[v], sub1[v * S * S + p]);
-          tmx[v] = tmax(tmx[v], sub1[v * S * S + p]);
-        }
+          for (int v = 0; v < V; ++v) {
+            const double x = sub1[v * S * S + p];
+            lo[v] = min(lo[v], okey_min(x));
+            hi[v] = max(hi[v], okey_max(x));
+          }
+#pragma unroll
+        for (int v = 0; v < V; ++v) { tmn[v] = okey_inv(lo[v]); tmx[v] = okey_inv(hi[v]); }
+      } else {
+#pragma unroll
+        for (int v = 0; v < V; ++v) { tmn[v] = T(kInf); tmx[v] = T(-kInf); }
+        for (int p = t; p < S * S; p += NT)
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            tmn[v] = tmin(tmn[v], sub1[v * S * S + p]);
+            tmx[v] = tmax(tmx[v], sub1[v * S * S + p]);
+          }
+      }
       warp_minmax_store<T, V, NW>(tmn, tmx, redt, t);
     }
     __syncthreads();
