@@ -16,6 +16,8 @@
 // predictor_tu.cu) and in FP32 in the FP32-wide mode.
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "physics.cuh"
 
@@ -259,16 +261,19 @@ __global__ void __launch_bounds__(256) k_faces(BatchArgs a, FaceConst fc) {
     R* dst = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
     dst[out] = (R)(CT(0.5) * ((FL0 + FR0) * nv0 + (FL1 + FR1) * nv1) - CT(0.5) * smax * (QR[0] - QL[0]));
   } else {
-    // Euler (FP64) and Baer-Nunziato (FP64 or FP32 compute, see above)
+    // Euler (FP64) and Baer-Nunziato (FP64 or FP32 compute, see above); FP32-mixed
+    // Baer-Nunziato (kRcp) keeps the FP32 states and widens them where it uses them
+    constexpr bool kRcp = sizeof(R) == 4 && sizeof(CT) == 8;
+    using LT = typename std::conditional<kRcp, float, CT>::type;
     const PhysC<CT> pc(ph);
-    CT QL[V], QR[V], FL[V], FR[V];
+    LT QL[V], QR[V], FL[V], FR[V];
     const bool is_dmr = (Sys::ID == kSysEuler) && in.bc_mode == 1;
     const long long cL = xdir ? cid(i - 1, j) : cid(i, j - 1);
     const long long cR = cid(i, j);
     if (pos == 0) {
       if (is_dmr) {
         if (xdir) {  // inflow, Euler/riemann_problem.f90:41-48
-          dmr_state(pc, fc.Va, 0, QL, FL);
+          if constexpr (Sys::ID == kSysEuler) dmr_state(pc, fc.Va, 0, QL, FL);
           load_face_state<V, R>(qb, fb, cR, P, l, fl, QR, FR);
         } else {     // transmissive / reflective wall, :76-86
           load_face_state<V, R>(qb, fb, cR, P, l, fl, QL, FL);
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(256) k_faces(BatchArgs a, FaceConst fc) {
       load_face_state<V, R>(qb, fb, cLast, P, l, fr, QL, FL);
       if (is_dmr && !xdir) {  // time-dependent top boundary, :88-100
         const double x_sw = fc.xsw0 + fc.xsw1 * a.st[k].time;
-        dmr_state(pc, ((double)(i + 1) * in.dx <= x_sw) ? fc.Va : fc.Vb, 1, QR, FR);
+        if constexpr (Sys::ID == kSysEuler) dmr_state(pc, ((double)(i + 1) * in.dx <= x_sw) ? fc.Va : fc.Vb, 1, QR, FR);
       } else if (!is_dmr && bcr == 3) {
         load_face_state<V, R>(qb, fb, xdir ? cid(0, j) : cid(i, 0), P, l, fl, QR, FR);
       } else {
@@ -302,29 +307,36 @@ __global__ void __launch_bounds__(256) k_faces(BatchArgs a, FaceConst fc) {
       load_face_state<V, R>(qb, fb, cL, P, l, fr, QL, FL);
       load_face_state<V, R>(qb, fb, cR, P, l, fl, QR, FR);
     }
-    // FP32-mixed Baer-Nunziato: FP64 with the reciprocal-sharing forms
-    constexpr bool kRcp = sizeof(R) == 4 && sizeof(CT) == 8;
-    // Rusanov: smax from both sides' eigenvalues (Euler/pde.f90:97-114)
-    CT smax;
-    if constexpr (kRcp) smax = tmax(Sys::max_eig_r(pc, QL, d), Sys::max_eig_r(pc, QR, d));
-    else smax = tmax(Sys::max_eig(pc, QL, d), Sys::max_eig(pc, QR, d));
-    if constexpr (Sys::ID == kSysBN) {
-      // path-conservative fluctuations, Baer-Nunziato/pde.f90:326-353
-      CT D[9];
-      if constexpr (kRcp) BNSys::roe_times_jump_r(pc, QL, QR, d, D);
-      else BNSys::roe_times_jump(pc, QL, QR, d, D);
+    if constexpr (kRcp) {
+      float fm[V], fp[V];
+      BNSys::face_mixed(pc, BNSys::FConst(ph), QL, QR, FL, FR, d, fm, fp);
       R* dm = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
       R* dp = reinterpret_cast<R*>(xdir ? a.fp : a.gp);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        const CT base = CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]);
-        dm[out + v] = (R)(base - CT(0.5) * D[v]);
-        dp[out + v] = (R)(base + CT(0.5) * D[v]);
+        dm[out + v] = fm[v];
+        dp[out + v] = fp[v];
       }
     } else {
-      R* dst = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
+      // Rusanov: smax from both sides' eigenvalues (Euler/pde.f90:97-114)
+      const CT smax = tmax(Sys::max_eig(pc, QL, d), Sys::max_eig(pc, QR, d));
+      if constexpr (Sys::ID == kSysBN) {
+        // path-conservative fluctuations, Baer-Nunziato/pde.f90:326-353
+        CT D[9];
+        BNSys::roe_times_jump(pc, QL, QR, d, D);
+        R* dm = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
+        R* dp = reinterpret_cast<R*>(xdir ? a.fp : a.gp);
 #pragma unroll
-      for (int v = 0; v < V; ++v) dst[out + v] = (R)(CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]));
+        for (int v = 0; v < V; ++v) {
+          const CT base = CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]);
+          dm[out + v] = (R)(base - CT(0.5) * D[v]);
+          dp[out + v] = (R)(base + CT(0.5) * D[v]);
+        }
+      } else {
+        R* dst = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
+#pragma unroll
+        for (int v = 0; v < V; ++v) dst[out + v] = (R)(CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]));
+      }
     }
   }
 }

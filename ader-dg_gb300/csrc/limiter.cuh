@@ -134,7 +134,6 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
   return ma < mb ? a : b;
 }
 
-__device__ __forceinline__ double max_nonneg(double a, double b);
 // Subgrid Rusanov flux (Euler/limiter.f90:361-378; BN :359-383 adds D = B~ dQ);
 // kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
 // flux (the update takes half its factor: one FP64 instruction less a variable)
@@ -167,19 +166,10 @@ __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const
 }
 
 // Keys that leave a NaN out of a minimum / maximum, as fmin / fmax do.
-__device__ __forceinline__ bool is_nan_bits(double x) {
-  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
-}
 __device__ __forceinline__ long long okey_min(double x) { return is_nan_bits(x) ? 0x7ff0000000000000LL : okey(x); }
 __device__ __forceinline__ long long okey_max(double x) {
   return is_nan_bits(x) ? okey(__longlong_as_double((long long)0xfff0000000000000ull)) : okey(x);
 }
-// fmax of two values that are >= 0 or NaN, on the integer pipe
-__device__ __forceinline__ double max_nonneg(double a, double b) {
-  const long long ka = is_nan_bits(a) ? -1 : __double_as_longlong(a), kb = is_nan_bits(b) ? -1 : __double_as_longlong(b);
-  return ka >= kb ? a : b;
-}
-
 // Warp-wide min/max of V values per lane (butterfly), then lane 0 of warp w
 // stores them at red[v * NW + w] (min) and red[(V + v) * NW + w] (max).  FP64
 // values as integer keys (okey, cells.cuh): the ten FP64 comparisons a value

@@ -53,18 +53,22 @@ template <class T> __device__ __forceinline__ T tsqrt(T x) {
 // the device by aderdg_probe_math); zeros, denormals, infinities and NaNs (the
 // exponent field all zeros or all ones, an integer test) take the correctly
 // rounded operation.  FP32: the correctly rounded operations.
-// FP32 -> FP64, exact, on the integer pipe (sign, exponent rebias, mantissa
-// shift) for zeros and normal values; infinities, NaNs and denormals take the
-// hardware conversion.  The FP64-bound kernels of the FP32-mixed mode read
-// FP32 inputs (the Baer-Nunziato face states): their conversions then leave
-// the FP64 pipe.
+// FP32 -> FP64, exact, without the FP64 pipe (sign, exponent rebias, mantissa
+// shift; denormals scaled in FP32 first; a NaN is quieted).  The FP64-bound kernels
+// of the FP32-mixed mode read FP32 inputs (the Baer-Nunziato face states): their
+// conversions then leave the FP64 pipe.  No case falls back to the hardware
+// conversion: as a rare branch it became a predicated instruction that the FP64
+// pipe issued for every value (a fifth of the face kernel's FP64 slots).
 __device__ __forceinline__ double widen_bits(float f) {
-  const unsigned u = __float_as_uint(f);
-  const unsigned e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
-  if (e == 0xffu || (e == 0u && m != 0u)) return (double)f;
-  unsigned long long d = (unsigned long long)(u & 0x80000000u) << 32;
-  if (e) d |= ((unsigned long long)(e + 896u) << 52) | ((unsigned long long)m << 29);
-  return __longlong_as_double((long long)d);
+  const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+  unsigned hi = (a >> 3) + (896u << 20), lo = a << 29;
+  if (a >= 0x7f800000u) hi += (896u << 20) + (a > 0x7f800000u ? 0x80000u & ~hi : 0u);
+  if (a < 0x00800000u) {
+    const unsigned g = __float_as_uint(__uint_as_float(a) * 1.8446744073709552e19f);  // 2^64
+    hi = g ? (g >> 3) + ((896u - 64u) << 20) : 0u;
+    lo = g << 29;
+  }
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
 template <class T, class R> __device__ __forceinline__ T widen(R x) {
   if constexpr (sizeof(T) == 8 && sizeof(R) == 4) return widen_bits(x);
@@ -96,6 +100,15 @@ template <class T> __device__ __forceinline__ T msqrt(T a) {
     const double h = fma(-s, y, 1.0);
     return fma(s * h, fma(h, 0.375, 0.5), s);
   }
+}
+
+__device__ __forceinline__ bool is_nan_bits(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+// fmax of two values that are >= 0 or NaN, on the integer pipe
+__device__ __forceinline__ double max_nonneg(double a, double b) {
+  const long long ka = is_nan_bits(a) ? -1 : __double_as_longlong(a), kb = is_nan_bits(b) ? -1 : __double_as_longlong(b);
+  return ka >= kb ? a : b;
 }
 
 // ---------------------------------------------------------------------------
@@ -514,6 +527,56 @@ struct BNSys {
     ex = tmax(tmax(tabs(u_g), tabs(u_g) + a_g), tmax(tabs(u_s), tabs(u_s) + a_s));
     ey = tmax(tmax(tabs(v_g), tabs(v_g) + a_g), tmax(tabs(v_s), tabs(v_s) + a_s));
   }
+  // maxval(abs(Lambda)) along d over two states, for FP32 states (widened on the
+  // integer pipe): FP32 estimates of the four speeds |u| + a with their error
+  // bounds, then the FP64 evaluation of those that may be the largest -- one or
+  // two of four, 19 FP64 instructions each.  A speed whose FP32 pressure is not
+  // settled (below 1e-3 of the terms it cancels) is always evaluated; a NaN is
+  // left out, as the maxima of max_eig_r do.
+  __device__ __forceinline__ static double max_speed(const PhysC<double>& pc, const FConst& fc, const float* qL,
+                                                     const float* qR, int d) {
+    float hi[4], lo = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float* q = k < 2 ? qL : qR;
+      const int o = (k & 1) ? 4 : 0;
+      const float g = (k & 1) ? fc.gg : fc.gs, g1 = (k & 1) ? fc.gg1 : fc.gs1, gpi = (k & 1) ? fc.ggpg : fc.gsps,
+                  pi = (k & 1) ? fc.pg : fc.ps, phi = (k & 1) ? 1.0f - q[8] : q[8];
+      const float i = 1.0f / q[o], u = (d == 0 ? q[o + 1] : q[o + 2]) * i;
+      const float ke = 0.5f * (q[o + 1] * q[o + 1] + q[o + 2] * q[o + 2]) * i;
+      const float pp = g1 * (q[o + 3] - ke) - gpi * phi + pi * phi;
+      const float mag = g1 * (fabsf(q[o + 3]) + fabsf(ke)) + fabsf(gpi) + fabsf(pi);
+      const float s = fabsf(u) + sqrtf(g * pp * i);
+      // relative error of s: half that of pp (a few roundings of its terms), and its own
+      const float rel = 1.0e-6f + 1.0e-6f * mag / pp;
+      const bool settled = pp > 1.0e-3f * mag && q[o] > 1.0e-30f && q[8] > 1.0e-3f && q[8] < 0.999f && s < 1.0e30f;
+      hi[k] = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
+      if (settled) lo = fmaxf(lo, s * (1.0f - rel));
+    }
+    unsigned cand = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (hi[k] >= lo) cand |= 1u << k;
+    // each lane takes its own candidates in turn (a branch per speed was turned
+    // into predicated instructions, which the FP64 pipe issued all the same)
+    long long best = -1;  // bits of the largest (>= 0)
+#pragma unroll 1
+    do {
+      const int k = __ffs(cand) - 1;
+      cand &= cand - 1u;
+      const bool gas = k & 1, right = k >> 1;
+      auto pick = [&](int s, int g) { return gas ? (right ? qR[g] : qL[g]) : (right ? qR[s] : qL[s]); };
+      const double m = widen_bits(pick(0, 4)), E = widen_bits(pick(3, 7)), a = widen_bits(right ? qR[8] : qL[8]);
+      const double mn = widen_bits(d == 0 ? pick(1, 5) : pick(2, 6)), mt = widen_bits(d == 0 ? pick(2, 6) : pick(1, 5));
+      const double phi = gas ? 1.0 - a : a;
+      const double i = mrcp<double>(m), u = mn * i;
+      const double pp = (gas ? pc.gg1 : pc.gs1) * (E - 0.5 * (mn * u + mt * (mt * i))) +
+                        (gas ? pc.pg - pc.ggpg : pc.ps - pc.gsps) * phi;  // phi (p + pi)
+      const double s = fabs(u) + msqrt<double>((gas ? pc.gg : pc.gs) * pp * i);
+      if (!is_nan_bits(s)) best = max(best, __double_as_longlong(s));
+    } while (cand);
+    return __longlong_as_double(best < 0 ? 0x7ff8000000000000LL : best);
+  }
   // The flux along axis d only, F[v] (the d-th half of flux_eig_r's F; Q1 v_s
   // = Q2 u_s), and maxval(abs(Lambda)) along d
   template <class T>
@@ -576,6 +639,57 @@ struct BNSys {
     D[6] = d == 1 ? bp * dq9 : T(0);
     D[7] = bpu * dq9;
     D[8] = bu * dq9;
+  }
+  // Path integrals of p_g, u_n and p_g u_n along QL + s jump (3-point
+  // Gauss-Legendre), the entries of the Roe matrix's column 9
+  __device__ __forceinline__ static void path_integrals(const PhysC<double>& pc, const double* QL, const double* jump,
+                                                        int d, double& bp, double& bu, double& bpu) {
+    const double sq = sqrt(15.0) / 10.;
+    const double sGP[3] = {0.5 - sq, 0.5, 0.5 + sq}, wGP[3] = {5. / 18.0, 8. / 18., 5. / 18.};
+    bp = bu = bpu = 0.0;
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+      const double s = sGP[g];
+      const double m = QL[0] + s * jump[0], mn = (d == 0 ? QL[1] : QL[2]) + s * (d == 0 ? jump[1] : jump[2]);
+      const double q4 = QL[4] + s * jump[4], q5 = QL[5] + s * jump[5], q6 = QL[6] + s * jump[6], q7 = QL[7] + s * jump[7];
+      const double b = q4 * (1.0 - (QL[8] + s * jump[8]));
+      const double r = mrcp<double>(b * m);
+      const double wp = (wGP[g] * pc.gg1) * (q7 * q4 - 0.5 * (q5 * q5 + q6 * q6)) * (m * r) - wGP[g] * pc.ggpg;
+      const double un = mn * (b * r);
+      bp = bp + wp;
+      bu = bu + wGP[g] * un;
+      bpu = bpu + wp * un;
+    }
+  }
+  // The FP32-mixed face fluxes Dm, Dp (Baer-Nunziato/pde.f90:326-353) of FP32
+  // face states and fluxes in FP64, rounded to FP32: twice the flux is formed
+  // and halved after the rounding, and the fluctuation's components that are
+  // zero along d are left out.
+  __device__ __forceinline__ static void face_mixed(const PhysC<double>& pc, const FConst& fc, const float* qL,
+                                                    const float* qR, const float* fL, const float* fR, int d, float* dm,
+                                                    float* dp) {
+    const double smax = max_speed(pc, fc, qL, qR, d);
+    double QL[9], jump[9];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      QL[v] = widen_bits(qL[v]);
+      jump[v] = widen_bits(qR[v]) - QL[v];
+    }
+    double bp, bu, bpu;
+    path_integrals(pc, QL, jump, d, bp, bu, bpu);
+    const double x = bp * jump[8], y = bpu * jump[8], z = bu * jump[8];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      const double t = (widen_bits(fL[v]) + widen_bits(fR[v])) - smax * jump[v];
+      const bool n = (v == 1 || v == 5) ? d == 0 : (v == 2 || v == 6) ? d == 1 : v != 0 && v != 4;
+      if (n) {
+        const double D = v == 1 || v == 2 ? -x : v == 3 ? -y : v == 5 || v == 6 ? x : v == 7 ? y : z;
+        dm[v] = 0.5f * (float)(t - D);
+        dp[v] = 0.5f * (float)(t + D);
+      } else {
+        dm[v] = dp[v] = 0.5f * (float)t;
+      }
+    }
   }
   template <class T>
   __device__ static void src_ncp_r(const PhysC<T>& pc, const T* Q, T ax, T ay, T* S) {
