@@ -152,7 +152,7 @@ __device__ void faces_euler_fp32(const BatchArgs& a, const FaceConst& fc, const 
 }
 
 template <class Sys, int N, class R, class CT>
-__global__ void __launch_bounds__(256) k_faces(BatchArgs a, FaceConst fc) {
+__global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && sizeof(CT) == 8 ? 3 : 1) k_faces(BatchArgs a, FaceConst fc) {
   constexpr int P = N + 1, V = Sys::V;
   const long long nx = a.nfx * P, ny = a.nfy * P;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;

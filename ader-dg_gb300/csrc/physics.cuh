@@ -70,6 +70,32 @@ __device__ __forceinline__ double widen_bits(float f) {
   }
   return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
+// FP64 -> FP32, round to nearest even as the hardware conversion, on the
+// integer pipe: the 24 leading bits plus the rounding carry; results below the
+// normal range take the shifted mantissa, too large ones are infinite.
+__device__ __forceinline__ float narrow_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  unsigned q = __funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 3);
+  q += ((lo & 0x1fffffffu) + 0x0fffffffu + (q & 1u)) >> 29;
+  unsigned r = ((e - 897u) << 23) + q;
+  if (e - 897u >= 253u) {  // outside [2^-126, 2^127): exponents near overflow, denormal results, infinities and NaNs
+    if (e >= 1023u + 127u) {
+      const bool nan = e == 0x7ffu && ((hi & 0xfffffu) | lo);
+      r = nan ? 0x7fc00000u : (e == 1023u + 127u && r < 0x7f800000u) ? r : 0x7f800000u;
+    } else {
+      const unsigned s = 897u - e + 29u;  // bits shifted out of the 53
+      const unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
+      if (s >= 55u) {
+        r = 0u;
+      } else {
+        const unsigned long long k = m >> s, rem = m & ((1ull << s) - 1ull), half = 1ull << (s - 1u);
+        r = (unsigned)(k + (rem > half || (rem == half && (k & 1ull)) ? 1ull : 0ull));
+      }
+    }
+  }
+  return __uint_as_float(r | (hi & 0x80000000u));
+}
 template <class T, class R> __device__ __forceinline__ T widen(R x) {
   if constexpr (sizeof(T) == 8 && sizeof(R) == 4) return widen_bits(x);
   else return (T)x;
@@ -684,10 +710,10 @@ struct BNSys {
       const bool n = (v == 1 || v == 5) ? d == 0 : (v == 2 || v == 6) ? d == 1 : v != 0 && v != 4;
       if (n) {
         const double D = v == 1 || v == 2 ? -x : v == 3 ? -y : v == 5 || v == 6 ? x : v == 7 ? y : z;
-        dm[v] = 0.5f * (float)(t - D);
-        dp[v] = 0.5f * (float)(t + D);
+        dm[v] = 0.5f * narrow_bits(t - D);
+        dp[v] = 0.5f * narrow_bits(t + D);
       } else {
-        dm[v] = dp[v] = 0.5f * (float)t;
+        dm[v] = dp[v] = 0.5f * narrow_bits(t);
       }
     }
   }
