@@ -138,8 +138,13 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
 // kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
 // flux (the update takes half its factor: one FP64 instruction less a variable)
 template <class Sys, class T, bool kRcp = false>
-__device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const T* QR, int d, T* F, T* D) {
+__device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const typename Sys::FConst& fcs, const T* QL, const T* QR,
+                                          int d, T* F, T* D) {
   constexpr int V = Sys::V;
+  if constexpr (kRcp && Sys::ID == kSysBN) {
+    BNSys::rusanov_mixed(pc, fcs, QL, QR, d, F, D);
+    return;
+  }
   T FLf[2 * V], FRf[2 * V], smax;
   if constexpr (kRcp) {
     // the flux along d only (the other direction's would be multiplied by 0)
@@ -160,8 +165,7 @@ __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const T* QL, const
       F[v] = T(0.5) * ((FLf[v] + FRf[v]) * nv0 + (FLf[V + v] + FRf[V + v]) * nv1) - T(0.5) * smax * (QR[v] - QL[v]);
   }
   if constexpr (Sys::ID == kSysBN) {
-    if constexpr (kRcp) BNSys::roe_times_jump_r(pc, QL, QR, d, D);
-    else BNSys::roe_times_jump(pc, QL, QR, d, D);
+    BNSys::roe_times_jump(pc, QL, QR, d, D);
   }
 }
 
@@ -277,6 +281,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     const InstState& st = a.st[k];
     const Phys ph = in.ph;
     const PhysC<T> pc(ph);
+    const typename Sys::FConst fcs(ph);
     const int par = parity(st);
     const long long lc = c - in.cell_base;
     const int ci = (int)(lc % in.imax), cj = (int)(lc / in.imax);
@@ -509,7 +514,8 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       flux(wr, 0, FR);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        if constexpr (BN) Qt[v] = src[v] - divx(FR[v] - FL[v]);
+        if (kRcp && BN && v == 8) Qt[v] = src[v];  // the volume fraction has no flux
+        else if constexpr (BN) Qt[v] = src[v] - divx(FR[v] - FL[v]);
         else Qt[v] = -divx(FR[v] - FL[v]);
         wLx[hx(v, ii, jj)] = wl[v];
         wRx[hx(v, ii, jj)] = wr[v];
@@ -525,7 +531,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       flux(wr, 1, FR);
 #pragma unroll
       for (int v = 0; v < V; ++v) {
-        Qt[v] = Qt[v] - divy(FR[V + v] - FL[V + v]);
+        if (!(kRcp && BN && v == 8)) Qt[v] = Qt[v] - divy(FR[V + v] - FL[V + v]);
         if constexpr (BN) slt[hx(v, ii, jj)] = Qt[v];
         wLx[hx(v, ii, jj)] = wLx[hx(v, ii, jj)] + T(0.5) * dt * Qt[v];
         wRx[hx(v, ii, jj)] = wRx[hx(v, ii, jj)] + T(0.5) * dt * Qt[v];
@@ -553,7 +559,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
           QL[v] = xd ? wRx[hx(v, ii - 1, jj)] : wRy[hx(v, ii, jj - 1)];
           QR[v] = xd ? wLx[hx(v, ii, jj)] : wLy[hx(v, ii, jj)];
         }
-        rusanov_s<Sys, T, kRcp>(pc, QL, QR, xd ? 0 : 1, F, Dd);
+        rusanov_s<Sys, T, kRcp>(pc, fcs, QL, QR, xd ? 0 : 1, F, Dd);
         T* dst = xd ? EX : EY;
 #pragma unroll
         for (int v = 0; v < V; ++v) dst[v * NE + q] = F[v];

@@ -96,6 +96,16 @@ __device__ __forceinline__ float narrow_bits(double x) {
   }
   return __uint_as_float(r | (hi & 0x80000000u));
 }
+// FP64 -> FP32 by truncation, for estimates: values below the normal range
+// give 0, beyond it (and infinities and NaNs) infinity.
+__device__ __forceinline__ float truncate_bits(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned a = hi & 0x7fffffffu;
+  unsigned r = __funnelshift_l(lo, a - (896u << 20), 3);
+  if (a < (897u << 20)) r = 0u;
+  if (a >= (1151u << 20)) r = 0x7f800000u;
+  return __uint_as_float(r | (hi & 0x80000000u));
+}
 template <class T, class R> __device__ __forceinline__ T widen(R x) {
   if constexpr (sizeof(T) == 8 && sizeof(R) == 4) return widen_bits(x);
   else return (T)x;
@@ -553,14 +563,12 @@ struct BNSys {
     ex = tmax(tmax(tabs(u_g), tabs(u_g) + a_g), tmax(tabs(u_s), tabs(u_s) + a_s));
     ey = tmax(tmax(tabs(v_g), tabs(v_g) + a_g), tmax(tabs(v_s), tabs(v_s) + a_s));
   }
-  // maxval(abs(Lambda)) along d over two states, for FP32 states (widened on the
-  // integer pipe): FP32 estimates of the four speeds |u| + a with their error
-  // bounds, then the FP64 evaluation of those that may be the largest -- one or
-  // two of four, 19 FP64 instructions each.  A speed whose FP32 pressure is not
-  // settled (below 1e-3 of the terms it cancels) is always evaluated; a NaN is
-  // left out, as the maxima of max_eig_r do.
-  __device__ __forceinline__ static double max_speed(const PhysC<double>& pc, const FConst& fc, const float* qL,
-                                                     const float* qR, int d) {
+  // Which of the four speeds |u| + a of two states (bit k: k & 1 the gas, k >> 1
+  // the right state) may be the largest along d, from FP32 estimates and their
+  // error bounds.  A speed whose FP32 pressure is not settled (below 1e-3 of the
+  // terms it cancels) always may.  The states may carry the relative error of an
+  // FP32 truncation.
+  __device__ __forceinline__ static unsigned fastest(const FConst& fc, const float* qL, const float* qR, int d) {
     float hi[4], lo = 0.0f;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -583,6 +591,15 @@ struct BNSys {
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (hi[k] >= lo) cand |= 1u << k;
+    return cand;
+  }
+  // maxval(abs(Lambda)) along d over two FP32 states (widened on the integer
+  // pipe): the FP64 evaluation of the one or two of four speeds that may be the
+  // largest, 19 FP64 instructions each; a NaN is left out, as the maxima of
+  // max_eig_r do.
+  __device__ __forceinline__ static double max_speed(const PhysC<double>& pc, const FConst& fc, const float* qL,
+                                                     const float* qR, int d) {
+    unsigned cand = fastest(fc, qL, qR, d);
     // each lane takes its own candidates in turn (a branch per speed was turned
     // into predicated instructions, which the FP64 pipe issued all the same)
     long long best = -1;  // bits of the largest (>= 0)
@@ -665,6 +682,69 @@ struct BNSys {
     D[6] = d == 1 ? bp * dq9 : T(0);
     D[7] = bpu * dq9;
     D[8] = bu * dq9;
+  }
+  // Twice the Rusanov flux along d of two FP64 states and the fluctuation (its
+  // components along d and 3, 7, 8; the others are zero), for the FP64 subcell
+  // re-solve: fluxes with one reciprocal a state, the sound speeds of the one or
+  // two speeds that may be the largest, the path integrals with the jumps shared.
+  __device__ __forceinline__ static void rusanov_mixed(const PhysC<double>& pc, const FConst& fc, const double* QL,
+                                                       const double* QR, int d, double* F, double* D) {
+    float fl[9], fr[9];
+#pragma unroll
+    for (int v = 0; v < 9; ++v) {
+      fl[v] = truncate_bits(QL[v]);
+      fr[v] = truncate_bits(QR[v]);
+    }
+    unsigned cand = fastest(fc, fl, fr, d);
+    double jump[9], un[4], aa[4];  // |u| and a^2 of the four speeds
+#pragma unroll
+    for (int v = 0; v < 9; ++v) jump[v] = QR[v] - QL[v];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const double* Q = k == 0 ? QL : QR;
+      const double r = mrcp<double>(Q[0] * Q[4]);
+      const double i0 = Q[4] * r, i4 = Q[0] * r;
+      const double u_s = Q[1] * i0, v_s = Q[2] * i0, u_g = Q[5] * i4, v_g = Q[6] * i4;
+      const double phi_s = Q[8], phi_g = 1.0 - Q[8];
+      const double pps = pc.gs1 * (Q[3] - 0.5 * (Q[1] * u_s + Q[2] * v_s)) - pc.gsps * phi_s;
+      const double ppg = pc.gg1 * (Q[7] - 0.5 * (Q[5] * u_g + Q[6] * v_g)) - pc.ggpg * phi_g;
+      const double us = d == 0 ? u_s : v_s, ug = d == 0 ? u_g : v_g;
+      const double f[8] = {d == 0 ? Q[1] : Q[2], Q[1] * us + (d == 0 ? pps : 0.0), Q[2] * us + (d == 1 ? pps : 0.0),
+                           us * (Q[3] + pps),    d == 0 ? Q[5] : Q[6],             Q[5] * ug + (d == 0 ? ppg : 0.0),
+                           Q[6] * ug + (d == 1 ? ppg : 0.0), ug * (Q[7] + ppg)};
+#pragma unroll
+      for (int v = 0; v < 8; ++v) F[v] = k == 0 ? f[v] : F[v] + f[v];
+      un[2 * k] = us;
+      un[2 * k + 1] = ug;
+      // gamma (phi p + pi phi) / (phi rho)
+      aa[2 * k] = (pps + pc.ps * phi_s) * i0;
+      aa[2 * k + 1] = (ppg + pc.pg * phi_g) * i4;
+    }
+    long long best = -1;
+#pragma unroll 1
+    do {
+      const int k = __ffs(cand) - 1;
+      cand &= cand - 1u;
+      const double a2 = k == 0 ? aa[0] : k == 1 ? aa[1] : k == 2 ? aa[2] : aa[3];
+      const double u = k == 0 ? un[0] : k == 1 ? un[1] : k == 2 ? un[2] : un[3];
+      const double s = fabs(u) + msqrt<double>(((k & 1) ? pc.gg : pc.gs) * a2);
+      if (!is_nan_bits(s)) best = max(best, __double_as_longlong(s));
+    } while (cand);
+    const double smax = __longlong_as_double(best < 0 ? 0x7ff8000000000000LL : best);
+#pragma unroll
+    for (int v = 0; v < 8; ++v) F[v] = F[v] - smax * jump[v];
+    F[8] = -smax * jump[8];
+    double bp, bu, bpu;
+    path_integrals(pc, QL, jump, d, bp, bu, bpu);
+    const double x = bp * jump[8];
+    D[0] = D[4] = 0.0;
+    D[1] = d == 0 ? -x : 0.0;
+    D[2] = d == 1 ? -x : 0.0;
+    D[3] = -(bpu * jump[8]);
+    D[5] = d == 0 ? x : 0.0;
+    D[6] = d == 1 ? x : 0.0;
+    D[7] = bpu * jump[8];
+    D[8] = bu * jump[8];
   }
   // Path integrals of p_g, u_n and p_g u_n along QL + s jump (3-point
   // Gauss-Legendre), the entries of the Roe matrix's column 9
