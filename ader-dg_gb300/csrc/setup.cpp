@@ -172,6 +172,8 @@ Dd operator/(Dd a, Dd b) {
   return Dd(q0, q1) + Dd(r.h / b.h);
 }
 
+}  // namespace
+
 // HostOps::Fine from the FP64 nodes and iK1: Newton steps on the Legendre
 // polynomial and on the inverse.
 void build_fine(HostOps& o) {
@@ -258,8 +260,6 @@ void build_fine(HostOps& o) {
   split(ts, o.fTs);
 }
 
-}  // namespace
-
 double pi_value() { return kPi; }
 
 double pnpm_cfl(int N) {
@@ -320,8 +320,6 @@ bool build_ops(int N, HostOps& o, std::string* err) {
   }
   o.K1 = K1.a;
   o.iK1 = iK1.a;
-
-  build_fine(o);
 
   // subcell limiter maps (Euler/initialize.f90:171-213)
   Mat U(S, P);
