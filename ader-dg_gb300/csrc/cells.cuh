@@ -59,9 +59,48 @@ struct Proj {
     else if constexpr (sizeof(T) == 8) return __dadd_rn(acc, __dmul_rn(a, b));
     else return acc + a * b;
   }
+  // T = float: U, LY and LB hold items of V values, four to a float4 in a plane
+  // of its own, the rest one to a plane (bases on 16 bytes): a load or store per
+  // four values, where one word each made the passes wait on shared memory.
+  // Rows of LY and LB are PS = P | 1 items apart, which leaves no bank conflict.
+  static constexpr int PS = P | 1, NU = P2, NLY = S * PS, NLB = P * PS;
+  static constexpr int UF = (V * NU + 3) / 4 * 4, LYF = (V * NLY + 3) / 4 * 4, LBF = (V * NLB + 3) / 4 * 4;
+  template <int n>
+  __device__ __forceinline__ static void ld(const float* b, int item, float* o) {
+#pragma unroll
+    for (int q = 0; q < V / 4; ++q) load_v<4>(b + 4 * (q * n + item), o + 4 * q);
+#pragma unroll
+    for (int v = V / 4 * 4; v < V; ++v) o[v] = b[v * n + item];
+  }
+  template <int n>
+  __device__ __forceinline__ static void st(float* b, int item, const float* x) {
+#pragma unroll
+    for (int q = 0; q < V / 4; ++q) store_v<4>(b + 4 * (q * n + item), x + 4 * q);
+#pragma unroll
+    for (int v = V / 4 * 4; v < V; ++v) b[v * n + item] = x[v];
+  }
   // y pass: LY[v][s][i] = sum_k U[v][i + P k] uh2lim(s,k); LB[v][s][i] likewise with uh2lob
   template <bool kFast = false>
   __device__ static void ypass(const T* U, T* LY, T* LB, const T* lim, const T* lob, int r, int nr) {
+    if constexpr (sizeof(T) == 4) {
+      for (int idx = r; idx < P * (S + P); idx += nr) {
+        const int ii = idx % P, s = idx / P;
+        float acc[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < P; ++k) {
+          const float c = s < S ? lim[s + S * k] : lob[s - S + P * k];
+          float x[V];
+          ld<NU>(U, ii + P * k, x);
+#pragma unroll
+          for (int v = 0; v < V; ++v) acc[v] = fmaf(x[v], c, acc[v]);
+        }
+        if (s < S) st<NLY>(LY, s * PS + ii, acc);
+        else st<NLB>(LB, (s - S) * PS + ii, acc);
+      }
+      return;
+    }
     for (int idx = r; idx < P * S; idx += nr) {
       const int ii = idx % P, s = idx / P;
 #pragma unroll
@@ -83,9 +122,27 @@ struct Proj {
       }
     }
   }
+  // T = float: sum over k of item (s2, k) times c[k * stride]
+  template <int n>
+  __device__ __forceinline__ static void row(const float* L, const float* c, int stride, int s2, float* out) {
+#pragma unroll
+    for (int v = 0; v < V; ++v) out[v] = 0.0f;
+#pragma unroll
+    for (int k = 0; k < P; ++k) {
+      const float ck = c[stride * k];
+      float x[V];
+      ld<n>(L, s2 * PS + k, x);
+#pragma unroll
+      for (int v = 0; v < V; ++v) out[v] = fmaf(x[v], ck, out[v]);
+    }
+  }
   // subcell value (s1, s2) from the y pass
   template <bool kFast = false>
   __device__ static void subcell(const T* LY, const T* lim, int s1, int s2, T* out) {
+    if constexpr (sizeof(T) == 4) {
+      row<NLY>(LY, lim + s1, S, s2, out);
+      return;
+    }
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       T acc = 0;
@@ -96,6 +153,10 @@ struct Proj {
   }
   template <bool kFast = false>
   __device__ static void lobatto(const T* LB, const T* lob, int s1, int s2, T* out) {
+    if constexpr (sizeof(T) == 4) {
+      row<NLB>(LB, lob + s1, P, s2, out);
+      return;
+    }
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       T acc = 0;
@@ -211,20 +272,21 @@ struct Proj {
 #pragma unroll
       for (int k = 0; k < P; ++k) c[q][k] = o < S ? lim[o + S * k] : o < S + P ? lob[o - S + P * k] : 0.0f;
     }
+    float x[P][V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      float x[P];
+    for (int k = 0; k < P; ++k) ld<NU>(U, ii + P * k, x[k]);
 #pragma unroll
-      for (int k = 0; k < P; ++k) x[k] = U[v * P2 + ii + P * k];
+    for (int q = 0; q < NO; ++q) {
+      const int o = o0 + q * P;
+      float acc[V];
 #pragma unroll
-      for (int q = 0; q < NO; ++q) {
-        const int o = o0 + q * P;
-        float acc = 0.0f;
+      for (int v = 0; v < V; ++v) {
+        acc[v] = 0.0f;
 #pragma unroll
-        for (int k = 0; k < P; ++k) acc = fmaf(x[k], c[q][k], acc);
-        if (o < S) LY[(v * S + o) * P + ii] = acc;
-        else if (o < S + P) LB[(v * P + o - S) * P + ii] = acc;
+        for (int k = 0; k < P; ++k) acc[v] = fmaf(x[k][v], c[q][k], acc[v]);
       }
+      if (o < S) st<NLY>(LY, o * PS + ii, acc);
+      else if (o < S + P) st<NLB>(LB, (o - S) * PS + ii, acc);
     }
   }
   template <class Sys>
@@ -237,13 +299,11 @@ struct Proj {
     float val[V];
     if (r < C * S) {
       const int s2 = r / C, c0 = r - s2 * C;
-      float e[V], ly[V][P];
+      float e[V], ly[P][V];
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        e[v] = err[v] + 2.5e-7f * fabsf(ubf[v]);
+      for (int v = 0; v < V; ++v) e[v] = err[v] + 2.5e-7f * fabsf(ubf[v]);
 #pragma unroll
-        for (int k = 0; k < P; ++k) ly[v][k] = LY[(v * S + s2) * P + k];
-      }
+      for (int k = 0; k < P; ++k) ld<NLY>(LY, s2 * PS + k, ly[k]);
       unsigned open = 0u;  // bit q: the chunk's q-th subcell needs the FP64 test
 #pragma unroll 1
       for (int q = 0; q < CH; ++q) {
@@ -256,7 +316,7 @@ struct Proj {
         for (int v = 0; v < V; ++v) {
           float acc = 0.0f;
 #pragma unroll
-          for (int k = 0; k < P; ++k) acc = fmaf(ly[v][k], c[k], acc);
+          for (int k = 0; k < P; ++k) acc = fmaf(ly[k][v], c[k], acc);
           mn[v] = fminf(mn[v], acc);
           mx[v] = fmaxf(mx[v], acc);
           qv[v] = ubf[v] + acc;
@@ -368,19 +428,30 @@ struct CellCfg {
   static constexpr int CPB = (CTA / P2) < 1 ? 1 : (CTA / P2);
   static constexpr int THREADS = ((CPB * P2 + 31) / 32) * 32;
   // per cell: U [V][P2], LY [V][S][P], LB [V][P][P], red [2][V][P2] (FP64);
-  // FP32-mixed: U64 [V][P2] then FP32 U [V][P2], LY, LB, red, |U| max [V]
-  // in the same room
-  static constexpr int CELL_DBL = V * P2 + V * S * P + V * P * P + 2 * V * P2;
-  static_assert(8 * V * P2 + 4 * (3 * V * P2 + V * S * P + V * P * P) <= 8 * CELL_DBL, "FP32 cell layout");
+  // the FP32 projections: U64 [V][P2] then FP32 U, LY, LB (Proj's items) and red
+  // [P2][2 V] in the same room, every part on 16 bytes.  Cells of a warp
+  // segment start 64 bytes apart modulo the banks' 128, so that the segments'
+  // accesses do not meet.
+  using PF = Proj<N, V, float>;
+  static constexpr int U_DBL = (V * P2 + 1) / 2 * 2, RED_F = U_DBL * 2 + PF::UF + PF::LYF + PF::LBF;
+  static constexpr int CELL_RAW = U_DBL + V * S * P + V * P * P + 2 * V * P2;
+  static constexpr int CELL_DBL = P2 == 16 ? (CELL_RAW + 7) / 16 * 16 + 8 : (CELL_RAW + 1) / 2 * 2;
+  static_assert(CELL_DBL >= CELL_RAW && 4 * (RED_F + 2 * V * P2) <= 8 * CELL_DBL, "FP32 cell layout");
   static constexpr int OPS_DBL = S * P + P * P;  // uh2lim, uh2lob (FP64, then FP32 in the FP32 modes)
   static constexpr int SMEM_BYTES = CPB * CELL_DBL * 8 + OPS_DBL * 12 + CPB * 8 /*cell max*/ + CPB * 4 /*flags*/ +
                                     CPB * V * 4 /*|U| max*/ + CPB * V * 4 /*FP32 reference state*/ +
                                     CPB * 4 /*instances*/ + 16;
-  // (cell, variable) pairs of the DMP comparison per thread: consecutive
-  // threads take them, so that they fill whole warps (with the pairs of a cell
-  // on its own first V threads every warp issued the comparison's FP64
-  // instructions for a few lanes: 2.5 of 6.8 FP64 slots per DOF)
-  static constexpr int NPAIR = (CPB * V + THREADS - 1) / THREADS;
+  // The DMP comparisons, (cell, variable) pairs on consecutive threads, so that
+  // they fill whole warps (with the pairs of a cell on its own first V threads
+  // every warp issued the comparison's FP64 instructions for a few lanes: 2.5 of
+  // 6.8 FP64 slots per DOF).  Euler, whose pairs leave lanes of a warp idle: the
+  // minimum and the maximum of a pair on neighbouring lanes (LPP = 2), which
+  // halves the serial part between barriers: N = 3 313 -> 281 us (Riemann problem
+  // 512^2), N = 4 144 -> 138 us, N = 5 291 -> 271 us; Baer-Nunziato's fill them:
+  // 410 -> 455 us (cylinder N = 3 400^2), so LPP = 1.
+  static constexpr int LPP = Sys::ID == kSysBN ? 1 : 2;          // lanes of a pair
+  static constexpr int SPL = 2 / LPP;                            // sides of a lane
+  static constexpr int NITEM = (LPP * CPB * V + THREADS - 1) / THREADS;
   // blocks per SM the register allocation aims at, in 256-thread units:
   // Euler's FP32-mixed cell kernel is latency-bound and gains from a fourth;
   // the other variants keep the allocation they reach unconstrained
@@ -407,10 +478,13 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   using C = CellCfg<Sys, N, VAR>;
   constexpr int P = N + 1, P2 = P * P, S = 2 * N + 1, V = Sys::V, CPB = C::CPB;
   constexpr bool kF32 = kFast && !kExact;  // FP32 storage and update
-  // the team passes where they are faster (measured): N = 3, 344 -> 328 us on the
-  // Riemann problem 512^2; at N = 4 their chunks leave a quarter of the lanes idle
-  // (156 -> 170 us on the vortex), at N = 5 and 2 they cost 7% and 6%
-  constexpr bool kTeam = P == 4;
+  // the team passes where they are faster (measured): Euler N = 3, 344 -> 328 us
+  // on the Riemann problem 512^2; at N = 4 their chunks leave a quarter of the
+  // lanes idle (156 -> 170 us on the vortex), at N = 5 and 2 they cost 7% and 6%.
+  // Baer-Nunziato N = 3 gains 2% on the 400^2 cylinder, but a chunk's subcells
+  // that need the FP64 test follow one another on one thread: 92 -> 137 us on a
+  // 281 x 103 cylinder in its first steps
+  constexpr bool kTeam = P == 4 && V == 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   double* sm = reinterpret_cast<double*>(smem_raw);
   double* opsm = sm + CPB * C::CELL_DBL;
@@ -440,43 +514,56 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   if (!__syncthreads_or(act)) return;  // nothing to do in this CTA
   const int par = parity(st);
   const long long lcell = cell - in.cell_base;
-  const int ci = valid ? (int)(lcell % in.imax) : 0, cj = valid ? (int)(lcell / in.imax) : 0;
+  const int ci = valid ? (int)((unsigned)lcell % (unsigned)in.imax) : 0, cj = valid ? (int)((unsigned)lcell / (unsigned)in.imax) : 0;
   const bool limiter = Sys::ID != kSysAD && a.mm[0] != nullptr;
   double* U = sm + (size_t)(in_cta ? lc : 0) * C::CELL_DBL;
-  double* LY = U + V * P2;
+  double* LY = U + C::U_DBL;
   double* LB = LY + V * S * P;
   double* RED = LB + V * P * P;
-  // FP32-mixed views of the same room
-  float* Uf = reinterpret_cast<float*>(U + V * P2);
-  float* LYf = Uf + V * P2;
-  float* LBf = LYf + V * S * P;
-  float* REDf = LBf + V * P * P;
+  // FP32 views of the same room
+  using PF = typename C::PF;
+  float* Uf = reinterpret_cast<float*>(U + C::U_DBL);
+  float* LYf = Uf + PF::UF;
+  float* LBf = LYf + PF::LYF;
+  float* REDf = LBf + PF::LBF;
   unsigned* amax = amax_all + (in_cta ? lc : 0) * V;
   float* ubs = ubs_all + (in_cta ? lc : 0) * V;
 
-  // DMP neighbourhood bounds (get_min_max step 2, Euler/limiter.f90:147-167):
-  // the thread of a (cell, variable) pair folds the cell's 3x3 Voronoi
-  // neighbourhood now, so the global loads overlap the update and the
-  // projections
-  double nlmin[C::NPAIR], nlmax[C::NPAIR];
-  float nen[C::NPAIR];  // largest error bound of the folded min/max
+  // DMP neighbourhood bounds (get_min_max step 2, Euler/limiter.f90:147-167): the
+  // threads of a (cell, variable) pair fold the minimum (side 0) and the maximum
+  // (side 1) over the cell's 3x3 Voronoi neighbourhood now, so the global loads
+  // overlap the update and the projections
+  constexpr int LPP = C::LPP, SPL = C::SPL;
+  double nbound[C::NITEM][SPL];
+  float nen[C::NITEM];  // largest error bound of the folded min/max
   if (limiter && (mode == kCellFused || mode == kCellUpdate)) {
 #pragma unroll
-    for (int q = 0; q < C::NPAIR; ++q) {
-      const int pr = t + q * C::THREADS, lc2 = pr / V, v = pr - lc2 * V;
-      nlmin[q] = nlmax[q] = 0.0;
+    for (int q = 0; q < C::NITEM; ++q) {
+      const int it = t + q * C::THREADS, pr = it / LPP, lc2 = pr / V, v = pr - lc2 * V;
+#pragma unroll
+      for (int s = 0; s < SPL; ++s) nbound[q][s] = 0.0;
       nen[q] = 0.0f;
       const int k2 = pr < CPB * V ? cinst[lc2] : -1;
       if (k2 < 0) continue;
       const InstDesc& in2 = a.inst[k2];
       const int par2 = parity(a.st[k2]);
-      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2, l2 = cell2 - in2.cell_base;
-      const int ci2 = (int)(l2 % in2.imax), cj2 = (int)(l2 / in2.imax);
-      const double* mmi = a.mm[par2];
+      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2;
+      const unsigned l2 = (unsigned)(cell2 - in2.cell_base);  // an instance has below 2^31 cells
+      const int ci2 = (int)(l2 % (unsigned)in2.imax), cj2 = (int)(l2 / (unsigned)in2.imax);
+      const int side0 = LPP == 2 ? it & 1 : 0;
+      const double* mmi = a.mm[par2] + side0 * V + v;
       const float* mei = a.mme[par2];
-      // integer-key min/max (the integer pipe, not FP64) in the fast kernels
-      double lo = mmi[(size_t)cell2 * 2 * V + v], hi = mmi[(size_t)cell2 * 2 * V + V + v];
-      long long klo = okey(lo), khi = okey(hi);
+      // the maximum as the minimum of the negated values (fast kernels: of the
+      // complemented integer keys, on the integer pipe, not FP64)
+      double b[SPL];
+      long long kb[SPL], kx[SPL];
+#pragma unroll
+      for (int s = 0; s < SPL; ++s) {
+        kx[s] = -(long long)(side0 + s);
+        const double x = mmi[(size_t)cell2 * 2 * V + s * V];
+        b[s] = kx[s] ? -x : x;
+        kb[s] = okey(x) ^ kx[s];
+      }
       float en = 0.0f;
 #pragma unroll
       for (int jj = -1; jj <= 1; ++jj)
@@ -485,18 +572,16 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const int in_ = nb_index(ci2, ii, in2.imax, in2.bc[0], in2.bc[1]);
           const int jn_ = nb_index(cj2, jj, in2.jmax, in2.bc[2], in2.bc[3]);
           const long long nc = in2.cell_base + in_ + (long long)in2.imax * jn_;
-          const double a_lo = mmi[(size_t)nc * 2 * V + v], a_hi = mmi[(size_t)nc * 2 * V + V + v];
-          if constexpr (kFast) {
-            klo = min(klo, okey(a_lo));
-            khi = max(khi, okey(a_hi));
-          } else {
-            lo = fmin(lo, a_lo);
-            hi = fmax(hi, a_hi);
+#pragma unroll
+          for (int s = 0; s < SPL; ++s) {
+            const double x = mmi[(size_t)nc * 2 * V + s * V];
+            if constexpr (kFast) kb[s] = min(kb[s], okey(x) ^ kx[s]);
+            else b[s] = fmin(b[s], kx[s] ? -x : x);
           }
           if (mei) en = fmaxf(en, mei[(size_t)nc * V + v]);
         }
-      nlmin[q] = kFast ? okey_inv(klo) : lo;
-      nlmax[q] = kFast ? okey_inv(khi) : hi;
+#pragma unroll
+      for (int s = 0; s < SPL; ++s) nbound[q][s] = kFast ? okey_inv(kb[s] ^ kx[s]) : (kx[s] ? -b[s] : b[s]);
       nen[q] = en;
     }
   }
@@ -539,38 +624,37 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         const float* YB = reinterpret_cast<const float*>(a.gu);
         const float* YT = reinterpret_cast<const float*>((Sys::ID == kSysBN) ? a.gp : a.gu);
         float d[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) d[v] = D32[off + v];
+        load_v<V>(D32 + off, d);
         if (mode != kCellUpdate) {
           const float cxf = op.wf[j] * in.idxf, cyf = op.wf[i] * in.idyf;
+          float fl[V], fr[V], gb[V], gt[V];
+          load_v<V>(XL + ((size_t)fxl * P + j) * V, fl);
+          load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, fr);
+          load_v<V>(YB + ((size_t)fyb * P + i) * V, gb);
+          load_v<V>(YT + ((size_t)fyt * P + i) * V, gt);
 #pragma unroll
           for (int v = 0; v < V; ++v) {
-            const float fl = XL[((size_t)fxl * P + j) * V + v], fr = XR[((size_t)(fxl + 1) * P + j) * V + v];
-            const float gb = YB[((size_t)fyb * P + i) * V + v], gt = YT[((size_t)fyt * P + i) * V + v];
-            const float sx = fr * op.FRf[i] - fl * op.FLf[i];
-            const float sy = gt * op.FRf[j] - gb * op.FLf[j];
+            const float sx = fr[v] * op.FRf[i] - fl[v] * op.FLf[i];
+            const float sy = gt[v] * op.FRf[j] - gb[v] * op.FLf[j];
             d[v] = d[v] - (cxf * sx + cyf * sy);
           }
         }
         if (mode == kCellSurface) {
           float* D32w = reinterpret_cast<float*>(a.duh);
-#pragma unroll
-          for (int v = 0; v < V; ++v) D32w[off + v] = d[v];
+          store_v<V>(D32w + off, d);
         } else {
           const double dt = st.dt;
           const double* uo = a.uh[par] + off;
           double* un = a.uh[par ^ 1] + off;
           const float iw = op.iwwf[i + P * j];
+          load_v<V>(uo, u);
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            u[v] = fma(dt, (double)(d[v] * iw), uo[v]);
-            un[v] = u[v];
-          }
+          for (int v = 0; v < V; ++v) u[v] = fma(dt, (double)(d[v] * iw), u[v]);
+          store_v<V>(un, u);
         }
       } else {
-        double d[V];
-#pragma unroll
-        for (int v = 0; v < V; ++v) d[v] = a.duh[off + v];
+        double d[V], p[V], q[V];
+        load_v<V>(a.duh + off, d);
         if (mode != kCellUpdate) {
           // surface_integral.f90:20-35: x faces then y faces
           const double* XL = a.fu;
@@ -578,36 +662,33 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const double* YB = a.gu;
           const double* YT = (Sys::ID == kSysBN) ? a.gp : a.gu;
           const double cx = in.wdx[j], cy = in.wdy[i];  // w_j / dx, w_i / dy
+          load_v<V>(XL + ((size_t)fxl * P + j) * V, p);
+          load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, q);
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            const double fl = XL[((size_t)fxl * P + j) * V + v], fr = XR[((size_t)(fxl + 1) * P + j) * V + v];
-            d[v] = d[v] - cx * (fr * op.FRd[i] - fl * op.FLd[i]);
-          }
+          for (int v = 0; v < V; ++v) d[v] = d[v] - cx * (q[v] * op.FRd[i] - p[v] * op.FLd[i]);
+          load_v<V>(YB + ((size_t)fyb * P + i) * V, p);
+          load_v<V>(YT + ((size_t)fyt * P + i) * V, q);
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            const double gb = YB[((size_t)fyb * P + i) * V + v], gt = YT[((size_t)fyt * P + i) * V + v];
-            d[v] = d[v] - cy * (gt * op.FRd[j] - gb * op.FLd[j]);
-          }
+          for (int v = 0; v < V; ++v) d[v] = d[v] - cy * (q[v] * op.FRd[j] - p[v] * op.FLd[j]);
         }
         if (mode == kCellSurface) {
-#pragma unroll
-          for (int v = 0; v < V; ++v) a.duh[off + v] = d[v];
+          store_v<V>(a.duh + off, d);
         } else {
           // element_update.f90:18-26
           const double dt = st.dt;
           const double* uo = a.uh[par] + off;
           double* un = a.uh[par ^ 1] + off;
+          load_v<V>(uo, p);
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             d[v] = div_by(d[v], op.wd[i] * op.wd[j], op.iwwd[i + P * j]);
-            u[v] = uo[v] + dt * d[v];
-            un[v] = u[v];
+            u[v] = p[v] + dt * d[v];
           }
+          store_v<V>(un, u);
         }
       }
     } else {
-#pragma unroll
-      for (int v = 0; v < V; ++v) u[v] = a.uh[par][off + v];
+      load_v<V>(a.uh[par] + off, u);
     }
   }
   if (mode == kCellSurface) return;  // uniform per launch: no barrier follows
@@ -630,6 +711,11 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   const bool want_cfl = mode != kCellInitDmp && mode != kCellPrimeLimited;
   // cells as aligned warp segments: per-cell maxima by shuffles, one store per
   // cell instead of P2 atomics on one shared address
+  // warp reductions ahead of the atomics on |du|: Euler N = 4 150 -> 144 us (vortex
+  // 256^2), N = 5 301 -> 291 us; Baer-Nunziato N = 2 342 -> 379 us (nine reductions
+  // of four groups each)
+  constexpr bool kRedux = P2 > 16 && V <= 4;
+  // (advection-diffusion's denominator is the instance's constant, folded below)
   constexpr bool kSeg = (32 % P2) == 0 && (C::THREADS % 32) == 0 && C::CPB * P2 == C::THREADS;
   if constexpr (kSeg && Sys::ID != kSysAD) {
     if (want_cfl) {
@@ -643,12 +729,25 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       bits = seg_max<P2>(bits);
       if (act && node == 0) cmax[lc] = bits;
     }
-  } else if (act && want_cfl) {
-    double dn;
-    if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
-    else dn = cfl_denom<Sys, N>(in, u);
-    // advection-diffusion: the denominator is the instance's constant, folded below
-    if constexpr (Sys::ID != kSysAD) atomicMax(&cmax[lc], (unsigned long long)__double_as_longlong(dn));
+  } else if constexpr (Sys::ID != kSysAD) {
+    if (want_cfl) {
+      unsigned long long bits = 0ull;
+      if (act) {
+        double dn;
+        if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+        else dn = cfl_denom<Sys, N>(in, u);
+        bits = (unsigned long long)__double_as_longlong(dn);
+      }
+      // the lanes of a cell within this warp by shuffles, then one atomic per
+      // cell and warp (every lane on its cell's address took turns)
+      const int lane = t & 31, rest = min(31 - lane, P2 - 1 - node);
+#pragma unroll
+      for (int o = 1; o < 32 && o < P2; o <<= 1) {
+        const unsigned long long y = __shfl_down_sync(0xffffffffu, bits, o);
+        if (o <= rest && y > bits) bits = y;
+      }
+      if (act && (lane == 0 || node == 0)) atomicMax(&cmax[lc], bits);
+    }
   }
 
   // ------------------------------------------------------------- DMP part
@@ -660,11 +759,21 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     if constexpr (kFast) {
       if (act) {
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-          U[v * P2 + node] = u[v];
-          Uf[v * P2 + node] = du[v];
-          if constexpr (!kSeg) atomicMax(&amax[v], __float_as_uint(fabsf(du[v])));
+        for (int v = 0; v < V; ++v) U[v * P2 + node] = u[v];
+        if constexpr (kRedux) {
+          // the lanes of a cell within this warp, then one atomic
+          const int lane = t & 31, first = max(lane - node, 0), last = min(lane + P2 - 1 - node, 31);
+          const unsigned m = (0xffffffffu >> (31 - last)) & (0xffffffffu << first);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const unsigned x = __reduce_max_sync(m, __float_as_uint(fabsf(du[v])));
+            if (lane == first) atomicMax(&amax[v], x);
+          }
+        } else if constexpr (!kSeg) {
+#pragma unroll
+          for (int v = 0; v < V; ++v) atomicMax(&amax[v], __float_as_uint(fabsf(du[v])));
         }
+        PF::template st<PF::NU>(Uf, node, du);
       }
       if constexpr (kSeg) {
         // du = 0 in lanes of inactive cells
@@ -722,11 +831,8 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
             Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, opsf, opsf + S * P, U, opsm,
                                                               typename Sys::FConst(in.ph), err, ubf, in.ph, node, P2,
                                                               mn, mx, posfail);
-#pragma unroll
-          for (int v = 0; v < V; ++v) {
-            REDf[v * P2 + node] = mn[v];
-            REDf[(V + v) * P2 + node] = mx[v];
-          }
+          store_v<V>(REDf + node * 2 * V, mn);
+          store_v<V>(REDf + node * 2 * V + V, mx);
         } else {
           double mn[V], mx[V];
 #pragma unroll
@@ -775,93 +881,131 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     }
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < C::NPAIR; ++q) {
-      const int pr = t + q * C::THREADS, lc2 = pr / V, v = pr - lc2 * V;
+    for (int q = 0; q < C::NITEM; ++q) {
+      const int it = t + q * C::THREADS, pr = it / LPP, lc2 = pr / V, v = pr - lc2 * V;
       const int k2 = pr < CPB * V ? cinst[lc2] : -1;
-      if (k2 < 0) continue;
-      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lc2;
-      const int par2 = parity(a.st[k2]);
-      const double* U2 = sm + (size_t)lc2 * C::CELL_DBL;
-      const double* RED2 = U2 + V * P2 + V * S * P + V * P * P;
-      const float* REDf2 = reinterpret_cast<const float*>(U2 + V * P2) + V * P2 + V * S * P + V * P * P;
-      const bool f32red = (cflag[lc2] & 8) != 0;
-      const float am = kFast ? __uint_as_float(amax_all[pr]) : 0.0f, ub32 = kFast ? ubs_all[pr] : 0.0f;
-      double cmn, cmx;
+      const bool on = k2 >= 0;
+      // LPP = 2: the lanes of a pair exchange their bounds, so the warp stays together
+      if (LPP == 2 ? !__any_sync(0xffffffffu, on) : !on) continue;
+      const int lcs = on ? lc2 : 0, prs = on ? pr : 0, side0 = LPP == 2 ? it & 1 : 0;
+      const long long cell2 = a.cell0 + (long long)blockIdx.x * CPB + lcs;
+      const int par2 = on ? parity(a.st[k2]) : 0;
+      const double* U2 = sm + (size_t)lcs * C::CELL_DBL;
+      const bool f32red = (cflag[lcs] & 8) != 0;
+      const float am = kFast ? __uint_as_float(amax_all[prs]) : 0.0f, ub32 = kFast ? ubs_all[prs] : 0.0f;
       const double ubar = kFast ? (double)ub32 : 0.0;  // the cell's FP32 reference state
-      // FP32 projections: the cell's deviation min/max from its FP32 reference
-      // state ubar, and a bound on |ubar + fmn - FP64 value| (and fmx): the
-      // projections' bound as formed above (rounded up), plus the FP64
-      // roundings of the reference-order values (generously 1e-12 relative)
-      float fmn = 0.0f, fmx = 0.0f, ecell = 0.0f;
-      if (f32red) {
-        fmn = REDf2[v * P2];
-        fmx = REDf2[(V + v) * P2];
+      // the cell's minimum and maximum.  FP32 projections: their deviations fx
+      // from the cell's FP32 reference state ubar, and a bound on |ubar + fx -
+      // FP64 value|: the projections' bound as formed above (rounded up), plus
+      // the FP64 roundings of the reference-order values (generously 1e-12
+      // relative)
+      double cm[SPL], bound[SPL];  // own value; lmin or lmax
+      float fx[SPL], en = 0.0f;
+      const float ecell = !f32red ? 0.0f
+                                  : (op.perr * am + op.pdev * (fabsf(ub32) + 2.0f * am)) * 1.0001f +
+                                        1.0e-12f * (fabsf(ub32) + am);
 #pragma unroll
-        for (int k = 1; k < P2; ++k) { fmn = fminf(fmn, REDf2[v * P2 + k]); fmx = fmaxf(fmx, REDf2[(V + v) * P2 + k]); }
-        cmn = ubar + (double)fmn;
-        cmx = ubar + (double)fmx;
-        ecell = (op.perr * am + op.pdev * (fabsf(ub32) + 2.0f * am)) * 1.0001f + 1.0e-12f * (fabsf(ub32) + am);
-      } else {
-        cmn = RED2[v * P2];
-        cmx = RED2[(V + v) * P2];
-#pragma unroll
-        for (int k = 1; k < P2; ++k) { cmn = fmin(cmn, RED2[v * P2 + k]); cmx = fmax(cmx, RED2[(V + v) * P2 + k]); }
+      for (int s = 0; s < SPL; ++s) {
+        cm[s] = 0.0;
+        fx[s] = 0.0f;
       }
-      if (mode == kCellPrime || mode == kCellPrimeLimited) {
-        a.mm[par2][(size_t)cell2 * 2 * V + v] = cmn;
-        a.mm[par2][(size_t)cell2 * 2 * V + V + v] = cmx;
-        if (a.mme[0]) a.mme[par2][(size_t)cell2 * V + v] = ecell;
-      } else {
-        double lmin, lmax, argmax;
-        float en = 0.0f;
-        if (mode == kCellInitDmp) {
+      if (on && f32red) {
+        const float* r = reinterpret_cast<const float*>(U2) + C::RED_F + side0 * V + v;
+#pragma unroll
+        for (int k = 0; k < P2; ++k)
+#pragma unroll
+          for (int s = 0; s < SPL; ++s) {
+            const float x = side0 + s ? -r[k * 2 * V + s * V] : r[k * 2 * V + s * V];
+            fx[s] = k == 0 ? x : fminf(fx[s], x);
+          }
+#pragma unroll
+        for (int s = 0; s < SPL; ++s) {
+          fx[s] = side0 + s ? -fx[s] : fx[s];
+          cm[s] = ubar + (double)fx[s];
+        }
+      } else if (on) {
+#pragma unroll
+        for (int s = 0; s < SPL; ++s) {
+          const double* r = U2 + C::U_DBL + V * S * P + V * P * P + ((side0 + s) * V + v) * P2;
+          double x = side0 + s ? -r[0] : r[0];
+#pragma unroll
+          for (int k = 1; k < P2; ++k) x = fmin(x, side0 + s ? -r[k] : r[k]);
+          cm[s] = side0 + s ? -x : x;
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < SPL; ++s) {
+        const int side = side0 + s;
+        bound[s] = 0.0;
+        if (mode == kCellPrime || mode == kCellPrimeLimited) {
+          if (on) {
+            a.mm[par2][((size_t)cell2 * 2 + side) * V + v] = cm[s];
+            if (a.mme[0] && side == 0) a.mme[par2][(size_t)cell2 * V + v] = ecell;
+          }
+        } else if (mode == kCellInitDmp) {
           // Euler/initialize.f90:291-294: the cell's own nodal min/max
-          lmin = U2[v * P2];
-          lmax = U2[v * P2];
-          for (int k = 1; k < P2; ++k) { lmin = fmin(lmin, U2[v * P2 + k]); lmax = fmax(lmax, U2[v * P2 + k]); }
-          argmax = 1.0e-1;
+          const double* Uv = U2 + v * P2;
+          double x = side ? -Uv[0] : Uv[0];
+          for (int k = 1; k < P2; ++k) x = fmin(x, side ? -Uv[k] : Uv[k]);
+          bound[s] = side ? -x : x;
         } else {
           // get_min_max step 2: the neighbourhood bounds folded at the start
-          lmin = nlmin[q];
-          lmax = nlmax[q];
+          bound[s] = nbound[q][s];
           en = nen[q];
-          argmax = 0.0;
-          if (a.lminmax) {
-            a.lminmax[(size_t)cell2 * 2 * V + v] = lmin;
-            a.lminmax[(size_t)cell2 * 2 * V + V + v] = lmax;
+          if (on) {
+            if (a.lminmax) a.lminmax[((size_t)cell2 * 2 + side) * V + v] = bound[s];
+            // candidate min/max for the next step (status 0)
+            a.mm[par2 ^ 1][((size_t)cell2 * 2 + side) * V + v] = cm[s];
+            if (a.mme[0] && side == 0) a.mme[par2 ^ 1][(size_t)cell2 * V + v] = ecell;
           }
-          // candidate min/max for the next step (status 0)
-          a.mm[par2 ^ 1][(size_t)cell2 * 2 * V + v] = cmn;
-          a.mm[par2 ^ 1][(size_t)cell2 * 2 * V + V + v] = cmx;
-          if (a.mme[0]) a.mme[par2 ^ 1][(size_t)cell2 * V + v] = ecell;
         }
-        if (a.mme[0] == nullptr || (!f32red && en == 0.0f)) {
-          // FP64 values (FP32-wide mode: FP32 projections taken as they are);
-          // Euler/limiter.f90:210-220
-          const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (lmax - lmin)), argmax);
-          if (cmn < lmin - ldiff || cmx > lmax + ldiff) atomicOr(&cflag[lc2], 2);
-        } else {
-          // FP32-mixed: the same comparisons in FP32, in the deviation space
-          // of the cell's FP32 reference state ub (FP64 work is the costly
-          // part of this kernel).  |own - FP64 value| <= ecell; |lmin - its
-          // FP64 value| <= en and likewise lmax, so the thresholds move by at
-          // most en (1 + 2e-3); the FP32 forms of lmin - ub, lmax - ub, ldiff,
-          // the thresholds and the differences add at most 2.5e-7 of the
-          // magnitudes involved, and the FP32 constants 1e-4 and 0.1 differ
-          // from their FP64 values by less than 1e-11 and 1e-8 of themselves.
-          // A comparison decides here only when it holds by that margin;
-          // otherwise k_settle decides the cell from FP64 values (bit 4).
-          const double ub = ubar;
-          const float Lmin = (float)(lmin - ub), Lmax = (float)(lmax - ub);
-          const float ld = fmaxf(fmaxf(1.0e-4f, 1.0e-3f * (Lmax - Lmin)), mode == kCellInitDmp ? 0.1f : 0.0f);
-          const float dl = Lmin - ld, dh = Lmax + ld;
-          const float xl = f32red ? fmn : (float)(cmn - ub), xh = f32red ? fmx : (float)(cmx - ub);
-          const float e = ecell + 1.002f * en + 2.5e-7f * (fabsf(Lmin) + fabsf(Lmax) + ld) + 1.0e-11f +
-                          1.0e-12f * fabsf(ub32);
-          const float ml = e + 1.2e-7f * fabsf(xl), mh = e + 1.2e-7f * fabsf(xh);
-          const float gl = xl - dl, gh = dh - xh;  // >= 0: not below lmin - ldiff / not above lmax + ldiff
-          if (gl < -ml || gh < -mh) atomicOr(&cflag[lc2], 2);
-          else if (!(gl >= ml) || !(gh >= mh)) atomicOr(&cflag[lc2], 4);
+      }
+      if (mode == kCellPrime || mode == kCellPrimeLimited) continue;
+      const bool in64 = a.mme[0] == nullptr || (!f32red && en == 0.0f);
+      // (no warp vote where the mode decides)
+      if (a.mme[0] == nullptr || (LPP == 2 ? __any_sync(0xffffffffu, on && in64) : in64)) {
+        // FP64 values (FP32-wide mode: FP32 projections taken as they are);
+        // Euler/limiter.f90:210-220
+        double other = bound[SPL - 1];
+        if constexpr (LPP == 2) other = __shfl_xor_sync(0xffffffffu, bound[0], 1);
+        if (on && in64) {
+          const double lmin = side0 ? other : bound[0], lmax = side0 ? bound[0] : other;
+          const double ldiff = fmax(fmax(1.0e-4, 1.0e-3 * (lmax - lmin)), mode == kCellInitDmp ? 1.0e-1 : 0.0);
+#pragma unroll
+          for (int s = 0; s < SPL; ++s)
+            if (side0 + s ? cm[s] > lmax + ldiff : cm[s] < lmin - ldiff) atomicOr(&cflag[lc2], 2);
+        }
+      }
+      if (LPP == 2 ? a.mme[0] != nullptr : !in64) {
+        // FP32-mixed: the same comparisons in FP32, in the deviation space
+        // of the cell's FP32 reference state ub (FP64 work is the costly
+        // part of this kernel).  |own - FP64 value| <= ecell; |lmin - its
+        // FP64 value| <= en and likewise lmax, so the thresholds move by at
+        // most en (1 + 2e-3); the FP32 forms of lmin - ub, lmax - ub, ldiff,
+        // the thresholds and the differences add at most 2.5e-7 of the
+        // magnitudes involved, and the FP32 constants 1e-4 and 0.1 differ
+        // from their FP64 values by less than 1e-11 and 1e-8 of themselves.
+        // A comparison decides here only when it holds by that margin;
+        // otherwise k_settle decides the cell from FP64 values (bit 4).
+        float L[SPL];
+#pragma unroll
+        for (int s = 0; s < SPL; ++s) L[s] = (float)(bound[s] - ubar);
+        float other = L[SPL - 1];
+        if constexpr (LPP == 2) other = __shfl_xor_sync(0xffffffffu, L[0], 1);
+        const float ld = fmaxf(fmaxf(1.0e-4f, 1.0e-3f * (side0 ? L[0] - other : other - L[0])),
+                               mode == kCellInitDmp ? 0.1f : 0.0f);
+        const float e = ecell + 1.002f * en + 2.5e-7f * (fabsf(L[0]) + fabsf(other) + ld) + 1.0e-11f +
+                        1.0e-12f * fabsf(ub32);
+#pragma unroll
+        for (int s = 0; s < SPL; ++s) {
+          const float sg = side0 + s ? -1.0f : 1.0f;
+          const float x = f32red ? fx[s] : (float)(cm[s] - ubar);
+          const float m = e + 1.2e-7f * fabsf(x);
+          const float g = sg * (x - (L[s] - sg * ld));  // >= 0: not below lmin - ldiff / not above lmax + ldiff
+          if (LPP == 1 || (on && !in64)) {
+            if (g < -m) atomicOr(&cflag[lc2], 2);
+            else if (!(g >= m)) atomicOr(&cflag[lc2], 4);
+          }
         }
       }
     }

@@ -198,6 +198,47 @@ __device__ __forceinline__ int find_inst_cell(const InstDesc* inst, int n, long 
   return lo;
 }
 
+// The V consecutive values of a node or face point: 16-byte accesses where V
+// allows them (every such array is an allocation of its own, so that a node's
+// 4 values start on a 16-byte boundary)
+template <int V, class T>
+__device__ __forceinline__ void load_v(const T* p, T* o) {
+  if constexpr (V % 4 == 0 && sizeof(T) == 4) {
+#pragma unroll
+    for (int q = 0; q < V / 4; ++q) {
+      const float4 x = reinterpret_cast<const float4*>(p)[q];
+      o[4 * q] = x.x;
+      o[4 * q + 1] = x.y;
+      o[4 * q + 2] = x.z;
+      o[4 * q + 3] = x.w;
+    }
+  } else if constexpr (V % 2 == 0 && sizeof(T) == 8) {
+#pragma unroll
+    for (int q = 0; q < V / 2; ++q) {
+      const double2 x = reinterpret_cast<const double2*>(p)[q];
+      o[2 * q] = x.x;
+      o[2 * q + 1] = x.y;
+    }
+  } else {
+#pragma unroll
+    for (int v = 0; v < V; ++v) o[v] = p[v];
+  }
+}
+template <int V, class T>
+__device__ __forceinline__ void store_v(T* p, const T* x) {
+  if constexpr (V % 4 == 0 && sizeof(T) == 4) {
+#pragma unroll
+    for (int q = 0; q < V / 4; ++q)
+      reinterpret_cast<float4*>(p)[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+  } else if constexpr (V % 2 == 0 && sizeof(T) == 8) {
+#pragma unroll
+    for (int q = 0; q < V / 2; ++q) reinterpret_cast<double2*>(p)[q] = make_double2(x[2 * q], x[2 * q + 1]);
+  } else {
+#pragma unroll
+    for (int v = 0; v < V; ++v) p[v] = x[v];
+  }
+}
+
 __device__ __forceinline__ void atomic_max_pos(unsigned long long* addr, double v) {
   atomicMax(addr, (unsigned long long)__double_as_longlong(v));
 }

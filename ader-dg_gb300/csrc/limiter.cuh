@@ -30,7 +30,7 @@ __global__ void __launch_bounds__(256) k_mark(BatchArgs a) {
     const InstDesc& in = a.inst[k];
     const int par = parity(a.st[k]);
     const long long lc = c - in.cell_base;
-    const int ci = (int)(lc % in.imax), cj = (int)(lc / in.imax);
+    const int ci = (int)((unsigned)lc % (unsigned)in.imax), cj = (int)((unsigned)lc / (unsigned)in.imax);
     int rec = 0;
     if (a.troubled[c]) {
       rec = 1;
@@ -81,7 +81,7 @@ struct SubCfg {
   // bytes spilled, 8% and 2% faster than 3 unspilled; N = 4: 2; N = 5: 1), so
   // that the CTAs' phases without FP64 work (gather loads, barriers) overlap
   // other CTAs' arithmetic.
-  static constexpr int MIN_BLOCKS = sizeof(T) == 4 ? (Sys::ID == kSysBN ? (N == 3 ? 4 : N == 2 ? 5 : 1) : 6)
+  static constexpr int MIN_BLOCKS = sizeof(T) == 4 ? (Sys::ID == kSysBN ? (N == 3 ? 4 : N == 2 ? 5 : 3) : 6)
                                                    : (Sys::ID == kSysBN ? (N <= 3 ? 4 : N == 4 ? 2 : 1) : 4);
   static constexpr int NE = (S + 1) * S;               // x edges (and y edges) of the subgrid
   static constexpr int NEF = (Sys::ID == kSysBN ? 4 : 2) * V * NE;  // edge fluxes (+ BN fluctuations)
@@ -99,7 +99,8 @@ struct SubCfg {
   static constexpr int TSTATE = 4 * TW + (Sys::ID == kSysBN ? TW + 2 * H * H : 0);
   static_assert(9 * V * P2 + 9 * V * P * S <= TSTATE + NEF, "gather staging room");
   static_assert(V * S * S <= TW && V * S * P <= TW, "subuh1 / luhy room");
-  static_assert(V * P2 + V * S * P + V * P * P <= 2 * TW, "FP32 DMP room");
+  using PF = Proj<N, V, float>;
+  static_assert(PF::UF + PF::LYF + PF::LBF + 3 <= 2 * TW, "FP32 DMP room");
   static constexpr int TEL = V * R * R + TSTATE + NEF + 2 * S * P + P * P;
   static constexpr int TBYTES = ((TEL * (int)sizeof(T) + 15) / 16) * 16;
   // FP64 elements: new polynomial UN [V][P2], DMP y pass LY [V][S][P], LB
@@ -254,9 +255,10 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
   int* nbs = reinterpret_cast<int*>(misc + 16 + 9 * 8);     // their status (0: project olduh)
   unsigned* amax = reinterpret_cast<unsigned*>(nbs + 9);     // max |UN - UN(node 0)| per variable
   float* limf = reinterpret_cast<float*>(amax + V);          // T = double: uh2lim and uh2lob in FP32
-  float* UNf = reinterpret_cast<float*>(wLy);                // FP32 DMP (after the re-solve)
-  float* LYf = UNf + V * P2;
-  float* LBf = LYf + V * S * P;
+  using PF = Proj<N, V, float>;                              // FP32 DMP (after the re-solve), on 16 bytes
+  float* UNf = reinterpret_cast<float*>(smem_raw + ((V * R * R + 2 * C::TW) * sizeof(T) + 15) / 16 * 16);
+  float* LYf = UNf + PF::UF;
+  float* LBf = LYf + PF::LYF;
   float* redf = reinterpret_cast<float*>(red);              // [2][V][NW]
 
   const int t = threadIdx.x;
@@ -284,7 +286,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     const typename Sys::FConst fcs(ph);
     const int par = parity(st);
     const long long lc = c - in.cell_base;
-    const int ci = (int)(lc % in.imax), cj = (int)(lc / in.imax);
+    const int ci = (int)((unsigned)lc % (unsigned)in.imax), cj = (int)((unsigned)lc / (unsigned)in.imax);
     const int rec = a.recompute[c];
     const T dt = (T)st.dt;
     const T ldx0 = (T)(in.dx / (double)S), ldx1 = (T)(in.dy / (double)S);
@@ -643,13 +645,15 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     const float* lim32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(limT) : limf;
     const float* lob32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(lobT) : limf + S * P;
     if (dmp && try32) {
-      for (int p = t; p < P2; p += NT)
+      for (int p = t; p < P2; p += NT) {
+        float d[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          const float d = (float)(UN[v * P2 + p] - UN[v * P2]);
-          UNf[v * P2 + p] = d;
-          atomicMax(&amax[v], __float_as_uint(fabsf(d)));
+          d[v] = (float)(UN[v * P2 + p] - UN[v * P2]);
+          atomicMax(&amax[v], __float_as_uint(fabsf(d[v])));
         }
+        PF::template st<PF::NU>(UNf, p, d);
+      }
     }
     __syncthreads();
     float err[V];
@@ -670,9 +674,12 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       float fmn[V], fmx[V], ubf[V];
 #pragma unroll
       for (int v = 0; v < V; ++v) { fmn[v] = __int_as_float(0x7f800000); fmx[v] = -__int_as_float(0x7f800000); }
-      for (int p = t; p < P2; p += NT)
+      for (int p = t; p < P2; p += NT) {
+        float d[V];
+        PF::template ld<PF::NU>(UNf, p, d);
 #pragma unroll
-        for (int v = 0; v < V; ++v) { fmn[v] = fminf(fmn[v], UNf[v * P2 + p]); fmx[v] = fmaxf(fmx[v], UNf[v * P2 + p]); }
+        for (int v = 0; v < V; ++v) { fmn[v] = fminf(fmn[v], d[v]); fmx[v] = fmaxf(fmx[v], d[v]); }
+      }
 #pragma unroll
       for (int v = 0; v < V; ++v) ubf[v] = (float)UN[v * P2];
       Proj<N, V, float>::template xpass_minmax_f32<Sys>(LYf, LBf, lim32, lob32, UN, opsm, typename Sys::FConst(ph), err,
@@ -931,7 +938,7 @@ __global__ void __launch_bounds__(128) k_settle(BatchArgs a, DevOps<N, double> o
     const InstDesc& in = a.inst[k];
     const int par = parity(a.st[k]);
     const long long lc = cell - in.cell_base;
-    const int ci = (int)(lc % in.imax), cj = (int)(lc / in.imax);
+    const int ci = (int)((unsigned)lc % (unsigned)in.imax), cj = (int)((unsigned)lc / (unsigned)in.imax);
     const double* un = (init ? a.uh[par] : a.uh[par ^ 1]) + (size_t)cell * P2 * V;
     __syncthreads();  // the previous cell's readers of U are done
     for (int p = t; p < P2 * V; p += NT) U[(p % V) * P2 + p / V] = un[p];
