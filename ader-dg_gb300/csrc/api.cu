@@ -202,12 +202,12 @@ int exact_lminmax(aderdg_ctx* c) {
 int launch_step(aderdg_ctx* c) {
   CK(c, control(c, aderdg::kCtlBegin));
   CK(c, aderdg::launch_predictor(c->kt, c->args, pred_ops(c), c->prec, c->stream));
-  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream));
+  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream, true));
   int r = cells(c, aderdg::kCellFused);
   if (r) return r;
   if (c->limiter) {
     CK(c, c->kt->mark(c->args, c->stream));
-    CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream));
+    CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, true));
   }
   CK(c, control(c, aderdg::kCtlEnd));
   return ADERDG_OK;
@@ -688,7 +688,7 @@ int aderdg_volume_integral(aderdg_ctx* c) {
 
 int aderdg_riemann_problem(aderdg_ctx* c) {
   if (!c) return fail(c, ADERDG_EINVAL, "null context");
-  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream));
+  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream, false));
   return ADERDG_OK;
 }
 
@@ -719,7 +719,7 @@ int aderdg_limiter(aderdg_ctx* c) {
   if (!c->pending) return fail(c, ADERDG_ESTATE, "run aderdg_element_update first");
   CK(c, cudaMemsetAsync(c->args.list_count, 0, sizeof(int), c->stream));
   CK(c, c->kt->mark(c->args, c->stream));
-  CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream));
+  CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, false));
   CK(c, control(c, aderdg::kCtlEnd));
   c->pending = false;
   return pull_state(c);
@@ -847,7 +847,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   CK(c, cudaEventRecord(ev[1], c->stream));
   CK(c, aderdg::launch_predictor(c->kt, c->args, pred_ops(c), c->prec, c->stream));
   CK(c, cudaEventRecord(ev[2], c->stream));
-  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream));
+  CK(c, aderdg::launch_faces(c->kt, c->args, c->fc, c->prec, c->stream, true));
   CK(c, cudaEventRecord(ev[3], c->stream));
   r = cells(c, aderdg::kCellFused);
   if (r) return r;
@@ -855,7 +855,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   if (c->limiter) CK(c, c->kt->mark(c->args, c->stream));
   CK(c, cudaEventRecord(ev[5], c->stream));
   if (c->limiter)
-    CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream));
+    CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, true));
   CK(c, cudaEventRecord(ev[6], c->stream));
   CK(c, control(c, aderdg::kCtlEnd));
   CK(c, cudaEventRecord(ev[7], c->stream));

@@ -221,12 +221,12 @@ int blaunch_step(aderdg_batch* b) {
   a.mode = aderdg::kCellFused;
   BK(b, bcontrol(b, aderdg::kCtlBegin, -1));
   BK(b, aderdg::launch_predictor(b->kt, a, bpred_ops(b), b->precision, b->stream));
-  BK(b, aderdg::launch_faces(b->kt, a, b->fc, b->precision, b->stream));
+  BK(b, aderdg::launch_faces(b->kt, a, b->fc, b->precision, b->stream, true));
   BK(b, aderdg::launch_cells(b->kt, a, b->ops64.data(), b->precision, b->stream));
   if (a.settle) BK(b, b->kt->settle(a, b->ops64.data(), b->num_sms, b->stream));
   if (b->limiter) {
     BK(b, b->kt->mark(a, b->stream));
-    BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream));
+    BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream, true));
   }
   BK(b, bcontrol(b, aderdg::kCtlEnd, -1));
   return ADERDG_OK;
@@ -774,7 +774,7 @@ int aderdg_batch_profile(aderdg_batch* b, double* phase_ms) {
   BK(b, cudaEventRecord(ev[1], b->stream));
   BK(b, aderdg::launch_predictor(b->kt, a, bpred_ops(b), b->precision, b->stream));
   BK(b, cudaEventRecord(ev[2], b->stream));
-  BK(b, aderdg::launch_faces(b->kt, a, b->fc, b->precision, b->stream));
+  BK(b, aderdg::launch_faces(b->kt, a, b->fc, b->precision, b->stream, true));
   BK(b, cudaEventRecord(ev[3], b->stream));
   BK(b, aderdg::launch_cells(b->kt, a, b->ops64.data(), b->precision, b->stream));
   if (a.settle) BK(b, b->kt->settle(a, b->ops64.data(), b->num_sms, b->stream));
@@ -782,7 +782,7 @@ int aderdg_batch_profile(aderdg_batch* b, double* phase_ms) {
   if (b->limiter) BK(b, b->kt->mark(a, b->stream));
   BK(b, cudaEventRecord(ev[5], b->stream));
   if (b->limiter)
-    BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream));
+    BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream, true));
   BK(b, cudaEventRecord(ev[6], b->stream));
   BK(b, bcontrol(b, aderdg::kCtlEnd, -1));
   BK(b, cudaEventRecord(ev[7], b->stream));

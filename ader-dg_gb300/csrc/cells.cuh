@@ -375,6 +375,20 @@ __device__ __forceinline__ double cfl_denom(const InstDesc& in, const double* Q)
     return denom;
   }
 }
+// The same from the reciprocal-sharing forms (the FP64 fused step): its divisions
+// and square roots were a third of the FP64 cell kernel's FP64 instructions (490 ->
+// 365 us on the Euler vortex N = 4 256^2, 453 -> 345 us on Baer-Nunziato N = 3 200^2)
+template <class Sys, int N>
+__device__ __forceinline__ double cfl_denom_r(const InstDesc& in, const double* Q) {
+  if constexpr (Sys::ID == kSysAD) {
+    return cfl_denom<Sys, N>(in, Q);
+  } else {
+    double ex, ey;
+    Sys::template max_eig2_r<true>(PhysC<double>(in.ph), Q, ex, ey);
+    return fma(ex, in.rdx, ey * in.rdy);
+  }
+}
+
 // FP32-mixed: eigenvalues and the node's denominator in FP32 (the maximum
 // over nodes, and dt, in FP64); states whose FP32 pressure is not settled
 // take the FP64 evaluation on Qd
@@ -468,10 +482,10 @@ using CellOps = typename std::conditional<kExact || !kFast, ExactOps<N>, DevOps<
 
 // kFast: DMP projections in FP32 with an error bound (settled from FP64 where
 // the bound leaves a decision open) and, without kExact, the FP32 modes'
-// storage and surface integral.  kExact: FP64 storage, surface integral, update
-// and CFL in reference order beside those projections: the FP64 mode's fused
-// step, whose decisions and state are those of the FP64 projections bit for
-// bit.
+// storage and surface integral.  kExact: FP64 storage, surface integral and
+// update in reference order beside those projections, and FP64 CFL eigenvalues:
+// the FP64 mode's fused step, whose decisions and state are those of the FP64
+// projections bit for bit.
 template <class Sys, int N, bool kFast, int VAR = 0, bool kExact = false>
 __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast && !kExact))
     k_cells(BatchArgs a, CellOps<N, kFast, kExact> op) {
@@ -723,6 +737,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       if (act) {
         double dn;
         if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+        else if constexpr (kExact) dn = cfl_denom_r<Sys, N>(in, u);
         else dn = cfl_denom<Sys, N>(in, u);
         bits = (unsigned long long)__double_as_longlong(dn);
       }
@@ -735,6 +750,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       if (act) {
         double dn;
         if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+        else if constexpr (kExact) dn = cfl_denom_r<Sys, N>(in, u);
         else dn = cfl_denom<Sys, N>(in, u);
         bits = (unsigned long long)__double_as_longlong(dn);
       }

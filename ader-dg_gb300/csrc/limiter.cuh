@@ -138,20 +138,20 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
 // Subgrid Rusanov flux (Euler/limiter.f90:361-378; BN :359-383 adds D = B~ dQ);
 // kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
 // flux (the update takes half its factor: one FP64 instruction less a variable)
-template <class Sys, class T, bool kRcp = false>
+template <class Sys, class T, int kRcp = 0>
 __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const typename Sys::FConst& fcs, const T* QL, const T* QR,
                                           int d, T* F, T* D) {
   constexpr int V = Sys::V;
   if constexpr (kRcp && Sys::ID == kSysBN) {
-    BNSys::rusanov_mixed(pc, fcs, QL, QR, d, F, D);
+    BNSys::rusanov_mixed<kRcp == 2>(pc, fcs, QL, QR, d, F, D);
     return;
   }
   T FLf[2 * V], FRf[2 * V], smax;
   if constexpr (kRcp) {
     // the flux along d only (the other direction's would be multiplied by 0)
     T eL, eR;
-    Sys::flux_dir_eig_r(pc, QL, d, FLf, eL);
-    Sys::flux_dir_eig_r(pc, QR, d, FRf, eR);
+    Sys::template flux_dir_eig_r<kRcp == 2>(pc, QL, d, FLf, eL);
+    Sys::template flux_dir_eig_r<kRcp == 2>(pc, QR, d, FRf, eR);
     if constexpr (sizeof(T) == 8) smax = max_nonneg(eL, eR);
     else smax = tmax(eL, eR);
 #pragma unroll
@@ -212,16 +212,19 @@ __device__ __forceinline__ void warp_minmax_store(R* mn, R* mx, R* red, int t) {
   }
 }
 
-// T = double: the reference's FP64 arithmetic in its order (bit for bit),
-// or, with kRcp (the FP32-mixed mode, instantiated with fused multiply-adds in
-// predictor_tu.cu), FP64 with the reciprocal-sharing physics forms and
-// multiplications by 1/ldx in place of divisions; the DMP projections keep
-// the reference order in both.
+// T = double: the reference's FP64 arithmetic in its order (bit for bit: the phase
+// API), or, with kRcp (instantiated with fused multiply-adds in predictor_tu.cu),
+// FP64 with the reciprocal-sharing physics forms and multiplications by 1/ldx in
+// place of divisions: 1 in the FP32-mixed mode, 2 in the FP64 fused step, whose
+// quotients are corrected (quot, physics.cuh) and where a NaN sound speed leaves
+// |u|, as the reference's maxima do.  FP64 fused step: 301 -> 168 us (Riemann
+// problem N = 3 257 x 193), 817 -> 326 us (Baer-Nunziato N = 3 200^2).  The DMP
+// projections keep the reference order in all.
 // T = float: the FP32-wide mode; the subcell re-solve, the DMP projections
 // of the new polynomial (while their error bound allows) and the CFL
 // eigenvalues (where the FP32 pressure is settled) in FP32; the state, Lh
 // and min/max in FP64.
-template <class Sys, int N, class T, bool kRcp = false>
+template <class Sys, int N, class T, int kRcp = 0>
 __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>::MIN_BLOCKS) k_subcell(BatchArgs a, DevOps<N, double> op, FaceConst fc) {
   using C = SubCfg<Sys, N, T>;
   constexpr int P = N + 1, P2 = P * P, S = 2 * N + 1, V = Sys::V, R = C::R, H = C::H, NT = C::THREADS, NE = C::NE;
@@ -299,14 +302,14 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     auto flux = [&](const T* Q, int d, T* F) {
       if constexpr (kRcp) {
         T e;
-        Sys::flux_dir_eig_r(pc, Q, d, F + d * V, e);
+        Sys::template flux_dir_eig_r<kRcp == 2>(pc, Q, d, F + d * V, e);
       } else {
         Sys::flux(pc, Q, F);
       }
     };
     auto ncp = [&](const T* Q, T ax, T ay, T* Sr) {
       if constexpr (Sys::ID == kSysBN) {
-        if constexpr (kRcp) BNSys::src_ncp_r(pc, Q, ax, ay, Sr);
+        if constexpr (kRcp) BNSys::src_ncp_r<kRcp == 2>(pc, Q, ax, ay, Sr);
         else BNSys::src_ncp(pc, Q, ax, ay, Sr);
       }
     };
@@ -705,7 +708,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
         dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(ph), q, Q);
       } else if constexpr (kRcp) {
         double ex, ey;
-        Sys::max_eig2_r(pc, Q, ex, ey);
+        Sys::template max_eig2_r<kRcp == 2>(pc, Q, ex, ey);
         dn = fma(ex, in.rdx, ey * in.rdy);
       } else {
         dn = cfl_denom<Sys, N>(in, Q);

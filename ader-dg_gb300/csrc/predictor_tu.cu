@@ -176,29 +176,40 @@ cudaError_t predictor(const BatchArgs& a, const void* ops, int fp32, bool phase,
 }
 
 #if ADERDG_SYS != 0
-// FP32-mixed subcell re-solve: FP64 with the reciprocal-sharing physics forms,
-// compiled here with fused multiply-adds (k_subcell's DMP projections keep
-// the reference order through rounded intrinsics)
-using SubMixed = SubCfg<Sys, N, double>;
-int subcell_grid_mixed(int num_sms) {
+// Subcell re-solve in FP64 with the reciprocal-sharing physics forms, compiled
+// here with fused multiply-adds (k_subcell's DMP projections keep the reference
+// order through rounded intrinsics): kRcp = 1 in the FP32-mixed mode, 2
+// (corrected quotients) in the FP64 fused step
+template <int kRcp>
+int subcell_grid_r(int num_sms) {
+  using C = SubCfg<Sys, N, double>;
+  auto kern = k_subcell<Sys, N, double, kRcp>;
   int per_sm = 0;
-  cudaFuncSetAttribute(k_subcell<Sys, N, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       SubMixed::SMEM_BYTES);
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_subcell<Sys, N, double, true>, SubMixed::THREADS,
-                                                    SubMixed::SMEM_BYTES) != cudaSuccess)
-    per_sm = 1;
+  cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM_BYTES) != cudaSuccess) per_sm = 1;
   return (per_sm < 1 ? 1 : per_sm) * num_sms;
 }
-cudaError_t subcell_mixed(const BatchArgs& a, const void* ops, const FaceConst& fc, int grid, cudaStream_t s) {
+template <int kRcp>
+cudaError_t subcell_r(const BatchArgs& a, const void* ops, const FaceConst& fc, int grid, cudaStream_t s) {
+  using C = SubCfg<Sys, N, double>;
+  auto kern = k_subcell<Sys, N, double, kRcp>;
   static bool attr = false;
   if (!attr) {
-    cudaError_t e = cudaFuncSetAttribute(k_subcell<Sys, N, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SubMixed::SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
     if (e != cudaSuccess) return e;
     attr = true;
   }
-  k_subcell<Sys, N, double, true><<<grid, SubMixed::THREADS, SubMixed::SMEM_BYTES, s>>>(
-      a, *reinterpret_cast<const DevOps<N, double>*>(ops), fc);
+  kern<<<grid, C::THREADS, C::SMEM_BYTES, s>>>(a, *reinterpret_cast<const DevOps<N, double>*>(ops), fc);
+  return cudaGetLastError();
+}
+#endif
+
+#if ADERDG_SYS != 0
+// FP64 faces of the fused step: reciprocal-sharing forms, fused multiply-adds
+cudaError_t faces_fused(const BatchArgs& a, const FaceConst& fc, cudaStream_t s) {
+  const long long n = (a.nfx + a.nfy) * (N + 1);
+  if (n <= 0) return cudaSuccess;
+  k_faces<Sys, N, double, double, true><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(a, fc);
   return cudaGetLastError();
 }
 #endif
@@ -235,8 +246,11 @@ void ADERDG_CAT(register_predictor_, ADERDG_SYS, ADERDG_N)(KernelTable& t) {
   t.faces_mixed = &faces_mixed;
 #endif
 #if ADERDG_SYS != 0
-  t.subcell_mixed = &subcell_mixed;
-  t.subcell_grid_mixed = &subcell_grid_mixed;
+  t.subcell_mixed = &subcell_r<1>;
+  t.subcell_grid_mixed = &subcell_grid_r<1>;
+  t.subcell_fused = &subcell_r<2>;
+  t.subcell_grid_fused = &subcell_grid_r<2>;
+  t.faces_fused = &faces_fused;
 #endif
 }
 

@@ -38,10 +38,16 @@ struct KernelTable {
   // FP32-mixed faces where they differ from the FP32 faces (Baer-Nunziato:
   // FP64 arithmetic on FP32 storage); null: use faces(..., fp32 = 1, ...)
   cudaError_t (*faces_mixed)(const BatchArgs&, const FaceConst&, cudaStream_t) = nullptr;
-  // FP32-mixed subcell re-solve (FP64, reciprocal-sharing physics, fused
-  // multiply-adds) and its persistent grid; null for advection-diffusion
+  // FP64 faces of the fused step (reciprocal-sharing physics, fused
+  // multiply-adds); null for advection-diffusion
+  cudaError_t (*faces_fused)(const BatchArgs&, const FaceConst&, cudaStream_t) = nullptr;
+  // Subcell re-solve of the FP32-mixed mode and of the FP64 fused step (FP64,
+  // reciprocal-sharing physics, fused multiply-adds) and their persistent grids;
+  // null for advection-diffusion
   cudaError_t (*subcell_mixed)(const BatchArgs&, const void* ops64, const FaceConst&, int grid, cudaStream_t) = nullptr;
+  cudaError_t (*subcell_fused)(const BatchArgs&, const void* ops64, const FaceConst&, int grid, cudaStream_t) = nullptr;
   int (*subcell_grid_mixed)(int num_sms) = nullptr;
+  int (*subcell_grid_fused)(int num_sms) = nullptr;
   // exact translation unit
   cudaError_t (*faces)(const BatchArgs&, const FaceConst&, int fp32, cudaStream_t) = nullptr;
   // fast: 0 FP64 in reference order, 1 the FP32 modes, 2 FP64 with certified FP32 projections
@@ -112,25 +118,30 @@ inline int subcell_launch_grid(const KernelTable* kt, int max_grid, int num_sms,
 
 // The face kernel of a precision mode (aderdg_precision).
 inline cudaError_t launch_faces(const KernelTable* kt, const BatchArgs& a, const FaceConst& fc, int precision,
-                                cudaStream_t s) {
+                                cudaStream_t s, bool fused) {
   if (precision == ADERDG_FP32_MIXED && kt->faces_mixed) return kt->faces_mixed(a, fc, s);
+  if (precision == ADERDG_FP64 && fused && kt->faces_fused) return kt->faces_fused(a, fc, s);
   return kt->faces(a, fc, precision != ADERDG_FP64 ? 1 : 0, s);
 }
 // The subcell re-solve of a precision mode: FP32 in the FP32-wide mode, FP64
-// with the reciprocal-sharing physics in the FP32-mixed mode, FP64 in the
-// reference's order otherwise.
+// with the reciprocal-sharing physics in the FP32-mixed mode and in the FP64
+// fused step, FP64 in the reference's order otherwise (the phase API).
 inline int subcell_fp32(int precision) { return precision == ADERDG_FP32_WIDE ? 1 : 0; }
 // max_grid: the most CTAs that fit (subcell_grid_of); the tuned CTAs per SM
 // apply within it
 inline cudaError_t launch_subcell(const KernelTable* kt, const BatchArgs& a, const void* ops64, const FaceConst& fc,
-                                  int max_grid, int num_sms, int precision, cudaStream_t s) {
+                                  int max_grid, int num_sms, int precision, cudaStream_t s, bool fused) {
   const int grid = subcell_launch_grid(kt, max_grid, num_sms, precision);
   if (precision == ADERDG_FP32_MIXED && kt->subcell_mixed) return kt->subcell_mixed(a, ops64, fc, grid, s);
+  if (precision == ADERDG_FP64 && fused && kt->subcell_fused) return kt->subcell_fused(a, ops64, fc, grid, s);
   return kt->subcell(a, ops64, fc, grid, subcell_fp32(precision), s);
 }
 inline int subcell_grid_of(const KernelTable* kt, int num_sms, int precision) {
   if (precision == ADERDG_FP32_MIXED && kt->subcell_grid_mixed) return kt->subcell_grid_mixed(num_sms);
-  return kt->subcell_grid(num_sms, subcell_fp32(precision));
+  const int g = kt->subcell_grid(num_sms, subcell_fp32(precision));
+  // FP64 launches both; a CTA that does not fit at once waits for one that leaves
+  const int f = precision == ADERDG_FP64 && kt->subcell_grid_fused ? kt->subcell_grid_fused(num_sms) : 0;
+  return g > f ? g : f;
 }
 
 }  // namespace aderdg
