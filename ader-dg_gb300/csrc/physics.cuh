@@ -132,8 +132,12 @@ template <class T> __device__ __forceinline__ T mrcp(T x) {
 // mean square over 4e5 random states; 0.93 to 1.10 uncorrected).
 template <bool kC, class T> __device__ __forceinline__ T quot(T a, T b, T i) {
   const T q = a * i;
-  if constexpr (kC) return fma(fma(-q, b, a), i, q);
-  else return q;
+  if constexpr (kC) {
+    const T r = fma(fma(-q, b, a), i, q);
+    return (__double2hiint(q) & 0x7ff00000) == 0x7ff00000 ? q : r;  // infinite quotients have no remainder
+  } else {
+    return q;
+  }
 }
 template <class T> __device__ __forceinline__ T msqrt(T a) {
   if constexpr (sizeof(T) == 4) {
