@@ -129,6 +129,9 @@ struct PredOps<N, double> : ExactOps<N> {  // the FP64 predictor
   static constexpr int P = N + 1;
   double iw[P];   // 1/w
   double tsx[P];  // sum_l T(l',l), rounded once
+  // advection-diffusion, rounded once from twice FP64: sum_k Kxi(k,i) dudx(k,m) at
+  // [i + P*m], Kxi and w (T and tw of its operators likewise)
+  double KG[P * P], Kx[P * P], wx[P];
   // Kxi, T, the end values FL and FR, and the time weights w and tw in 60-bit
   // fixed point (predictor_fix.cuh): entry = (h 2^31 + l) 2^-s, 0 <= l < 2^31
   int Kh[P * P], Kl[P * P], Th[P * P], Tl[P * P], Eh[2 * P], El[2 * P], Wh[P], Wl[P], TWh[P], TWl[P];

@@ -125,6 +125,15 @@ void make_ops(const HostOps& h, void* out) {
       o.El[k] = end_l[k];
     }
     for (int k = 0; k < P; ++k) o.iw[k] = 1.0 / h.w[k];
+    for (int k = 0; k < P * P; ++k) {
+      o.KG[k] = h.fKG.hi[k];
+      o.Kx[k] = h.fKxi.hi[k];
+      if (Sys::ID == kSysAD) o.T[k] = h.fT.hi[k];
+    }
+    for (int l = 0; l < P; ++l) {
+      o.wx[l] = h.fTimes.hi[l];
+      if (Sys::ID == kSysAD) o.tw[l] = h.fTimes.hi[P + l];
+    }
   }
   for (int k = 0; k < S * P; ++k) {
     o.uh2lim[k] = h.uh2lim[k];

@@ -258,6 +258,11 @@ void build_fine(HostOps& o) {
   split(ends, o.fEnds);
   split(times, o.fTimes);
   split(ts, o.fTs);
+  std::vector<Dd> KG(P * P);  // dudx(k,m) = Kxi(m,k) / w(k)
+  for (int i = 0; i < P; ++i)
+    for (int m = 0; m < P; ++m)
+      for (int k = 0; k < P; ++k) KG[i + P * m] = KG[i + P * m] + K[k + P * i] * K[m + P * k] / w[k];
+  split(KG, o.fKG);
 }
 
 double pi_value() { return kPi; }

@@ -31,6 +31,7 @@ struct HostOps {
   Fine fEnds;        // FL, FR
   Fine fTimes;       // w(l), tw(l) = sum_l' w(l') T(l',l)
   Fine fTs;          // sum_l T(l',l)
+  Fine fKG;          // sum_k Kxi(k,i) dudx(k,m) at [i + P*m]: the stiffness of a gradient
 };
 
 bool build_ops(int N, HostOps& ops, std::string* err);
