@@ -302,6 +302,7 @@ InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops) {
   if (cfg->system == ADERDG_SYS_ADVDIFF) {
     // the expressions of the face kernel and of calc_time_step, evaluated once
     const double pi = 4.0 * std::atan(1.0);
+    in.ad_pi = pi;
     const double factor = (double)(2 * cfg->N + 1);
     const double eta = factor / (in.dx * std::sqrt(0.5 * pi));
     for (int d = 0; d < 2; ++d) {

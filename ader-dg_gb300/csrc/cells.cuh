@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "faces.cuh"
 #include "physics.cuh"
 
 namespace aderdg {
@@ -100,8 +101,7 @@ struct Proj {
         if (s < S) st<NLY>(LY, s * PS + ii, acc);
         else st<NLB>(LB, (s - S) * PS + ii, acc);
       }
-      return;
-    }
+    } else {
     for (int idx = r; idx < P * S; idx += nr) {
       const int ii = idx % P, s = idx / P;
 #pragma unroll
@@ -121,6 +121,7 @@ struct Proj {
         for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, U[v * P2 + ii + P * k], lob[s + P * k]);
         LB[(v * P + s) * P + ii] = acc;
       }
+    }
     }
   }
   // T = float: sum over k of item (s2, k) times c[k * stride]
@@ -142,8 +143,7 @@ struct Proj {
   __device__ static void subcell(const T* LY, const T* lim, int s1, int s2, T* out) {
     if constexpr (sizeof(T) == 4) {
       row<NLY>(LY, lim + s1, S, s2, out);
-      return;
-    }
+    } else {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       T acc = 0;
@@ -151,19 +151,20 @@ struct Proj {
       for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LY[(v * S + s2) * P + k], lim[s1 + S * k]);
       out[v] = acc;
     }
+    }
   }
   template <bool kFast = false>
   __device__ static void lobatto(const T* LB, const T* lob, int s1, int s2, T* out) {
     if constexpr (sizeof(T) == 4) {
       row<NLB>(LB, lob + s1, P, s2, out);
-      return;
-    }
+    } else {
 #pragma unroll
     for (int v = 0; v < V; ++v) {
       T acc = 0;
 #pragma unroll
       for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LB[(v * P + s2) * P + k], lob[s1 + P * k]);
       out[v] = acc;
+    }
     }
   }
   // x pass fused with min/max (integer keys) and the positivity test of every subcell (FP64)
@@ -626,6 +627,29 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   // ---------------------------------------------------------------- update
   double u[V];
   const size_t off = ((size_t)(valid ? cell : 0) * P2 + node) * V;
+  // Advection-diffusion, fused step on small grids (faces_in_cells): the cell's
+  // face fluxes [4][P] from the predictor's face states; a cell stores those of its
+  // left and bottom faces, the last ones of a row or column also the others
+  using FR_ = typename std::conditional<kF32, float, double>::type;
+  FR_* sF = reinterpret_cast<FR_*>(U);
+  const bool own_faces = Sys::ID == kSysAD && mode == kCellFused && faces_in_cells(a, P2, kF32);
+  if constexpr (Sys::ID == kSysAD) {
+    if (own_faces) {
+      if (act) {
+        for (int idx = node; idx < 4 * P; idx += P2) {
+          const int f = idx / P, l = idx - f * P, fi = ci + (f == 1), fj = cj + (f == 3);
+          const bool xdir = f < 2;
+          const FR_ x = ad_face_flux<FR_, FR_>(a, in, in.ad_pi, op.xid[l], xdir, fi, fj, l, P);
+          sF[idx] = x;
+          if (f == 0 || f == 2 || (f == 1 ? fi == in.imax : fj == in.jmax)) {
+            const long long face = xdir ? in.fx_base + fi + (long long)(in.imax + 1) * fj : in.fy_base + fi + (long long)in.imax * fj;
+            reinterpret_cast<FR_*>(xdir ? a.fu : a.gu)[(size_t)face * P + l] = x;
+          }
+        }
+      }
+      __syncthreads();
+    }
+  }
   if (act) {
     if (mode == kCellFused || mode == kCellSurface || mode == kCellUpdate) {
       const long long fxl = in.fx_base + ci + (long long)(in.imax + 1) * cj;
@@ -645,10 +669,17 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         if (mode != kCellUpdate) {
           const float cxf = op.wf[j] * in.idxf, cyf = op.wf[i] * in.idyf;
           float fl[V], fr[V], gb[V], gt[V];
-          load_v<V>(XL + ((size_t)fxl * P + j) * V, fl);
-          load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, fr);
-          load_v<V>(YB + ((size_t)fyb * P + i) * V, gb);
-          load_v<V>(YT + ((size_t)fyt * P + i) * V, gt);
+          if (own_faces) {
+            fl[0] = sF[j];
+            fr[0] = sF[P + j];
+            gb[0] = sF[2 * P + i];
+            gt[0] = sF[3 * P + i];
+          } else {
+            load_v<V>(XL + ((size_t)fxl * P + j) * V, fl);
+            load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, fr);
+            load_v<V>(YB + ((size_t)fyb * P + i) * V, gb);
+            load_v<V>(YT + ((size_t)fyt * P + i) * V, gt);
+          }
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             const float sx = fr[v] * op.FRf[i] - fl[v] * op.FLf[i];
@@ -679,15 +710,25 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
           const double* YB = a.gu;
           const double* YT = (Sys::ID == kSysBN) ? a.gp : a.gu;
           const double cx = in.wdx[j], cy = in.wdy[i];  // w_j / dx, w_i / dy
-          load_v<V>(XL + ((size_t)fxl * P + j) * V, p);
-          load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, q);
+          if (own_faces) {
+            p[0] = sF[j];
+            q[0] = sF[P + j];
+          } else {
+            load_v<V>(XL + ((size_t)fxl * P + j) * V, p);
+            load_v<V>(XR + ((size_t)(fxl + 1) * P + j) * V, q);
+          }
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             if constexpr (kExact) d[v] = fma(-cx, fma(-p[v], op.FLd[i], q[v] * op.FRd[i]), d[v]);
             else d[v] = d[v] - cx * (q[v] * op.FRd[i] - p[v] * op.FLd[i]);
           }
-          load_v<V>(YB + ((size_t)fyb * P + i) * V, p);
-          load_v<V>(YT + ((size_t)fyt * P + i) * V, q);
+          if (own_faces) {
+            p[0] = sF[2 * P + i];
+            q[0] = sF[3 * P + i];
+          } else {
+            load_v<V>(YB + ((size_t)fyb * P + i) * V, p);
+            load_v<V>(YT + ((size_t)fyt * P + i) * V, q);
+          }
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             if constexpr (kExact) d[v] = fma(-cy, fma(-p[v], op.FLd[j], q[v] * op.FRd[j]), d[v]);

@@ -56,6 +56,7 @@ struct InstDesc {
   // (Advection-Diffusion/calc_time_step.f90:37-50)
   double ad_smax[2];
   double ad_denom;
+  double ad_pi;                // 4 atan(1) as the host computes it
   double rdx, rdy;             // 1/dx, 1/dy (the FP64 predictor)
   double wdx[6], wdy[6];       // w_k/dx, w_k/dy (the FP64 surface integral)
 };
@@ -184,6 +185,15 @@ struct BatchArgs {
   long long cell0;                   // first cell of a launch over part of the cell range (K1, K3)
   int only_inst;                     // >= 0: the priming modes of K3 touch this instance only
 };
+
+// Advection-diffusion's fused step: whether the cell kernel forms its cells' face
+// fluxes itself.  It forms each twice, from scattered loads, but saves a launch:
+// on small grids 2 us of a step's 18 to 60 (FP32 modes, 16 K to 147 K nodes: 1.00 to
+// 1.13 times as fast, beyond 0.89 to 1.00; FP64, to 65 K nodes 1.00 to 1.07, from 83 K on
+// 0.86 to 1.00; N = 2 to 5, 32^2 to 512^2).
+__host__ __device__ inline bool faces_in_cells(const BatchArgs& a, int P2, bool fp32) {
+  return a.ncells * P2 <= (fp32 ? 131072 : 65536);
+}
 
 __device__ __forceinline__ int parity(const InstState& s) { return (int)(s.steps & 1); }
 

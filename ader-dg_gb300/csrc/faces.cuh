@@ -156,6 +156,79 @@ __device__ void faces_euler_fp32(const BatchArgs& a, const FaceConst& fc, const 
   store_v<V>(dst, out);
 }
 
+// Advection-diffusion's numerical flux at point l of face (i, j) along x (xdir)
+// or y, as stored: Advection-Diffusion/riemann_problem.f90 with
+// PDEViscLLFRiemannSolver (pde.f90:121-152); compute type CT: FP64 (reference
+// order), FP32 in the FP32 modes.  xi = the point's coordinate in its face, P the
+// points of a face.  On small grids the fused step's cell kernel forms its cells'
+// face fluxes from it, too.
+template <class R, class CT>
+__device__ __forceinline__ R ad_face_flux(const BatchArgs& a, const InstDesc& in, double pi, double xi, bool xdir, int i,
+                                          int j, int l, int P) {
+  const R* qb = reinterpret_cast<const R*>(a.qbnd);
+  const R* fb = reinterpret_cast<const R*>(a.fbnd);
+  const int I = in.imax, J = in.jmax;
+  auto cid = [&](int ci, int cj) { return in.cell_base + (long long)ci + (long long)I * cj; };
+  const int pos = xdir ? i : j, last = xdir ? I : J;
+  const int bcl = in.bc[xdir ? 0 : 2], bcr = in.bc[xdir ? 1 : 3];
+  const int fl = xdir ? 0 : 2, fr = xdir ? 1 : 3;  // left/bottom and right/top face ids
+  CT QL[1], QR[1], gL[2], gR[2];
+  auto get = [&](long long c, int f, CT* Q, CT* gq) {
+    const size_t o = (((size_t)c * 4 + f) * P + l);
+    Q[0] = (CT)qb[o];
+    gq[0] = (CT)fb[o * 2 + 0];
+    gq[1] = (CT)fb[o * 2 + 1];
+  };
+  const long long cL = xdir ? cid(i - 1, j) : cid(i, j - 1);
+  const long long cR = cid(i, j);
+  if (pos == 0) {
+    if (bcl == 1) {
+      get(cR, fl, QL, gL);
+      get(cR, fl, QR, gR);
+    } else if (bcl == 2) {
+      if (xdir) {
+        // QR from the right face of cell IMAX, QL = -QR + 2 sin(pi y),
+        // y = (j-1 + xi_l) dy (Advection-Diffusion/riemann_problem.f90:37-40)
+        get(cid(I - 1, j), 1, QR, gR);
+        const double y = ((double)j + xi) * in.dy;
+        QL[0] = -QR[0] + (CT)(2.0 * sin(pi * y));
+      } else {
+        get(cR, fl, QR, gR);
+        QL[0] = -QR[0];
+      }
+      gL[0] = gR[0];
+      gL[1] = gR[1];
+    } else {
+      get(xdir ? cid(I - 1, j) : cid(i, J - 1), fr, QL, gL);
+      get(cR, fl, QR, gR);
+    }
+  } else if (pos == last) {
+    const long long cLast = xdir ? cid(I - 1, j) : cid(i, J - 1);
+    if (bcr == 1) {
+      get(cLast, fr, QL, gL);
+      get(cLast, fr, QR, gR);
+    } else if (bcr == 2) {
+      get(cLast, fr, QL, gL);
+      QR[0] = -QL[0];
+      gR[0] = gL[0];
+      gR[1] = gL[1];
+    } else {
+      get(cLast, fr, QL, gL);
+      get(xdir ? cid(0, j) : cid(i, 0), fl, QR, gR);
+    }
+  } else {
+    get(cL, fr, QL, gL);
+    get(cR, fl, QR, gR);
+  }
+  const CT nv0 = xdir ? CT(1) : CT(0), nv1 = xdir ? CT(0) : CT(1);
+  // smax = max(|c.n|) + 2 eta a, eta = (2N+1) / (dx sqrt(pi/2)): formed on the host
+  const CT smax = (CT)in.ad_smax[xdir ? 0 : 1];
+  const CT cx = (CT)in.ph.cx, cy = (CT)in.ph.cy, ca = (CT)in.ph.a;
+  const CT FL0 = cx * QL[0] + -ca * gL[0], FL1 = cy * QL[0] + -ca * gL[1];
+  const CT FR0 = cx * QR[0] + -ca * gR[0], FR1 = cy * QR[0] + -ca * gR[1];
+  return (R)(CT(0.5) * ((FL0 + FR0) * nv0 + (FL1 + FR1) * nv1) - CT(0.5) * smax * (QR[0] - QL[0]));
+}
+
 // kRec (FP64): the reciprocal-sharing forms, for the fused step (the phase API
 // keeps the reference's operation order): Euler N = 4 256^2 139 -> 96 us,
 // Baer-Nunziato N = 3 200^2 432 -> 143 us
@@ -211,64 +284,7 @@ __global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && si
   }
 
   if constexpr (Sys::ID == kSysAD) {
-    // Advection-Diffusion/riemann_problem.f90 with PDEViscLLFRiemannSolver (pde.f90:121-152);
-    // compute type: FP64 (reference order), FP32 in the FP32 modes
-    CT QL[1], QR[1], gL[2], gR[2];
-    auto get = [&](long long c, int f, CT* Q, CT* gq) {
-      const size_t o = (((size_t)c * 4 + f) * P + l);
-      Q[0] = (CT)qb[o];
-      gq[0] = (CT)fb[o * 2 + 0];
-      gq[1] = (CT)fb[o * 2 + 1];
-    };
-    const long long cL = xdir ? cid(i - 1, j) : cid(i, j - 1);
-    const long long cR = cid(i, j);
-    if (pos == 0) {
-      if (bcl == 1) {
-        get(cR, fl, QL, gL);
-        get(cR, fl, QR, gR);
-      } else if (bcl == 2) {
-        if (xdir) {
-          // QR from the right face of cell IMAX, QL = -QR + 2 sin(pi y),
-          // y = (j-1 + xi_l) dy (Advection-Diffusion/riemann_problem.f90:37-40)
-          get(cid(I - 1, j), 1, QR, gR);
-          const double y = ((double)j + fc.xi[l]) * in.dy;
-          QL[0] = -QR[0] + (CT)(2.0 * sin(fc.pi * y));
-        } else {
-          get(cR, fl, QR, gR);
-          QL[0] = -QR[0];
-        }
-        gL[0] = gR[0];
-        gL[1] = gR[1];
-      } else {
-        get(xdir ? cid(I - 1, j) : cid(i, J - 1), fr, QL, gL);
-        get(cR, fl, QR, gR);
-      }
-    } else if (pos == nfaces_side) {
-      const long long cLast = xdir ? cid(I - 1, j) : cid(i, J - 1);
-      if (bcr == 1) {
-        get(cLast, fr, QL, gL);
-        get(cLast, fr, QR, gR);
-      } else if (bcr == 2) {
-        get(cLast, fr, QL, gL);
-        QR[0] = -QL[0];
-        gR[0] = gL[0];
-        gR[1] = gL[1];
-      } else {
-        get(cLast, fr, QL, gL);
-        get(xdir ? cid(0, j) : cid(i, 0), fl, QR, gR);
-      }
-    } else {
-      get(cL, fr, QL, gL);
-      get(cR, fl, QR, gR);
-    }
-    const CT nv0 = xdir ? CT(1) : CT(0), nv1 = xdir ? CT(0) : CT(1);
-    // smax = max(|c.n|) + 2 eta a, eta = (2N+1) / (dx sqrt(pi/2)): formed on the host
-    const CT smax = (CT)in.ad_smax[xdir ? 0 : 1];
-    const CT cx = (CT)ph.cx, cy = (CT)ph.cy, ca = (CT)ph.a;
-    const CT FL0 = cx * QL[0] + -ca * gL[0], FL1 = cy * QL[0] + -ca * gL[1];
-    const CT FR0 = cx * QR[0] + -ca * gR[0], FR1 = cy * QR[0] + -ca * gR[1];
-    R* dst = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
-    dst[out] = (R)(CT(0.5) * ((FL0 + FR0) * nv0 + (FL1 + FR1) * nv1) - CT(0.5) * smax * (QR[0] - QL[0]));
+    reinterpret_cast<R*>(xdir ? a.fu : a.gu)[out] = ad_face_flux<R, CT>(a, in, fc.pi, fc.xi[l], xdir, i, j, l, P);
   } else {
     // Euler (FP64) and Baer-Nunziato (FP64 or FP32 compute, see above); FP32-mixed
     // Baer-Nunziato (kRcp) keeps the FP32 states and widens them where it uses them

@@ -120,6 +120,8 @@ inline int subcell_launch_grid(const KernelTable* kt, int max_grid, int num_sms,
 inline cudaError_t launch_faces(const KernelTable* kt, const BatchArgs& a, const FaceConst& fc, int precision,
                                 cudaStream_t s, bool fused) {
   if (precision == ADERDG_FP32_MIXED && kt->faces_mixed) return kt->faces_mixed(a, fc, s);
+  if (fused && kt->sys == ADERDG_SYS_ADVDIFF && faces_in_cells(a, (kt->N + 1) * (kt->N + 1), precision != ADERDG_FP64))
+    return cudaSuccess;
   if (precision == ADERDG_FP64 && fused && kt->faces_fused) return kt->faces_fused(a, fc, s);
   return kt->faces(a, fc, precision != ADERDG_FP64 ? 1 : 0, s);
 }
