@@ -761,7 +761,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
   }
   if (mode == kCellSurface) return;  // uniform per launch: no barrier follows
 
-  // FP32-mixed: the node's state in FP32, and its deviation from the cell's
+  // kFast: the node's state in FP32, and its deviation from the cell's
   // FP32 reference state ubar, formed in FP32 (one conversion per value)
   float uf[V], du[V], ubf[V];
   if constexpr (kFast && Sys::ID != kSysAD) {
@@ -1047,7 +1047,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         }
       }
       if (LPP == 2 ? a.mme[0] != nullptr : !in64) {
-        // FP32-mixed: the same comparisons in FP32, in the deviation space
+        // FP64 and FP32-mixed: the same comparisons in FP32, in the deviation space
         // of the cell's FP32 reference state ub (FP64 work is the costly
         // part of this kernel).  |own - FP64 value| <= ecell; |lmin - its
         // FP64 value| <= en and likewise lmax, so the thresholds move by at

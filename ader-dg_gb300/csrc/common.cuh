@@ -68,7 +68,7 @@ struct InstState {
   unsigned long long denom_next;     // accumulator for the next step
   int active;                        // 1 while time < tend
   int n_recompute;                   // troubled cells of the last step (nRecompute)
-  int n_settled;                     // FP32-mixed: DMP decisions of the last step settled from FP64 values
+  int n_settled;                     // FP64, FP32-mixed: DMP decisions of the last step settled from FP64 values
   int n_list;                        // cells the last step's limiter re-solved (recompute > 0)
   int nonfinite;                     // set when dt came out non-finite
   long long steps;

@@ -7,9 +7,9 @@
 // Advection-Diffusion/riemann_problem.f90:8-113 (viscous LLF).  One thread per
 // (face, point); the x faces of all instances come first, then the y faces.
 // R is the storage type of the face states and fluxes, CT the compute type.
-// FP64 (R = CT = double) is compiled with --fmad=false: every value agrees bit
-// for bit with the reference expression evaluated in FP64 from the same face
-// states.  The FP32 modes store states and fluxes in FP32; Euler and
+// FP64 (R = CT = double) is compiled with --fmad=false for the phase API: every
+// value agrees bit for bit with the reference expression evaluated in FP64 from
+// the same face states; the fused step takes the kRec form.  The FP32 modes store states and fluxes in FP32; Euler and
 // advection-diffusion compute in FP32, and Baer-Nunziato computes its
 // path-conservative flux (Roe-matrix path integral included) in FP64 in the
 // FP32-mixed mode (CT = double, instantiated with fused multiply-adds in

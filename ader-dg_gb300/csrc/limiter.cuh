@@ -8,10 +8,11 @@
 //     cell, persistent over the list; then put_subcell_data, the DMP of
 //     recompute = 2 cells, the next step's min/max and CFL contribution.
 //     update_limiter (Lh = NewLh) is the parity flip of the Lh buffers.
-// Compiled with --fmad=false, reference operation order throughout.  The FP64
-// and FP32-mixed modes run K4b in FP64 (T = double); the FP32-mixed mode adds
-// the settling of DMP comparisons against neighbourhood bounds that carry an
-// FP32 error bound.  The FP32-wide mode runs the re-solve in FP32 (T = float).
+// The FP64 and FP32-mixed modes run K4b in FP64 (T = double): the phase API with
+// --fmad=false in the reference's operation order, the FP64 fused step and the
+// FP32-mixed mode with the reciprocal-sharing forms (kRcp); DMP comparisons
+// against bounds that carry an FP32 error bound are settled from FP64 values.
+// The FP32-wide mode runs the re-solve in FP32 (T = float).
 #pragma once
 
 #include "cells.cuh"
@@ -136,7 +137,7 @@ __device__ __forceinline__ double minmod_bits(double a, double b) {
 }
 
 // Subgrid Rusanov flux (Euler/limiter.f90:361-378; BN :359-383 adds D = B~ dQ);
-// kRcp: the reciprocal-sharing physics forms (FP32-mixed mode), and F twice the
+// kRcp: the reciprocal-sharing physics forms, and F twice the
 // flux (the update takes half its factor: one FP64 instruction less a variable)
 template <class Sys, class T, int kRcp = 0>
 __device__ __forceinline__ void rusanov_s(const PhysC<T>& pc, const typename Sys::FConst& fcs, const T* QL, const T* QR,
@@ -486,7 +487,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       T Qt[V], FL[2 * V], FR[2 * V];
       // Euler computes slopes for interior subcells only (halo slopes stay 0,
       // Euler/limiter.f90:529-536); BN also on the halo (BN :486-492)
-      // FP32-mixed (FP64 re-solve): minmod on the bit patterns
+      // kRcp (FP64 re-solve): minmod on the bit patterns
       auto mm = [](T a, T b) -> T {
         if constexpr (kRcp && sizeof(T) == 8) return minmod_bits(a, b);
         else return minmod(a, b);
@@ -894,7 +895,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
 }
 
 
-// FP32-mixed: the DMP decisions k_cells left open (a.settle, a.list_count[1]
+// FP64 fused step and FP32-mixed: the DMP decisions k_cells left open (a.settle, a.list_count[1]
 // entries), from FP64 values in the reference's order.  One CTA per listed
 // cell, persistent over the list.  The cell's own subcell / Gauss-Lobatto /
 // nodal min and max come from its new state (fused step: uh[par ^ 1]; initial

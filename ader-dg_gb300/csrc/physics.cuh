@@ -41,9 +41,9 @@ template <class T> __device__ __forceinline__ T tmin(T a, T b) {
 template <class T> __device__ __forceinline__ T tsqrt(T x) {
   if constexpr (sizeof(T) == 4) return sqrtf(x); else return sqrt(x);
 }
-// Reciprocal and square root of the FP32-mixed mode's FP64 arithmetic (the
-// reciprocal-sharing physics *_r; the FP64 mode keeps the correctly rounded
-// operations and the reference's divisions).  The hardware's approximations
+// Reciprocal and square root of the FP64 arithmetic of the FP32-mixed mode and of
+// the FP64 fused step (the reciprocal-sharing physics *_r; the phase API keeps the
+// correctly rounded operations and the reference's divisions).  The hardware's approximations
 // (rcp.approx.ftz.f64, rsqrt.approx.ftz.f64) are refined by one third-order
 // Newton step, derived from the series of the exact quotients:
 //   1/x:     e = 1 - x r0,        1/x     = r0 / (1 - e)    ~ r0 (1 + e + e^2)
@@ -501,9 +501,10 @@ struct BNSys {
     roe_times_jump<double>(PhysC<double>(ph), QL, QR, d, D);
   }
   // Reciprocal-sharing forms for the FP64 face flux, subcell re-solve and CFL
-  // eigenvalues of the FP32-mixed mode and of the FP64 fused step (compiled with fused multiply-adds; values agree with the
-  // reference order to rounding).  Algebraically the reference expressions of
-  // Baer-Nunziato/pde.f90 with phi = alpha_s (Q8), phi_g = 1 - phi:
+  // eigenvalues of the FP32-mixed mode and of the FP64 fused step (compiled with
+  // fused multiply-adds; values agree with the reference order to rounding).
+  // Algebraically the reference expressions of Baer-Nunziato/pde.f90 with phi =
+  // alpha_s (Q8), phi_g = 1 - phi:
   //   phi p_s = (gamma_s - 1) (Q3 - (Q1^2 + Q2^2) / (2 Q0)) - gamma_s pi_s phi,
   //   phi rho_s u_s = Q1, (p_s + pi_s) / rho_s = (phi p_s + pi_s phi) / Q0,
   // and likewise for the gas with Q4..Q7 and phi_g; so a state needs 1/Q0

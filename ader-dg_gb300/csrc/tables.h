@@ -56,7 +56,7 @@ struct KernelTable {
   cudaError_t (*mark)(const BatchArgs&, cudaStream_t) = nullptr;
   cudaError_t (*subcell)(const BatchArgs&, const void* ops64, const FaceConst&, int grid, int fp32, cudaStream_t) = nullptr;
   int (*subcell_grid)(int num_sms, int fp32) = nullptr;
-  // FP32-mixed: DMP decisions k_cells left open, from FP64 values (k_settle);
+  // FP64 and FP32-mixed: DMP decisions k_cells left open, from FP64 values (k_settle);
   // grid CTAs persistent over the list
   cudaError_t (*settle)(const BatchArgs&, const void* ops64, int grid, cudaStream_t) = nullptr;
 };

@@ -454,16 +454,20 @@ def _profile_groups(groups):
     return tot, listed
 
 
+def _step_launches(aderdg, system, prec, limiter=True, nodes=None):
+    """Kernel launches of one step: control, predictor, faces, cells, [settle (FP64
+    and FP32-mixed), mark, subcell,] control; a small advection-diffusion grid's
+    cell kernel forms its face fluxes itself (common.cuh: faces_in_cells)."""
+    if system == aderdg.SYS_ADVDIFF:
+        return 4 if nodes is not None and nodes <= (65536 if prec == aderdg.FP64 else 131072) else 5
+    if not limiter:
+        return 5
+    return 7 if prec == aderdg.FP32_WIDE else 8
+
+
 def _launches_per_step(groups, prec, aderdg):
-    """Kernel launches of one step of every group: control, predictor, faces,
-    cells, [settle (FP32-mixed), mark, subcell,] control."""
-    n = 0
-    for key in groups:
-        if key[0] == aderdg.SYS_ADVDIFF:
-            n += 5
-        else:
-            n += 8 if prec == aderdg.FP32_MIXED else 7
-    return n
+    """Kernel launches of one step of every group (its simulations together)."""
+    return sum(_step_launches(aderdg, key[0], prec) for key in groups)
 
 
 def _err_stats(errs):
@@ -574,8 +578,7 @@ def run_single(args, aderdg, dist, rank, ws, lr):
                        "precision": args.precision, "l2": "flushed before every timed step"},
             "latency_ms": {"p50": float(np.percentile(ms, 50)), "p99": float(np.percentile(ms, 99))},
             "phase_ms": phases,
-            "gpu_launches": ((8 if prec == aderdg.FP32_MIXED else 7)
-                             if cfg.limiter and cfg.system != aderdg.SYS_ADVDIFF else 5) * args.steps,
+            "gpu_launches": _step_launches(aderdg, cfg.system, prec, cfg.limiter, cfg.cells * (cfg.N + 1) ** 2) * args.steps,
             "roofline": {"bound": "fp32" if prec == aderdg.FP32_MIXED else "fp64", "kernel": "k_predictor",
                          "achieved": ach, "peak": fpeak, "unit": "GFLOP/s", "frac": ach / fpeak, "traffic": None,
                          "peak_source": "aderdg_probe_peaks on this GPU"},

@@ -42,7 +42,12 @@ enum aderdg_status {
 };
 
 enum aderdg_system { ADERDG_SYS_ADVDIFF = 0, ADERDG_SYS_EULER = 1, ADERDG_SYS_BN = 2 };
-/* ADERDG_FP64: every phase in FP64 (the reference's arithmetic).
+/* ADERDG_FP64: every phase to FP64 accuracy.  The phase API evaluates the face
+ *   fluxes, surface integral, update, limiter and time step in the reference's
+ *   operation order; the fused step (aderdg_step, aderdg_run, batches) forms the
+ *   same values with fused multiply-adds, shared reciprocals and, in the
+ *   predictor, 60-bit fixed point, with rounding errors no larger, and takes the
+ *   DMP and positivity decisions of an FP64 evaluation of its state.
  * ADERDG_FP32_MIXED: the predictor, volume and surface contractions and the
  *   Euler / advection-diffusion face fluxes in FP32 with FP32 accumulation;
  *   FP64 for the update of the state (conservation), the Baer-Nunziato
@@ -199,7 +204,10 @@ enum aderdg_array {
   ADERDG_A_FP,           /* Fp(nVar,P,I+1,J) (BN) */
   ADERDG_A_GP,           /* Gp(nVar,P,I,J+1) (BN) */
   ADERDG_A_LH,           /* Lh(nVar,S,S,I,J) */
-  ADERDG_A_LMIN,         /* lmin(nVar,I,J): neighbourhood minimum used by the DMP */
+  /* lmin(nVar,I,J), lmax(nVar,I,J): neighbourhood minimum and maximum of the DMP.
+   * After a fused FP64 step, whose decisions need no exact values, they are formed
+   * on request from the state the step started from. */
+  ADERDG_A_LMIN,
   ADERDG_A_LMAX,
   ADERDG_A_RECOMPUTE,    /* int recompute(I,J) */
   ADERDG_A_STATUS        /* int status(I,J) */
@@ -224,8 +232,8 @@ typedef struct aderdg_info {
   double dt;
   int n_recompute;      /* last step */
   int n_limited;        /* cells with status != 0 after the last step */
-  int n_settled;        /* FP32-mixed: DMP decisions of the last step that the FP32
-                           error bounds left open and FP64 values settled */
+  int n_settled;        /* FP64 fused step and FP32-mixed: DMP decisions of the last step
+                           that the FP32 error bounds left open and FP64 values settled */
   int n_listed;         /* cells the last step's limiter re-solved (recompute > 0) */
 } aderdg_info;
 int aderdg_get_info(aderdg_ctx* ctx, aderdg_info* info);
@@ -276,7 +284,7 @@ int aderdg_batch_query(aderdg_batch* b, int slot, double* time, double* dt, long
 int aderdg_batch_download(aderdg_batch* b, int slot, double* uh);
 /* Sums over the batch's simulations of the last step's counters: troubled
  * cells (nRecompute), cells the limiter re-solved (recompute > 0) and, in the
- * FP32-mixed mode, DMP decisions settled from FP64 values. */
+ * FP64 and FP32-mixed modes, DMP decisions settled from FP64 values. */
 int aderdg_batch_counters(aderdg_batch* b, int* n_recompute, int* n_listed, int* n_settled);
 /* The simulation's limiter status(IMAX,JMAX) (as aderdg_download's status):
  * 1 for the cells its last step limited; zeros without the limiter. */
