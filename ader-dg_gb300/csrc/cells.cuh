@@ -377,6 +377,12 @@ __device__ __forceinline__ double cfl_denom(const InstDesc& in, const double* Q)
     return denom;
   }
 }
+// out of line, for kernels whose registers it would raise (the priming pass of the
+// FP64 fused step's kernel)
+template <class Sys, int N>
+static __device__ __noinline__ double cfl_denom_call(const InstDesc& in, const double* Q) {
+  return cfl_denom<Sys, N>(in, Q);
+}
 // The same from the reciprocal-sharing forms (the FP64 fused step): its divisions
 // and square roots were a third of the FP64 cell kernel's FP64 instructions (490 ->
 // 365 us on the Euler vortex N = 4 256^2, 453 -> 345 us on Baer-Nunziato N = 3 200^2)
@@ -791,7 +797,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       if (act) {
         double dn;
         if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
-        else if constexpr (kExact) dn = cfl_denom_r<Sys, N>(in, u);
+        else if constexpr (kExact) dn = mode == kCellFused ? cfl_denom_r<Sys, N>(in, u) : cfl_denom_call<Sys, N>(in, u);
         else dn = cfl_denom<Sys, N>(in, u);
         bits = (unsigned long long)__double_as_longlong(dn);
       }
@@ -804,7 +810,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       if (act) {
         double dn;
         if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
-        else if constexpr (kExact) dn = cfl_denom_r<Sys, N>(in, u);
+        else if constexpr (kExact) dn = mode == kCellFused ? cfl_denom_r<Sys, N>(in, u) : cfl_denom_call<Sys, N>(in, u);
         else dn = cfl_denom<Sys, N>(in, u);
         bits = (unsigned long long)__double_as_longlong(dn);
       }

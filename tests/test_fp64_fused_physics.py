@@ -79,3 +79,25 @@ def test_inadmissible_states(name, N, grid):
     # as the admissible states' comparison of both orders (sums of a step's few
     # hundred roundings)
     assert np.abs(a[ok] - b[ok]).max() <= 1e-12 * np.abs(b[ok]).max()
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 3, (17, 12)), ("bn_cylinder", 2, (13, 14)), ("euler_rp2d", 5, (8, 8))])
+def test_host_step(name, N, grid):
+    """A host step primes with certified bounds, upload with FP64 projections: the
+    same time step, decisions and state, bit for bit (every comparison the bounds
+    leave open is settled from FP64 values)."""
+    cfg, (uh, lh) = build(name, N, grid)
+    h, d = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (h, d):
+        s.upload(uh)
+        s.init_limiter(lh)
+    u, t = uh.copy(), 0.0
+    for _ in range(3):
+        st, l = h.download_limiter()
+        d.upload(u)
+        d.upload_limiter(st, l)
+        td, dtd, nd = d.step(t, 1e30)
+        t, dt, n = h.step_host(u, t, 1e30)
+        assert (t, dt, n) == (td, dtd, nd)
+        assert np.array_equal(u, d.download()[0]) and np.array_equal(h.get(aderdg.A_STATUS), d.get(aderdg.A_STATUS))
+        assert np.array_equal(h.get(aderdg.A_LMIN), d.get(aderdg.A_LMIN))
