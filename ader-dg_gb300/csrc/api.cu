@@ -41,6 +41,7 @@ struct aderdg_ctx {
   size_t bytes = 0;
   bool uploaded = false;
   bool pending = false;  // between element_update and the limiter commit (phase API)
+  bool mm_bounds = false;    // mm carries error bounds (FP64: the phase API forms the exact values first)
   bool lmin_bounds = false;  // lminmax holds a fused step's bounds (FP64: exact values on request)
   cudaGraphExec_t gexec = nullptr;
   void* flush_buf = nullptr;
@@ -138,8 +139,13 @@ int cells(aderdg_ctx* c, int mode) {
 }
 
 // min/max of the current state for the DMP neighbourhood and the CFL
-// denominators (get_min_max step 1 + calc_time_step's node loop)
+// denominators (get_min_max step 1 + calc_time_step's node loop).  FP64: the
+// min/max from certified FP32 projections, with their error bounds, which every
+// decision takes into account; the denominators, and so the next dt, in the
+// reference's order.  A host step of the Euler vortex N = 3 128^2 0.77 -> 0.62 ms,
+// the initial condition of the vortex N = 4 256^2 4.9 -> 1.5 ms.
 int prime(aderdg_ctx* c) {
+  c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
   CK(c, control(c, aderdg::kCtlPrimeReset));
   int r = cells(c, aderdg::kCellPrime);
   if (r) return r;
@@ -147,17 +153,12 @@ int prime(aderdg_ctx* c) {
   return ADERDG_OK;
 }
 
-// prime for a fused step that follows at once: the FP64 mode's certified FP32
-// projections (min/max with their error bounds, which the step's decisions take
-// into account); the CFL denominators, and so dt, in the reference's order as in
-// prime. A host step of the Euler vortex
-// N = 3 128^2 0.77 -> 0.62 ms (the FP64 projections took 0.2 ms of it).
-int prime_fused(aderdg_ctx* c) {
-  if (c->prec != ADERDG_FP64 || !c->args.mme[0]) return prime(c);
-  CK(c, control(c, aderdg::kCtlPrimeReset));
+// the min/max again for the phase API: FP64 projections in the reference's order
+int prime_exact(aderdg_ctx* c) {
+  if (c->prec != ADERDG_FP64) return cells(c, aderdg::kCellPrime);
+  c->mm_bounds = false;
   c->args.mode = aderdg::kCellPrime;
-  CK(c, c->kt->cells(c->args, c->ops64.data(), 2, c->stream));
-  CK(c, control(c, aderdg::kCtlPrimeCommit));
+  CK(c, c->kt->cells(c->args, c->ops64.data(), 0, c->stream));
   return ADERDG_OK;
 }
 
@@ -237,7 +238,7 @@ void free_all(aderdg_ctx* c) {
 }
 
 int ensure_graph(aderdg_ctx* c) {
-  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
+  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
   if (c->gexec) return ADERDG_OK;
   cudaGraph_t g = nullptr;
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -681,7 +682,7 @@ int aderdg_limiter_prepare(aderdg_ctx* c) {
   // get_min_max step 1 into the current min/max buffer; the CFL accumulator
   // it also feeds is cleared again by the next calc_time_step
   CK(c, control(c, aderdg::kCtlPrimeReset));
-  return cells(c, aderdg::kCellPrime);
+  return prime_exact(c);
 }
 
 int aderdg_space_time_predictor(aderdg_ctx* c) {
@@ -716,6 +717,8 @@ int aderdg_element_update(aderdg_ctx* c, int* n_recompute) {
   if (!c) return fail(c, ADERDG_EINVAL, "null context");
   if (c->pending) return fail(c, ADERDG_ESTATE, "element update already applied");
   c->lmin_bounds = false;
+  if (c->mm_bounds)  // a caller that left out aderdg_limiter_prepare
+    if (int r = prime_exact(c)) return r;
   CK(c, cudaMemsetAsync(&c->d_st->n_recompute, 0, sizeof(int), c->stream));
   CK(c, cudaMemsetAsync(&c->d_st->denom_next, 0, sizeof(unsigned long long), c->stream));
   int r = cells(c, aderdg::kCellUpdate);
@@ -747,7 +750,7 @@ int aderdg_step(aderdg_ctx* c, double* time, double tend, double* dt, int* n_rec
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
-  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
+  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
   r = launch_step(c);
   if (r) return r;
   r = pull_state(c);
@@ -792,7 +795,7 @@ int aderdg_step_host(aderdg_ctx* c, double* uh, double* time, double tend, doubl
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   const size_t n = (size_t)c->ncells * c->P * c->P * c->V * sizeof(double);
   CK(c, cudaMemcpyAsync(c->args.uh[cur_par(c)], uh, n, cudaMemcpyHostToDevice, c->stream));
-  int r = prime_fused(c);
+  int r = prime(c);
   if (!r) r = set_clock(c, *time, tend);
   if (!r) r = ensure_graph(c);
   if (r) return r;
@@ -854,7 +857,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
-  c->lmin_bounds = c->limiter && c->prec == ADERDG_FP64;
+  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
   cudaEvent_t ev[8];
   for (auto& e : ev) CK(c, cudaEventCreate(&e));
   CK(c, cudaEventRecord(ev[0], c->stream));

@@ -104,8 +104,10 @@ inline cudaError_t launch_cells(const KernelTable* kt, const BatchArgs& a, const
   if (fast) {
     const int v = tuning_of(kt->sys, kt->N, precision).cells;
     if (v > 0 && v < kCellVariantsMax && kt->cells_var[v]) return kt->cells_var[v](a, ops64, s);
-  } else if (a.mode == kCellFused && a.mme[0]) {
-    return kt->cells(a, ops64, 2, s);  // FP64 update, certified FP32 projections
+  } else if (a.mme[0] && a.mode != kCellSurface && a.mode != kCellUpdate && a.mode != kCellCfl) {
+    // the fused step, priming and the initial limiter: certified FP32 projections
+    // (the phase API's passes stay in the reference's FP64 order)
+    return kt->cells(a, ops64, 2, s);
   }
   return kt->cells(a, ops64, fast, s);
 }

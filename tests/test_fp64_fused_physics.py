@@ -101,3 +101,26 @@ def test_host_step(name, N, grid):
         assert (t, dt, n) == (td, dtd, nd)
         assert np.array_equal(u, d.download()[0]) and np.array_equal(h.get(aderdg.A_STATUS), d.get(aderdg.A_STATUS))
         assert np.array_equal(h.get(aderdg.A_LMIN), d.get(aderdg.A_LMIN))
+
+
+@pytest.mark.parametrize("fused_first", [False, True])
+def test_phases_without_limiter_prepare(gpu_lib, fused_first):
+    """The phase API forms exact minima and maxima itself where the caller leaves out
+    limiter_prepare after an upload or a fused step."""
+    cfg, (uh, lh) = build("euler_rp2d", 3, (13, 10))
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (a, b):
+        s.upload(uh)
+        s.init_limiter(lh)
+        t = s.step(0.0, 1e30)[0] if fused_first else 0.0
+        s.calc_time_step(t, 1e30)
+        if s is a:
+            s.limiter_prepare()
+        s.space_time_predictor()
+        s.volume_integral()
+        s.riemann_problem()
+        s.surface_integral()
+        s.element_update()
+        s.limiter()
+    for w in (aderdg.A_UH, aderdg.A_LMIN, aderdg.A_LMAX, aderdg.A_STATUS, aderdg.A_RECOMPUTE):
+        assert np.array_equal(a.get(w), b.get(w)), w
