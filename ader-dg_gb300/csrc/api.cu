@@ -384,7 +384,6 @@ int aderdg_create(const aderdg_config* cfg, aderdg_ctx** out) {
     delete c;
     return fail(nullptr, ADERDG_EINVAL, why);
   }
-  aderdg::build_fine(c->ops);
   auto bail = [&](int code) {
     free_all(c);
     delete c;

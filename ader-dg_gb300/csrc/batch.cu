@@ -320,7 +320,6 @@ int aderdg_batch_create(int system, int N, int precision, int limiter, long capa
     return code;
   };
   if (!aderdg::build_ops(N, b->ops, &why)) return bail(bfail(nullptr, ADERDG_EINVAL, why));
-  aderdg::build_fine(b->ops);
   b->fc = aderdg::make_face_const(b->ops);
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

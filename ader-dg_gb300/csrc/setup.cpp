@@ -12,6 +12,7 @@
 #include "ic_eval.h"
 
 #include <cmath>
+#include <mutex>
 
 #include "../../include/aderdg_gpu.h"
 
@@ -172,8 +173,6 @@ Dd operator/(Dd a, Dd b) {
   return Dd(q0, q1) + Dd(r.h / b.h);
 }
 
-}  // namespace
-
 // HostOps::Fine from the FP64 nodes and iK1: Newton steps on the Legendre
 // polynomial and on the inverse.
 void build_fine(HostOps& o) {
@@ -265,18 +264,7 @@ void build_fine(HostOps& o) {
   split(KG, o.fKG);
 }
 
-double pi_value() { return kPi; }
-
-double pnpm_cfl(int N) {
-  static const double t[10] = {1.0, 0.33, 0.17, 0.1, 0.069, 0.045, 0.038, 0.03, 0.02, 0.015};
-  return (N >= 0 && N <= 9) ? t[N] : 0.0;
-}
-
-bool build_ops(int N, HostOps& o, std::string* err) {
-  if (N < 1 || N > 9) {
-    if (err) *err = "N out of range";
-    return false;
-  }
+bool compute_ops(int N, HostOps& o, std::string* err) {
   const int P = N + 1, S = 2 * N + 1;
   o.N = N;
   o.P = P;
@@ -371,6 +359,39 @@ bool build_ops(int N, HostOps& o, std::string* err) {
   o.xilimbary.assign(S, 0.0);
   for (int s = 1; s <= S; ++s) o.xilimbary[s - 1] = 0.0 + 0.5 / (double)S + (double)(s - 1) * 1.0 / (double)S;
   return true;
+}
+
+}  // namespace
+
+double pi_value() { return kPi; }
+
+double pnpm_cfl(int N) {
+  static const double t[10] = {1.0, 0.33, 0.17, 0.1, 0.069, 0.045, 0.038, 0.03, 0.02, 0.015};
+  return (N >= 0 && N <= 9) ? t[N] : 0.0;
+}
+
+// The operators depend on the degree alone: computed once per degree and process
+// (20 to 200 us), since every context, initial field and output call asks for them.
+bool build_ops(int N, HostOps& o, std::string* err) {
+  if (N < 1 || N > 9) {
+    if (err) *err = "N out of range";
+    return false;
+  }
+  struct Entry {
+    std::once_flag once;
+    bool ok = false;
+    HostOps ops;
+    std::string why;
+  };
+  static Entry table[10];
+  Entry& t = table[N];
+  std::call_once(t.once, [&] {
+    t.ok = compute_ops(N, t.ops, &t.why);
+    if (t.ok) build_fine(t.ops);
+  });
+  if (t.ok) o = t.ops;
+  else if (err) *err = t.why;
+  return t.ok;
 }
 
 }  // namespace aderdg

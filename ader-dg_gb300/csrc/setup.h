@@ -35,10 +35,6 @@ struct HostOps {
 };
 
 bool build_ops(int N, HostOps& ops, std::string* err);
-// The operators to twice FP64 (HostOps::Fine), after build_ops: contexts only,
-// which keep them; the calls that build operators anew (initial fields, outputs)
-// do without.
-void build_fine(HostOps& ops);
 
 // Maximum CFL numbers of the PNPM schemes, Euler/ader_dg.f90:28.
 double pnpm_cfl(int N);
