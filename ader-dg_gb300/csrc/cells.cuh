@@ -102,26 +102,26 @@ struct Proj {
         else st<NLB>(LB, (s - S) * PS + ii, acc);
       }
     } else {
-    for (int idx = r; idx < P * S; idx += nr) {
-      const int ii = idx % P, s = idx / P;
+      for (int idx = r; idx < P * S; idx += nr) {
+        const int ii = idx % P, s = idx / P;
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        T acc = 0;
+        for (int v = 0; v < V; ++v) {
+          T acc = 0;
 #pragma unroll
-        for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, U[v * P2 + ii + P * k], lim[s + S * k]);
-        LY[(v * S + s) * P + ii] = acc;
+          for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, U[v * P2 + ii + P * k], lim[s + S * k]);
+          LY[(v * S + s) * P + ii] = acc;
+        }
       }
-    }
-    for (int idx = r; idx < P * P; idx += nr) {
-      const int ii = idx % P, s = idx / P;
+      for (int idx = r; idx < P * P; idx += nr) {
+        const int ii = idx % P, s = idx / P;
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        T acc = 0;
+        for (int v = 0; v < V; ++v) {
+          T acc = 0;
 #pragma unroll
-        for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, U[v * P2 + ii + P * k], lob[s + P * k]);
-        LB[(v * P + s) * P + ii] = acc;
+          for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, U[v * P2 + ii + P * k], lob[s + P * k]);
+          LB[(v * P + s) * P + ii] = acc;
+        }
       }
-    }
     }
   }
   // T = float: sum over k of item (s2, k) times c[k * stride]
@@ -145,12 +145,12 @@ struct Proj {
       row<NLY>(LY, lim + s1, S, s2, out);
     } else {
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      T acc = 0;
+      for (int v = 0; v < V; ++v) {
+        T acc = 0;
 #pragma unroll
-      for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LY[(v * S + s2) * P + k], lim[s1 + S * k]);
-      out[v] = acc;
-    }
+        for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LY[(v * S + s2) * P + k], lim[s1 + S * k]);
+        out[v] = acc;
+      }
     }
   }
   template <bool kFast = false>
@@ -159,12 +159,12 @@ struct Proj {
       row<NLB>(LB, lob + s1, P, s2, out);
     } else {
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-      T acc = 0;
+      for (int v = 0; v < V; ++v) {
+        T acc = 0;
 #pragma unroll
-      for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LB[(v * P + s2) * P + k], lob[s1 + P * k]);
-      out[v] = acc;
-    }
+        for (int k = 0; k < P; ++k) acc = madd<kFast>(acc, LB[(v * P + s2) * P + k], lob[s1 + P * k]);
+        out[v] = acc;
+      }
     }
   }
   // x pass fused with min/max (integer keys) and the positivity test of every subcell (FP64)

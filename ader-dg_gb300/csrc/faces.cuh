@@ -231,7 +231,9 @@ __device__ __forceinline__ R ad_face_flux(const BatchArgs& a, const InstDesc& in
 
 // kRec (FP64): the reciprocal-sharing forms, for the fused step (the phase API
 // keeps the reference's operation order): Euler N = 4 256^2 139 -> 96 us,
-// Baer-Nunziato N = 3 200^2 432 -> 143 us
+// Baer-Nunziato N = 3 200^2 432 -> 143 us.  FP32-mixed Baer-Nunziato: three CTAs an
+// SM (80 registers, 16 bytes spilled) and the rounding on the integer pipe: 462 ->
+// 405 us, cylinder N = 3 400^2
 template <class Sys, int N, class R, class CT, bool kRec = false>
 __global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && sizeof(CT) == 8 ? 3 : 1) k_faces(BatchArgs a, FaceConst fc) {
   constexpr int P = N + 1, V = Sys::V;

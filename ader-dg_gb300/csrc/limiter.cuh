@@ -76,7 +76,8 @@ struct SubCfg {
   static constexpr int H = S + 2;  // reconstructed region: 0 .. S+1
   static constexpr int THREADS = 128;
   // CTAs per SM the register allocation aims at.  FP32: one more than the
-  // unconstrained allocation allows where that does not spill.  FP64 (the
+  // unconstrained allocation allows where that does not spill (Baer-Nunziato N = 4:
+  // 3 CTAs at 158 registers 59 us, 2 at 175 82 us, cylinder 97 x 61).  FP64 (the
   // FP64 pipe bounds it): as many as shared memory admits, up to 4 (Euler:
   // 128 registers; Baer-Nunziato N = 2 and 3: 4 at 128 registers, about 130
   // bytes spilled, 8% and 2% faster than 3 unspilled; N = 4: 2; N = 5: 1), so
