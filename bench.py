@@ -581,7 +581,11 @@ def run_single(args, aderdg, dist, rank, ws, lr):
             "gpu_launches": _step_launches(aderdg, cfg.system, prec, cfg.limiter, cfg.cells * (cfg.N + 1) ** 2) * args.steps,
             "roofline": {"bound": "fp32" if prec == aderdg.FP32_MIXED else "fp64", "kernel": "k_predictor",
                          "achieved": ach, "peak": fpeak, "unit": "GFLOP/s", "frac": ach / fpeak, "traffic": None,
-                         "peak_source": "aderdg_probe_peaks on this GPU"},
+                         "peak_source": "aderdg_probe_peaks on this GPU",
+                         **({"note": "the flop model's operations over the kernel's time against the FP64 FMA peak: "
+                                     "the contractions run in fixed point on the integer pipe (Euler and "
+                                     "Baer-Nunziato, N >= 3) or as one operator a direction (advection-diffusion), "
+                                     "so that peak is no bound"} if prec == aderdg.FP64 else {})},
             "e2e": {"value": cfg.dofs * n_e / e2e_s, "unit": UNIT, "h2d_bytes_per_step": cfg.dofs * 8,
                     "d2h_bytes_per_step": cfg.dofs * 8, "api": "aderdg_step_host"},
             "clocks": clk.summary(), "limited_cells": info["n_limited"], "to_tend": to_tend}
