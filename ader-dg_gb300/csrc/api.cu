@@ -719,7 +719,11 @@ int aderdg_element_update(aderdg_ctx* c, int* n_recompute) {
   if (c->mm_bounds)  // a caller that left out aderdg_limiter_prepare
     if (int r = prime_exact(c)) return r;
   CK(c, cudaMemsetAsync(&c->d_st->n_recompute, 0, sizeof(int), c->stream));
+  CK(c, cudaMemsetAsync(&c->d_st->n_settled, 0, sizeof(int), c->stream));
   CK(c, cudaMemsetAsync(&c->d_st->denom_next, 0, sizeof(unsigned long long), c->stream));
+  // a caller that gave the time step itself may have issued no reset since the
+  // pass that last filled the settle list (ncells entries: one pass at a time)
+  CK(c, cudaMemsetAsync(c->args.list_count + 1, 0, sizeof(int), c->stream));
   int r = cells(c, aderdg::kCellUpdate);
   if (r) return r;
   if (!c->limiter) CK(c, control(c, aderdg::kCtlEnd));
