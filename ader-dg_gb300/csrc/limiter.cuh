@@ -641,12 +641,13 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     // its subcell data), uniform per CTA.  FP32 projections of the deviations
     // from the new polynomial's node-0 state when their error bound stays
     // within the DMP's absolute tolerance, else FP64 (as in the cell kernel).
-    // T = double: a comparison the bounds leave open is decided from FP64 values
-    // below; T = float (FP32-wide): the FP32 values are taken as they are.  (The
-    // FP64 re-solve projected in FP64 throughout before: a fifth of its FP64
-    // instructions on a recompute = 2 cell.)
+    // kRcp: a comparison the bounds leave open is decided from FP64 values below
+    // (FP64 projections are a fifth of the FP64 instructions of a recompute = 2
+    // cell).  T = float (FP32-wide): the FP32 values are taken as they are.  The
+    // phase API (T = double without kRcp) projects in FP64: its next step may take
+    // the stored min/max as they are.
     const bool dmp = rec == 2;
-    const bool try32 = sizeof(T) == 4 || a.mme[0] != nullptr;
+    const bool try32 = sizeof(T) == 4 || (kRcp && a.mme[0] != nullptr);
     const float* lim32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(limT) : limf;
     const float* lob32 = sizeof(T) == 4 ? reinterpret_cast<const float*>(lobT) : limf + S * P;
     if (dmp && try32) {

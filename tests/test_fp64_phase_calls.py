@@ -62,3 +62,25 @@ def test_given_time_step_after_settled_cells(name, N, grid):
         for w in (aderdg.A_RECOMPUTE, aderdg.A_STATUS, aderdg.A_UH):
             assert np.array_equal(a.get(w), b.get(w)), (k, w)
         t = ra[0]
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 3, (13, 10)), ("bn_cylinder", 2, (13, 14))])
+def test_phase_steps_without_prepare(name, N, grid):
+    """Consecutive phase steps form the same minima and maxima with and without
+    limiter_prepare, recompute = 2 cells that stay unlimited among them."""
+    cfg, (uh, lh) = build(name, N, grid)
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (a, b):
+        s.upload(uh)
+        s.init_limiter(lh)
+    t, kept = 0.0, 0
+    for k in range(4):
+        ra, rb = phase_step(a, t), phase_step(b, t, prepare=False)
+        assert ra[:4] == rb[:4], k
+        for x, y in zip(ra[4], rb[4]):
+            assert np.array_equal(x, y), k
+        for w in (aderdg.A_RECOMPUTE, aderdg.A_STATUS, aderdg.A_UH):
+            assert np.array_equal(a.get(w), b.get(w)), (k, w)
+        kept += int(((a.get(aderdg.A_RECOMPUTE) == 2) & (a.get(aderdg.A_STATUS) == 0)).sum())
+        t = ra[0]
+    assert kept > 0
