@@ -42,7 +42,10 @@ struct aderdg_ctx {
   bool uploaded = false;
   bool pending = false;  // between element_update and the limiter commit (phase API)
   bool mm_bounds = false;    // mm carries error bounds (FP64: the phase API forms the exact values first)
-  bool lmin_bounds = false;  // lminmax holds a fused step's bounds (FP64: exact values on request)
+  // lminmax holds the bounds of the last step, a fused FP64 one, whose exact values
+  // are formed on request.  Nothing but a step writes uh, mm and mme of the other
+  // parity, so uploads and initial fields leave it as it is.
+  bool lmin_bounds = false;
   cudaGraphExec_t gexec = nullptr;
   void* flush_buf = nullptr;
   size_t flush_bytes = 0;
@@ -172,45 +175,62 @@ int set_clock(aderdg_ctx* c, double time, double tend) {
   return ADERDG_OK;
 }
 
-// neighbourhood min/max (get_min_max step 2, Euler/limiter.f90:147-167) of the
-// per-cell values mm[par ^ 1] of a context's single instance
-__global__ void k_neighbourhood(BatchArgs a, int V) {
+// neighbourhood min/max (get_min_max step 2, Euler/limiter.f90:147-167) of the last
+// step of a context's single instance, from the per-cell values it started with,
+// mm of the other parity; of a cell whose values carry an error bound, from exact
+__global__ void k_neighbourhood(BatchArgs a, int V, const double* exact) {
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= a.ncells * V) return;
   const long long cell = k / V;
   const int v = (int)(k - cell * V);
   const InstDesc& in = a.inst[0];
-  const int ci = (int)(cell % in.imax), cj = (int)(cell / in.imax);
-  const double* mm = a.mm[aderdg::parity(a.st[0])];
-  double lo = mm[cell * 2 * V + v], hi = mm[cell * 2 * V + V + v];
-  for (int jj = -1; jj <= 1; ++jj)
-    for (int ii = -1; ii <= 1; ++ii) {
-      const long long nc = aderdg::nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]) +
-                           (long long)in.imax * aderdg::nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
-      lo = fmin(lo, mm[nc * 2 * V + v]);
-      hi = fmax(hi, mm[nc * 2 * V + V + v]);
-    }
+  const int ci = (int)(cell % in.imax), cj = (int)(cell / in.imax), par = aderdg::parity(a.st[0]) ^ 1;
+  double lo = 0.0, hi = 0.0;
+  for (int n = 0; n < 10; ++n) {  // the cell, then its neighbourhood
+    const int ii = n ? (n - 1) % 3 - 1 : 0, jj = n ? (n - 1) / 3 - 1 : 0;
+    const long long nc = aderdg::nb_index(ci, ii, in.imax, in.bc[0], in.bc[1]) +
+                         (long long)in.imax * aderdg::nb_index(cj, jj, in.jmax, in.bc[2], in.bc[3]);
+    bool bounded = false;
+    for (int w = 0; w < V; ++w) bounded = bounded || a.mme[par][nc * V + w] > 0.0f;
+    const double* m = (bounded ? exact : a.mm[par]) + nc * 2 * V;
+    lo = n ? fmin(lo, m[v]) : m[v];
+    hi = n ? fmax(hi, m[V + v]) : m[V + v];
+  }
   a.lminmax[cell * 2 * V + v] = lo;
   a.lminmax[cell * 2 * V + V + v] = hi;
 }
 
 // FP64: a fused step decides its DMP from bounds on the per-cell min/max; the
-// exact lmin/lmax of that step, from its start-of-step state, which the other
-// parity's buffers still hold
+// exact lmin/lmax of that step.  Its start-of-step state and min/max are those of
+// the other parity; limited cells, whose min/max come from their subcell data,
+// carry no bound (the status and Lh of that parity may be those of a new initial
+// field).
 int exact_lminmax(aderdg_ctx* c) {
+  const long long n = c->ncells * c->V;
+  double* tmp = nullptr;  // exact min/max of the projections, and a status of zeros
+  const size_t bytes = 2 * n * sizeof(double);
+  CK(c, cudaMallocAsync(&tmp, bytes + c->ncells * sizeof(int), c->stream));
   BatchArgs z = c->args;
   std::swap(z.uh[0], z.uh[1]);
-  std::swap(z.status[0], z.status[1]);
-  std::swap(z.lh[0], z.lh[1]);
-  std::swap(z.mm[0], z.mm[1]);
-  std::swap(z.mme[0], z.mme[1]);
+  z.mm[0] = z.mm[1] = tmp;
+  z.mme[0] = z.mme[1] = nullptr;
+  z.status[0] = z.status[1] = reinterpret_cast<int*>(tmp + 2 * n);
   z.mode = aderdg::kCellPrime;
-  CK(c, c->kt->cells(z, c->ops64.data(), 0, c->stream));
-  const long long n = c->ncells * c->V;
-  k_neighbourhood<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(z, c->V);
-  CK(c, cudaGetLastError());
+  cudaError_t e = cudaMemsetAsync(z.status[0], 0, c->ncells * sizeof(int), c->stream);
+  if (e == cudaSuccess) e = c->kt->cells(z, c->ops64.data(), 0, c->stream);
+  if (e == cudaSuccess) {
+    k_neighbourhood<<<(unsigned)((n + 255) / 256), 256, 0, c->stream>>>(c->args, c->V, tmp);
+    e = cudaGetLastError();
+  }
+  cudaFreeAsync(tmp, c->stream);
+  CK(c, e);
   c->lmin_bounds = false;
   return ADERDG_OK;
+}
+
+// after a call that took fused steps (state pulled): what the last one left
+void stepped(aderdg_ctx* c, long long steps_before) {
+  if (c->limiter && c->prec == ADERDG_FP64 && c->h_st->steps > steps_before) c->lmin_bounds = c->mm_bounds = true;
 }
 
 // one fused loop body of main.f90
@@ -238,7 +258,6 @@ void free_all(aderdg_ctx* c) {
 }
 
 int ensure_graph(aderdg_ctx* c) {
-  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
   if (c->gexec) return ADERDG_OK;
   cudaGraph_t g = nullptr;
   CK(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
@@ -489,7 +508,6 @@ int aderdg_destroy(aderdg_ctx* ctx) {
 
 int aderdg_upload(aderdg_ctx* c, const double* uh) {
   if (!c || !uh) return fail(c, ADERDG_EINVAL, "null argument");
-  c->lmin_bounds = false;
   const int par = cur_par(c);
   const size_t n = (size_t)c->ncells * c->P * c->P * c->V;
   CK(c, cudaMemcpyAsync(c->args.uh[par], uh, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
@@ -533,7 +551,6 @@ int aderdg_init_limiter(aderdg_ctx* c, const double* lh_ic, int* n_limited) {
 int aderdg_initial_condition(aderdg_ctx* c, int ic, const double* params, int* n_limited) {
   if (!c) return fail(c, ADERDG_EINVAL, "null context");
   if (n_limited) *n_limited = 0;
-  c->lmin_bounds = false;
   const int par = cur_par(c);
   // the subcell candidates are formed after the initial DMP, for the cells it
   // limits only, in both Lh buffers
@@ -753,11 +770,12 @@ int aderdg_step(aderdg_ctx* c, double* time, double tend, double* dt, int* n_rec
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
-  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
+  const long long steps0 = c->h_st->steps;
   r = launch_step(c);
   if (r) return r;
   r = pull_state(c);
   if (r) return r;
+  stepped(c, steps0);
   *time = c->h_st->time;
   if (dt) *dt = c->h_st->dt;
   if (n_recompute) *n_recompute = c->h_st->n_recompute;
@@ -784,6 +802,7 @@ int aderdg_run(aderdg_ctx* c, double* time, double tend, int max_steps, int sync
     launched += n;
     r = pull_state(c);
     if (r) return r;
+    stepped(c, steps0);
     if (c->h_st->nonfinite || !(c->h_st->time < tend)) break;
   }
   *time = c->h_st->time;
@@ -802,9 +821,11 @@ int aderdg_step_host(aderdg_ctx* c, double* uh, double* time, double tend, doubl
   if (!r) r = set_clock(c, *time, tend);
   if (!r) r = ensure_graph(c);
   if (r) return r;
+  const long long steps0 = c->h_st->steps;
   CK(c, cudaGraphLaunch(c->gexec, c->stream));
-  CK(c, cudaMemcpyAsync(c->h_st, c->d_st, sizeof(InstState), cudaMemcpyDeviceToHost, c->stream));
-  CK(c, cudaStreamSynchronize(c->stream));
+  r = pull_state(c);
+  if (r) return r;
+  stepped(c, steps0);
   CK(c, cudaMemcpyAsync(uh, c->args.uh[cur_par(c)], n, cudaMemcpyDeviceToHost, c->stream));
   CK(c, cudaStreamSynchronize(c->stream));
   *time = c->h_st->time;
@@ -821,6 +842,7 @@ int aderdg_time_steps(aderdg_ctx* c, double* time, double tend, int steps, int f
   int r = set_clock(c, *time, tend);
   if (!r) r = ensure_graph(c);
   if (r) return r;
+  const long long steps0 = c->h_st->steps;
   if (flush_l2 && !c->flush_buf) {
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c->device);
@@ -849,6 +871,7 @@ int aderdg_time_steps(aderdg_ctx* c, double* time, double tend, int steps, int f
   for (auto& e : ev) cudaEventDestroy(e);
   r = pull_state(c);
   if (r) return r;
+  stepped(c, steps0);
   *time = c->h_st->time;
   if (c->h_st->nonfinite) return fail(c, ADERDG_ENONFINITE, "the time step became non-finite");
   return ADERDG_OK;
@@ -860,7 +883,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   if (c->pending) return fail(c, ADERDG_ESTATE, "finish the phase-API step first");
   int r = set_clock(c, *time, tend);
   if (r) return r;
-  c->lmin_bounds = c->mm_bounds = c->limiter && c->prec == ADERDG_FP64;
+  const long long steps0 = c->h_st->steps;
   cudaEvent_t ev[8];
   for (auto& e : ev) CK(c, cudaEventCreate(&e));
   CK(c, cudaEventRecord(ev[0], c->stream));
@@ -889,6 +912,7 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   for (auto& e : ev) cudaEventDestroy(e);
   r = pull_state(c);
   if (r) return r;
+  stepped(c, steps0);
   *time = c->h_st->time;
   return ADERDG_OK;
 }

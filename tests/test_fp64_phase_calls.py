@@ -84,3 +84,67 @@ def test_phase_steps_without_prepare(name, N, grid):
         kept += int(((a.get(aderdg.A_RECOMPUTE) == 2) & (a.get(aderdg.A_STATUS) == 0)).sum())
         t = ra[0]
     assert kept > 0
+
+
+BOUNDS = (aderdg.A_LMIN, aderdg.A_LMAX)
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 3, (13, 10)), ("bn_cylinder", 2, (13, 14))])
+@pytest.mark.parametrize("then", ["no_step", "no_run", "no_host_step", "upload", "upload_no_step", "initial_condition",
+                                  "init_limiter", "upload_limiter", "limiter_prepare"])
+def test_bounds_of_the_last_step_on_request(name, N, grid, then):
+    """lmin and lmax stay those of the last step taken, whatever comes between it
+    and the request short of another step."""
+    cfg, ic, params, _ = aderdg.workloads.make(name, side=8, N=N)
+    cfg = dataclasses.replace(cfg, imax=grid[0], jmax=grid[1])
+    uh, lh = aderdg.project_initial_condition(cfg, ic, params)
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (a, b):
+        s.upload(uh)
+        s.init_limiter(lh)
+        t = s.run(0.0, 1e30, 5)[0]
+    want = [a.get(w) for w in BOUNDS]
+    st, l = a.download_limiter()
+    assert st.any()
+    other = 1.5 * uh
+    if then == "no_step":
+        b.step(t, t)
+    elif then == "no_run":
+        b.run(t, t, 3)
+    elif then == "no_host_step":
+        b.step_host(b.download()[0], t, t)
+    elif then == "upload":
+        b.upload(other)
+    elif then == "upload_no_step":
+        b.upload(other)
+        b.step(t, t)
+    elif then == "initial_condition":
+        b.initial_condition(ic, params)
+    elif then == "init_limiter":
+        b.upload(other)
+        b.init_limiter(2.0 * lh)
+    elif then == "upload_limiter":
+        b.upload_limiter(np.zeros_like(st), 2.0 * l)
+    else:
+        b.calc_time_step(t, 1e30)
+        b.limiter_prepare()
+    for w, x in zip(BOUNDS, want):
+        assert np.array_equal(b.get(w), x), w
+    assert all(np.array_equal(a.get(w), x) for w, x in zip(BOUNDS, want))  # a second request: the same
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 3, (13, 10)), ("bn_cylinder", 2, (13, 14))])
+def test_bounds_are_those_of_the_phases(name, N, grid):
+    """After several fused steps on one trajectory, lmin and lmax of the last equal
+    those the phase API forms from its start state."""
+    cfg, (uh, lh) = build(name, N, grid)
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    a.upload(uh)
+    a.init_limiter(lh)
+    t = a.run(0.0, 1e30, 4)[0]
+    b.upload(a.download()[0])
+    b.upload_limiter(*a.download_limiter())
+    a.step(t, 1e30)
+    r = phase_step(b, t)
+    for w, x in zip(BOUNDS, r[4]):
+        assert np.array_equal(a.get(w), x), w
