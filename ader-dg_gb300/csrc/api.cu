@@ -241,8 +241,9 @@ int launch_step(aderdg_ctx* c) {
   int r = cells(c, aderdg::kCellFused);
   if (r) return r;
   if (c->limiter) {
-    CK(c, c->kt->mark(c->args, c->stream));
+    CK(c, aderdg::launch_mark(c->kt, c->args, c->prec, c->stream, true));
     CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, true));
+    CK(c, aderdg::launch_cfl(c->kt, c->args, c->prec, c->stream));
   }
   CK(c, control(c, aderdg::kCtlEnd));
   return ADERDG_OK;
@@ -756,7 +757,7 @@ int aderdg_limiter(aderdg_ctx* c) {
   if (!c->limiter) return ADERDG_OK;
   if (!c->pending) return fail(c, ADERDG_ESTATE, "run aderdg_element_update first");
   CK(c, cudaMemsetAsync(c->args.list_count, 0, sizeof(int), c->stream));
-  CK(c, c->kt->mark(c->args, c->stream));
+  CK(c, aderdg::launch_mark(c->kt, c->args, c->prec, c->stream, false));
   CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, false));
   CK(c, control(c, aderdg::kCtlEnd));
   c->pending = false;
@@ -896,11 +897,12 @@ int aderdg_profile_step(aderdg_ctx* c, double* time, double tend, double* phase_
   r = cells(c, aderdg::kCellFused);
   if (r) return r;
   CK(c, cudaEventRecord(ev[4], c->stream));
-  if (c->limiter) CK(c, c->kt->mark(c->args, c->stream));
+  if (c->limiter) CK(c, aderdg::launch_mark(c->kt, c->args, c->prec, c->stream, true));
   CK(c, cudaEventRecord(ev[5], c->stream));
   if (c->limiter)
     CK(c, aderdg::launch_subcell(c->kt, c->args, c->ops64.data(), c->fc, c->subcell_grid, c->num_sms, c->prec, c->stream, true));
   CK(c, cudaEventRecord(ev[6], c->stream));
+  if (c->limiter) CK(c, aderdg::launch_cfl(c->kt, c->args, c->prec, c->stream));
   CK(c, control(c, aderdg::kCtlEnd));
   CK(c, cudaEventRecord(ev[7], c->stream));
   CK(c, cudaStreamSynchronize(c->stream));

@@ -225,8 +225,9 @@ int blaunch_step(aderdg_batch* b) {
   BK(b, aderdg::launch_cells(b->kt, a, b->ops64.data(), b->precision, b->stream));
   if (a.settle) BK(b, b->kt->settle(a, b->ops64.data(), b->num_sms, b->stream));
   if (b->limiter) {
-    BK(b, b->kt->mark(a, b->stream));
+    BK(b, aderdg::launch_mark(b->kt, a, b->precision, b->stream, true));
     BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream, true));
+    BK(b, aderdg::launch_cfl(b->kt, a, b->precision, b->stream));
   }
   BK(b, bcontrol(b, aderdg::kCtlEnd, -1));
   return ADERDG_OK;
@@ -778,11 +779,12 @@ int aderdg_batch_profile(aderdg_batch* b, double* phase_ms) {
   BK(b, aderdg::launch_cells(b->kt, a, b->ops64.data(), b->precision, b->stream));
   if (a.settle) BK(b, b->kt->settle(a, b->ops64.data(), b->num_sms, b->stream));
   BK(b, cudaEventRecord(ev[4], b->stream));
-  if (b->limiter) BK(b, b->kt->mark(a, b->stream));
+  if (b->limiter) BK(b, aderdg::launch_mark(b->kt, a, b->precision, b->stream, true));
   BK(b, cudaEventRecord(ev[5], b->stream));
   if (b->limiter)
     BK(b, aderdg::launch_subcell(b->kt, a, b->ops64.data(), b->fc, b->subcell_grid, b->num_sms, b->precision, b->stream, true));
   BK(b, cudaEventRecord(ev[6], b->stream));
+  if (b->limiter) BK(b, aderdg::launch_cfl(b->kt, a, b->precision, b->stream));
   BK(b, bcontrol(b, aderdg::kCtlEnd, -1));
   BK(b, cudaEventRecord(ev[7], b->stream));
   BK(b, cudaStreamSynchronize(b->stream));

@@ -383,18 +383,17 @@ template <class Sys, int N>
 static __device__ __noinline__ double cfl_denom_call(const InstDesc& in, const double* Q) {
   return cfl_denom<Sys, N>(in, Q);
 }
-// The same from the reciprocal-sharing forms (the FP64 fused step): its divisions
-// and square roots were a third of the FP64 cell kernel's FP64 instructions (490 ->
-// 365 us on the Euler vortex N = 4 256^2, 453 -> 345 us on Baer-Nunziato N = 3 200^2)
-template <class Sys, int N>
-__device__ __forceinline__ double cfl_denom_r(const InstDesc& in, const double* Q) {
-  if constexpr (Sys::ID == kSysAD) {
-    return cfl_denom<Sys, N>(in, Q);
-  } else {
-    double ex, ey;
-    Sys::template max_eig2_r<true>(PhysC<double>(in.ph), Q, ex, ey);
-    return fma(ex, in.rdx, ey * in.rdy);
-  }
+// FP64 fused step: bounds on a node's denominator from FP32 (hi in the upper half,
+// lo in the lower: the maximum of keys is that of hi).  The time step is the
+// reference's, bit for bit, from the one maximum over all nodes, so that nearly
+// all nodes need no FP64 evaluation: k_cfl evaluates the cells whose hi reaches the
+// largest lo, and restarts, host steps and the phase API's calc_time_step give the
+// time steps of an uninterrupted run.
+template <class Sys>
+__device__ __forceinline__ unsigned long long cfl_key(const InstDesc& in, const float* q) {
+  float lo, hi;
+  Sys::cfl_bounds(typename Sys::FConst(in.ph), q, in.idxf, in.idyf, lo, hi);
+  return (unsigned long long)__float_as_uint(hi) << 32 | __float_as_uint(lo);
 }
 
 // FP32-mixed: eigenvalues and the node's denominator in FP32 (the maximum
@@ -783,6 +782,18 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
 
   // ------------------------------------------------------------- CFL part
   const bool want_cfl = mode != kCellInitDmp && mode != kCellPrimeLimited;
+  auto cfl_bits = [&]() -> unsigned long long {
+    double dn;
+    if constexpr (kExact && Sys::ID != kSysAD) {
+      if (mode == kCellFused) return cfl_key<Sys>(in, uf);
+      dn = cfl_denom_call<Sys, N>(in, u);
+    } else if constexpr (kF32) {
+      dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
+    } else {
+      dn = cfl_denom<Sys, N>(in, u);
+    }
+    return (unsigned long long)__double_as_longlong(dn);
+  };
   // cells as aligned warp segments: per-cell maxima by shuffles, one store per
   // cell instead of P2 atomics on one shared address
   // warp reductions ahead of the atomics on |du|: Euler N = 4 150 -> 144 us (vortex
@@ -795,11 +806,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     if (want_cfl) {
       unsigned long long bits = 0ull;
       if (act) {
-        double dn;
-        if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
-        else if constexpr (kExact) dn = mode == kCellFused ? cfl_denom_r<Sys, N>(in, u) : cfl_denom_call<Sys, N>(in, u);
-        else dn = cfl_denom<Sys, N>(in, u);
-        bits = (unsigned long long)__double_as_longlong(dn);
+        bits = cfl_bits();
       }
       bits = seg_max<P2>(bits);
       if (act && node == 0) cmax[lc] = bits;
@@ -808,11 +815,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
     if (want_cfl) {
       unsigned long long bits = 0ull;
       if (act) {
-        double dn;
-        if constexpr (kF32) dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(in.ph), uf, u);
-        else if constexpr (kExact) dn = mode == kCellFused ? cfl_denom_r<Sys, N>(in, u) : cfl_denom_call<Sys, N>(in, u);
-        else dn = cfl_denom<Sys, N>(in, u);
-        bits = (unsigned long long)__double_as_longlong(dn);
+        bits = cfl_bits();
       }
       // the lanes of a cell within this warp by shuffles, then one atomic per
       // cell and warp (every lane on its cell's address took turns)

@@ -66,6 +66,7 @@ struct InstState {
   double time, dt, tend;
   unsigned long long denom_bits;     // max over nodes of sum_d lambda_max/dx_d (positive double bits)
   unsigned long long denom_next;     // accumulator for the next step
+  unsigned long long denom_floor;    // FP64 fused step: a lower bound on denom_next (FP32 bits; k_cfl)
   int active;                        // 1 while time < tend
   int n_recompute;                   // troubled cells of the last step (nRecompute)
   int n_settled;                     // FP64, FP32-mixed: DMP decisions of the last step settled from FP64 values
@@ -179,7 +180,7 @@ struct BatchArgs {
   int* list_count;                   // [0]: entries of list, [1]: entries of settle
   int* settle;                       // with mme (null otherwise): cells whose DMP
                                      // decision k_settle takes from FP64 values
-  double* denom;                     // per-cell CFL denominator
+  double* denom;                     // per-cell CFL denominator (FP64 fused step: bounds on it, cfl_key)
   const double* lh_ic;               // initial-limiter candidates
   int mode;                          // kernel mode switch
   long long cell0;                   // first cell of a launch over part of the cell range (K1, K3)

@@ -40,6 +40,7 @@ static __global__ void k_control(InstDesc* inst, InstState* st, int ninst, int* 
   switch (mode) {
     case kCtlBegin: {
       s.denom_next = 0ull;
+      s.denom_floor = 0ull;
       s.n_recompute = 0;
       s.n_settled = 0;
       s.n_list = 0;

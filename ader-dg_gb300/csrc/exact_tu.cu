@@ -98,9 +98,17 @@ cudaError_t volume(const BatchArgs& a, const void* ops, cudaStream_t s) {
 }
 
 #if ADERDG_SYS != 0
-cudaError_t mark(const BatchArgs& a, cudaStream_t s) {
+cudaError_t mark(const BatchArgs& a, bool cfl_bounds, cudaStream_t s) {
   if (a.ncells <= 0) return cudaSuccess;
-  k_mark<Sys, N><<<(unsigned)((a.ncells + 255) / 256), 256, 0, s>>>(a);
+  const unsigned grid = (unsigned)((a.ncells + 255) / 256);
+  if (cfl_bounds) k_mark<Sys, N, true><<<grid, 256, 0, s>>>(a);
+  else k_mark<Sys, N, false><<<grid, 256, 0, s>>>(a);
+  return cudaGetLastError();
+}
+
+cudaError_t cfl(const BatchArgs& a, cudaStream_t s) {
+  if (a.ncells <= 0) return cudaSuccess;
+  k_cfl<Sys, N><<<(unsigned)((a.ncells + 127) / 128), 128, 0, s>>>(a);
   return cudaGetLastError();
 }
 
@@ -151,6 +159,7 @@ void ADERDG_CAT(register_exact_, ADERDG_SYS, ADERDG_N)(KernelTable& t) {
   t.volume = &volume;
 #if ADERDG_SYS != 0
   t.mark = &mark;
+  t.cfl = &cfl;
   t.subcell = &subcell;
   t.subcell_grid = &subcell_grid;
   t.settle = &settle;

@@ -8,6 +8,7 @@
 //     cell, persistent over the list; then put_subcell_data, the DMP of
 //     recompute = 2 cells, the next step's min/max and CFL contribution.
 //     update_limiter (Lh = NewLh) is the parity flip of the Lh buffers.
+// K4c k_cfl (FP64 fused step): the CFL denominators that may be the largest.
 // The FP64 and FP32-mixed modes run K4b in FP64 (T = double): the phase API with
 // --fmad=false in the reference's operation order, the FP64 fused step and the
 // FP32-mixed mode with the reciprocal-sharing forms (kRcp); DMP comparisons
@@ -21,7 +22,9 @@
 
 namespace aderdg {
 
-template <class Sys, int N>
+// kBounds: the cells' denominators are cfl_key bounds (FP64 fused step): the fold is
+// that of the lower ones
+template <class Sys, int N, bool kBounds>
 __global__ void __launch_bounds__(256) k_mark(BatchArgs a) {
   const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int k = c < a.ncells ? find_inst_cell(a.inst, a.ninst, c) : -1;
@@ -52,8 +55,10 @@ __global__ void __launch_bounds__(256) k_mark(BatchArgs a) {
       atomicAdd(&a.st[k].n_list, 1);
     } else {
       val = (unsigned long long)__double_as_longlong(a.denom[c]);
+      if constexpr (kBounds) val &= 0xffffffffull;
     }
   }
+  auto target = [&](int inst) { return kBounds ? &a.st[inst].denom_floor : &a.st[inst].denom_next; };
   // warp fold of the CFL denominators when the warp holds one instance
   const unsigned full = 0xffffffffu;
   const int k0 = __shfl_sync(full, k, 0);
@@ -63,9 +68,46 @@ __global__ void __launch_bounds__(256) k_mark(BatchArgs a) {
       const unsigned long long other = __shfl_down_sync(full, val, o);
       val = val > other ? val : other;
     }
-    if ((threadIdx.x & 31) == 0 && k0 >= 0 && val) atomicMax(&a.st[k0].denom_next, val);
+    if ((threadIdx.x & 31) == 0 && k0 >= 0 && val) atomicMax(target(k0), val);
   } else if (act && val) {
-    atomicMax(&a.st[k].denom_next, val);
+    atomicMax(target(k), val);
+  }
+}
+
+// FP64 fused step: the CFL denominators, in the reference's order, of the cells
+// whose bound reaches the largest lower bound (cells.cuh: cfl_key); the others'
+// are smaller than the maximum.  A thread looks at a cell, then the CTA evaluates
+// the nodes of those it found.  Twenty steps of the Euler vortex N = 4 256^2 take
+// 48.2 ms (49.5 with reciprocal-sharing FP64 forms at every node, whose last bits
+// were others), Baer-Nunziato N = 3 200^2 51.6 ms (53.1): the cell kernel's and the
+// re-solve's FP64 pipe has this part no more.
+template <class Sys, int N>
+__global__ void __launch_bounds__(128) k_cfl(BatchArgs a) {
+  constexpr int P2 = (N + 1) * (N + 1), V = Sys::V, NT = 128;
+  __shared__ int found[NT], inst[NT], count;
+  const int t = threadIdx.x;
+  const long long first = (long long)blockIdx.x * NT, c = first + t;
+  const int k = c < a.ncells ? find_inst_cell(a.inst, a.ninst, c) : -1;
+  if (t == 0) count = 0;
+  __syncthreads();
+  if (k >= 0 && a.st[k].active) {
+    const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(a.denom[c]) >> 32);
+    if (hi >= (unsigned)a.st[k].denom_floor) {
+      const int pos = atomicAdd(&count, 1);
+      found[pos] = t;
+      inst[pos] = k;
+    }
+  }
+  __syncthreads();
+  for (int q = t; q < count * P2; q += NT) {
+    const int f = q / P2, node = q - f * P2, kf = inst[f];
+    InstState& st = a.st[kf];
+    const double* un = a.uh[parity(st) ^ 1] + ((size_t)(first + found[f]) * P2 + node) * V;
+    double Q[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) Q[v] = un[v];
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(cfl_denom<Sys, N>(a.inst[kf], Q));
+    if (bits > *(volatile unsigned long long*)&st.denom_next) atomicMax(&st.denom_next, bits);
   }
 }
 
@@ -698,20 +740,26 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
       warp_minmax_store<double, V, NW>(mn, mx, red, t);
     }
     // CFL denominator of the new polynomial (FP32-wide: FP32 eigenvalues
-    // where the FP32 pressure is settled; FP64 in the other modes)
+    // where the FP32 pressure is settled; FP64 fused step: bounds on it for
+    // k_cfl; FP64 in the other modes)
     for (int p = t; p < P2; p += NT) {
       double Q[V];
 #pragma unroll
       for (int v = 0; v < V; ++v) Q[v] = UN[v * P2 + p];
       double dn;
-      if constexpr (sizeof(T) == 4) {
+      if constexpr (kRcp == 2) {
+        float q[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) q[v] = narrow_bits(Q[v]);
+        dn = __longlong_as_double((long long)cfl_key<Sys>(in, q));
+      } else if constexpr (sizeof(T) == 4) {
         float q[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) q[v] = (float)Q[v];
         dn = cfl_denom_f32<Sys, N>(in, typename Sys::FConst(ph), q, Q);
       } else if constexpr (kRcp) {
         double ex, ey;
-        Sys::template max_eig2_r<kRcp == 2>(pc, Q, ex, ey);
+        Sys::max_eig2_r(pc, Q, ex, ey);
         dn = fma(ex, in.rdx, ey * in.rdy);
       } else {
         dn = cfl_denom<Sys, N>(in, Q);
@@ -890,7 +938,12 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     }
     if (t == 0) {
       a.status[par ^ 1][c] = limited ? 1 : 0;
-      atomicMax(&a.st[k].denom_next, *cmaxp);
+      if constexpr (kRcp == 2) {
+        a.denom[c] = __longlong_as_double((long long)*cmaxp);
+        atomicMax(&a.st[k].denom_floor, *cmaxp & 0xffffffffull);
+      } else {
+        atomicMax(&a.st[k].denom_next, *cmaxp);
+      }
     }
     __syncthreads();
   }

@@ -199,14 +199,14 @@ struct EulerSys {
     ex = fmax(fmax(fabs(u - c), fabs(u)), fabs(u + c));
     ey = fmax(fmax(fabs(v - c), fabs(v)), fabs(v + c));
   }
-  // maxval(abs(Lambda)) along both axes; a NaN sound speed leaves the velocity,
-  // as the maxima of max_eig2 do
-  template <bool kC, class T>
+  // maxval(abs(Lambda)) along both axes (FP32-mixed); a NaN sound speed leaves the
+  // velocity, as the maxima of max_eig2 do
+  template <class T>
   __device__ static void max_eig2_r(const PhysC<T>& pc, const T* Q, T& ex, T& ey) {
     const T irho = mrcp<T>(Q[0]);
-    const T u = quot<kC>(Q[1], Q[0], irho), v = quot<kC>(Q[2], Q[0], irho);
+    const T u = Q[1] * irho, v = Q[2] * irho;
     const T p = pc.gm1 * (Q[3] - T(0.5) * (Q[1] * u + Q[2] * v));
-    const T c = msqrt<T>(quot<kC>(pc.gamma * p, Q[0], irho));
+    const T c = msqrt<T>(pc.gamma * p * irho);
     ex = tmax(tabs(u), tabs(u) + c);
     ey = tmax(tabs(v), tabs(v) + c);
   }
@@ -254,6 +254,23 @@ struct EulerSys {
     ex = fabsf(q[1] * iq) + c;
     ey = fabsf(q[2] * iq) + c;
     return ex < 1.0e30f && ey < 1.0e30f;
+  }
+  // Bounds on the CFL denominator ex/dx + ey/dy (as max_eig2 forms it) of the FP64
+  // states that round to q, from FP32 with 1/dx, 1/dy.  The velocities carry four
+  // roundings of 2^-24, the sound speed half the pressure's relative error (below
+  // 10 2^-24 mag / p for its terms of magnitude mag) and six roundings, the sum
+  // four: 2e-6 + 1e-6 mag / p is three times that.  Outside the ranges in which no
+  // product under- or overflows the bounds are 0 and infinity.
+  __device__ static void cfl_bounds(const FConst& fc, const float* q, float idx, float idy, float& lo, float& hi) {
+    const float i = 1.0f / q[0];
+    const float ke = 0.5f * (q[1] * q[1] + q[2] * q[2]) * i;
+    const float p = fc.gm1 * (q[3] - ke), mag = fc.gm1 * (fabsf(q[3]) + ke), c2 = fc.gamma * p * i;
+    const float c = sqrtf(c2), s = (fabsf(q[1]) * i + c) * idx + (fabsf(q[2]) * i + c) * idy;
+    const float rel = 2.0e-6f + 1.0e-6f * mag / p;
+    const bool settled = p > 1.0e-3f * mag && mag > 1.0e-18f && c2 > 1.0e-30f && q[0] > 1.0e-12f && q[0] < 1.0e30f &&
+                         s > 1.0e-30f && s < 1.0e30f;
+    lo = settled ? s * (1.0f - rel) : 0.0f;
+    hi = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
   }
   // True when every state within e (componentwise) of the FP32 state q passes
   // positive()'s test, with a margin for this evaluation's own rounding.  False
@@ -438,6 +455,29 @@ struct BNSys {
     ey = fmaxf(fabsf(vg) + ag, fabsf(vs) + as);
     return ex < 1.0e30f && ey < 1.0e30f;
   }
+  // Bounds on the CFL denominator, as EulerSys::cfl_bounds; a fraction's pressure
+  // phi (p + pi) has terms of magnitude mag, and its 1 - phi an absolute error of
+  // 2^-23, which mag's unscaled pi terms cover
+  __device__ static void cfl_bounds(const FConst& fc, const float* q, float idx, float idy, float& lo, float& hi) {
+    float ex = 0.0f, ey = 0.0f, ratio = 0.0f;
+    bool settled = q[8] > 1.0e-3f && q[8] < 0.999f;
+#pragma unroll
+    for (int o = 0; o < 8; o += 4) {
+      const float g = o ? fc.gg : fc.gs, g1 = o ? fc.gg1 : fc.gs1, gpi = o ? fc.ggpg : fc.gsps, pi = o ? fc.pg : fc.ps;
+      const float phi = o ? 1.0f - q[8] : q[8], i = 1.0f / q[o];
+      const float ke = 0.5f * (q[o + 1] * q[o + 1] + q[o + 2] * q[o + 2]) * i;
+      const float pp = g1 * (q[o + 3] - ke) - gpi * phi + pi * phi;
+      const float mag = g1 * (fabsf(q[o + 3]) + ke) + fabsf(gpi) + fabsf(pi), c2 = g * pp * i, c = sqrtf(c2);
+      settled = settled && pp > 1.0e-3f * mag && mag > 1.0e-18f && c2 > 1.0e-30f && q[o] > 1.0e-12f && q[o] < 1.0e30f;
+      ex = fmaxf(ex, fabsf(q[o + 1]) * i + c);
+      ey = fmaxf(ey, fabsf(q[o + 2]) * i + c);
+      ratio = fmaxf(ratio, mag / pp);
+    }
+    const float s = ex * idx + ey * idy, rel = 2.0e-6f + 1.0e-6f * ratio;
+    settled = settled && s > 1.0e-30f && s < 1.0e30f;
+    lo = settled ? s * (1.0f - rel) : 0.0f;
+    hi = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
+  }
   // True when every state within e (componentwise) of the FP32 state q passes
   // positive()'s test (rho_s, rho_g, p_s + pi_s, p_g + pi_g above 1e-12 and
   // 0 < phi_s < 1), with a margin for this evaluation's own rounding.  With
@@ -509,19 +549,19 @@ struct BNSys {
   //   phi rho_s u_s = Q1, (p_s + pi_s) / rho_s = (phi p_s + pi_s phi) / Q0,
   // and likewise for the gas with Q4..Q7 and phi_g; so a state needs 1/Q0
   // and 1/Q4 only, both from one reciprocal of Q0 Q4.
-  // maxval(abs(Lambda)) along both axes; a NaN sound speed leaves the velocity,
-  // as the maxima of max_eig2 do
-  template <bool kC, class T>
+  // maxval(abs(Lambda)) along both axes (FP32-mixed); a NaN sound speed leaves the
+  // velocity, as the maxima of max_eig2 do
+  template <class T>
   __device__ static void max_eig2_r(const PhysC<T>& pc, const T* Q, T& ex, T& ey) {
     const T r = mrcp<T>(Q[0] * Q[4]);
     const T i0 = Q[4] * r, i4 = Q[0] * r;
-    const T u_s = quot<kC>(Q[1], Q[0], i0), v_s = quot<kC>(Q[2], Q[0], i0);
-    const T u_g = quot<kC>(Q[5], Q[4], i4), v_g = quot<kC>(Q[6], Q[4], i4);
+    const T u_s = Q[1] * i0, v_s = Q[2] * i0;
+    const T u_g = Q[5] * i4, v_g = Q[6] * i4;
     const T phi_s = Q[8], phi_g = T(1) - Q[8];
     const T pps = pc.gs1 * (Q[3] - T(0.5) * (Q[1] * u_s + Q[2] * v_s)) - pc.gsps * phi_s;
     const T ppg = pc.gg1 * (Q[7] - T(0.5) * (Q[5] * u_g + Q[6] * v_g)) - pc.ggpg * phi_g;
-    const T a_s = msqrt<T>(quot<kC>(pc.gs * (pps + pc.ps * phi_s), Q[0], i0));
-    const T a_g = msqrt<T>(quot<kC>(pc.gg * (ppg + pc.pg * phi_g), Q[4], i4));
+    const T a_s = msqrt<T>(pc.gs * (pps + pc.ps * phi_s) * i0);
+    const T a_g = msqrt<T>(pc.gg * (ppg + pc.pg * phi_g) * i4);
     ex = tmax(tmax(tabs(u_g), tabs(u_g) + a_g), tmax(tabs(u_s), tabs(u_s) + a_s));
     ey = tmax(tmax(tabs(v_g), tabs(v_g) + a_g), tmax(tabs(v_s), tabs(v_s) + a_s));
   }

@@ -53,7 +53,8 @@ struct KernelTable {
   // fast: 0 FP64 in reference order, 1 the FP32 modes, 2 FP64 with certified FP32 projections
   cudaError_t (*cells)(const BatchArgs&, const void* ops64, int fast, cudaStream_t) = nullptr;
   cudaError_t (*volume)(const BatchArgs&, const void* ops64, cudaStream_t) = nullptr;
-  cudaError_t (*mark)(const BatchArgs&, cudaStream_t) = nullptr;
+  cudaError_t (*mark)(const BatchArgs&, bool cfl_bounds, cudaStream_t) = nullptr;
+  cudaError_t (*cfl)(const BatchArgs&, cudaStream_t) = nullptr;  // FP64 fused step (k_cfl)
   cudaError_t (*subcell)(const BatchArgs&, const void* ops64, const FaceConst&, int grid, int fp32, cudaStream_t) = nullptr;
   int (*subcell_grid)(int num_sms, int fp32) = nullptr;
   // FP64 and FP32-mixed: DMP decisions k_cells left open, from FP64 values (k_settle);
@@ -139,6 +140,14 @@ inline cudaError_t launch_subcell(const KernelTable* kt, const BatchArgs& a, con
   if (precision == ADERDG_FP32_MIXED && kt->subcell_mixed) return kt->subcell_mixed(a, ops64, fc, grid, s);
   if (precision == ADERDG_FP64 && fused && kt->subcell_fused) return kt->subcell_fused(a, ops64, fc, grid, s);
   return kt->subcell(a, ops64, fc, grid, subcell_fp32(precision), s);
+}
+// The FP64 fused step folds the CFL denominators' FP32 bounds and evaluates the
+// cells that may hold the largest one after the re-solve.
+inline cudaError_t launch_mark(const KernelTable* kt, const BatchArgs& a, int precision, cudaStream_t s, bool fused) {
+  return kt->mark(a, fused && precision == ADERDG_FP64, s);
+}
+inline cudaError_t launch_cfl(const KernelTable* kt, const BatchArgs& a, int precision, cudaStream_t s) {
+  return precision == ADERDG_FP64 ? kt->cfl(a, s) : cudaSuccess;
 }
 inline int subcell_grid_of(const KernelTable* kt, int num_sms, int precision) {
   if (precision == ADERDG_FP32_MIXED && kt->subcell_grid_mixed) return kt->subcell_grid_mixed(num_sms);

@@ -456,13 +456,13 @@ def _profile_groups(groups):
 
 def _step_launches(aderdg, system, prec, limiter=True, nodes=None):
     """Kernel launches of one step: control, predictor, faces, cells, [settle (FP64
-    and FP32-mixed), mark, subcell,] control; a small advection-diffusion grid's
+    and FP32-mixed), mark, subcell, cfl (FP64),] control; a small advection-diffusion grid's
     cell kernel forms its face fluxes itself (common.cuh: faces_in_cells)."""
     if system == aderdg.SYS_ADVDIFF:
         return 4 if nodes is not None and nodes <= (65536 if prec == aderdg.FP64 else 131072) else 5
     if not limiter:
         return 5
-    return 7 if prec == aderdg.FP32_WIDE else 8
+    return {aderdg.FP32_WIDE: 7, aderdg.FP32_MIXED: 8, aderdg.FP64: 9}[prec]
 
 
 def _launches_per_step(groups, prec, aderdg):

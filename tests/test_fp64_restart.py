@@ -1,0 +1,128 @@
+"""The FP64 mode's time steps do not depend on how a state was reached: a run
+continued from its downloaded state, steps on a host array and the phase API's
+calc_time_step give the time step of the uninterrupted run, bit for bit (the
+fused step finds the cells that may hold the largest CFL denominator from FP32
+bounds and evaluates those in the reference's order)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import aderdg
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _gpu(gpu_lib):
+    return gpu_lib
+
+
+CASES = [("euler_vortex", 1, (9, 7)), ("euler_vortex", 4, (16, 13)), ("euler_rp2d", 2, (40, 33)), ("euler_rp2d", 3, (33, 21)),
+         ("euler_rp2d", 5, (11, 9)), ("bn_cylinder", 1, (17, 12)), ("bn_cylinder", 2, (24, 31)), ("bn_cylinder", 3, (20, 17)),
+         ("bn_cylinder", 5, (9, 8))]
+
+
+def build(name, N, grid, limiter=1):
+    cfg, ic, params, _ = aderdg.workloads.make(name, side=8, N=N)
+    cfg = dataclasses.replace(cfg, imax=grid[0], jmax=grid[1], limiter=limiter)
+    return cfg, aderdg.project_initial_condition(cfg, ic, params)
+
+
+def start(cfg, uh, lh):
+    s = aderdg.Solver(cfg)
+    s.upload(uh)
+    if cfg.limiter:
+        s.init_limiter(lh)
+    return s
+
+
+def same_state(a, b):
+    (ua, sa), (ub, sb) = a.download(), b.download()
+    return np.array_equal(ua, ub) and np.array_equal(sa, sb)
+
+
+@pytest.mark.parametrize("name,N,grid", CASES)
+def test_continued_run(name, N, grid):
+    cfg, (uh, lh) = build(name, N, grid)
+    a, b, c = start(cfg, uh, lh), start(cfg, uh, lh), aderdg.Solver(cfg)
+    t = a.run(0.0, 1e30, 12)[0]
+    tb = b.run(0.0, 1e30, 7)[0]
+    c.upload(b.download()[0])
+    c.upload_limiter(*b.download_limiter())
+    assert c.run(tb, 1e30, 5)[0] == t
+    assert same_state(a, c)
+
+
+@pytest.mark.parametrize("name,N,grid", CASES)
+def test_host_steps(name, N, grid):
+    cfg, (uh, lh) = build(name, N, grid)
+    a, b = start(cfg, uh, lh), start(cfg, uh, lh)
+    t = a.run(0.0, 1e30, 6)[0]
+    u, tb = uh.copy(), 0.0
+    for _ in range(6):
+        tb, _, _ = b.step_host(u, tb, 1e30)
+    assert tb == t and np.array_equal(u, a.download()[0])
+
+
+@pytest.mark.parametrize("limiter", [1, 0])
+@pytest.mark.parametrize("name,N,grid", CASES)
+def test_calc_time_step_is_the_next_step(name, N, grid, limiter):
+    cfg, (uh, lh) = build(name, N, grid, limiter)
+    a, b = start(cfg, uh, lh), start(cfg, uh, lh)
+    t = 0.0
+    for k in range(5):
+        want = b.calc_time_step(t, 1e30)
+        ta, dt, _ = a.step(t, 1e30)
+        assert dt == want, k
+        b.upload(a.download()[0])
+        t = ta
+
+
+def random_states(cfg, rng):
+    """Independent nodes: densities and pressures over eight decades, Mach numbers up
+    to 1e3, a tenth of the cells uniform, one cell inadmissible."""
+    n, P2, V = cfg.cells, cfg.P * cfg.P, cfg.nvar
+    u = np.empty((n, P2, V))
+
+    def phase(gamma, pi):
+        r, p = 10.0 ** rng.uniform(-4, 4, (n, P2)), 10.0 ** rng.uniform(-4, 4, (n, P2))
+        c = np.sqrt(gamma * (p + pi) / r)
+        m, phi = c * 10.0 ** rng.uniform(-3, 3, (n, P2)), rng.uniform(0, 2 * np.pi, (n, P2))
+        vx, vy = m * np.cos(phi), m * np.sin(phi)
+        return r, r * vx, r * vy, (p + gamma * pi) / (gamma - 1) + 0.5 * r * m * m
+
+    if cfg.system == aderdg.SYS_EULER:
+        u[..., :4] = np.stack(phase(cfg.gamma, 0.0), -1)
+    else:
+        a = np.where(rng.uniform(size=(n, P2)) < 0.1, 10.0 ** rng.uniform(-6, -1, (n, P2)), rng.uniform(0.05, 0.95, (n, P2)))
+        u[..., 8] = a
+        u[..., :4] = np.stack(phase(cfg.gamma_s, cfg.pi_s), -1) * a[..., None]
+        u[..., 4:8] = np.stack(phase(cfg.gamma_g, cfg.pi_g), -1) * (1 - a[..., None])
+    flat = rng.uniform(size=n) < 0.1
+    u[flat] = u[flat][:, :1]
+    u[n // 3, :, 3] *= -0.5
+    return u.ravel()
+
+
+@pytest.mark.parametrize("name,N", [("euler_vortex", 2), ("euler_rp2d", 3), ("bn_cylinder", 2), ("bn_cylinder", 3)])
+@pytest.mark.parametrize("seed", range(6))
+@pytest.mark.parametrize("scale", [1.0, 1e-12, 1e25])
+def test_random_states(name, N, seed, scale):
+    """The time step after one very short step from random states is the reference
+    order's, with the largest denominator in re-solved and other cells alike."""
+    cfg, _ = build(name, N, (9, 7))
+    uh = random_states(cfg, np.random.default_rng(seed))
+    if scale != 1.0 and cfg.system == aderdg.SYS_EULER:
+        uh = uh * scale
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (a, b):
+        s.upload(uh)
+    short = 1e-9 * a.calc_time_step(0.0, 1e30)
+    assert short > 0.0
+    for s in (a, b):
+        t, _, n = s.step(0.0, short)
+    assert n > 0 and np.array_equal(a.download()[0], b.download()[0], equal_nan=True)
+    want = b.calc_time_step(t, 1e30)
+    if np.isfinite(want) and want < 1e19:  # no NaN among the denominators
+        assert a.step(t, 1e30)[1] == want
