@@ -229,11 +229,41 @@ __device__ __forceinline__ R ad_face_flux(const BatchArgs& a, const InstDesc& in
   return (R)(CT(0.5) * ((FL0 + FR0) * nv0 + (FL1 + FR1) * nv1) - CT(0.5) * smax * (QR[0] - QL[0]));
 }
 
-// kRec (FP64): the reciprocal-sharing forms, for the fused step (the phase API
-// keeps the reference's operation order): Euler N = 4 256^2 139 -> 96 us,
-// Baer-Nunziato N = 3 200^2 432 -> 143 us.  FP32-mixed Baer-Nunziato: three CTAs an
-// SM (80 registers, 16 bytes spilled) and the rounding on the integer pipe: 462 ->
-// 405 us, cylinder N = 3 400^2
+// Baer-Nunziato's path-conservative face fluxes F-, F+ (pde.f90:326-353) in the
+// reference's order
+template <class CT>
+__device__ __forceinline__ void bn_face(const PhysC<CT>& pc, const CT* QL, const CT* QR, const CT* FL, const CT* FR, int d,
+                                        CT* fm, CT* fp) {
+  const CT smax = tmax(BNSys::max_eig(pc, QL, d), BNSys::max_eig(pc, QR, d));
+  CT D[9];
+  BNSys::roe_times_jump(pc, QL, QR, d, D);
+#pragma unroll
+  for (int v = 0; v < 9; ++v) {
+    const CT base = CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]);
+    fm[v] = base - CT(0.5) * D[v];
+    fp[v] = base + CT(0.5) * D[v];
+  }
+}
+// out of line, for the states of the FP64 fused step's faces that are not ordinary:
+// q holds QL, QR, FL, FR, then F- and F+
+static __device__ __noinline__ void face_reference(const Phys& ph, int d, double* q) {
+  double fm[9], fp[9];
+  bn_face(PhysC<double>(ph), q, q + 9, q + 18, q + 27, d, fm, fp);
+  for (int v = 0; v < 9; ++v) {
+    q[v] = fm[v];
+    q[9 + v] = fp[v];
+  }
+}
+static __device__ __noinline__ double max_eig_call(const Phys& ph, double q0, double q1, double q2, double q3, int d) {
+  const double Q[4] = {q0, q1, q2, q3};
+  return EulerSys::max_eig(ph, Q, d);
+}
+
+// kRec (FP64): the reciprocal-sharing forms, for the fused step (the phase API, and
+// states that are not ordinary, take the reference's operation order): Euler N = 4
+// 256^2 139 -> 96 us, Baer-Nunziato N = 3 200^2 432 -> 143 us.  FP32-mixed
+// Baer-Nunziato: three CTAs an SM (80 registers, 16 bytes spilled) and the rounding
+// on the integer pipe: 462 -> 405 us, cylinder N = 3 400^2
 template <class Sys, int N, class R, class CT, bool kRec = false>
 __global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && sizeof(CT) == 8 ? 3 : 1) k_faces(BatchArgs a, FaceConst fc) {
   constexpr int P = N + 1, V = Sys::V;
@@ -347,7 +377,24 @@ __global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && si
     } else {
       if constexpr (kRec && Sys::ID == kSysBN) {
         double fm[V], fp[V];
-        BNSys::face_r(pc, BNSys::FConst(ph), QL, QR, FL, FR, d, fm, fp);
+        if (ordinary<Sys>(QL) && ordinary<Sys>(QR)) {
+          BNSys::face_r(pc, BNSys::FConst(ph), QL, QR, FL, FR, d, fm, fp);
+        } else {
+          double q[4 * V];  // (a copy: the call's arguments lie in memory)
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            q[v] = QL[v];
+            q[V + v] = QR[v];
+            q[2 * V + v] = FL[v];
+            q[3 * V + v] = FR[v];
+          }
+          face_reference(in.ph, d, q);
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            fm[v] = q[v];
+            fp[v] = q[V + v];
+          }
+        }
         double* dm = xdir ? a.fu : a.gu;
         double* dp = xdir ? a.fp : a.gp;
 #pragma unroll
@@ -359,19 +406,21 @@ __global__ void __launch_bounds__(256, Sys::ID == kSysBN && sizeof(R) == 4 && si
       }
       // Rusanov: smax from both sides' eigenvalues (Euler/pde.f90:97-114)
       CT smax;
-      if constexpr (kRec && Sys::ID == kSysEuler) smax = max_nonneg(Sys::max_speed_r(pc, QL, d), Sys::max_speed_r(pc, QR, d));
-      else smax = tmax(Sys::max_eig(pc, QL, d), Sys::max_eig(pc, QR, d));
+      if constexpr (kRec && Sys::ID == kSysEuler) {
+        if (ordinary<Sys>(QL) && ordinary<Sys>(QR)) smax = max_nonneg(Sys::max_speed_r(pc, QL, d), Sys::max_speed_r(pc, QR, d));
+        else smax = tmax(max_eig_call(in.ph, QL[0], QL[1], QL[2], QL[3], d), max_eig_call(in.ph, QR[0], QR[1], QR[2], QR[3], d));
+      } else if constexpr (Sys::ID == kSysEuler) {
+        smax = tmax(Sys::max_eig(pc, QL, d), Sys::max_eig(pc, QR, d));
+      }
       if constexpr (Sys::ID == kSysBN) {
-        // path-conservative fluctuations, Baer-Nunziato/pde.f90:326-353
-        CT D[9];
-        BNSys::roe_times_jump(pc, QL, QR, d, D);
         R* dm = reinterpret_cast<R*>(xdir ? a.fu : a.gu);
         R* dp = reinterpret_cast<R*>(xdir ? a.fp : a.gp);
+        CT fm[V], fp[V];
+        bn_face(pc, QL, QR, FL, FR, d, fm, fp);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-          const CT base = CT(0.5) * (FL[v] + FR[v]) - CT(0.5) * smax * (QR[v] - QL[v]);
-          dm[out + v] = (R)(base - CT(0.5) * D[v]);
-          dp[out + v] = (R)(base + CT(0.5) * D[v]);
+          dm[out + v] = (R)fm[v];
+          dp[out + v] = (R)fp[v];
         }
       } else {
         R r[V];

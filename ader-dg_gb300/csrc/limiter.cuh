@@ -171,7 +171,8 @@ __device__ __forceinline__ T minmod(T a, T b) {
 // pipe): 0 when the signs differ or either is 0, else the smaller magnitude
 // (magnitude bits order like the magnitudes).  It differs from minmod only
 // where a * b underflows to 0 for same-signed |a b| < 2^-1074 (the smaller
-// slope instead of 0).
+// slope instead of 0) and where either is a NaN; neither occurs between ordinary
+// states (FP64 mode).
 __device__ __forceinline__ double minmod_bits(double a, double b) {
   const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
   const long long ma = ia & 0x7fffffffffffffffLL, mb = ib & 0x7fffffffffffffffLL;
@@ -256,12 +257,40 @@ __device__ __forceinline__ void warp_minmax_store(R* mn, R* mx, R* red, int t) {
   }
 }
 
+// The finite-volume step of one cell in the reference's order, out of line: cells of
+// the FP64 fused step whose subcells hold values that are not ordinary.  sub0: the
+// gathered subcells, at the head of k_subcell's layout.
+template <class Sys, int N>
+static __device__ __noinline__ void fv_update_reference(const InstDesc& in, double* sub0, double dt) {
+  using T = double;
+  using C = SubCfg<Sys, N, T>;
+  constexpr int kRcp = 0, S = 2 * N + 1, V = Sys::V, R = C::R, H = C::H, NT = C::THREADS, NE = C::NE;
+  constexpr bool BN = Sys::ID == kSysBN;
+  T* wLx = sub0 + V * R * R;
+  T* wRx = wLx + C::TW;
+  T* wLy = wRx + C::TW;
+  T* wRy = wLy + C::TW;
+  T* slt = wRy + C::TW;              // BN: half-step increment [V][H*H]
+  T* sa8 = slt + C::TW;              // BN: volume-fraction slopes x [H*H], y [H*H]
+  T* EF = wLx + C::TSTATE;           // x edges: F [V][NE] (BN: then D [V][NE]); then the y edges
+  T* sub1 = wLx;                     // [V][S*S], after the edge fluxes
+  const int t = threadIdx.x;
+  auto SU = [&](int v, int ii, int jj) -> T& { return sub0[v * R * R + (ii + 1) + R * (jj + 1)]; };  // ii,jj in -1..S+2
+  auto hx = [&](int v, int ii, int jj) { return v * H * H + ii + H * jj; };                         // ii,jj in 0..S+1
+  const Phys ph = in.ph;
+  const PhysC<T> pc(ph);
+  const typename Sys::FConst fcs(ph);
+  const T ldx0 = in.dx / (double)S, ldx1 = in.dy / (double)S, ix0 = 0.0, ix1 = 0.0;
+#include "fv_update.cuh"
+}
+
 // T = double: the reference's FP64 arithmetic in its order (bit for bit: the phase
 // API), or, with kRcp (instantiated with fused multiply-adds in predictor_tu.cu),
 // FP64 with the reciprocal-sharing physics forms and multiplications by 1/ldx in
 // place of divisions: 1 in the FP32-mixed mode, 2 in the FP64 fused step, whose
-// quotients are corrected (quot, physics.cuh) and where a NaN sound speed leaves
-// |u|, as the reference's maxima do.  FP64 fused step: 301 -> 168 us (Riemann
+// quotients are corrected (quot, physics.cuh), where a NaN sound speed leaves |u|,
+// as the reference's maxima do, and whose cells with subcells that are not ordinary
+// take the reference's order.  FP64 fused step: 301 -> 168 us (Riemann
 // problem N = 3 257 x 193), 817 -> 326 us (Baer-Nunziato N = 3 200^2).  The DMP
 // projections keep the reference order in all.
 // T = float: the FP32-wide mode; the subcell re-solve, the DMP projections
@@ -338,25 +367,6 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     const T dt = (T)st.dt;
     const T ldx0 = (T)(in.dx / (double)S), ldx1 = (T)(in.dy / (double)S);
     const T ix0 = T(1) / ldx0, ix1 = T(1) / ldx1;  // kRcp only
-    auto divx = [&](T q) -> T { if constexpr (kRcp) return q * ix0; else return q / ldx0; };
-    auto divy = [&](T q) -> T { if constexpr (kRcp) return q * ix1; else return q / ldx1; };
-    // the flux of Q into F[d * V + v]; kRcp: along d only (the MUSCL half step
-    // uses the x flux of the x-reconstructed states and the y flux of the
-    // y-reconstructed ones), otherwise both directions as the reference
-    auto flux = [&](const T* Q, int d, T* F) {
-      if constexpr (kRcp) {
-        T e;
-        Sys::template flux_dir_eig_r<kRcp == 2>(pc, Q, d, F + d * V, e);
-      } else {
-        Sys::flux(pc, Q, F);
-      }
-    };
-    auto ncp = [&](const T* Q, T ax, T ay, T* Sr) {
-      if constexpr (Sys::ID == kSysBN) {
-        if constexpr (kRcp) BNSys::src_ncp_r<kRcp == 2>(pc, Q, ax, ay, Sr);
-        else BNSys::src_ncp(pc, Q, ax, ay, Sr);
-      }
-    };
     const bool dmr = (Sys::ID == kSysEuler) && in.bc_mode == 1;
 
     // ---- gather the subcell data of the 3x3 neighbourhood (only the strip
@@ -433,6 +443,7 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
     // the four strips beside it (columns 1..S of rows 0..S+1, then columns 0
     // and S+1 of rows 1..S)
     constexpr int NX = BN ? H * H + 4 * S : S * S + 4 * S;
+    bool odd = false;  // kRcp = 2: a subcell that is not ordinary
     for (int p = t; p < NX; p += NT) {
       int ii, jj;
       if constexpr (BN) {
@@ -488,173 +499,17 @@ __global__ void __launch_bounds__(SubCfg<Sys, N, T>::THREADS, SubCfg<Sys, N, T>:
           }
         }
       }
+      if constexpr (kRcp == 2) odd = odd || !ordinary<Sys>(val);
 #pragma unroll
       for (int v = 0; v < V; ++v) SU(v, ii, jj) = val[v];
     }
-    __syncthreads();
+    if constexpr (kRcp == 2) odd = __syncthreads_or(odd);
+    else __syncthreads();
 
-    // ---- MUSCL-Hancock reconstruction on subcells 0..S+1; the slopes of
-    // one direction at a time in registers.  The S*S interior subcells come
-    // first, then the ring of halo subcells, so that the interior ones fill
-    // whole warps: Euler's halo subcells have zero slopes (Euler/limiter.f90:
-    // 529-536), so their two face states per direction are the subcell value,
-    // the half-step flux differences vanish exactly and their evolved face
-    // states are the subcell value itself; they are copied, and only the
-    // warps holding interior subcells evaluate fluxes.
-    for (int p = t; p < H * H; p += NT) {
-      int ii, jj;
-      if (p < S * S) {
-        ii = 1 + p % S;
-        jj = 1 + p / S;
-      } else {
-        const int r = p - S * S;  // the ring: bottom row, top row, left column, right column
-        if (r < H) { ii = r; jj = 0; }
-        else if (r < 2 * H) { ii = r - H; jj = H - 1; }
-        else if (r < 2 * H + S) { ii = 0; jj = 1 + (r - 2 * H); }
-        else { ii = H - 1; jj = 1 + (r - 2 * H - S); }
-      }
-      const bool interior = p < S * S;
-      // the corners of the ring feed no edge (Euler does not gather them)
-      if (!interior && (ii == 0 || ii == H - 1) && (jj == 0 || jj == H - 1)) continue;
-      if (!BN && !interior) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const T q = SU(v, ii, jj);
-          wLx[hx(v, ii, jj)] = q;
-          wRx[hx(v, ii, jj)] = q;
-          wLy[hx(v, ii, jj)] = q;
-          wRy[hx(v, ii, jj)] = q;
-        }
-        continue;
-      }
-      T Qt[V], FL[2 * V], FR[2 * V];
-      // Euler computes slopes for interior subcells only (halo slopes stay 0,
-      // Euler/limiter.f90:529-536); BN also on the halo (BN :486-492)
-      // kRcp (FP64 re-solve): minmod on the bit patterns
-      auto mm = [](T a, T b) -> T {
-        if constexpr (kRcp && sizeof(T) == 8) return minmod_bits(a, b);
-        else return minmod(a, b);
-      };
-      auto slope_x = [&](int v) -> T {
-        return (BN || interior) ? mm(SU(v, ii + 1, jj) - SU(v, ii, jj), SU(v, ii, jj) - SU(v, ii - 1, jj)) : T(0);
-      };
-      auto slope_y = [&](int v) -> T {
-        return (BN || interior) ? mm(SU(v, ii, jj + 1) - SU(v, ii, jj), SU(v, ii, jj) - SU(v, ii, jj - 1)) : T(0);
-      };
-      T q0[V], wl[V], wr[V], sl[V];
-#pragma unroll
-      for (int v = 0; v < V; ++v) q0[v] = SU(v, ii, jj);
-      T src[V];
-      if constexpr (BN) {
-        // Baer-Nunziato/limiter.f90:494-497
-        const T ax = slope_x(8), ay = slope_y(8);
-        sa8[ii + H * jj] = ax;
-        sa8[H * H + ii + H * jj] = ay;
-        ncp(q0, divx(ax), divy(ay), src);
-      }
-#pragma unroll
-      for (int v = 0; v < V; ++v) sl[v] = slope_x(v);
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        wl[v] = q0[v] - T(0.5) * sl[v];
-        wr[v] = q0[v] + T(0.5) * sl[v];
-      }
-      flux(wl, 0, FL);
-      flux(wr, 0, FR);
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        if (kRcp && BN && v == 8) Qt[v] = src[v];  // the volume fraction has no flux
-        else if constexpr (BN) Qt[v] = src[v] - divx(FR[v] - FL[v]);
-        else Qt[v] = -divx(FR[v] - FL[v]);
-        wLx[hx(v, ii, jj)] = wl[v];
-        wRx[hx(v, ii, jj)] = wr[v];
-      }
-#pragma unroll
-      for (int v = 0; v < V; ++v) sl[v] = slope_y(v);
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        wl[v] = q0[v] - T(0.5) * sl[v];
-        wr[v] = q0[v] + T(0.5) * sl[v];
-      }
-      flux(wl, 1, FL);
-      flux(wr, 1, FR);
-#pragma unroll
-      for (int v = 0; v < V; ++v) {
-        if (!(kRcp && BN && v == 8)) Qt[v] = Qt[v] - divy(FR[V + v] - FL[V + v]);
-        if constexpr (BN) slt[hx(v, ii, jj)] = Qt[v];
-        wLx[hx(v, ii, jj)] = wLx[hx(v, ii, jj)] + T(0.5) * dt * Qt[v];
-        wRx[hx(v, ii, jj)] = wRx[hx(v, ii, jj)] + T(0.5) * dt * Qt[v];
-        wLy[hx(v, ii, jj)] = wl[v] + T(0.5) * dt * Qt[v];
-        wRy[hx(v, ii, jj)] = wr[v] + T(0.5) * dt * Qt[v];
-      }
-    }
-    __syncthreads();
-
-    // ---- edge fluxes Fx(1..S+1, 1..S), Fy(1..S, 1..S+1) (Euler/limiter.f90:571-588);
-    // BN's four Rusanov fluxes per subcell (Baer-Nunziato/limiter.f90:526-545)
-    // are those of its edges, each formed once here from the same states
-    {
-      T* EX = EF;
-      T* EY = EF + (BN ? 2 : 1) * V * NE;
-      for (int p = t; p < 2 * NE; p += NT) {
-        const bool xd = p < NE;
-        const int q = xd ? p : p - NE;
-        T QL[V], QR[V], F[V], Dd[V];
-        int ii, jj;
-        if (xd) { ii = q % (S + 1) + 1; jj = q / (S + 1) + 1; }
-        else { ii = q % S + 1; jj = q / S + 1; }
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          QL[v] = xd ? wRx[hx(v, ii - 1, jj)] : wRy[hx(v, ii, jj - 1)];
-          QR[v] = xd ? wLx[hx(v, ii, jj)] : wLy[hx(v, ii, jj)];
-        }
-        rusanov_s<Sys, T, kRcp>(pc, fcs, QL, QR, xd ? 0 : 1, F, Dd);
-        T* dst = xd ? EX : EY;
-#pragma unroll
-        for (int v = 0; v < V; ++v) dst[v * NE + q] = F[v];
-        if constexpr (BN) {
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-            if (!kRcp || (v != 0 && v != 4)) dst[(V + v) * NE + q] = Dd[v];
-        }
-      }
-      __syncthreads();
-      for (int p = t; p < S * S; p += NT) {
-        const int ii = p % S + 1, jj = p / S + 1;
-        const int xp = ii + (S + 1) * (jj - 1), xm = (ii - 1) + (S + 1) * (jj - 1);
-        const int yp = (ii - 1) + S * jj, ym = (ii - 1) + S * (jj - 1);
-        // kRcp: EX, EY hold twice the flux
-        const T fX = kRcp ? T(0.5) * divx(dt) : divx(dt), fY = kRcp ? T(0.5) * divy(dt) : divy(dt);
-        if constexpr (!BN) {
-          // first-order FV update, Euler/limiter.f90:592-597
-#pragma unroll
-          for (int v = 0; v < V; ++v)
-            sub1[v * S * S + p] = SU(v, ii, jj) - fX * (EX[v * NE + xp] - EX[v * NE + xm]) -
-                                  fY * (EY[v * NE + yp] - EY[v * NE + ym]);
-        } else {
-          T qh[V], src[V];
-#pragma unroll
-          for (int v = 0; v < V; ++v) qh[v] = SU(v, ii, jj) + T(0.5) * dt * slt[hx(v, ii, jj)];
-          ncp(qh, divx(sa8[ii + H * jj]), divy(sa8[H * H + ii + H * jj]), src);
-#pragma unroll
-          for (int v = 0; v < V; ++v) {
-            if constexpr (kRcp) {
-              // the fluctuation of an x (y) edge has no component along y (x),
-              // nor in the two densities
-              T q = SU(v, ii, jj) - fX * (EX[v * NE + xp] - EX[v * NE + xm]) - fY * (EY[v * NE + yp] - EY[v * NE + ym]);
-              if (v != 0 && v != 2 && v != 4 && v != 6) q = q - fX * (EX[(V + v) * NE + xp] + EX[(V + v) * NE + xm]);
-              if (v != 0 && v != 1 && v != 4 && v != 5) q = q - fY * (EY[(V + v) * NE + yp] + EY[(V + v) * NE + ym]);
-              sub1[v * S * S + p] = v != 0 && v != 4 ? q + dt * src[v] : q;
-            } else {
-              sub1[v * S * S + p] = SU(v, ii, jj) - divx(dt) * (EX[v * NE + xp] - EX[v * NE + xm]) -
-                                    divy(dt) * (EY[v * NE + yp] - EY[v * NE + ym]) -
-                                    divx(dt) * T(0.5) * (EX[(V + v) * NE + xp] + EX[(V + v) * NE + xm]) -
-                                    divy(dt) * T(0.5) * (EY[(V + v) * NE + yp] + EY[(V + v) * NE + ym]) +
-                                    dt * src[v];
-            }
-          }
-        }
-      }
+    if constexpr (kRcp == 2)
+      if (odd) fv_update_reference<Sys, N>(in, sub0, st.dt);
+    if (!odd) {
+#include "fv_update.cuh"
     }
     __syncthreads();
 

@@ -161,6 +161,28 @@ __device__ __forceinline__ double max_nonneg(double a, double b) {
   return ka >= kb ? a : b;
 }
 
+// The states for which the FP64 fused step's reciprocal-sharing forms stand in for
+// the reference's order: every value zero or within 2^-400 .. 2^100 in magnitude
+// (differences of such values are zero or at least 2^-452: no product of two
+// underflows), the densities at least 2^-100 (no product of two and a fraction
+// under- or overflows), a volume fraction in (0, 1).  NaN and infinities are
+// outside: the reference's order multiplies the other direction's flux by 0, which
+// spreads them.  Integer pipe.
+template <class Sys>
+__device__ __forceinline__ bool ordinary(const double* Q) {
+  constexpr unsigned top = (1023u + 100u) << 20;
+  bool ok = true;
+#pragma unroll
+  for (int v = 0; v < Sys::V; ++v) {
+    const unsigned a = (unsigned)__double2hiint(Q[v]) & 0x7fffffffu;
+    const unsigned low = ((v & 3) == 0 ? 1023u - 100u : 1023u - 400u) << 20;
+    const bool in = a - low < top - low;
+    ok = ok && ((v & 3) == 0 ? in : in || (a | (unsigned)__double2loint(Q[v])) == 0u);
+    if (v == 8) ok = ok && __double_as_longlong(Q[v]) < 0x3ff0000000000000LL && __double_as_longlong(Q[v]) > 0;
+  }
+  return ok;
+}
+
 // ---------------------------------------------------------------------------
 struct EulerSys {
   static constexpr int V = 4;
