@@ -577,7 +577,12 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
       const double* mmi = a.mm[par2] + side0 * V + v;
       const float* mei = a.mme[par2];
       // the maximum as the minimum of the negated values (fast kernels: of the
-      // complemented integer keys, on the integer pipe, not FP64)
+      // complemented integer keys, on the integer pipe, not FP64; FP64: a NaN is
+      // the largest key on either side, left out as fmin and fmax leave it out)
+      auto key = [](double x, long long flip) -> long long {
+        if (kExact && is_nan_bits(x)) return 0x7fffffffffffffffLL;
+        return okey(x) ^ flip;
+      };
       double b[SPL];
       long long kb[SPL], kx[SPL];
 #pragma unroll
@@ -585,7 +590,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
         kx[s] = -(long long)(side0 + s);
         const double x = mmi[(size_t)cell2 * 2 * V + s * V];
         b[s] = kx[s] ? -x : x;
-        kb[s] = okey(x) ^ kx[s];
+        kb[s] = key(x, kx[s]);
       }
       float en = 0.0f;
 #pragma unroll
@@ -598,7 +603,7 @@ __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N,
 #pragma unroll
           for (int s = 0; s < SPL; ++s) {
             const double x = mmi[(size_t)nc * 2 * V + s * V];
-            if constexpr (kFast) kb[s] = min(kb[s], okey(x) ^ kx[s]);
+            if constexpr (kFast) kb[s] = min(kb[s], key(x, kx[s]));
             else b[s] = fmin(b[s], kx[s] ? -x : x);
           }
           if (mei) en = fmaxf(en, mei[(size_t)nc * V + v]);

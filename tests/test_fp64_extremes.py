@@ -140,3 +140,28 @@ def test_faces(system, N, value, v):
         size = np.abs(b)
         ok = np.isfinite(b)
         assert np.all(np.abs(a - b)[ok] <= 64 * 2.0 ** -53 * 16.0 + 1e-10 * size[ok] * (size[ok] > 10.0)), w
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 1, (15, 12)), ("euler_rp2d", 3, (12, 14)), ("euler_vortex", 4, (9, 10)),
+                                         ("bn_cylinder", 2, (13, 12)), ("bn_cylinder", 3, (9, 11))])
+@pytest.mark.parametrize("seed", range(6))
+def test_nan_neighbour(name, N, grid, seed):
+    """Cells of NaN energy (either sign) among noisy ones, all of magnitudes whose DMP
+    is decided in FP64: the neighbourhoods' minima and maxima leave the NaN out."""
+    cfg, ic, params = config(name, N, grid)
+    uh, _ = aderdg.project_initial_condition(cfg, ic, params)
+    rng = np.random.default_rng(seed)
+    V = cfg.nvar
+    u = uh.reshape(cfg.cells, -1, V) * (1.0 + 0.02 * 0.1 ** seed * rng.uniform(-1, 1, (cfg.cells, cfg.P ** 2, 1)))
+    u[..., : 8 if V == 9 else 4] *= 1.0e6
+    u[rng.choice(cfg.cells, 8, replace=False), :, 3] = -np.nan if seed % 2 else np.nan
+    out = []
+    for fused in (True, False):
+        s = aderdg.Solver(cfg)
+        s.upload(u.ravel())
+        r = s.step(0.0, 1e30) if fused else by_phases(s, 0.0, 1e30)
+        out.append((r, s.get(aderdg.A_RECOMPUTE), s.get(aderdg.A_STATUS), s.get(aderdg.A_LMIN), s.get(aderdg.A_LMAX)))
+    (ra, *a), (rb, *b) = out
+    assert ra == rb
+    for x, y in zip(a, b):
+        assert np.array_equal(x, y, equal_nan=True)
