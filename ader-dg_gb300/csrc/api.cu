@@ -293,8 +293,15 @@ int ensure_phase_buffers(aderdg_ctx* c) {
 namespace aderdg {
 void set_last_error(const std::string& msg) { g_err = msg; }
 int validate_config(const aderdg_config* c, std::string* why) { return validate(c, why); }
+// 1 / (a b) rounded once: the rounded quotient of the rounded product, corrected by
+// the remainder of both
+static double inverse_of_product(double a, double b) {
+  const double p = a * b, r = 1.0 / p;
+  const double c = std::fma(r, std::fma(-p, r, 1.0) - std::fma(a, b, -p) * r, r);
+  return std::isfinite(c) ? c : r;
+}
 // Instance description of a configuration (cell and face bases 0; without
-// ops, the surface integral's w/dx and w/dy are left 0).
+// ops, the factors of w are left 0).
 InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops) {
   InstDesc in{};
   in.imax = cfg->imax;
@@ -309,6 +316,8 @@ InstDesc make_inst_desc(const aderdg_config* cfg, const HostOps* ops) {
   for (int k = 0; k < 6; ++k) {
     in.wdx[k] = ops && k < ops->P ? ops->w[k] / in.dx : 0.0;
     in.wdy[k] = ops && k < ops->P ? ops->w[k] / in.dy : 0.0;
+    in.iwdx[k] = ops && k < ops->P ? inverse_of_product(ops->w[k], in.dx) : 0.0;
+    in.iwdy[k] = ops && k < ops->P ? inverse_of_product(ops->w[k], in.dy) : 0.0;
   }
   in.xl0 = cfg->xl[0];
   in.xl1 = cfg->xl[1];

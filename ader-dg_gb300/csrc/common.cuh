@@ -59,6 +59,7 @@ struct InstDesc {
   double ad_pi;                // 4 atan(1) as the host computes it
   double rdx, rdy;             // 1/dx, 1/dy (the FP64 predictor)
   double wdx[6], wdy[6];       // w_k/dx, w_k/dy (the FP64 surface integral)
+  double iwdx[6], iwdy[6];     // 1/(w_k dx), 1/(w_k dy), rounded once (the FP64 predictor)
 };
 
 // Mutable per-instance state, device resident.

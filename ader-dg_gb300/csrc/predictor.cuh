@@ -447,9 +447,9 @@ __global__ void __launch_bounds__(PredCfg<Sys, N, R, Tune>::THREADS, PredCfg<Sys
   R Dx[P], Dy[P], Gx[P], Gy[P];
   R cxw, cyw;  // dt/(dx w_i), dt/(dy w_j)
   if constexpr (C::FIX) {
-    // 1 in inactive lanes: their arithmetic stays in the fixed-point range
-    cxw = (act ? dt * in.rdx : 1.0) * op.iw[i];
-    cyw = (act ? dt * in.rdy : 1.0) * op.iw[j];
+    // two roundings; 1 in inactive lanes: their arithmetic stays in the fixed-point range
+    cxw = act ? dt * in.iwdx[i] : 1.0;
+    cyw = act ? dt * in.iwdy[j] : 1.0;
     if constexpr (C::MAT_ELEMS > 0)
       for (int k = t; k < P2; k += C::THREADS) sm[C::SLOTS * C::CELL_ELEMS + k] = op.dudx[k];
   } else if constexpr (C::LIN) {
