@@ -70,16 +70,18 @@ __device__ __forceinline__ double widen_bits(float f) {
   }
   return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
-// FP64 -> FP32, round to nearest even as the hardware conversion, on the
-// integer pipe: the 24 leading bits plus the rounding carry; results below the
+// FP64 -> FP32 of x 2^-kDown, round to nearest even as the hardware conversion, on
+// the integer pipe: the 24 leading bits plus the rounding carry; results below the
 // normal range take the shifted mantissa, too large ones are infinite.
+template <unsigned kDown = 0>
 __device__ __forceinline__ float narrow_bits(double x) {
   const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-  const unsigned e = (hi >> 20) & 0x7ffu;
+  unsigned e = (hi >> 20) & 0x7ffu;
   unsigned q = __funnelshift_l(lo, (hi & 0xfffffu) | 0x100000u, 3);
   q += ((lo & 0x1fffffffu) + 0x0fffffffu + (q & 1u)) >> 29;
-  unsigned r = ((e - 897u) << 23) + q;
-  if (e - 897u >= 253u) {  // outside [2^-126, 2^127): exponents near overflow, denormal results, infinities and NaNs
+  unsigned r = ((e - 897u - kDown) << 23) + q;
+  if (e - 897u - kDown >= 253u) {  // outside [2^-126, 2^127): exponents near overflow, denormal results, infinities and NaNs
+    if (e != 0x7ffu) e = e > kDown ? e - kDown : 0u;
     if (e >= 1023u + 127u) {
       const bool nan = e == 0x7ffu && ((hi & 0xfffffu) | lo);
       r = nan ? 0x7fc00000u : (e == 1023u + 127u && r < 0x7f800000u) ? r : 0x7f800000u;
@@ -831,7 +833,7 @@ struct BNSys {
   }
   // The FP32-mixed face fluxes Dm, Dp (Baer-Nunziato/pde.f90:326-353) of FP32
   // face states and fluxes in FP64, rounded to FP32: twice the flux is formed
-  // and halved after the rounding, and the fluctuation's components that are
+  // and halved as it is rounded, and the fluctuation's components that are
   // zero along d are left out.  The FP64 pipe bounds it, about 160 of its slots a
   // point: 616 -> 405 us on the 400^2 cylinder, N = 3.
   __device__ __forceinline__ static void face_mixed(const PhysC<double>& pc, const FConst& fc, const float* qL,
@@ -853,10 +855,10 @@ struct BNSys {
       const bool n = (v == 1 || v == 5) ? d == 0 : (v == 2 || v == 6) ? d == 1 : v != 0 && v != 4;
       if (n) {
         const double D = v == 1 || v == 2 ? -x : v == 3 ? -y : v == 5 || v == 6 ? x : v == 7 ? y : z;
-        dm[v] = 0.5f * narrow_bits(t - D);
-        dp[v] = 0.5f * narrow_bits(t + D);
+        dm[v] = narrow_bits<1>(t - D);
+        dp[v] = narrow_bits<1>(t + D);
       } else {
-        dm[v] = dp[v] = 0.5f * narrow_bits(t);
+        dm[v] = dp[v] = narrow_bits<1>(t);
       }
     }
   }
