@@ -489,12 +489,13 @@ using CellOps = typename std::conditional<kExact || !kFast, ExactOps<N>, DevOps<
 
 // kFast: DMP projections in FP32 with an error bound (settled from FP64 where
 // the bound leaves a decision open) and, without kExact, the FP32 modes'
-// storage and surface integral.  kExact: FP64 storage, surface integral, update
-// and CFL eigenvalues beside those projections: the FP64 mode's fused step, whose
-// decisions are those of the FP64 projections of its state.  Its surface integral
-// and update are fused multiply-adds (7 roundings a value in place of 12; the FP64
-// pipe bounds the kernel: 365 -> 255 us on the Euler vortex N = 4 256^2, 345 -> 248
-// us on Baer-Nunziato N = 3 200^2); the phase API keeps the reference's order.
+// storage and surface integral.  kExact: FP64 storage, surface integral and update
+// beside those projections: the FP64 mode's fused step, whose decisions are those of
+// the FP64 projections of its state.  Its surface integral and update are fused
+// multiply-adds (7 roundings a value in place of 12; the FP64 pipe bounds the kernel:
+// 365 -> 255 us on the Euler vortex N = 4 256^2, 345 -> 248 us on Baer-Nunziato N = 3
+// 200^2), its CFL denominators FP32 bounds (cfl_key: 255 -> 196 and 248 -> 198 us); the
+// phase API keeps the reference's order.
 template <class Sys, int N, bool kFast, int VAR = 0, bool kExact = false>
 __global__ void __launch_bounds__(CellCfg<Sys, N, VAR>::THREADS, CellCfg<Sys, N, VAR>::min_blocks(kFast && !kExact))
     k_cells(BatchArgs a, CellOps<N, kFast, kExact> op) {

@@ -82,7 +82,9 @@ cudaError_t launch_cells(const BatchArgs& a, const void* ops, cudaStream_t s) {
 
 // fast = 1 (the FP32 modes): FP32 surface integral and DMP projections, the
 // FP64 update as one fused multiply-add; fast = 0: FP64 in reference order;
-// fast = 2: FP64 in reference order with certified FP32 DMP projections
+// fast = 2: FP64 with certified FP32 DMP projections, the surface integral and the
+// update as fused multiply-adds and, in the fused step, FP32 bounds on the CFL
+// denominators
 cudaError_t cells(const BatchArgs& a, const void* ops, int fast, cudaStream_t s) {
 #if ADERDG_SYS != 0
   if (fast == 2) return launch_cells<true, true>(a, ops, s);

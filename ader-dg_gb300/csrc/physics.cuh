@@ -564,9 +564,10 @@ struct BNSys {
   __device__ static void roe_times_jump(const Phys& ph, const double* QL, const double* QR, int d, double* D) {
     roe_times_jump<double>(PhysC<double>(ph), QL, QR, d, D);
   }
-  // Reciprocal-sharing forms for the FP64 face flux, subcell re-solve and CFL
-  // eigenvalues of the FP32-mixed mode and of the FP64 fused step (compiled with
-  // fused multiply-adds; values agree with the reference order to rounding).
+  // Reciprocal-sharing forms for the FP64 face flux and subcell re-solve of the
+  // FP32-mixed mode and of the FP64 fused step, and the former's CFL eigenvalues
+  // (compiled with fused multiply-adds; values agree with the reference order to
+  // rounding).
   // Algebraically the reference expressions of Baer-Nunziato/pde.f90 with phi =
   // alpha_s (Q8), phi_g = 1 - phi:
   //   phi p_s = (gamma_s - 1) (Q3 - (Q1^2 + Q2^2) / (2 Q0)) - gamma_s pi_s phi,

@@ -87,9 +87,10 @@ const KernelTable* kernel_table(int sys, int N);
 // The tuner's choice for (system, N, precision) (registry.cu; zeros: the defaults).
 aderdg_tuning tuning_of(int sys, int N, int precision);
 
-// The FP32 modes' predictor and cell kernel in the tuned variant; FP64 has
-// kernels of its own (the cell kernel: reference order throughout in the phase
-// API and the priming passes, whose min/max are introspection outputs).
+// The FP32 modes' predictor and cell kernel in the tuned variant; FP64 has kernels
+// of its own.  Its cell kernel is that with certified FP32 projections in the fused
+// step, the priming passes (whose CFL denominators are in the reference's order) and
+// the initial limiter; the phase API's passes are in the reference's order throughout.
 inline cudaError_t launch_predictor(const KernelTable* kt, const BatchArgs& a, const void* ops, int precision,
                                     cudaStream_t s) {
   const int fp32 = precision != ADERDG_FP64 ? 1 : 0;

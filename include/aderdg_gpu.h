@@ -46,8 +46,11 @@ enum aderdg_system { ADERDG_SYS_ADVDIFF = 0, ADERDG_SYS_EULER = 1, ADERDG_SYS_BN
  *   fluxes, surface integral, update, limiter and time step in the reference's
  *   operation order; the fused step (aderdg_step, aderdg_run, batches) forms the
  *   same values with fused multiply-adds, shared reciprocals and, in the
- *   predictor, 60-bit fixed point, with rounding errors no larger, and takes the
- *   DMP and positivity decisions of an FP64 evaluation of its state.
+ *   predictor, 60-bit fixed point.  Its rounding errors are smaller in the root
+ *   mean square (a single value may be rounded less well).  It takes the DMP and
+ *   positivity decisions of an FP64 evaluation of its state, and its time steps are
+ *   those of the reference's order bit for bit, so that a run continued from a
+ *   downloaded state and limiter, or by host steps, equals the uninterrupted one.
  * ADERDG_FP32_MIXED: the predictor, volume and surface contractions and the
  *   Euler / advection-diffusion face fluxes in FP32 with FP32 accumulation;
  *   FP64 for the update of the state (conservation), the Baer-Nunziato
