@@ -607,10 +607,12 @@ struct BNSys {
       const float ke = 0.5f * (q[o + 1] * q[o + 1] + q[o + 2] * q[o + 2]) * i;
       const float pp = g1 * (q[o + 3] - ke) - gpi * phi + pi * phi;
       const float mag = g1 * (fabsf(q[o + 3]) + fabsf(ke)) + fabsf(gpi) + fabsf(pi);
-      const float s = fabsf(u) + sqrtf(g * pp * i);
+      const float c2 = g * pp * i, s = fabsf(u) + sqrtf(c2);
       // relative error of s: half that of pp (a few roundings of its terms), and its own
       const float rel = 1.0e-6f + 1.0e-6f * mag / pp;
-      const bool settled = pp > 1.0e-3f * mag && mag > 1.0e-25f && q[o] > 1.0e-30f && q[8] > 1.0e-3f && q[8] < 0.999f && s < 1.0e30f;
+      // (densities at which no square of a momentum that counts underflows)
+      const bool settled = pp > 1.0e-3f * mag && mag > 1.0e-18f && c2 > 1.0e-30f && q[o] > 1.0e-12f && q[8] > 1.0e-3f &&
+                           q[8] < 0.999f && s < 1.0e30f;
       hi[k] = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
       if (settled) lo = fmaxf(lo, s * (1.0f - rel));
     }
