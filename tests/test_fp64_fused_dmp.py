@@ -1,8 +1,8 @@
 """The FP64 mode's fused step decides the DMP from certified FP32 projections;
-its state, time step, flags and neighbourhood min/max are those of the phase
-API, which projects every cell in FP64, bit for bit: on states with shocks,
-uniform regions and smooth flow, on magnitudes beyond the FP32 bound's reach
-(x 1e4), and on states placed within 1e-9 of the DMP thresholds."""
+its time step, flags and neighbourhood min/max are those of the phase API, which
+projects every cell in FP64, bit for bit, and its state to 1e-12: on states with
+shocks, uniform regions and smooth flow, on magnitudes beyond the FP32 bound's
+reach (x 1e4), and on states placed within 1e-9 of the DMP thresholds."""
 import dataclasses
 
 import numpy as np

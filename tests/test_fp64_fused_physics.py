@@ -83,9 +83,9 @@ def test_inadmissible_states(name, N, grid):
 
 @pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 3, (17, 12)), ("bn_cylinder", 2, (13, 14)), ("euler_rp2d", 5, (8, 8))])
 def test_host_step(name, N, grid):
-    """A host step primes with certified bounds, upload with FP64 projections: the
-    same time step, decisions and state, bit for bit (every comparison the bounds
-    leave open is settled from FP64 values)."""
+    """A host step and upload, upload_limiter and a step: the same time step, decisions
+    and state, bit for bit.  (Both prime with certified bounds; against exact ones:
+    test_fp64_restart.py.)"""
     cfg, (uh, lh) = build(name, N, grid)
     h, d = aderdg.Solver(cfg), aderdg.Solver(cfg)
     for s in (h, d):

@@ -126,3 +126,30 @@ def test_random_states(name, N, seed, scale):
     want = b.calc_time_step(t, 1e30)
     if np.isfinite(want) and want < 1e19:  # no NaN among the denominators
         assert a.step(t, 1e30)[1] == want
+
+
+@pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 2, (17, 12)), ("euler_vortex", 4, (9, 8)), ("bn_cylinder", 2, (13, 14)),
+                                         ("bn_cylinder", 3, (10, 9))])
+@pytest.mark.parametrize("noise", [2e-5, 1e-4, 1e-3])
+def test_priming_bounds(name, N, grid, noise):
+    """A host step primes with certified FP32 bounds on the minima and maxima; the same
+    step from exact ones (limiter_prepare: FP64 projections in the reference's order)
+    takes the same decisions and gives the same state bit for bit, on states with
+    noise about the DMP's tolerance, where the bounds leave comparisons open."""
+    cfg, (uh, lh) = build(name, N, grid)
+    uh = uh * (1.0 + noise * np.random.default_rng(1).uniform(-1, 1, uh.size))
+    h, d = start(cfg, uh, lh), start(cfg, uh, lh)
+    u, t, marked = uh.copy(), 0.0, 0
+    for _ in range(4):
+        st, l = h.download_limiter()
+        d.upload(u)
+        d.upload_limiter(st, l)
+        d.limiter_prepare()
+        want = d.step(t, 1e30)
+        got = h.step_host(u, t, 1e30)
+        assert got == want
+        assert np.array_equal(u, d.download()[0])
+        for w in (aderdg.A_STATUS, aderdg.A_RECOMPUTE, aderdg.A_LMIN, aderdg.A_LMAX):
+            assert np.array_equal(h.get(w), d.get(w)), w
+        t, marked = got[0], marked + got[2]
+    assert marked > 0 or noise < 1e-4
