@@ -284,7 +284,8 @@ struct EulerSys {
   // roundings of 2^-24, the sound speed half the pressure's relative error (below
   // 10 2^-24 mag / p for its terms of magnitude mag) and six roundings, the sum
   // four: 2e-6 + 1e-6 mag / p is three times that.  Outside the ranges in which no
-  // product under- or overflows the bounds are 0 and infinity.
+  // product under- or overflows, and where 1/dx or 1/dy is denormal (cells beyond
+  // 1e37: its error is that of few bits), the bounds are 0 and infinity.
   __device__ static void cfl_bounds(const FConst& fc, const float* q, float idx, float idy, float& lo, float& hi) {
     const float i = 1.0f / q[0];
     const float ke = 0.5f * (q[1] * q[1] + q[2] * q[2]) * i;
@@ -292,7 +293,7 @@ struct EulerSys {
     const float c = sqrtf(c2), s = (fabsf(q[1]) * i + c) * idx + (fabsf(q[2]) * i + c) * idy;
     const float rel = 2.0e-6f + 1.0e-6f * mag / p;
     const bool settled = p > 1.0e-3f * mag && mag > 1.0e-18f && c2 > 1.0e-30f && q[0] > 1.0e-12f && q[0] < 1.0e30f &&
-                         s > 1.0e-30f && s < 1.0e30f;
+                         s > 1.0e-30f && s < 1.0e30f && idx > 1.0e-37f && idy > 1.0e-37f;
     lo = settled ? s * (1.0f - rel) : 0.0f;
     hi = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
   }
@@ -498,7 +499,7 @@ struct BNSys {
       ratio = fmaxf(ratio, mag / pp);
     }
     const float s = ex * idx + ey * idy, rel = 2.0e-6f + 1.0e-6f * ratio;
-    settled = settled && s > 1.0e-30f && s < 1.0e30f;
+    settled = settled && s > 1.0e-30f && s < 1.0e30f && idx > 1.0e-37f && idy > 1.0e-37f;
     lo = settled ? s * (1.0f - rel) : 0.0f;
     hi = settled ? s * (1.0f + rel) : __int_as_float(0x7f800000);
   }

@@ -128,6 +128,50 @@ def test_random_states(name, N, seed, scale):
         assert a.step(t, 1e30)[1] == want
 
 
+def largest_along_x(system, N):
+    """Cells so large that FP32's 1/dx, 1/dy are denormal numbers, the first 2e-4 too
+    small, the second 2e-4 too large; a cell whose flow along x gives the largest CFL
+    denominator and one whose flow along y gives 5e-5 less (by those FP32 values 1e-4
+    more), among cells at rest."""
+    unit = 2.0 ** -149
+    dx, dy = 1.0 / (2000.4 * unit), 1.0 / (2000.6 * unit)
+    x, y = float(np.float32(1 / dx)), float(np.float32(1 / dy))
+    assert x == 2000 * unit and y == 2001 * unit
+    cfg = aderdg.Config(system=system, N=N, imax=8, jmax=6, bc=(3, 3, 3, 3), xr=(8 * dx, 6 * dy), cfl=1e-8)
+    c, U = 1e15, 3e15
+    V = (((U + c) / dx + c / dy) * (1 - 5e-5) - c / dx) * dy - c
+    assert (U + c) * x + c * y < (c * x + (V + c) * y) * (1 - 1e-4)
+    u = np.zeros((cfg.cells, cfg.P ** 2, cfg.nvar))
+    mom = np.zeros((cfg.cells, 2))
+    mom[11], mom[29] = (U, 0.0), (0.0, V)
+    phases = [(0, cfg.gamma, 1.0)] if system == aderdg.SYS_EULER else [(0, cfg.gamma_s, 0.6), (4, cfg.gamma_g, 0.4)]
+    for o, g, a in phases:
+        u[..., o] = a
+        u[..., o + 1:o + 3] = a * mom[:, None]
+        u[..., o + 3] = a * (c * c / g / (g - 1) + 0.5 * (mom ** 2).sum(1))[:, None]
+    if system == aderdg.SYS_BN:
+        u[..., 8] = 0.6
+    return cfg, u.ravel()
+
+
+@pytest.mark.parametrize("system", [aderdg.SYS_EULER, aderdg.SYS_BN])
+@pytest.mark.parametrize("N", [2, 4])
+def test_huge_cells(system, N):
+    """The time step where 1/dx has few bits in FP32."""
+    cfg, uh = largest_along_x(system, N)
+    a, b = aderdg.Solver(cfg), aderdg.Solver(cfg)
+    for s in (a, b):
+        s.upload(uh)
+    short = 1e-9 * a.calc_time_step(0.0, 1e30)
+    for s in (a, b):
+        t, _, _ = s.step(0.0, short)
+    assert np.array_equal(a.download()[0], b.download()[0])
+    b.upload(b.download()[0])
+    want = b.calc_time_step(t, 1e30)
+    assert 0.0 < want < 1e19  # below the scheme's largest time step
+    assert a.step(t, 1e30)[1] == want
+
+
 @pytest.mark.parametrize("name,N,grid", [("euler_rp2d", 2, (17, 12)), ("euler_vortex", 4, (9, 8)), ("bn_cylinder", 2, (13, 14)),
                                          ("bn_cylinder", 3, (10, 9))])
 @pytest.mark.parametrize("noise", [2e-5, 1e-4, 1e-3])
