@@ -33,6 +33,7 @@ static __global__ void k_control(InstDesc* inst, InstState* st, int ninst, int* 
   if (k == 0 && list_count && (mode == kCtlBegin || (mode == kCtlPrimeReset && only < 0))) list_count[0] = 0;
   // the settle list serves one cell-kernel pass at a time: every pass that
   // fills it follows a begin or a priming reset on the same stream
+  // (aderdg_element_update, which either may be missing before, clears it itself)
   if (k == 0 && list_count && (mode == kCtlBegin || mode == kCtlPrimeReset)) list_count[1] = 0;
   if (k >= ninst) return;
   if (only >= 0 && k != only) return;
