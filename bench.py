@@ -756,7 +756,7 @@ def run_mix(args, aderdg, dist, rank, ws, lr):
                 "phase_share": {k: v / sum(kern_ms.values()) for k, v in kern_ms.items()},
                 "phase_ms_one_step": ph, "traffic": sub_traffic,
                 "traffic_source": "profiles/traffic.json: DRAM bytes per re-solved cell of k_subcell per (system, N) "
-                                  "group from one ncu capture of the batched mix, times each group's re-solved cells",
+                                  "group from an ncu capture of one simulation of each, times each group's re-solved cells",
                 "limiter": sub_limiter}
     roof = {"bound": "fp32" if mixed else "fp64", "kernel": "k_predictor (all (system, N) groups of the mix)",
             "achieved": ach, "peak": peak, "unit": "GFLOP/s", "frac": (ach / peak) if ach else None,
